@@ -36,6 +36,15 @@ int32_t sw_host_check_checkpoint(const void* buffer, size_t bytes);
 int64_t sw_host_schedule_order(const uint16_t* task_level, uint32_t np, uint32_t n, uint32_t d, int32_t levels,
                                int32_t groups, uint32_t* order, uint32_t* seg, int64_t seg_cap);
 
+/* The direction streams of a grid: every (direction, part) pair's tasks by Kahn level and
+ * within a level by number of upwind faces (`up`, as task_level), in groups.
+ * parts[0..num_parts]: offsets of the closed cell ranges.  Writes order[n * d] and one row
+ * of five numbers per group, in order: stream, first position, the stream's groups in
+ * earlier levels, tasks and slots per task (at most plan_cap rows).  Returns the number of
+ * groups, -1 on an invalid argument. */
+int64_t sw_host_stream_plan(const uint16_t* task_level, const uint8_t* up, uint32_t np, uint32_t n, uint32_t d,
+                            const uint32_t* parts, uint32_t num_parts, uint32_t* order, int64_t* plan, int64_t plan_cap);
+
 /* Task spaces of fewer than 2^31 tasks that sw_create splits the mixed path's
  * directions into at the least (0: more than eight would be needed); -1 on an invalid
  * argument. */

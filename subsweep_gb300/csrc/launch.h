@@ -93,6 +93,21 @@ struct DevicePtrs {
   uint32_t* space_lvl[kMaxSpaces];      // segment offsets of each space's schedule
   uint32_t space_segments[kMaxSpaces];
   uint32_t space_lvl_words[kMaxSpaces];
+  // direction streams (sweep_stream.cuh): stream_mode != 0 when the handle's schedule is
+  // laid out in streams; pull_rec then holds the streams' records
+  int stream_mode;
+  void* streams;             // StreamDesc per stream, in launch order (longest first)
+  void* stream_groups;       // StreamGroup per group
+  uint32_t* seg_group;       // first group of every level segment
+  unsigned char* stream_data;  // the groups' pieces
+  unsigned long long stream_bytes;
+  uint32_t num_streams, num_groups;
+  void* cell_att;            // attenuation of every cell or the inactive mark (R)
+  double* cell_rate;         // rate of every cell summed over the directions
+  uint8_t* cell_periodic;    // whether the cell has a LOCAL_PERIODIC face
+  uint32_t stream_shape[5];  // StreamShape: ring, magic, far, warps, buffer
+  // per level, lazily allocated: the active positions' bitmap, and their range in each stream
+  uint32_t *act_bits_lv[32], *act_range[32];
   int sparse_sweep;          // pull path: this launch runs over the compacted list of its level
   int compact_now;           // pull path: ... and builds that list first
   uint32_t* chunk;           // pull path: compaction chunk offsets, count at [num_chunks]
@@ -107,6 +122,11 @@ struct DevicePtrs {
   swk::SweepCtl* ctl;
   int coop_blocks;
   unsigned long long timeout_ns;
+};
+
+// device scratch of the streams' build (StreamBuild)
+struct StreamScratch {
+  uint32_t *gseg, *sbase, *sgroup;
 };
 
 struct PrecisionOps {
@@ -144,6 +164,10 @@ struct PrecisionOps {
   // push path, once per grid: precomputed downwind fractions (phases as records);
   // nullptr on the pull path
   cudaError_t (*push_records)(const DevicePtrs&, int phase, unsigned long long* scratch, cudaStream_t);
+  // direction streams, once per grid: phase 0 writes the inverse order and the groups'
+  // segments; phase 1 finds the groups' flags and far words for the shape set; phase 2, with
+  // stream_data allocated, writes the groups' pieces
+  cudaError_t (*stream_build)(const DevicePtrs&, int phase, const StreamScratch&, cudaStream_t);
 };
 
 // pull path: transport kernel variant used without autotuning (the lockstep kernel with

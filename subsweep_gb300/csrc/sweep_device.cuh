@@ -623,19 +623,24 @@ __global__ void k_fold_periodic(R* periodic, R* pending, const uint32_t* cells, 
   }
 }
 
+// attenuation of a cell that is not active in the sweep (a NaN that no arithmetic gives)
+__device__ __forceinline__ float inactive_mark(float) { return __uint_as_float(0xffffffffu); }
+__device__ __forceinline__ double inactive_mark(double) { return __longlong_as_double(-1ll); }
+
 // Per-cell attenuation factor exp(-n_HI sigma size) of HydrogenOnly::get_outgoing_rate
 // (hydrogen_only/mod.rs:72-88); direction-independent, so computed once per cell.
-template <bool kCarryNeutral>
+template <bool kCarryNeutral, typename AttR>
 __global__ void k_attenuation(uint32_t n, const uint8_t* level, int current_level, const double* density,
                               const double* xhii, const double* yneu, const double* size, double* att,
                               uint32_t* cell_sweep, const uint32_t* epoch_base, uint32_t epoch, uint2* cellpack,
-                              const float* src32) {
+                              const float* src32, AttR* cell_att) {
   // pull path: the number of the sweep that solves each active cell, and per cell the
   // pair {(float) attenuation, source / D} (attenuation 0xffffffff: inactive)
   const uint32_t sweep = cell_sweep ? (epoch_base ? *epoch_base + epoch : epoch) : 0u;
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
     if (level[c] < current_level) {
       if (cellpack) cellpack[c] = make_uint2(0xffffffffu, 0u);
+      if (cell_att) cell_att[c] = inactive_mark(AttR(0));
       continue;
     }
     if (cell_sweep) cell_sweep[c] = sweep;
@@ -644,7 +649,56 @@ __global__ void k_attenuation(uint32_t n, const uint8_t* level, int current_leve
     const double at = exp(-nhn * Units::kSigma * size[c]);
     att[c] = at;
     if (cellpack) cellpack[c] = make_uint2(__float_as_uint((float)at), __float_as_uint(src32[c]));
+    if (cell_att) cell_att[c] = (AttR)at;
   }
+}
+
+// Rate of cell c summed over the directions (Sweep::get_solver, src/sweep/mod.rs:613-631): FP64
+// in direction order; mixed path: a compensated FP32 sum of the scaled transported rates, the
+// source added in FP64.  `pos`: the incoming rates are indexed by position, else by task;
+// `has_periodic`: the cell has periodic faces (else its periodic sources are 0).  The rates are
+// loaded eight directions at a time.
+template <typename R>
+__device__ __forceinline__ double cell_sum(const R* incoming, const uint32_t* pos, const R* periodic, bool has_periodic,
+                                           double source, int D, uint32_t Np, uint32_t c, double rate_scale) {
+  constexpr int kBatch = 8;
+  const double src = source / (double)D;
+  double rate = 0.0;
+  float s = 0.f, comp = 0.f;
+  for (int d0 = 0; d0 < D; d0 += kBatch) {
+    R in[kBatch], per[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const size_t t = (size_t)min(d0 + j, D - 1) * Np + c;
+      in[j] = incoming[pos ? pos[t] : t];
+      per[j] = has_periodic ? periodic[t] : R(0);
+    }
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      if (d0 + j >= D) break;
+      if (sizeof(R) == 8) {
+        rate += ((double)in[j] + src) + (double)per[j];  // Site::get_rate
+      } else {
+        const float yv = ((float)in[j] + (float)per[j]) - comp;
+        const float tt = s + yv;
+        comp = (tt - s) - yv;
+        s = tt;
+      }
+    }
+  }
+  return sizeof(R) == 8 ? rate : (double)s * rate_scale + source;
+}
+
+// The same for every active cell, ahead of the chemistry: the gather over the positions wants
+// more threads in flight than the chemistry's registers allow.
+template <typename R>
+__global__ void __launch_bounds__(128) k_cell_sums(uint32_t n, const uint8_t* level, int current_level,
+                                                   const R* incoming, const uint32_t* pos, const R* periodic,
+                                                   const uint8_t* cell_periodic, const double* source, int D,
+                                                   uint32_t Np, double rate_scale, double* out) {
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
+    if (level[c] >= current_level)
+      out[c] = cell_sum(incoming, pos, periodic, cell_periodic[c] != 0, source[c], D, Np, c, rate_scale);
 }
 
 template <typename R>
@@ -654,6 +708,7 @@ struct ChemArgs {
   int current_level;
   int D;
   uint32_t Np;
+  const double* cell_rate;     // rate of every active cell (k_cell_sums), or null: summed here
   const R* incoming;           // incoming rate of task t at incoming[t]
   const R* periodic;
   double rate_scale;
@@ -684,37 +739,9 @@ __global__ void k_chemistry(ChemArgs<R> a) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < a.n; c += gridDim.x * blockDim.x) {
     if (a.level[c] < a.current_level) continue;
     const double timestep = ldexp(a.max_timestep, -(int)a.level[c]);  // timestep_level.rs:42-48
-    double rate;
-    if (sizeof(R) == 8) {
-      const double src = a.source[c] / (double)a.D;
-      rate = 0.0;  // sum over directions of Site::get_rate, in direction order
-      for (int d = 0; d < a.D; ++d) {
-        const size_t t = (size_t)d * a.Np + c;
-        rate += ((double)a.incoming[t] + src) + (double)a.periodic[t];
-      }
-    } else {
-      // compensated FP32 sum of the scaled transported rates in direction order, the
-      // source added in FP64; the rates are loaded eight directions at a time
-      constexpr int kBatch = 8;
-      float s = 0.f, comp = 0.f;
-      for (int d0 = 0; d0 < a.D; d0 += kBatch) {
-        float v[kBatch];
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-          const size_t t = (size_t)(d0 + j) * a.Np + c;
-          v[j] = d0 + j < a.D ? (float)a.incoming[t] + (float)a.periodic[t] : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-          if (d0 + j >= a.D) break;
-          const float yv = v[j] - comp;
-          const float tt = s + yv;
-          comp = (tt - s) - yv;
-          s = tt;
-        }
-      }
-      rate = (double)s * a.rate_scale + a.source[c];
-    }
+    const double rate = a.cell_rate ? a.cell_rate[c]
+                                    : cell_sum(a.incoming, nullptr, a.periodic, true, a.source[c], a.D, a.Np, c,
+                                               a.rate_scale);
     double relative_change;
     // chemistry/mod.rs:79-81.  The mixed path also treats a rate below the smallest
     // value its FP32 transport carries at full precision as insignificant: there the

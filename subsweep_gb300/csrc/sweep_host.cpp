@@ -108,6 +108,13 @@ struct sw_handle {
   std::string last_error;
   double* scratch = nullptr;  // N doubles for field export
   uint32_t stats_schedule_levels = 0;
+  // direction streams: whether the schedule is to be laid out in streams, the closed cell
+  // ranges of the grid ([parts] offsets), and the layout until the records are built
+  bool want_streams = false, force_streams = false;
+  std::vector<uint32_t> parts;
+  std::vector<uint32_t> stream_seg;
+  std::vector<std::vector<uint8_t>> stream_gmax;  // per stream: the largest count of every group
+  std::vector<swk::StreamDesc> streams;
   // fingerprint of the levelled schedule (direction groups and segment offsets): the pull
   // path's checkpointed words are indexed by schedule position
   uint64_t schedule_hash = 0;
@@ -357,6 +364,95 @@ static uint64_t grouped_level_order(const uint16_t* level, uint32_t Np, uint32_t
   return base;
 }
 
+// Closed parts of a grid: contiguous cell ranges that no LOCAL face leaves (the boxes of
+// a batch; the whole grid otherwise), at least `min_cells` each.  Returns their offsets.
+static std::vector<uint32_t> closed_parts(const sw_grid_csr* g, int64_t min_cells) {
+  std::vector<uint32_t> parts = {0};
+  int64_t reach = 0;
+  for (int64_t c = 0; c < g->num_cells; ++c) {
+    for (int64_t f = g->row_ptr[c]; f < g->row_ptr[c + 1]; ++f)
+      if (g->kind[f] == SW_FACE_LOCAL) reach = std::max<int64_t>(reach, g->nbr[f]);
+    if (reach <= c && c + 1 - parts.back() >= min_cells && g->num_cells - (c + 1) >= min_cells)
+      parts.push_back((uint32_t)(c + 1));
+  }
+  parts.push_back((uint32_t)g->num_cells);
+  return parts;
+}
+
+// The positions in direction streams: direction by direction, part by part, each stream's
+// tasks by Kahn level, within a level by number of upwind LOCAL faces (`up`), then by id.
+// Writes order[N * D]; the streams' descriptors (base, count, dir, seg0, segs) and the
+// level segments' offsets (seg[0] = 0, the end of every segment) are appended; gmax: the
+// largest count of every group of kStreamGroup tasks of a level, per stream.  A stream's
+// levels are contiguous from 0: every level has a task whose upwind neighbour lies one
+// level below, in the same stream.
+static void stream_order(const uint16_t* level, const uint8_t* up, uint32_t Np, uint32_t N, uint32_t D,
+                         const std::vector<uint32_t>& parts, uint32_t* order, std::vector<uint32_t>& seg,
+                         std::vector<swk::StreamDesc>& streams, std::vector<std::vector<uint8_t>>& gmax) {
+  const uint32_t np = (uint32_t)parts.size() - 1, ns = D * np;
+  std::vector<std::vector<uint32_t>> ends(ns);
+  gmax.assign(ns, {});
+  std::atomic<uint32_t> next{0};
+  const int nt = (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+  std::vector<std::thread> th;
+  for (int t = 0; t < nt; ++t)
+    th.emplace_back([&]() {
+      std::vector<uint32_t> tmp, at;
+      for (uint32_t s; (s = next.fetch_add(1)) < ns;) {
+        const uint32_t d = s / np, c0 = parts[s % np], n = parts[s % np + 1] - c0;
+        const uint32_t t0 = d * Np + c0;
+        tmp.resize(n);
+        uint32_t by_count[257] = {0};
+        uint32_t depth = 0;
+        for (uint32_t i = 0; i < n; ++i) {
+          ++by_count[up[t0 + i] + 1u];
+          depth = std::max<uint32_t>(depth, level[t0 + i] + 1u);
+        }
+        for (int k = 0; k < 256; ++k) by_count[k + 1] += by_count[k];
+        for (uint32_t i = 0; i < n; ++i) tmp[by_count[up[t0 + i]]++] = t0 + i;
+        at.assign(depth + 1, 0u);
+        for (uint32_t i = 0; i < n; ++i) ++at[level[t0 + i] + 1u];
+        for (uint32_t l = 0; l < depth; ++l) at[l + 1] += at[l];
+        const uint32_t base = d * N + c0;
+        for (uint32_t l = 1; l <= depth; ++l) ends[s].push_back(base + at[l]);
+        for (uint32_t i = 0; i < n; ++i) order[base + at[level[tmp[i]]]++] = tmp[i];
+        // the last task of a group has its largest count
+        uint32_t p = base;
+        for (uint32_t e : ends[s])
+          while (p < e) {
+            p = std::min(p + swk::kStreamGroup, e);
+            gmax[s].push_back(up[order[p - 1]]);
+          }
+      }
+    });
+  for (auto& x : th) x.join();
+  seg.assign(1, 0u);
+  streams.clear();
+  for (uint32_t s = 0; s < ns; ++s) {
+    swk::StreamDesc x{};
+    x.dir = s / np;
+    x.base = x.dir * N + parts[s % np];
+    x.count = parts[s % np + 1] - parts[s % np];
+    x.seg0 = (uint32_t)seg.size() - 1;
+    x.segs = (uint32_t)ends[s].size();
+    seg.insert(seg.end(), ends[s].begin(), ends[s].end());
+    streams.push_back(x);
+  }
+}
+
+// Whether direction streams are faster than the lockstep kernels over the levelled schedule:
+// the longest stream, at 3.6 ns a task of its block, against the time of a level (0.85 us
+// from word to word) times the levels, plus the tasks at the lockstep kernels' 17 per ns.
+// Measured on uniform boxes (mixed path, ms per sweep, lockstep and streams): 84 directions
+// 24^3 0.32 and 0.15, 48^3 0.89 and 0.52, 64^3 1.56 and 1.01, 128^3 10.3 and 7.6; 16
+// directions 64^3 0.95 and 0.87, but 101^3 1.87 and 2.98: sixteen blocks cannot keep up
+// with the whole device where levels are wide.
+static bool streams_pay(const std::vector<uint32_t>& parts, uint64_t tasks, size_t levels) {
+  uint32_t longest = 0;
+  for (size_t k = 1; k < parts.size(); ++k) longest = std::max(longest, parts[k] - parts[k - 1]);
+  return 3.6 * longest < 850.0 * (double)levels + (double)tasks / 17.0;
+}
+
 // Compact state (mixed path): task spaces hold fewer than kSpaceTasks tasks each.  The
 // fewest spaces of evenly split directions that do, 0 when kMaxSpaces are not enough.
 constexpr uint64_t kSpaceTasks = 1ull << 31;
@@ -381,6 +477,14 @@ static int schedule_dir_groups(int D, uint64_t tasks, size_t levels) {
   return std::max(1, std::min(g, D));
 }
 
+// Fingerprint of a schedule: FNV-1a over the state kind, spaces, groups and offsets.
+struct ScheduleHash {
+  uint64_t value = 0xcbf29ce484222325ull;
+  void mix(uint32_t v) {
+    for (int k = 0; k < 4; ++k) value = (value ^ ((v >> (8 * k)) & 0xffu)) * 0x100000001b3ull;
+  }
+};
+
 // Levelled schedule (Kahn levels of all N*D tasks with every cell active), built once
 // per grid on the device, per task space (one space unless the compact state splits the
 // directions; task ids and positions are local to a space).  A dependency cycle leaves
@@ -399,12 +503,9 @@ sw_status build_schedule(sw_handle* h) {
   for (int sp = 0; sp < p.num_spaces; ++sp) max_ds = std::max(max_ds, p.space_d0[sp + 1] - p.space_d0[sp]);
   SW_CUDA(h, cudaMalloc(&level_scratch.ptr, (size_t)h->Np * max_ds * sizeof(uint16_t)), "schedule scratch");
   uint16_t* task_level = static_cast<uint16_t*>(level_scratch.ptr);
-  uint64_t hash = 0xcbf29ce484222325ull;  // FNV-1a over the state kind, spaces, groups and offsets
-  auto mix = [&](uint32_t v) {
-    for (int k = 0; k < 4; ++k) hash = (hash ^ ((v >> (8 * k)) & 0xffu)) * 0x100000001b3ull;
-  };
-  mix((uint32_t)p.geo_mode);
-  mix((uint32_t)p.num_spaces);
+  ScheduleHash hash;
+  hash.mix((uint32_t)p.geo_mode);
+  hash.mix((uint32_t)p.num_spaces);
   uint32_t depth = 0;
   for (int sp = 0; sp < p.num_spaces; ++sp) {
     const swh::DevicePtrs q = swh::space_view(p, sp);
@@ -416,6 +517,11 @@ sw_status build_schedule(sw_handle* h) {
     unsigned long long tail = 0;
     SW_CUDA(h, cudaMemcpyAsync(&tail, &p.ctl->tail, sizeof(tail), cudaMemcpyDeviceToHost, h->stream), "read tail");
     SW_CUDA(h, cudaStreamSynchronize(h->stream), "schedule seed");
+    std::vector<uint8_t> up;  // upwind LOCAL faces of every task (the rounds count them down)
+    if (h->want_streams) {
+      up.resize((size_t)h->Np * q.D);
+      SW_CUDA(h, cudaMemcpy(up.data(), p.counters, up.size(), cudaMemcpyDeviceToHost), "read upwind counts");
+    }
     uint32_t begin = 0;
     uint32_t round = 0;
     while (tail > begin) {
@@ -436,6 +542,7 @@ sw_status build_schedule(sw_handle* h) {
       // dependency-driven queue; the pull path visits tasks in id order and its waits run
       // out, so either reports the stall at the first sweep, where the reference deadlocks.
       p.num_sched_levels = 0;
+      h->want_streams = false;
       if (h->ops->pull) {
         std::vector<uint32_t> ids;
         ids.reserve(total);
@@ -458,6 +565,7 @@ sw_status build_schedule(sw_handle* h) {
     // and checkpoints hold them in that order.
     const size_t L = lvl.size() - 1;
     depth = std::max(depth, (uint32_t)L);
+    if (h->want_streams) h->want_streams = h->force_streams || streams_pay(h->parts, total, L);
     int groups = schedule_dir_groups(q.D, total, L);
     if (p.geo_mode && !std::getenv("SUBSWEEP_DIR_GROUPS")) groups = 1;
     std::vector<uint32_t> seg = {0};
@@ -466,9 +574,14 @@ sw_status build_schedule(sw_handle* h) {
       SW_CUDA(h, cudaMemcpy(tl.data(), task_level, tl.size() * sizeof(uint16_t), cudaMemcpyDeviceToHost),
               "read task levels");
       std::vector<uint32_t> order(total);
-      const uint64_t base =
-          grouped_level_order(tl.data(), h->Np, (uint32_t)h->N, (uint32_t)q.D, L, groups, order.data(), seg);
-      if (base != total) return h->fail(SW_ERR_CUDA, "schedule order incomplete");
+      if (h->want_streams) {
+        stream_order(tl.data(), up.data(), h->Np, (uint32_t)h->N, (uint32_t)q.D, h->parts, order.data(), seg,
+                     h->streams, h->stream_gmax);
+        h->stream_seg = seg;
+      } else if (grouped_level_order(tl.data(), h->Np, (uint32_t)h->N, (uint32_t)q.D, L, groups, order.data(), seg) !=
+                 total) {
+        return h->fail(SW_ERR_CUDA, "schedule order incomplete");
+      }
       SW_CUDA(h, cudaMemcpy(q.order, order.data(), order.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
               "upload order");
     }
@@ -482,15 +595,15 @@ sw_status build_schedule(sw_handle* h) {
     p.space_lvl[sp] = d_lvl;
     p.space_segments[sp] = (uint32_t)(seg.size() - 1);
     p.space_lvl_words[sp] = (uint32_t)lvl_words;
-    mix((uint32_t)groups);
-    for (uint32_t o : seg) mix(o);
+    hash.mix((uint32_t)groups);
+    for (uint32_t o : seg) hash.mix(o);
   }
   SW_CUDA(h, cudaMemsetAsync(p.ctl, 0, offsetof(swk::SweepCtl, tasks), h->stream), "reset control");
   p.lvl = p.space_lvl[0];
   p.num_sched_levels = p.space_segments[0];
   p.lvl_words = p.space_lvl_words[0];
   h->stats_schedule_levels = depth;  // the dependency depth
-  h->schedule_hash = hash;
+  h->schedule_hash = hash.value;
   return SW_OK;
 }
 
@@ -561,9 +674,198 @@ sw_status build_push_records(sw_handle* h) {
   return SW_OK;
 }
 
+// The groups of one stream, in order (data and the flags of the shape follow later).
+static void plan_stream(const swk::StreamDesc& sd, const uint32_t* seg, const std::vector<uint8_t>& gmax,
+                        swk::StreamGroup* out) {
+  uint32_t g = 0;
+  for (uint32_t k = sd.seg0; k < sd.seg0 + sd.segs; ++k) {
+    const uint32_t need = g;
+    for (uint32_t p = seg[k]; p < seg[k + 1]; p += swk::kStreamGroup, ++g) {
+      const uint32_t n = std::min(swk::kStreamGroup, seg[k + 1] - p), slots = (gmax[g] + 3u) & ~3u;
+      out[g] = {need, 0u, p, (n - 1) | (slots << 5)};
+    }
+  }
+}
+
+// bytes of a group's piece (StreamPiece), rb bytes a rate
+static uint32_t piece_bytes(uint32_t shape, uint32_t rb) {
+  const uint32_t slots = (shape >> 5) & 0x7fu, far = shape >> 17;
+  return (uint32_t)sizeof(swk::StreamGroup) +
+         32u * (rb + (rb == 4 ? 4u : 0u) + slots * (rb + 2u) + ((shape & swk::kGroupExt) ? 2u * rb : 0u) + far * 4u);
+}
+
+// Direction streams: groups and their pieces, and the launch shape (after the schedule is in
+// place).
+sw_status build_streams(sw_handle* h) {
+  swh::DevicePtrs& p = h->p;
+  const std::vector<uint32_t>& seg = h->stream_seg;
+  const uint32_t segs = (uint32_t)seg.size() - 1;
+  const uint32_t rb = (uint32_t)h->ops->rate_bytes;
+  const double width = (double)h->N * h->D / segs;  // of a level, on average
+  uint32_t warps = width <= 32 ? 4 : (width <= 96 ? 8 : 16);
+  if (const char* env = std::getenv("SUBSWEEP_STREAM_WARPS")) {
+    const int v = std::atoi(env);
+    if (v == 4 || v == 8 || v == 16) warps = (uint32_t)v;
+  }
+  uint32_t slots = 0;  // per task of the largest group
+  for (const auto& m : h->stream_gmax)
+    for (uint8_t v : m) slots = std::max<uint32_t>(slots, (v + 3u) & ~3u);
+  std::vector<uint32_t> seg_group(segs + 1), sbase(segs), sgroup(segs);
+  uint32_t longest = 0, widest = 0;
+  for (swk::StreamDesc& s : h->streams) {
+    s.group0 = seg_group[s.seg0];
+    for (uint32_t k = s.seg0; k < s.seg0 + s.segs; ++k) {
+      widest = std::max(widest, seg[k + 1] - seg[k]);
+      seg_group[k + 1] = seg_group[k] + (seg[k + 1] - seg[k] + swk::kStreamGroup - 1) / swk::kStreamGroup;
+      sbase[k] = s.base;
+      sgroup[k] = s.group0;
+    }
+    s.groups = seg_group[s.seg0 + s.segs] - s.group0;
+    longest = std::max(longest, s.count);
+  }
+  // Shared memory of a block: its share of the SM's (several blocks share an SM when there are
+  // more streams than SMs); the warps' buffers, the rest words: ring, unless that leaves far
+  // words, for which the warps then get room.
+  int optin = 0, per_sm = 0;
+  SW_CUDA(h, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device), "attribute");
+  SW_CUDA(h, cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device), "attribute");
+  const uint32_t buffer = piece_bytes(31u | (slots << 5) | swk::kGroupExt, rb);
+  auto words_for = [&](size_t room, uint32_t far) -> int64_t {
+    return std::min<int64_t>(((int64_t)room - 272 - 4 * rb - (int64_t)warps * buffer) / rb - (int64_t)warps * far * 32,
+                             60000 - (int64_t)warps * far * 32);
+  };
+  size_t room = 0;
+  const int most = std::max(1, std::min(8, (int)(48 / warps)));  // blocks per SM that their registers allow
+  for (int k = std::max(1, std::min(most, (int)((h->streams.size() + p.num_sms - 1) / p.num_sms))); k >= 1; --k) {
+    room = std::min((size_t)optin, (size_t)per_sm / k - 1024);
+    if (words_for(room, swk::kStreamFar) >= (int64_t)std::min(longest, 8192u)) break;
+  }
+  // a ring must not wrap inside a level: with a wider one the grid keeps the levelled schedule
+  if (words_for(room, swk::kStreamFar) < (int64_t)std::min(longest, widest)) {
+    h->want_streams = false;
+    return SW_OK;
+  }
+  std::vector<swk::StreamGroup> groups(seg_group[segs]);
+  {
+    std::atomic<size_t> next{0};
+    const int nt = (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    std::vector<std::thread> th;
+    for (int t = 0; t < nt; ++t)
+      th.emplace_back([&]() {
+        for (size_t s; (s = next.fetch_add(1)) < h->streams.size();)
+          plan_stream(h->streams[s], seg.data(), h->stream_gmax[s], groups.data() + h->streams[s].group0);
+      });
+    for (auto& x : th) x.join();
+  }
+  h->stream_gmax.clear();
+  struct Scratch {
+    std::vector<void*> mem;
+    ~Scratch() {
+      for (void* m : mem) cudaFree(m);
+    }
+    cudaError_t get(void** out, size_t bytes, const void* src) {
+      cudaError_t e = cudaMalloc(out, std::max<size_t>(bytes, 4));
+      if (e != cudaSuccess) return e;
+      mem.push_back(*out);
+      return src ? cudaMemcpy(*out, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
+    }
+  } scratch;
+  swh::StreamScratch b{};
+  SW_CUDA(h, scratch.get((void**)&b.gseg, groups.size() * 4, nullptr), "stream scratch");
+  SW_CUDA(h, scratch.get((void**)&b.sbase, sbase.size() * 4, sbase.data()), "stream scratch");
+  SW_CUDA(h, scratch.get((void**)&b.sgroup, sgroup.size() * 4, sgroup.data()), "stream scratch");
+  swk::StreamDesc* d_streams = nullptr;
+  swk::StreamGroup* d_groups = nullptr;
+  if (!h->alloc(&d_streams, h->streams.size()) || !h->alloc(&d_groups, groups.size() + 1) ||
+      !h->alloc(&p.seg_group, seg_group.size()))
+    return h->fail(SW_ERR_OOM, "device allocation of the streams failed");
+  p.streams = d_streams;
+  p.stream_groups = d_groups;
+  p.num_streams = (uint32_t)h->streams.size();
+  p.num_groups = (uint32_t)groups.size();
+  const size_t group_bytes = groups.size() * sizeof(groups[0]);
+  std::stable_sort(h->streams.begin(), h->streams.end(),  // launch order: the longest first
+                   [](const swk::StreamDesc& x, const swk::StreamDesc& y) { return x.count > y.count; });
+  SW_CUDA(h, cudaMemcpy(d_streams, h->streams.data(), h->streams.size() * sizeof(h->streams[0]), cudaMemcpyHostToDevice),
+          "streams");
+  SW_CUDA(h, cudaMemcpy(p.seg_group, seg_group.data(), seg_group.size() * 4, cudaMemcpyHostToDevice), "streams");
+  SW_CUDA(h, h->ops->stream_build(p, 0, b, h->stream), "stream position kernels");
+  uint32_t* shape = p.stream_shape;
+  shape[3] = warps;
+  bool far = false;
+  int64_t late = 0, slow = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    shape[2] = pass == 0 ? 0u : swk::kStreamFar;
+    shape[4] = buffer;
+    shape[0] = (uint32_t)std::min<int64_t>(words_for(room, shape[2]), longest);
+    shape[1] = (uint32_t)((1ull << 32) / shape[0]) + 1u;
+    for (swk::StreamGroup& g : groups) g.shape &= 0xfffu;
+    SW_CUDA(h, cudaMemcpy(d_groups, groups.data(), group_bytes, cudaMemcpyHostToDevice), "groups");
+    SW_CUDA(h, h->ops->stream_build(p, 1, b, h->stream), "stream flag kernel");
+    SW_CUDA(h, cudaStreamSynchronize(h->stream), "stream flags");
+    SW_CUDA(h, cudaMemcpy(groups.data(), d_groups, group_bytes, cudaMemcpyDeviceToHost), "groups");
+    far = false;
+    late = slow = 0;
+    for (const swk::StreamGroup& g : groups) {
+      far = far || (g.shape >> 17) != 0;
+      late += (g.shape & swk::kGroupLate) != 0;
+      slow += (g.shape & swk::kGroupSlow) != 0;
+    }
+    if (!far) break;
+  }
+  uint64_t at = 0;
+  for (swk::StreamGroup& g : groups) {
+    g.data = (uint32_t)(at / 16);
+    at += piece_bytes(g.shape, rb);
+  }
+  groups.push_back({0u, (uint32_t)(at / 16), 0u, 0u});  // where the last piece ends
+  if (at / 16 > 0xffffffffull) {  // past the pieces' 32-bit offsets: the levelled schedule
+    h->want_streams = false;
+    return SW_OK;
+  }
+  SW_CUDA(h, cudaMemcpy(d_groups, groups.data(), groups.size() * sizeof(groups[0]), cudaMemcpyHostToDevice), "groups");
+  groups.pop_back();
+  if (!h->alloc(&p.stream_data, at)) {  // no room: the levelled schedule (smaller, unless groups are full)
+    (void)cudaGetLastError();
+    p.stream_data = nullptr;
+    h->want_streams = false;
+    return SW_OK;
+  }
+  char* cell_att = nullptr;
+  std::vector<uint32_t> pcells(p.n_periodic_cells);
+  std::vector<uint8_t> has_periodic(h->N, 0);
+  SW_CUDA(h, cudaMemcpy(pcells.data(), p.periodic_cells, pcells.size() * 4, cudaMemcpyDeviceToHost), "periodic cells");
+  for (uint32_t c : pcells) has_periodic[c] = 1;
+  if (!h->alloc(&cell_att, (size_t)h->N * rb) || !h->alloc(&p.cell_rate, h->N) || !h->alloc(&p.cell_periodic, h->N))
+    return h->fail(SW_ERR_OOM, "device allocation of the streams failed");
+  p.stream_bytes = at;
+  p.cell_att = cell_att;
+  SW_CUDA(h, cudaMemcpy(p.cell_periodic, has_periodic.data(), h->N, cudaMemcpyHostToDevice), "periodic cells");
+  SW_CUDA(h, h->ops->stream_build(p, 2, b, h->stream), "upwind slot kernel");
+  SW_CUDA(h, cudaStreamSynchronize(h->stream), "upwind slots");
+  uint32_t err = 0;
+  SW_CUDA(h, cudaMemcpy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
+  if (err & swk::kErrRecords) return h->fail(SW_ERR_CUDA, "upwind slot classification disagrees with its count");
+  int64_t all_slots = 0;
+  for (const swk::StreamGroup& g : groups) all_slots += (int64_t)((g.shape & 31u) + 1u) * ((g.shape >> 5) & 0x7fu);
+  h->stats_upwind_slots = all_slots;
+  if (h->trace)
+    std::fprintf(stderr, "subsweep streams: %u of %u warps, buffer %u, ring %u, far %u, %zu groups (%lld late, %lld slow), %llu bytes\n",
+                 p.num_streams, warps, shape[4], shape[0], shape[2], groups.size(), (long long)late, (long long)slow,
+                 (unsigned long long)at);
+  p.stream_mode = 1;
+  return SW_OK;
+}
+
 // Pull path: task records and upwind slots of every schedule position (after the
 // schedule, or the id order of a cyclic grid, is in place).
 sw_status build_records(sw_handle* h) {
+  if (h->want_streams) {
+    sw_status st = build_streams(h);
+    if (st != SW_OK || h->want_streams) return st;
+    st = build_schedule(h);  // a level too wide for a ring: the levelled schedule
+    if (st != SW_OK) return st;
+  }
   if (!h->ops->records) return SW_OK;
   swh::DevicePtrs& p = h->p;
   if (p.geo_mode) {  // compact state: only the periodic fold's entries
@@ -580,6 +882,11 @@ sw_status build_records(sw_handle* h) {
   } off_scratch;
   SW_CUDA(h, cudaMalloc(&off_scratch.ptr, (nc + 1) * sizeof(unsigned long long)), "record scratch");
   auto* chunk_off = static_cast<unsigned long long*>(off_scratch.ptr);
+  if (!p.pull_rec) {  // a cyclic grid that was to be laid out in streams
+    uint4* rec = nullptr;
+    if (!h->alloc(&rec, (size_t)h->Np * h->D)) return h->fail(SW_ERR_OOM, "device allocation of the task records failed");
+    p.pull_rec = rec;
+  }
   SW_CUDA(h, h->ops->records(p, 0, chunk_off, h->stream), "task record kernels");
   unsigned long long total = 0;
   SW_CUDA(h, cudaMemcpyAsync(&total, chunk_off + nc, sizeof(total), cudaMemcpyDeviceToHost, h->stream),
@@ -1056,6 +1363,16 @@ sw_status sw_create(const sw_params* params, const sw_grid_csr* grid, const sw_c
       h->autotune = false;
     }
   }
+  // Direction streams (SUBSWEEP_STREAMS=0 turns them off; so does pinning a transport
+  // kernel variant or the direction groups of the levelled schedule).
+  if (h->ops->stream_build && !p.geo_mode) {
+    h->want_streams = !std::getenv("SUBSWEEP_PULL_VARIANT") && !std::getenv("SUBSWEEP_DIR_GROUPS");
+    if (const char* env = std::getenv("SUBSWEEP_STREAMS")) {
+      h->want_streams = h->want_streams && std::atoi(env) != 0;
+      h->force_streams = h->want_streams;
+    }
+    if (h->want_streams) h->parts = closed_parts(grid, 256);
+  }
   {
     const size_t nd = (size_t)Np * D;
     const size_t rb = (size_t)h->ops->rate_bytes;
@@ -1080,7 +1397,7 @@ sw_status sw_create(const sw_params* params, const sw_grid_csr* grid, const sw_c
       ok = h->alloc(&qe, nd) && h->alloc(&act_counts, 32) && h->alloc(&cell_sweep, (size_t)h->Np) &&
            h->alloc(&cellpack, (size_t)h->Np);
     else if (ok && pull)
-      ok = h->alloc(&qe, nd) && h->alloc(&rec, nd) && h->alloc(&act_counts, 32) && h->alloc(&pos_of_task, nd) &&
+      ok = h->alloc(&qe, nd) && (h->want_streams || h->alloc(&rec, nd)) && h->alloc(&act_counts, 32) && h->alloc(&pos_of_task, nd) &&
            h->alloc(&act_bits, (nd + 31) / 32) && h->alloc(&cell_sweep, (size_t)h->Np) &&
            h->alloc(&cellpack, (size_t)h->Np) &&
            // per-position periodic sources: only for the staged wavefront kernel (78)
@@ -1158,11 +1475,22 @@ static bool pull_sparse(sw_handle* h, int level) {
   if (level <= 0) return false;
   if (p.compact_mode == 1) return true;
   if (p.compact_mode == 2) return false;
+  // Streams: a dense sweep takes the time of all tasks, 23 per ns, a sparse one ~5 per ns of
+  // the active ones (128^3 x 84: 7.9 ms dense; sparse 14 ms with 39% of the cells active, the
+  // crossing near 20%; 64^3 x 84: 1.03 ms dense, 0.13 ms with 0.2% active).
+  if (p.stream_mode) return (int64_t)h->n_ge_host[level] * 5 < h->N;
   return h->n_ge_host[level] * 2 < h->N;
 }
 
 static sw_status ensure_act_list(sw_handle* h, int level) {
   if (h->p.act_lv[level]) return SW_OK;
+  if (h->p.stream_mode) {
+    uint32_t *bits = nullptr, *range = nullptr;
+    if (!h->alloc(&bits, ((size_t)h->Np * h->D + 31) / 32) || !h->alloc(&range, 2 * (size_t)h->p.num_streams))
+      return h->fail(SW_ERR_OOM, "device allocation of the active positions of level %d failed", level);
+    h->p.act_bits_lv[level] = bits;
+    h->p.act_range[level] = range;
+  }
   uint32_t* buf = nullptr;
   if (!h->alloc(&buf, (size_t)h->Np * h->D))
     return h->fail(SW_ERR_OOM, "device allocation of the active positions of level %d failed", level);
@@ -1234,7 +1562,7 @@ static sw_status step_graph(sw_handle* h, double* time_elapsed_out) {
       } else if (variants[k] && !((compacted >> levels[k]) & 1u)) {
         compact_now[k] = 1;
         compacted |= 1u << levels[k];
-        kernels += 4;
+        kernels += p.stream_mode ? 5 : 4;
       }
     }
     for (size_t k = 0; k < levels.size() && ce == cudaSuccess; ++k) {
@@ -1402,7 +1730,7 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
     if (h->force_path == 2) levelled = false;
     // autotuning trials on dense sweeps only: sparse ones always run the lockstep kernel
     const bool trial = ops.pull && h->autotune && !h->tuned && !pull_sparse(h, level);
-    if (trial) h->p.pull_variant = ops.tune_variants[h->tune_index];
+    if (trial && !h->p.stream_mode) h->p.pull_variant = ops.tune_variants[h->tune_index];
     if (ops.pull) {
       levelled = true;  // the pull path always walks the schedule (or the id order)
       h->p.epoch += 1;
@@ -1416,7 +1744,7 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
         if (!((h->act_valid >> level) & 1u)) {  // first sweep of this level in the step
           h->p.compact_now = 1;
           h->act_valid |= 1u << level;
-          launches += 4;  // compaction of the active positions
+          launches += h->p.stream_mode ? 5 : 4;  // compaction of the active positions
         }
       }
     }
@@ -1449,7 +1777,9 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
     sweep_ms += a;
     chem_ms += b;
     kernel_ms += k;
-    if (trial) {  // one autotuning trial per sweep; the fastest variant per task is kept
+    if (trial && h->p.stream_mode) {  // the streams have one shape: nothing to choose
+      h->tuned = true;
+    } else if (trial) {  // one autotuning trial per sweep; the fastest variant per task is kept
       h->tune_ns.push_back(1e6 * k / std::max(1.0, (double)h->n_ge_host[level] * h->D));
       if (++h->tune_index == ops.num_tune_variants) {
         int best = 0;
@@ -1669,6 +1999,57 @@ static std::vector<CheckpointSection> checkpoint_sections(sw_handle* h) {
   return v;
 }
 
+// Checkpoints hold the words by position of the levelled schedule and the incoming rates by
+// task, whatever the handle's own layout.  Direction streams: the levelled order, from the
+// streams' (a stream's segments are its levels), and its fingerprint.
+static sw_status levelled_schedule(sw_handle* h, std::vector<uint32_t>& own, std::vector<uint32_t>& order,
+                                   uint64_t& fingerprint) {
+  const swh::DevicePtrs& p = h->p;
+  const uint32_t total = (uint32_t)(h->N * (int64_t)h->D);
+  own.resize(total);
+  SW_CUDA(h, cudaMemcpy(own.data(), p.order, (size_t)total * 4, cudaMemcpyDeviceToHost), "read order");
+  std::vector<uint16_t> level((size_t)h->Np * h->D, 0);
+  uint32_t depth = 0;
+  for (const swk::StreamDesc& s : h->streams) {
+    for (uint32_t k = 0; k < s.segs; ++k)
+      for (uint32_t i = h->stream_seg[s.seg0 + k]; i < h->stream_seg[s.seg0 + k + 1]; ++i) level[own[i]] = (uint16_t)k;
+    depth = std::max(depth, s.segs);
+  }
+  const int groups = schedule_dir_groups(h->D, total, depth);
+  order.resize(total);
+  std::vector<uint32_t> seg = {0};
+  grouped_level_order(level.data(), h->Np, (uint32_t)h->N, (uint32_t)h->D, depth, groups, order.data(), seg);
+  ScheduleHash hash;
+  hash.mix(0u);
+  hash.mix(1u);
+  hash.mix((uint32_t)groups);
+  for (uint32_t o : seg) hash.mix(o);
+  fingerprint = hash.value;
+  return SW_OK;
+}
+
+// Words and incoming rates of a checkpoint from the streams' layout, and back.
+static void stream_to_checkpoint(const std::vector<uint32_t>& own, const std::vector<uint32_t>& order,
+                                 const uint64_t* words, const uint32_t* inc, uint64_t* cp_words, uint32_t* cp_inc,
+                                 size_t nd) {
+  std::vector<uint32_t> pos(nd, 0);
+  for (size_t i = 0; i < own.size(); ++i) pos[own[i]] = (uint32_t)i;
+  std::memset(cp_words, 0, nd * 8);
+  std::memset(cp_inc, 0, nd * 4);
+  for (size_t i = 0; i < order.size(); ++i) cp_words[i] = words[pos[order[i]]];
+  for (size_t i = 0; i < own.size(); ++i) cp_inc[own[i]] = inc[i];
+}
+static void checkpoint_to_stream(const std::vector<uint32_t>& own, const std::vector<uint32_t>& order,
+                                 const uint64_t* cp_words, const uint32_t* cp_inc, uint64_t* words, uint32_t* inc,
+                                 size_t nd) {
+  std::vector<uint32_t> pos(nd, 0);
+  for (size_t i = 0; i < own.size(); ++i) pos[own[i]] = (uint32_t)i;
+  std::memset(words, 0, nd * 8);
+  std::memset(inc, 0, nd * 4);
+  for (size_t i = 0; i < order.size(); ++i) words[pos[order[i]]] = cp_words[i];
+  for (size_t i = 0; i < own.size(); ++i) inc[i] = cp_inc[own[i]];
+}
+
 static size_t checkpoint_bytes(sw_handle* h) {
   size_t total = sizeof(CheckpointHeader);
   for (const CheckpointSection& s : checkpoint_sections(h)) total += s.bytes;
@@ -1724,6 +2105,30 @@ int64_t sw_host_schedule_order(const uint16_t* task_level, uint32_t np, uint32_t
   return (int64_t)s.size() - 1;
 }
 
+int64_t sw_host_stream_plan(const uint16_t* task_level, const uint8_t* up, uint32_t np, uint32_t n, uint32_t d,
+                            const uint32_t* parts, uint32_t num_parts, uint32_t* order, int64_t* plan, int64_t plan_cap) {
+  if (!task_level || !up || !parts || !order || !plan || n == 0 || np < n || d == 0 || num_parts == 0 ||
+      parts[0] != 0 || parts[num_parts] != n || (uint64_t)np * d >= (1ull << 32))
+    return -1;
+  std::vector<uint32_t> seg;
+  std::vector<swk::StreamDesc> streams;
+  std::vector<std::vector<uint8_t>> gmax;
+  stream_order(task_level, up, np, n, d, std::vector<uint32_t>(parts, parts + num_parts + 1), order, seg, streams, gmax);
+  int64_t rows = 0;
+  for (size_t s = 0; s < streams.size(); ++s) {
+    std::vector<swk::StreamGroup> groups(gmax[s].size());
+    plan_stream(streams[s], seg.data(), gmax[s], groups.data());
+    for (const swk::StreamGroup& g : groups) {
+      if (rows < plan_cap) {
+        const int64_t row[5] = {(int64_t)s, g.pos, g.need, (g.shape & 31u) + 1, g.shape >> 5};
+        std::copy(row, row + 5, plan + 5 * rows);
+      }
+      ++rows;
+    }
+  }
+  return rows;
+}
+
 int32_t sw_host_task_spaces(uint32_t np, int32_t d) {
   if (np == 0 || d < 1) return -1;
   return min_task_spaces(np, d);
@@ -1766,6 +2171,11 @@ sw_status sw_save_state(sw_handle* h, void* buffer, size_t bytes) {
   hd.epoch = h->p.epoch;
   hd.last_epoch = h->last_epoch;
   hd.schedule_hash = h->ops->pull ? h->schedule_hash : 0;
+  std::vector<uint32_t> own, order;
+  if (h->p.stream_mode) {
+    const sw_status st = levelled_schedule(h, own, order, hd.schedule_hash);
+    if (st != SW_OK) return st;
+  }
   char* out = static_cast<char*>(buffer);
   std::memcpy(out, &hd, sizeof(hd));
   size_t off = sizeof(hd);
@@ -1774,6 +2184,19 @@ sw_status sw_save_state(sw_handle* h, void* buffer, size_t bytes) {
     off += s.bytes;
   }
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "save state");
+  if (h->p.stream_mode) {  // the words and incoming rates, the sections before the last
+    const size_t nd = (size_t)h->Np * h->D;
+    char* at = out + off - (size_t)h->N * 4 - nd * 12;
+    std::vector<uint64_t> words(nd);
+    std::vector<uint32_t> inc(nd);
+    std::memcpy(words.data(), at, nd * 8);
+    std::memcpy(inc.data(), at + nd * 8, nd * 4);
+    std::vector<uint64_t> cp_words(nd);
+    std::vector<uint32_t> cp_inc(nd);
+    stream_to_checkpoint(own, order, words.data(), inc.data(), cp_words.data(), cp_inc.data(), nd);
+    std::memcpy(at, cp_words.data(), nd * 8);
+    std::memcpy(at + nd * 8, cp_inc.data(), nd * 4);
+  }
   return SW_OK;
 }
 
@@ -1791,7 +2214,14 @@ sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) {
     return h->fail(SW_ERR_INVALID_ARG, "checkpoint was written by a handle with another grid, parameters or precision");
   if (checkpoint_bytes_for(hd) != checkpoint_bytes(h))
     return h->fail(SW_ERR_INVALID_ARG, "checkpoint layout does not match this handle");
-  if (h->ops->pull && hd.schedule_hash != h->schedule_hash)
+  std::vector<uint32_t> own, order;
+  uint64_t schedule = h->schedule_hash;
+  if (h->p.stream_mode) {
+    SW_DEVICE_SCOPE(h);
+    const sw_status st = levelled_schedule(h, own, order, schedule);
+    if (st != SW_OK) return st;
+  }
+  if (h->ops->pull && hd.schedule_hash != schedule)
     return h->fail(SW_ERR_INVALID_ARG, "checkpoint was written with another transport schedule (direction groups)");
   if (check == 1) return h->fail(SW_ERR_INVALID_ARG, "corrupt checkpoint header");
   if (check == 2) return h->fail(SW_ERR_INVALID_ARG, "checkpoint buffer too small");
@@ -1804,6 +2234,17 @@ sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) {
     off += s.bytes;
   }
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "load state");
+  if (h->p.stream_mode) {
+    const size_t nd = (size_t)h->Np * h->D;
+    const char* at = in + off - (size_t)h->N * 4 - nd * 12;
+    std::vector<uint64_t> cp_words(nd), words(nd);
+    std::vector<uint32_t> cp_inc(nd), inc(nd);
+    std::memcpy(cp_words.data(), at, nd * 8);
+    std::memcpy(cp_inc.data(), at + nd * 8, nd * 4);
+    checkpoint_to_stream(own, order, cp_words.data(), cp_inc.data(), words.data(), inc.data(), nd);
+    SW_CUDA(h, cudaMemcpy(h->p.qe, words.data(), nd * 8, cudaMemcpyHostToDevice), "load state");
+    SW_CUDA(h, cudaMemcpy(h->p.incoming, inc.data(), nd * 4, cudaMemcpyHostToDevice), "load state");
+  }
   h->sim_time = hd.sim_time;
   h->ts.lowest = hd.ts_lowest;
   h->ts.first_done = hd.ts_first_done != 0;

@@ -11,6 +11,7 @@
 #if SWK_PULL
 #include "sweep_pull.cuh"
 #include "sweep_pull_setup.cuh"
+#include "sweep_stream.cuh"
 #include "sweep_pull_lockstep.cuh"
 #include "sweep_pull_wavefront.cuh"
 #include "sweep_pull_geometry.cuh"
@@ -76,9 +77,10 @@ bool staged_inputs(const DevicePtrs& p) {
 }
 
 cudaError_t attenuation(const DevicePtrs& p, int level, cudaStream_t s) {
-  swk::k_attenuation<kCarry><<<grid_for(p.num_cells, 256), 256, 0, s>>>(
+  swk::k_attenuation<kCarry, R><<<grid_for(p.num_cells, 256), 256, 0, s>>>(
       (uint32_t)p.num_cells, p.level, level, p.density, p.xhii, p.yneu, p.size, p.att, p.cell_sweep,
-      p.epoch_base, p.epoch, static_cast<uint2*>(p.cellpack), static_cast<const float*>(p.src_dir));
+      p.epoch_base, p.epoch, static_cast<uint2*>(p.cellpack), static_cast<const float*>(p.src_dir),
+      static_cast<R*>(p.cell_att));
   return cudaGetLastError();
 }
 
@@ -180,6 +182,13 @@ cudaError_t fold_periodic(const DevicePtrs& p, cudaStream_t s) {
 
 cudaError_t chemistry(const DevicePtrs& p, int level, cudaStream_t s) {
   swk::ChemArgs<R> a;
+  a.cell_rate = nullptr;
+  if (p.stream_mode) {
+    swk::k_cell_sums<R><<<grid_for(p.num_cells, 128), 128, 0, s>>>(
+        (uint32_t)p.num_cells, p.level, level, static_cast<const R*>(p.incoming), p.pos_of_task,
+        static_cast<const R*>(p.periodic), p.cell_periodic, p.source, p.D, p.Np, p.rate_scale, p.cell_rate);
+    a.cell_rate = p.cell_rate;
+  }
   a.n = (uint32_t)p.num_cells;
   a.ctl = p.ctl;
   a.current_level = level;
@@ -246,6 +255,7 @@ swk::PullArgs pull_args(const DevicePtrs& p, int level) {
   a.cellpack = static_cast<const uint2*>(p.cellpack);
   a.per_pos = p.per_pos;
   a.pos_of_task = p.pos_of_task;
+  a.inc_pos = p.stream_mode ? p.pos_of_task : nullptr;
   a.order = p.order;
   return a;
 }
@@ -418,29 +428,120 @@ cudaError_t sweep_pull_geo(const DevicePtrs& p, int level, cudaStream_t s) {
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(swk::kGeoThreads), args, 0, s);
 }
 
+// The compacted list of the level's active positions: mark the active cells' positions,
+// then compact the bitmap.
+cudaError_t compact_active(const DevicePtrs& p, int level, cudaStream_t s) {
+  uint32_t* act = p.act_lv[level];
+  uint32_t* cnt = p.act_counts + level;
+  if (!act) return cudaErrorInvalidValue;
+  if (!p.compact_now) return cudaSuccess;
+  const uint32_t words = (uint32_t)((p.num_cells * p.D + 31) / 32);
+  const uint32_t nb = (words + swk::kBitsThreads - 1) / swk::kBitsThreads;
+  uint32_t* bits = p.stream_mode ? p.act_bits_lv[level] : p.act_bits;
+  cudaError_t e = cudaMemsetAsync(bits, 0, (size_t)words * sizeof(uint32_t), s);
+  if (e != cudaSuccess) return e;
+  swk::k_mark_active<<<grid_for(p.num_cells, 256), 256, 0, s>>>(p.level, level, (uint32_t)p.num_cells, p.D, p.Np,
+                                                                  p.pos_of_task, bits);
+  swk::k_bits_count<<<nb, swk::kBitsThreads, 0, s>>>(bits, words, p.chunk);
+  swk::k_compact_scan<<<1, swk::kScanThreads, 0, s>>>(p.chunk, nb, cnt);
+  swk::k_bits_scatter<<<nb, swk::kBitsThreads, 0, s>>>(bits, words, p.chunk, act);
+  if (p.stream_mode)
+    swk::k_stream_act_range<<<grid_for((int64_t)p.num_streams * 64, 256), 256, 0, s>>>(
+        bits, p.chunk, static_cast<const swk::StreamDesc*>(p.streams), p.num_streams, (uint32_t)(p.num_cells * p.D),
+        cnt, p.act_range[level]);
+  return cudaGetLastError();
+}
+
+swk::StreamShape stream_shape(const DevicePtrs& p) {
+  return {p.stream_shape[0], p.stream_shape[1], p.stream_shape[2], p.stream_shape[3], p.stream_shape[4]};
+}
+
+swk::StreamArgs<R> stream_args(const DevicePtrs& p) {
+  swk::StreamArgs<R> a{};
+  a.streams = static_cast<const swk::StreamDesc*>(p.streams);
+  a.groups = static_cast<const swk::StreamGroup*>(p.stream_groups);
+  a.data = p.stream_data;
+  a.bytes = p.stream_bytes;
+  a.evict_first = p.stream_bytes > (64ull << 20);
+  a.seg_group = p.seg_group;
+  a.word = reinterpret_cast<swk::StreamArgs<R>::Word*>(p.qe);
+  a.inc = static_cast<R*>(p.incoming);
+  a.threshold = (R)(p.threshold / p.rate_scale);
+  a.ctl = p.ctl;
+  a.timeout_ns = p.timeout_ns;
+  a.epoch = p.epoch;
+  a.epoch_base = p.epoch_base;
+  a.shape = stream_shape(p);
+  return a;
+}
+
+template <int W>
+cudaError_t launch_stream(const DevicePtrs& p, bool all, cudaStream_t s) {
+  const swk::StreamArgs<R> a = stream_args(p);
+  const size_t smem = swk::stream_smem_bytes<R>(a.shape);
+  auto fn = a.shape.far ? (all ? swk::k_sweep_stream<R, W, true, true> : swk::k_sweep_stream<R, W, true, false>)
+                        : (all ? swk::k_sweep_stream<R, W, false, true> : swk::k_sweep_stream<R, W, false, false>);
+  cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  fn<<<p.num_streams, 32 * W, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t sweep_stream(const DevicePtrs& p, int level, cudaStream_t s) {
+  if (p.sparse_sweep) {
+    cudaError_t e = compact_active(p, level, s);
+    if (e != cudaSuccess) return e;
+    swk::StreamArgs<R> a = stream_args(p);
+    a.act = p.act_lv[level];
+    a.act_range = p.act_range[level];
+    a.act_bits = p.act_bits_lv[level];
+    a.seg = p.lvl;
+    a.order = p.order;
+    a.cell_att = static_cast<const R*>(p.cell_att);
+    a.periodic = static_cast<const R*>(p.periodic);
+    a.Np = p.Np;
+    swk::k_sweep_stream_sparse<R><<<p.num_streams, swk::kStreamSparseThreads, 0, s>>>(a);
+    return cudaGetLastError();
+  }
+  swk::k_stream_gather<R><<<grid_for((int64_t)p.num_groups * 32, 256), 256, 0, s>>>(
+      static_cast<const swk::StreamGroup*>(p.stream_groups), p.num_groups, p.stream_data, p.order, p.Np,
+      static_cast<const R*>(p.cell_att), static_cast<const R*>(p.periodic));
+  const bool all = p.active_cells >= p.num_cells;
+  switch (p.stream_shape[3]) {
+    case 4: return launch_stream<4>(p, all, s);
+    case 8: return launch_stream<8>(p, all, s);
+    default: return launch_stream<16>(p, all, s);
+  }
+}
+
+cudaError_t stream_build(const DevicePtrs& p, int phase, const StreamScratch& b, cudaStream_t s) {
+  const uint32_t total = (uint32_t)(p.num_cells * p.D);
+  swk::PullArgs a = pull_args(p, 0);
+  if (phase == 0) {
+    swk::k_invert_order<<<grid_for(total, 256), 256, 0, s>>>(p.order, total, p.pos_of_task);
+    swk::k_stream_group_segs<<<grid_for((int64_t)p.num_sched_levels * 32, 256), 256, 0, s>>>(
+        p.seg_group, p.num_sched_levels, b.gseg);
+    return cudaGetLastError();
+  }
+  const swk::StreamBuild sb{static_cast<swk::StreamGroup*>(p.stream_groups), p.num_groups, b.gseg, p.lvl, p.seg_group,
+                            b.sbase, b.sgroup, p.num_sched_levels, phase == 2 ? p.stream_data : nullptr, stream_shape(p)};
+  swk::k_stream_slots<<<grid_for((int64_t)p.num_groups * 32, 256), 256, 0, s>>>(a, sb);
+  if (phase == 2 && p.n_periodic_cells > 0)
+    swk::k_fold_build<<<grid_for((int64_t)p.n_periodic_cells * p.D, 256), 256, 0, s>>>(
+        a, p.periodic_cells, p.n_periodic_cells, p.fold_cnt, static_cast<uint2*>(p.fold_slots));
+  return cudaGetLastError();
+}
+
 cudaError_t sweep_pull(const DevicePtrs& p, int level, cudaStream_t s) {
   if (p.geo_mode) return sweep_pull_geo(p, level, s);
+  if (p.stream_mode) return sweep_stream(p, level, s);
   swk::PullArgs a = pull_args(p, level);
   const int variant = pull_variant(&p);
   if (p.sparse_sweep) {
-    uint32_t* act = p.act_lv[level];
-    uint32_t* cnt = p.act_counts + level;
-    if (!act) return cudaErrorInvalidValue;
-    if (p.compact_now) {  // mark the active cells' positions, then compact the bitmap
-      const uint32_t words = (a.count + 31) / 32;
-      const uint32_t nb = (words + swk::kBitsThreads - 1) / swk::kBitsThreads;
-      cudaError_t e = cudaMemsetAsync(p.act_bits, 0, (size_t)words * sizeof(uint32_t), s);
-      if (e != cudaSuccess) return e;
-      swk::k_mark_active<<<grid_for(p.num_cells, 256), 256, 0, s>>>(p.level, level, (uint32_t)p.num_cells, p.D,
-                                                                      p.Np, p.pos_of_task, p.act_bits);
-      swk::k_bits_count<<<nb, swk::kBitsThreads, 0, s>>>(p.act_bits, words, p.chunk);
-      swk::k_compact_scan<<<1, swk::kScanThreads, 0, s>>>(p.chunk, nb, cnt);
-      swk::k_bits_scatter<<<nb, swk::kBitsThreads, 0, s>>>(p.act_bits, words, p.chunk, act);
-      e = cudaGetLastError();
-      if (e != cudaSuccess) return e;
-    }
-    a.act = act;
-    a.act_count = cnt;
+    cudaError_t e = compact_active(p, level, s);
+    if (e != cudaSuccess) return e;
+    a.act = p.act_lv[level];
+    a.act_count = p.act_counts + level;
   }
   // the wavefront kernels run dense sweeps over a levelled schedule only; sparse sweeps
   // run the handle's lockstep variant (which tests the upwind cells' levels) or the
@@ -541,14 +642,14 @@ extern const PrecisionOps SWK_OPS = {
     SWK_NAME,       (int)sizeof(R), true,       occupancy,     attenuation, init_counts, sweep,
     occupancy_pull, sweep_pull,     kahn_round, schedule_seed, fold_pull,   chemistry,   photon_rate,
     export_rates,   records,        cell_rates, SWK_CARRY != 0,
-    (int)(sizeof(kTuneVariants) / sizeof(int)), kTuneVariants, nullptr,
+    (int)(sizeof(kTuneVariants) / sizeof(int)), kTuneVariants, nullptr, stream_build,
 };
 #else
 extern const PrecisionOps SWK_OPS = {
     SWK_NAME,         (int)sizeof(R), false,      occupancy,     attenuation,   init_counts, sweep,
     occupancy_levels, sweep_levels,   kahn_round, schedule_seed, fold_periodic, chemistry,   photon_rate,
     export_rates,     nullptr,        cell_rates, SWK_CARRY != 0,
-    0, nullptr,       push_records,
+    0, nullptr,       push_records, nullptr,
 };
 #endif
 

@@ -73,6 +73,7 @@ struct PullArgs {
   // schedule position of every task, or null in the compact state, whose words are
   // indexed by task
   const uint32_t* pos_of_task;
+  const uint32_t* inc_pos;    // direction streams: inc is indexed by position; null: by task
   const uint32_t* order;      // compact state: the task at every schedule position
 };
 
@@ -162,6 +163,9 @@ __device__ __forceinline__ bool rec_periodic(const uint4& r) { return (r.w & kRe
 __device__ __forceinline__ size_t word_of_task(const PullArgs& a, size_t t) {
   return a.pos_of_task ? (size_t)a.pos_of_task[t] : t;
 }
+
+// incoming rate of task t
+__device__ __forceinline__ float inc_of_task(const PullArgs& a, size_t t) { return a.inc[a.inc_pos ? a.inc_pos[t] : t]; }
 
 // commit of the task with record r at position p
 __device__ __forceinline__ void commit_slot(const PullArgs& a, size_t p, const uint4& r, unsigned long long word,

@@ -114,8 +114,8 @@ __device__ __forceinline__ bool cell_current(const PullArgs& a, uint32_t c) {
 __device__ __forceinline__ float current_incoming(const PullArgs& a, uint32_t c, uint32_t d, uint32_t last_epoch,
                                                   bool cell_is_current) {
   const size_t t = (size_t)d * a.Np + c;
-  if (cell_is_current) return a.inc[t];
-  if ((uint32_t)(*word_ptr(a.qe, word_of_task(a, t)) >> 32) == (last_epoch << 1)) return a.inc[t];  // solved
+  if (cell_is_current) return inc_of_task(a, t);
+  if ((uint32_t)(*word_ptr(a.qe, word_of_task(a, t)) >> 32) == (last_epoch << 1)) return inc_of_task(a, t);  // solved
   return gather_in(a, c, d, false);
 }
 

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "sweep_pull.cuh"
+#include "sweep_stream.cuh"
 
 namespace swk {
 
@@ -146,8 +147,82 @@ __global__ void __launch_bounds__(kCompactThreads) k_pull_slots(PullArgs a, uint
 }
 
 // ---------------------------------------------------------------------------------------
+// Direction streams: finds the flags and far words of every group (b.data null), or writes
+// the groups' pieces, one warp each (sweep_stream.cuh).  Classification, order and roundings
+// are those of k_pull_rec_count and k_pull_slots.
+__global__ void k_stream_slots(PullArgs a, StreamBuild b) {
+  const uint32_t lane = threadIdx.x & 31;
+  const float inv_np = 1.0f / (float)a.Np;
+  for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / 32; g < b.num_groups; g += gridDim.x * blockDim.x / 32) {
+    const StreamGroup gr = b.groups[g];
+    const StreamPiece<float> piece(b.data + 16ull * gr.data, gr);
+    const uint32_t n = group_tasks(gr.shape), padded = group_slots(gr.shape);
+    StreamSlot s = stream_slots(b, g);
+    bool ext = false;
+    uint32_t* far = const_cast<uint32_t*>(piece.far()) + lane;
+    uint16_t* idx = const_cast<uint16_t*>(piece.idx());
+    float* w = const_cast<float*>(piece.w());
+    uint32_t written = 0;
+    float inv = 0.f, source = 0.f;
+    if (lane < n) {
+      uint32_t c, d, beg, nf;
+      classify_task(a, a.order[gr.pos + lane], inv_np, c, d, beg, nf);
+      const uint32_t dnp = d * a.Np;
+      const float fx = a.dir32[3 * d], fy = a.dir32[3 * d + 1], fz = a.dir32[3 * d + 2];
+      const double dx = a.dir64[3 * d], dy = a.dir64[3 * d + 1], dz = a.dir64[3 * d + 2];
+      float area_down = 0.f;
+      source = a.src_dir[c];
+      ext = source != 0.f;
+      for (uint32_t j = 0; j < nf; ++j) {
+        const uint4 f = a.geo16[beg + j];
+        const uint32_t kind = f.w >> kKindShift;
+        const float sj = face_eff(f, fx, fy, fz, a.geo64 + beg + j, dx, dy, dz);
+        if (sj > 0.f) {
+          area_down += sj;
+        } else if (sj < 0.f && kind == kKindLocal) {
+          if (written < padded) {
+            const uint32_t up = a.pos_of_task[dnp + (f.w & kNbrMask)] - s.base, f0 = s.far;
+            const uint32_t x = stream_slot(b, s, gr.shape, lane, up);
+            if (b.data) {
+              idx[piece.slot(written, lane)] = (uint16_t)x;
+              w[piece.slot(written, lane)] = -sj;
+              if (s.far > f0) far[f0 * 32] = up;
+            }
+          }
+          ++written;
+        } else if (sj < 0.f && kind == kKindPeriodic) {
+          ext = true;
+        }
+      }
+      if (written > padded) atomicOr(&a.ctl->error, kErrRecords);
+      inv = area_down > 0.f ? 1.0f / area_down : 0.f;
+    }
+    if (b.data) {
+      for (uint32_t j = written; j < padded; ++j) {
+        idx[piece.slot(j, lane)] = (uint16_t)b.shape.ring;  // the zero word
+        w[piece.slot(j, lane)] = 0.f;
+      }
+      for (uint32_t f = s.far; f < group_far(gr.shape); ++f) far[f * 32] = 0xffffffffu;
+      const_cast<float*>(piece.inv())[lane] = inv;
+      const_cast<float*>(piece.att())[lane] = 0.f;
+      if (gr.shape & kGroupExt) {
+        const_cast<float*>(piece.per())[lane] = 0.f;
+        const_cast<float*>(piece.src())[lane] = source;
+      }
+    }
+    if (b.data && lane == 0) *reinterpret_cast<uint4*>(b.data + 16ull * gr.data) = reinterpret_cast<const uint4*>(b.groups)[g];
+    const uint32_t flags = stream_flags(ext, s, b.shape.far);
+    if (!b.data) {
+      if (lane == 0) atomicOr(&b.groups[g].shape, flags);
+    } else if (((gr.shape ^ flags) & ~(0xfffu | kGroupKeep)) != 0u) {
+      if (lane == 0) atomicOr(&a.ctl->error, kErrRecords);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------
 // exclusive scan of the chunk counts in place (one block); the total goes to *count
-__global__ void __launch_bounds__(kScanThreads) k_compact_scan(uint32_t* chunk, uint32_t n, uint32_t* count) {
+static __global__ void __launch_bounds__(kScanThreads) k_compact_scan(uint32_t* chunk, uint32_t n, uint32_t* count) {
   __shared__ uint32_t warp_sum[kScanThreads / 32];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t carry = 0;
@@ -180,12 +255,12 @@ __global__ void __launch_bounds__(kScanThreads) k_compact_scan(uint32_t* chunk, 
 // the bitmap words then yields the active positions in schedule order.  The work is the
 // active cells' tasks plus one pass over N*D/8 bytes.
 
-__global__ void k_invert_order(const uint32_t* order, uint32_t total, uint32_t* pos_of_task) {
+static __global__ void k_invert_order(const uint32_t* order, uint32_t total, uint32_t* pos_of_task) {
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x)
     pos_of_task[order[p]] = p;
 }
 
-__global__ void k_mark_active(const uint8_t* level, int cur, uint32_t n, int D, uint32_t Np,
+static __global__ void k_mark_active(const uint8_t* level, int cur, uint32_t n, int D, uint32_t Np,
                               const uint32_t* pos_of_task, uint32_t* bitmap) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
     if (level[c] < cur) continue;
@@ -198,7 +273,7 @@ __global__ void k_mark_active(const uint8_t* level, int cur, uint32_t n, int D, 
 
 constexpr int kBitsThreads = 256;  // one bitmap word per thread, kBitsThreads words per chunk
 
-__global__ void __launch_bounds__(kBitsThreads) k_bits_count(const uint32_t* bitmap, uint32_t words, uint32_t* chunk) {
+static __global__ void __launch_bounds__(kBitsThreads) k_bits_count(const uint32_t* bitmap, uint32_t words, uint32_t* chunk) {
   const uint32_t w = blockIdx.x * kBitsThreads + threadIdx.x;
   uint32_t n = w < words ? __popc(bitmap[w]) : 0u;
   for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
@@ -212,7 +287,7 @@ __global__ void __launch_bounds__(kBitsThreads) k_bits_count(const uint32_t* bit
   }
 }
 
-__global__ void __launch_bounds__(kBitsThreads) k_bits_scatter(const uint32_t* bitmap, uint32_t words,
+static __global__ void __launch_bounds__(kBitsThreads) k_bits_scatter(const uint32_t* bitmap, uint32_t words,
                                                                const uint32_t* chunk, uint32_t* act) {
   const uint32_t w = blockIdx.x * kBitsThreads + threadIdx.x;
   uint32_t bits = w < words ? bitmap[w] : 0u;

@@ -22,6 +22,29 @@ constexpr int kCompactThreads = 256;
 constexpr int kCompactPer = 8;
 constexpr uint32_t kCompactChunk = kCompactThreads * kCompactPer;
 
+// Direction streams (sweep_stream.cuh): the tasks of one direction over one closed range
+// of cells, positions [base, base + count), in groups of up to kStreamGroup consecutive
+// positions of one level (the tasks of a warp).
+struct StreamDesc {
+  uint32_t base, count;
+  uint32_t group0, groups;
+  uint32_t dir;
+  uint32_t seg0, segs;  // its dependency levels: segments [seg0, seg0 + segs)
+  uint32_t pad;
+};
+struct alignas(16) StreamGroup {
+  uint32_t need;   // groups of the stream in earlier levels: solved before this one
+  uint32_t data;   // its piece of data, in units of 16 bytes
+  uint32_t pos;    // first position
+  uint32_t shape;  // tasks - 1 | slots per task << 5 | kGroup* flags | far words per task << 17
+};
+constexpr uint32_t kStreamGroup = 32;
+constexpr uint32_t kGroupExt = 1u << 12;   // a task has a periodic source or a cell with a source
+constexpr uint32_t kGroupLate = 1u << 13;  // a far word may be solved after the warp's previous group
+constexpr uint32_t kGroupSlow = 1u << 14;  // more far words than the buffer holds
+constexpr uint32_t kGroupKeep = 1u << 15;  // a word of it is a far word of another group
+constexpr uint32_t kStreamFar = 8;         // far words of a task in the buffer at most
+
 enum : uint32_t { kErrStall = 1u, kErrQueue = 2u, kErrClamp = 8u, kErrRecords = 16u };
 
 // Control block of one handle (device memory).
