@@ -81,6 +81,7 @@ struct DevicePtrs {
   uint32_t* pos_of_task;     // pull path: schedule position of every task (inverse order)
   uint8_t* fold_cnt;         // pull path: upwind periodic faces per (periodic cell, direction)
   void* fold_slots;          // pull path: their uint2 {upwind schedule position, weight}, 4 per entry
+  uint32_t* fold_off;        // FP64 streams: first slot of every (periodic cell, direction)
   uint8_t* fold_changed;     // pull path: per periodic cell, a periodic neighbour was active
   uint32_t* act_bits;        // pull path: one bit per schedule position (sparse compaction)
   // pull path, compact state (geo_mode): no task records, upwind slots or inverse order
@@ -94,7 +95,8 @@ struct DevicePtrs {
   uint32_t space_segments[kMaxSpaces];
   uint32_t space_lvl_words[kMaxSpaces];
   // direction streams (sweep_stream.cuh): stream_mode != 0 when the handle's schedule is
-  // laid out in streams; pull_rec then holds the streams' records
+  // laid out in streams.  The FP64 path then keeps incoming and outgoing by schedule position,
+  // the sparse sweeps' stamps in queue, and no pending rates
   int stream_mode;
   void* streams;             // StreamDesc per stream, in launch order (longest first)
   void* stream_groups;       // StreamGroup per group
@@ -105,6 +107,7 @@ struct DevicePtrs {
   void* cell_att;            // attenuation of every cell or the inactive mark (R)
   double* cell_rate;         // rate of every cell summed over the directions
   uint8_t* cell_periodic;    // whether the cell has a LOCAL_PERIODIC face
+  uint8_t* stale;            // FP64 streams: cells whose incoming rates are out of date (scratch)
   uint32_t stream_shape[5];  // StreamShape: ring, magic, far, warps, buffer
   // per level, lazily allocated: the active positions' bitmap, and their range in each stream
   uint32_t *act_bits_lv[32], *act_range[32];
@@ -166,8 +169,11 @@ struct PrecisionOps {
   cudaError_t (*push_records)(const DevicePtrs&, int phase, unsigned long long* scratch, cudaStream_t);
   // direction streams, once per grid: phase 0 writes the inverse order and the groups'
   // segments; phase 1 finds the groups' flags and far words for the shape set; phase 2, with
-  // stream_data allocated, writes the groups' pieces
+  // stream_data allocated, writes the groups' pieces; FP64: phase 3 counts the periodic fold's
+  // slots, phase 4 writes them
   cudaError_t (*stream_build)(const DevicePtrs&, int phase, const StreamScratch&, cudaStream_t);
+  // FP64 streams: brings the incoming rates of inactive cells up to date; nullptr on the pull path
+  cudaError_t (*refresh)(const DevicePtrs&, cudaStream_t);
 };
 
 // pull path: transport kernel variant used without autotuning (the lockstep kernel with

@@ -865,10 +865,14 @@ static __global__ void k_ionization_time(uint32_t n, const double* xhii, double*
 
 // PhotonRate = sum over directions of the incoming rate (src/sweep/mod.rs:727-730).
 template <typename R>
-__global__ void k_photon_rate(uint32_t n, const R* incoming, int D, uint32_t Np, double rate_scale, double* out) {
+__global__ void k_photon_rate(uint32_t n, const R* incoming, const uint32_t* pos, int D, uint32_t Np, double rate_scale,
+                              double* out) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
     double r = 0.0;
-    for (int d = 0; d < D; ++d) r += (double)incoming[(size_t)d * Np + c];
+    for (int d = 0; d < D; ++d) {
+      const size_t t = (size_t)d * Np + c;
+      r += (double)incoming[pos ? pos[t] : t];
+    }
     out[c] = r * rate_scale;
   }
 }
@@ -877,13 +881,13 @@ __global__ void k_photon_rate(uint32_t n, const R* incoming, int D, uint32_t Np,
 // (src/sweep/mod.rs:616-620): sum over d of get_rate(d) = (incoming + source/D) +
 // periodic (site.rs:53-56), in photons/s.
 template <typename R>
-__global__ void k_cell_rates(uint32_t n, const R* incoming, const R* periodic, const R* src_dir, int D, uint32_t Np,
-                             double rate_scale, double* out) {
+__global__ void k_cell_rates(uint32_t n, const R* incoming, const uint32_t* pos, const R* periodic, const R* src_dir,
+                             int D, uint32_t Np, double rate_scale, double* out) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
     double r = 0.0;
     for (int d = 0; d < D; ++d) {
       const size_t t = (size_t)d * Np + c;
-      r += ((double)incoming[t] + (double)src_dir[c]) + (double)periodic[t];
+      r += ((double)incoming[pos ? pos[t] : t] + (double)src_dir[c]) + (double)periodic[t];
     }
     out[c] = r * rate_scale;
   }
@@ -949,11 +953,12 @@ static __global__ void k_time_series_final(const double* partial, int blocks, do
 
 // Convert a per-task array to FP64 photons/s in [cell][D] layout.
 template <typename R>
-__global__ void k_export_rates(uint32_t n, const R* src, int D, uint32_t Np, double rate_scale, double* out) {
+__global__ void k_export_rates(uint32_t n, const R* src, const uint32_t* pos, int D, uint32_t Np, double rate_scale, double* out) {
   const size_t total = (size_t)n * D;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t c = i / D, d = i % D;
-    out[i] = (double)src[d * (size_t)Np + c] * rate_scale;
+    const size_t t = d * (size_t)Np + c;
+    out[i] = (double)src[pos ? pos[t] : t] * rate_scale;
   }
 }
 

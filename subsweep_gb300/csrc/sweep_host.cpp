@@ -111,6 +111,8 @@ struct sw_handle {
   // direction streams: whether the schedule is to be laid out in streams, the closed cell
   // ranges of the grid ([parts] offsets), and the layout until the records are built
   bool want_streams = false, force_streams = false;
+  // whether sweeps pull (and are numbered): the mixed path and the FP64 streams
+  bool pulls() const { return ops->pull || p.stream_mode; }
   std::vector<uint32_t> parts;
   std::vector<uint32_t> stream_seg;
   std::vector<std::vector<uint8_t>> stream_gmax;  // per stream: the largest count of every group
@@ -440,16 +442,19 @@ static void stream_order(const uint16_t* level, const uint8_t* up, uint32_t Np, 
   }
 }
 
-// Whether direction streams are faster than the lockstep kernels over the levelled schedule:
-// the longest stream, at 3.6 ns a task of its block, against the time of a level (0.85 us
-// from word to word) times the levels, plus the tasks at the lockstep kernels' 17 per ns.
-// Measured on uniform boxes (mixed path, ms per sweep, lockstep and streams): 84 directions
-// 24^3 0.32 and 0.15, 48^3 0.89 and 0.52, 64^3 1.56 and 1.01, 128^3 10.3 and 7.6; 16
-// directions 64^3 0.95 and 0.87, but 101^3 1.87 and 2.98: sixteen blocks cannot keep up
-// with the whole device where levels are wide.
-static bool streams_pay(const std::vector<uint32_t>& parts, uint64_t tasks, size_t levels) {
+// Whether direction streams are faster than the kernels over the levelled schedule: the longest
+// stream, at 3.6 ns a task of its block (FP64 7.7), against the time of a level, from word to word
+// 0.85 us (FP64 push form, from atomic to atomic: 4), times the levels, plus the tasks at 17 per
+// ns (12).  Measured on uniform boxes, ms per sweep, levelled and streams.  Mixed path: 84
+// directions 24^3 0.32 and 0.15, 48^3 0.89 and 0.52, 64^3 1.56 and 1.01, 128^3 10.3 and 7.6; 16
+// directions 64^3 0.95 and 0.87, but 101^3 1.87 and 2.98: sixteen blocks cannot keep up with the
+// whole device where levels are wide.  FP64: 84 directions 16^3 0.97 and 0.18, 24^3 1.61 and 0.31,
+// 32^3 2.10 and 0.46, 64^3 5.4 and 2.0, 96^3 13.8 and 7.9; 16 directions 64^3 4.8 and 1.8, 101^3
+// 7.8 and 7.5.
+static bool streams_pay(const std::vector<uint32_t>& parts, uint64_t tasks, size_t levels, bool mixed) {
   uint32_t longest = 0;
   for (size_t k = 1; k < parts.size(); ++k) longest = std::max(longest, parts[k] - parts[k - 1]);
+  if (!mixed) return 7.7 * longest < 4000.0 * (double)levels + (double)tasks / 12.0;
   return 3.6 * longest < 850.0 * (double)levels + (double)tasks / 17.0;
 }
 
@@ -565,7 +570,7 @@ sw_status build_schedule(sw_handle* h) {
     // and checkpoints hold them in that order.
     const size_t L = lvl.size() - 1;
     depth = std::max(depth, (uint32_t)L);
-    if (h->want_streams) h->want_streams = h->force_streams || streams_pay(h->parts, total, L);
+    if (h->want_streams) h->want_streams = h->force_streams || streams_pay(h->parts, total, L, h->ops->pull);
     int groups = schedule_dir_groups(q.D, total, L);
     if (p.geo_mode && !std::getenv("SUBSWEEP_DIR_GROUPS")) groups = 1;
     std::vector<uint32_t> seg = {0};
@@ -613,7 +618,7 @@ sw_status build_schedule(sw_handle* h) {
 // Without them the transport computes the geometry on the fly.
 sw_status build_push_records(sw_handle* h) {
   swh::DevicePtrs& p = h->p;
-  if (!h->ops->push_records || p.num_sched_levels == 0) return SW_OK;
+  if (!h->ops->push_records || p.num_sched_levels == 0 || p.stream_mode) return SW_OK;
   int mode = -1;
   if (const char* env = std::getenv("SUBSWEEP_FP64_RECORDS")) mode = std::atoi(env) != 0 ? 1 : 0;
   if (mode == 0) return SW_OK;
@@ -690,7 +695,7 @@ static void plan_stream(const swk::StreamDesc& sd, const uint32_t* seg, const st
 // bytes of a group's piece (StreamPiece), rb bytes a rate
 static uint32_t piece_bytes(uint32_t shape, uint32_t rb) {
   const uint32_t slots = (shape >> 5) & 0x7fu, far = shape >> 17;
-  return (uint32_t)sizeof(swk::StreamGroup) +
+  return (uint32_t)sizeof(swk::StreamGroup) + (rb == 8 ? 16u : 0u) +
          32u * (rb + (rb == 4 ? 4u : 0u) + slots * (rb + 2u) + ((shape & swk::kGroupExt) ? 2u * rb : 0u) + far * 4u);
 }
 
@@ -702,7 +707,11 @@ sw_status build_streams(sw_handle* h) {
   const uint32_t segs = (uint32_t)seg.size() - 1;
   const uint32_t rb = (uint32_t)h->ops->rate_bytes;
   const double width = (double)h->N * h->D / segs;  // of a level, on average
-  uint32_t warps = width <= 32 ? 4 : (width <= 96 ? 8 : 16);
+  // warps of a block: as many as find a group of a level to work on.  Mixed path, 84 directions,
+  // ms per sweep with 4, 8 and 16: 24^3 (35 tasks a level) 0.159, 0.152, 0.185; 32^3 (62) 0.289,
+  // 0.235, 0.274; 48^3 (138) 0.80, 0.57, 0.52; 64^3 (250) 2.5, 1.55, 1.01.  FP64, whose warps also
+  // sum ahead: 24^3 0.36, 0.31, 0.31; 32^3 0.69, 0.48, 0.46; 48^3 2.2, 1.38, 1.02.
+  uint32_t warps = width <= 32 ? 4 : (width <= (rb == 4 ? 96 : 48) ? 8 : 16);
   if (const char* env = std::getenv("SUBSWEEP_STREAM_WARPS")) {
     const int v = std::atoi(env);
     if (v == 4 || v == 8 || v == 16) warps = (uint32_t)v;
@@ -776,9 +785,24 @@ sw_status build_streams(sw_handle* h) {
   SW_CUDA(h, scratch.get((void**)&b.sgroup, sgroup.size() * 4, sgroup.data()), "stream scratch");
   swk::StreamDesc* d_streams = nullptr;
   swk::StreamGroup* d_groups = nullptr;
+  uint32_t* d_cell_sweep = nullptr;
   if (!h->alloc(&d_streams, h->streams.size()) || !h->alloc(&d_groups, groups.size() + 1) ||
       !h->alloc(&p.seg_group, seg_group.size()))
     return h->fail(SW_ERR_OOM, "device allocation of the streams failed");
+  if (rb == 8) {  // what the push form does without
+    uint32_t *pos = nullptr, *counts = nullptr, *cell_sweep = nullptr;
+    if (!h->alloc(&pos, (size_t)h->Np * h->D) || !h->alloc(&counts, 32) || !h->alloc(&cell_sweep, h->Np) ||
+        !h->alloc(&p.stale, h->N) || !h->alloc(&p.fold_changed, p.n_periodic_cells) ||
+        !h->alloc(&p.fold_off, (size_t)p.n_periodic_cells * h->D + 1)) {
+      (void)cudaGetLastError();
+      h->want_streams = false;
+      return SW_OK;
+    }
+    SW_CUDA(h, cudaMemset(cell_sweep, 0, h->Np * sizeof(uint32_t)), "streams");
+    p.pos_of_task = pos;
+    p.act_counts = counts;
+    d_cell_sweep = cell_sweep;
+  }
   p.streams = d_streams;
   p.stream_groups = d_groups;
   p.num_streams = (uint32_t)h->streams.size();
@@ -825,7 +849,12 @@ sw_status build_streams(sw_handle* h) {
   }
   SW_CUDA(h, cudaMemcpy(d_groups, groups.data(), groups.size() * sizeof(groups[0]), cudaMemcpyHostToDevice), "groups");
   groups.pop_back();
-  if (!h->alloc(&p.stream_data, at)) {  // no room: the levelled schedule (smaller, unless groups are full)
+  // no room: the levelled schedule.  FP64: as for the push form's records, room is what leaves a
+  // reserve of 1/16 of the device (at least 4 GiB) for later allocations.
+  size_t free_b = 0, total_b = 0;
+  SW_CUDA(h, cudaMemGetInfo(&free_b, &total_b), "memory info");
+  const size_t reserve = rb == 8 ? std::max(total_b / 16, (size_t)4 << 30) : 0;
+  if (at + reserve > free_b || !h->alloc(&p.stream_data, at)) {
     (void)cudaGetLastError();
     p.stream_data = nullptr;
     h->want_streams = false;
@@ -841,8 +870,42 @@ sw_status build_streams(sw_handle* h) {
   p.stream_bytes = at;
   p.cell_att = cell_att;
   SW_CUDA(h, cudaMemcpy(p.cell_periodic, has_periodic.data(), h->N, cudaMemcpyHostToDevice), "periodic cells");
+  SW_CUDA(h, cudaMemsetAsync(p.ctl, 0, offsetof(swk::SweepCtl, tasks), h->stream), "reset control");
   SW_CUDA(h, h->ops->stream_build(p, 2, b, h->stream), "upwind slot kernel");
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "upwind slots");
+  if (rb == 8 && p.n_periodic_cells > 0) {  // the periodic fold's slots
+    const size_t entries = (size_t)p.n_periodic_cells * h->D;
+    void* cnt = nullptr;
+    SW_CUDA(h, scratch.get(&cnt, entries, nullptr), "fold scratch");
+    p.fold_cnt = static_cast<uint8_t*>(cnt);
+    SW_CUDA(h, h->ops->stream_build(p, 3, b, h->stream), "periodic fold entries");
+    SW_CUDA(h, cudaStreamSynchronize(h->stream), "periodic fold entries");
+    p.fold_cnt = nullptr;
+    std::vector<uint8_t> n(entries);
+    SW_CUDA(h, cudaMemcpy(n.data(), cnt, entries, cudaMemcpyDeviceToHost), "periodic fold entries");
+    std::vector<uint32_t> off(entries + 1, 0u);
+    for (size_t e = 0; e < entries; ++e) off[e + 1] = off[e] + n[e];
+    SW_CUDA(h, cudaMemcpy(p.fold_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice), "periodic fold entries");
+    uint4* fslots = nullptr;
+    if (!h->alloc(&fslots, off[entries])) return h->fail(SW_ERR_OOM, "device allocation of the periodic fold slots failed");
+    p.fold_slots = fslots;
+    SW_CUDA(h, h->ops->stream_build(p, 4, b, h->stream), "periodic fold entries");
+    SW_CUDA(h, cudaStreamSynchronize(h->stream), "periodic fold entries");
+  }
+  if (rb == 8) {
+    unsigned long long faces[2] = {0, 0};  // handed out, found
+    SW_CUDA(h, cudaMemcpy(&faces[0], &p.ctl->head, 8, cudaMemcpyDeviceToHost), "upwind slots");
+    SW_CUDA(h, cudaMemcpy(&faces[1], &p.ctl->tail, 8, cudaMemcpyDeviceToHost), "upwind slots");
+    const size_t nd = (size_t)h->Np * h->D;
+    SW_CUDA(h, cudaMemset(p.pending, 0, nd * 8), "pending rates");
+    SW_CUDA(h, cudaMemset(p.ctl, 0, offsetof(swk::SweepCtl, error)), "reset control");
+    if (faces[0] != faces[1]) {  // faces without a partner of their own: only the push form tells them apart
+      h->want_streams = false;
+      p.cell_att = nullptr;
+      return SW_OK;
+    }
+    p.cell_sweep = d_cell_sweep;
+  }
   uint32_t err = 0;
   SW_CUDA(h, cudaMemcpy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
   if (err & swk::kErrRecords) return h->fail(SW_ERR_CUDA, "upwind slot classification disagrees with its count");
@@ -1364,9 +1427,11 @@ sw_status sw_create(const sw_params* params, const sw_grid_csr* grid, const sw_c
     }
   }
   // Direction streams (SUBSWEEP_STREAMS=0 turns them off; so does pinning a transport
-  // kernel variant or the direction groups of the levelled schedule).
+  // kernel variant, the direction groups of the levelled schedule, the FP64 path's push form
+  // or its records).
   if (h->ops->stream_build && !p.geo_mode) {
-    h->want_streams = !std::getenv("SUBSWEEP_PULL_VARIANT") && !std::getenv("SUBSWEEP_DIR_GROUPS");
+    h->want_streams = !std::getenv("SUBSWEEP_PULL_VARIANT") && !std::getenv("SUBSWEEP_DIR_GROUPS") &&
+                      !std::getenv("SUBSWEEP_FP64_RECORDS") && h->force_path == 0;
     if (const char* env = std::getenv("SUBSWEEP_STREAMS")) {
       h->want_streams = h->want_streams && std::atoi(env) != 0;
       h->force_streams = h->want_streams;
@@ -1477,8 +1542,9 @@ static bool pull_sparse(sw_handle* h, int level) {
   if (p.compact_mode == 2) return false;
   // Streams: a dense sweep takes the time of all tasks, 23 per ns, a sparse one ~5 per ns of
   // the active ones (128^3 x 84: 7.9 ms dense; sparse 14 ms with 39% of the cells active, the
-  // crossing near 20%; 64^3 x 84: 1.03 ms dense, 0.13 ms with 0.2% active).
-  if (p.stream_mode) return (int64_t)h->n_ge_host[level] * 5 < h->N;
+  // crossing near 20%; 64^3 x 84: 1.03 ms dense, 0.13 ms with 0.2% active).  FP64: a sparse sweep
+  // of all tasks takes twice a dense one's time (24^3 x 84, 32 sweeps: 19.8 and 9.8 ms).
+  if (p.stream_mode) return (int64_t)h->n_ge_host[level] * 5 < (h->ops->pull ? 1 : 2) * h->N;
   return h->n_ge_host[level] * 2 < h->N;
 }
 
@@ -1513,7 +1579,7 @@ static sw_status step_graph(sw_handle* h, double* time_elapsed_out) {
     expected += (uint64_t)h->n_ge_host[level] * (uint64_t)h->D;
     // pull path: compaction or not; push path: levelled schedule or ready queue
     bool variant;
-    if (ops.pull) {
+    if (h->pulls()) {
       variant = pull_sparse(h, level);
       if (variant) {
         sw_status st = ensure_act_list(h, level);  // allocations stay outside the capture
@@ -1555,9 +1621,10 @@ static sw_status step_graph(sw_handle* h, double* time_elapsed_out) {
       // attenuation, transport, chemistry, the periodic fold, and the counts (push) or
       // the compaction at a sparse level's first sweep (pull)
       kernels += 3 + (p.n_periodic_cells > 0 ? 1 : 0);
+      if (p.stream_mode) kernels += variants[k] ? 1 : 2;  // rates of the cells, gather of a dense sweep
       // the fold's mark pass after a sweep that leaves cells inactive (pull path)
-      if (ops.pull && p.n_periodic_cells > 0 && h->n_ge_host[levels[k]] < h->N) kernels += 1;
-      if (!ops.pull) {
+      if (h->pulls() && p.n_periodic_cells > 0 && h->n_ge_host[levels[k]] < h->N) kernels += 1;
+      if (!h->pulls()) {
         kernels += 1;
       } else if (variants[k] && !((compacted >> levels[k]) & 1u)) {
         compact_now[k] = 1;
@@ -1569,14 +1636,14 @@ static sw_status step_graph(sw_handle* h, double* time_elapsed_out) {
       const int level = levels[k];
       q.epoch = (uint32_t)(k + 1);
       q.active_cells = h->n_ge_host[level];
-      q.sparse_sweep = (ops.pull && variants[k]) ? 1 : 0;
+      q.sparse_sweep = (h->pulls() && variants[k]) ? 1 : 0;
       q.compact_now = compact_now[k];
       ce = cudaMemsetAsync(p.ctl, 0, offsetof(swk::SweepCtl, error), h->stream);
       if (ce == cudaSuccess) ce = ops.attenuation(q, level, h->stream);
-      if (ce == cudaSuccess && !ops.pull) ce = ops.init_counts(q, level, nullptr, !variants[k], h->stream);
+      if (ce == cudaSuccess && !h->pulls()) ce = ops.init_counts(q, level, nullptr, !variants[k], h->stream);
       // external records: event nodes that are recorded when the graph runs
       if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(h->graph_ev[2 * k], h->stream, cudaEventRecordExternal);
-      if (ce == cudaSuccess) ce = (ops.pull || variants[k]) ? ops.sweep_levels(q, level, h->stream)
+      if (ce == cudaSuccess) ce = (h->pulls() || variants[k]) ? ops.sweep_levels(q, level, h->stream)
                                                             : ops.sweep(q, level, h->stream);
       if (ce == cudaSuccess) ce = cudaEventRecordWithFlags(h->graph_ev[2 * k + 1], h->stream, cudaEventRecordExternal);
       if (ce == cudaSuccess) ce = ops.fold_periodic(q, h->stream);
@@ -1601,6 +1668,7 @@ static sw_status step_graph(sw_handle* h, double* time_elapsed_out) {
   h->graph_scalars->epoch_base = p.epoch;
   h->graph_scalars->time = h->sim_time + elapsed;
   const unsigned long long tasks_before = h->ctl_host.tasks;
+  if (!levels.empty()) p.active_cells = h->n_ge_host[levels.back()];  // of the step's last sweep
   SW_CUDA(h, cudaEventRecord(h->ev[5], h->stream), "event");
   SW_CUDA(h, cudaGraphLaunch(h->graph_exec, h->stream), "graph launch");
   SW_CUDA(h, cudaEventRecord(h->ev[1], h->stream), "event");
@@ -1633,7 +1701,7 @@ static sw_status step_graph(sw_handle* h, double* time_elapsed_out) {
   h->stats.step_ms += step_ms;
   h->stats.steps += 1;
   h->stats.level_sweeps += n;
-  for (bool v : variants) h->stats.levelled_sweeps += (ops.pull || v) ? 1 : 0;
+  for (bool v : variants) h->stats.levelled_sweeps += (h->pulls() || v) ? 1 : 0;
   h->stats.transport_launches += n;
   h->stats.graph_launches += 1;
   h->stats.kernel_launches += h->graph_kernels;
@@ -1731,7 +1799,7 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
     // autotuning trials on dense sweeps only: sparse ones always run the lockstep kernel
     const bool trial = ops.pull && h->autotune && !h->tuned && !pull_sparse(h, level);
     if (trial && !h->p.stream_mode) h->p.pull_variant = ops.tune_variants[h->tune_index];
-    if (ops.pull) {
+    if (h->pulls()) {
       levelled = true;  // the pull path always walks the schedule (or the id order)
       h->p.epoch += 1;
       h->last_epoch = h->p.epoch;
@@ -1750,7 +1818,7 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
     }
     // after the pull path's sweep number advanced: attenuation records it per solved cell
     SW_CUDA(h, ops.attenuation(h->p, level, h->stream), "attenuation kernel");
-    if (!ops.pull) {
+    if (!h->pulls()) {
       SW_CUDA(h, ops.init_counts(h->p, level, nullptr, !levelled, h->stream), "init_counts kernel");
       launches += 1;
     }
@@ -1764,7 +1832,8 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
     SW_CUDA(h, cudaEventRecord(h->ev[7], h->stream), "event");
     SW_CUDA(h, ops.fold_periodic(h->p, h->stream), "periodic fold kernel");
     launches += 3 + (h->p.n_periodic_cells > 0 ? 1 : 0);
-    if (ops.pull && h->p.n_periodic_cells > 0 && h->p.active_cells < h->N) launches += 1;  // fold marks
+    if (h->p.stream_mode) launches += h->p.sparse_sweep ? 1 : 2;  // rates of the cells, gather of a dense sweep
+    if (h->pulls() && h->p.n_periodic_cells > 0 && h->p.active_cells < h->N) launches += 1;  // fold marks
     SW_CUDA(h, cudaEventRecord(h->ev[1], h->stream), "event");
     SW_CUDA(h, ops.chemistry(h->p, level, h->stream), "chemistry kernel");
     SW_CUDA(h, cudaEventRecord(h->ev[2], h->stream), "event");
@@ -2028,26 +2097,33 @@ static sw_status levelled_schedule(sw_handle* h, std::vector<uint32_t>& own, std
   return SW_OK;
 }
 
-// Words and incoming rates of a checkpoint from the streams' layout, and back.
-static void stream_to_checkpoint(const std::vector<uint32_t>& own, const std::vector<uint32_t>& order,
-                                 const uint64_t* words, const uint32_t* inc, uint64_t* cp_words, uint32_t* cp_inc,
-                                 size_t nd) {
-  std::vector<uint32_t> pos(nd, 0);
-  for (size_t i = 0; i < own.size(); ++i) pos[own[i]] = (uint32_t)i;
-  std::memset(cp_words, 0, nd * 8);
-  std::memset(cp_inc, 0, nd * 4);
-  for (size_t i = 0; i < order.size(); ++i) cp_words[i] = words[pos[order[i]]];
-  for (size_t i = 0; i < own.size(); ++i) cp_inc[own[i]] = inc[i];
+// The rates of a checkpoint, from the streams' layout (by position) or back to it: mixed path
+// words by position of the levelled schedule and incoming rates by task, FP64 incoming and
+// outgoing rates by task.
+static void reorder(char* at, size_t nd, size_t elem, const std::vector<uint32_t>& own,
+                    const std::vector<uint32_t>* order, bool save) {
+  std::vector<uint32_t> to(own);  // index in the checkpoint of every position
+  if (order) {
+    std::vector<uint32_t> rank(nd, 0);
+    for (size_t i = 0; i < order->size(); ++i) rank[(*order)[i]] = (uint32_t)i;
+    for (uint32_t& t : to) t = rank[t];
+  }
+  const std::vector<char> in(at, at + nd * elem);
+  std::memset(at, 0, nd * elem);
+  for (size_t i = 0; i < to.size(); ++i)
+    std::memcpy(at + (save ? to[i] : i) * elem, in.data() + (save ? i : to[i]) * elem, elem);
 }
-static void checkpoint_to_stream(const std::vector<uint32_t>& own, const std::vector<uint32_t>& order,
-                                 const uint64_t* cp_words, const uint32_t* cp_inc, uint64_t* words, uint32_t* inc,
-                                 size_t nd) {
-  std::vector<uint32_t> pos(nd, 0);
-  for (size_t i = 0; i < own.size(); ++i) pos[own[i]] = (uint32_t)i;
-  std::memset(words, 0, nd * 8);
-  std::memset(inc, 0, nd * 4);
-  for (size_t i = 0; i < order.size(); ++i) words[pos[order[i]]] = cp_words[i];
-  for (size_t i = 0; i < own.size(); ++i) inc[i] = cp_inc[own[i]];
+static void reorder_rates(sw_handle* h, char* end, const std::vector<uint32_t>& own, const std::vector<uint32_t>& order,
+                          bool save) {
+  const size_t nd = (size_t)h->Np * h->D;
+  if (h->ops->pull) {  // the sections before the last
+    char* words = end - (size_t)h->N * 4 - nd * 12;
+    reorder(words, nd, 8, own, &order, save);
+    reorder(words + nd * 8, nd, 4, own, nullptr, save);
+  } else {
+    reorder(end - 3 * nd * 8, nd, 8, own, nullptr, save);
+    reorder(end - 2 * nd * 8, nd, 8, own, nullptr, save);
+  }
 }
 
 static size_t checkpoint_bytes(sw_handle* h) {
@@ -2168,13 +2244,16 @@ sw_status sw_save_state(sw_handle* h, void* buffer, size_t bytes) {
   hd.sim_time = h->sim_time;
   hd.ts_lowest = h->ts.lowest;
   hd.ts_first_done = h->ts.first_done ? 1 : 0;
-  hd.epoch = h->p.epoch;
-  hd.last_epoch = h->last_epoch;
+  hd.epoch = h->ops->pull ? h->p.epoch : 0u;
+  hd.last_epoch = h->ops->pull ? h->last_epoch : 0u;
   hd.schedule_hash = h->ops->pull ? h->schedule_hash : 0;
   std::vector<uint32_t> own, order;
   if (h->p.stream_mode) {
-    const sw_status st = levelled_schedule(h, own, order, hd.schedule_hash);
+    uint64_t schedule = 0;
+    const sw_status st = levelled_schedule(h, own, order, schedule);
     if (st != SW_OK) return st;
+    if (h->ops->pull) hd.schedule_hash = schedule;
+    if (h->ops->refresh) SW_CUDA(h, h->ops->refresh(h->p, h->stream), "incoming rates");
   }
   char* out = static_cast<char*>(buffer);
   std::memcpy(out, &hd, sizeof(hd));
@@ -2184,19 +2263,7 @@ sw_status sw_save_state(sw_handle* h, void* buffer, size_t bytes) {
     off += s.bytes;
   }
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "save state");
-  if (h->p.stream_mode) {  // the words and incoming rates, the sections before the last
-    const size_t nd = (size_t)h->Np * h->D;
-    char* at = out + off - (size_t)h->N * 4 - nd * 12;
-    std::vector<uint64_t> words(nd);
-    std::vector<uint32_t> inc(nd);
-    std::memcpy(words.data(), at, nd * 8);
-    std::memcpy(inc.data(), at + nd * 8, nd * 4);
-    std::vector<uint64_t> cp_words(nd);
-    std::vector<uint32_t> cp_inc(nd);
-    stream_to_checkpoint(own, order, words.data(), inc.data(), cp_words.data(), cp_inc.data(), nd);
-    std::memcpy(at, cp_words.data(), nd * 8);
-    std::memcpy(at + nd * 8, cp_inc.data(), nd * 4);
-  }
+  if (h->p.stream_mode) reorder_rates(h, out + off, own, order, true);
   return SW_OK;
 }
 
@@ -2228,22 +2295,22 @@ sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) {
   if (check == 3) return h->fail(SW_ERR_INVALID_ARG, "corrupt checkpoint: a cell's timestep level is out of range");
   SW_DEVICE_SCOPE(h);
   const char* in = static_cast<const char*>(buffer);
+  std::vector<char> reordered;
+  if (h->p.stream_mode) {
+    reordered.assign(in, in + checkpoint_bytes(h));
+    in = reordered.data();
+    reorder_rates(h, reordered.data() + reordered.size(), own, order, false);
+  }
   size_t off = sizeof(hd);
   for (const CheckpointSection& s : checkpoint_sections(h)) {
     SW_CUDA(h, cudaMemcpyAsync(s.dev, in + off, s.bytes, cudaMemcpyHostToDevice, h->stream), "load state");
     off += s.bytes;
   }
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "load state");
-  if (h->p.stream_mode) {
-    const size_t nd = (size_t)h->Np * h->D;
-    const char* at = in + off - (size_t)h->N * 4 - nd * 12;
-    std::vector<uint64_t> cp_words(nd), words(nd);
-    std::vector<uint32_t> cp_inc(nd), inc(nd);
-    std::memcpy(cp_words.data(), at, nd * 8);
-    std::memcpy(cp_inc.data(), at + nd * 8, nd * 4);
-    checkpoint_to_stream(own, order, cp_words.data(), cp_inc.data(), words.data(), inc.data(), nd);
-    SW_CUDA(h, cudaMemcpy(h->p.qe, words.data(), nd * 8, cudaMemcpyHostToDevice), "load state");
-    SW_CUDA(h, cudaMemcpy(h->p.incoming, inc.data(), nd * 4, cudaMemcpyHostToDevice), "load state");
+  if (h->p.stream_mode && !h->ops->pull) {  // every incoming rate is current, no sweep is stamped
+    h->p.active_cells = h->N;
+    SW_CUDA(h, cudaMemset(h->p.cell_sweep, 0, (size_t)h->Np * 4), "load state");
+    SW_CUDA(h, cudaMemset(h->p.queue, 0xff, (size_t)h->Np * h->D * 4), "load state");
   }
   h->sim_time = hd.sim_time;
   h->ts.lowest = hd.ts_lowest;

@@ -3,21 +3,24 @@
 // (R = float, carried neutral fraction); each defines SWK_R, SWK_CARRY and SWK_OPS.
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 
 #include "launch.h"
+#include "sweep_compact.cuh"
 #include "sweep_device.cuh"
+#include "sweep_stream.cuh"
 #if SWK_PULL
 #include "sweep_pull.cuh"
 #include "sweep_pull_setup.cuh"
-#include "sweep_stream.cuh"
 #include "sweep_pull_lockstep.cuh"
 #include "sweep_pull_wavefront.cuh"
 #include "sweep_pull_geometry.cuh"
 #include "sweep_pull_fold.cuh"
 #else
 #include "sweep_push_records.cuh"
+#include "sweep_stream_fp64.cuh"
 #endif
 
 namespace swh {
@@ -59,6 +62,97 @@ int grid_for(int64_t work, int block) {
   if (g < 1) g = 1;
   if (g > 152 * 32) g = 152 * 32;
   return (int)g;
+}
+
+// The compacted list of the level's active positions: mark the active cells' positions,
+// then compact the bitmap.
+cudaError_t compact_active(const DevicePtrs& p, int level, cudaStream_t s) {
+  uint32_t* act = p.act_lv[level];
+  uint32_t* cnt = p.act_counts + level;
+  if (!act) return cudaErrorInvalidValue;
+  if (!p.compact_now) return cudaSuccess;
+  const uint32_t words = (uint32_t)((p.num_cells * p.D + 31) / 32);
+  const uint32_t nb = (words + swk::kBitsThreads - 1) / swk::kBitsThreads;
+  uint32_t* bits = p.stream_mode ? p.act_bits_lv[level] : p.act_bits;
+  cudaError_t e = cudaMemsetAsync(bits, 0, (size_t)words * sizeof(uint32_t), s);
+  if (e != cudaSuccess) return e;
+  swk::k_mark_active<<<grid_for(p.num_cells, 256), 256, 0, s>>>(p.level, level, (uint32_t)p.num_cells, p.D, p.Np,
+                                                                  p.pos_of_task, bits);
+  swk::k_bits_count<<<nb, swk::kBitsThreads, 0, s>>>(bits, words, p.chunk);
+  swk::k_compact_scan<<<1, swk::kScanThreads, 0, s>>>(p.chunk, nb, cnt);
+  swk::k_bits_scatter<<<nb, swk::kBitsThreads, 0, s>>>(bits, words, p.chunk, act);
+  if (p.stream_mode)
+    swk::k_stream_act_range<<<grid_for((int64_t)p.num_streams * 64, 256), 256, 0, s>>>(
+        bits, p.chunk, static_cast<const swk::StreamDesc*>(p.streams), p.num_streams, (uint32_t)(p.num_cells * p.D),
+        cnt, p.act_range[level]);
+  return cudaGetLastError();
+}
+
+swk::StreamShape stream_shape(const DevicePtrs& p) {
+  return {p.stream_shape[0], p.stream_shape[1], p.stream_shape[2], p.stream_shape[3], p.stream_shape[4]};
+}
+
+swk::StreamArgs<R> stream_args(const DevicePtrs& p) {
+  swk::StreamArgs<R> a{};
+  a.streams = static_cast<const swk::StreamDesc*>(p.streams);
+  a.groups = static_cast<const swk::StreamGroup*>(p.stream_groups);
+  a.data = p.stream_data;
+  a.bytes = p.stream_bytes;
+  a.evict_first = p.stream_bytes > (64ull << 20);
+  a.seg_group = p.seg_group;
+#if SWK_PULL
+  a.word = p.qe;
+#else
+  a.word = static_cast<double*>(p.outgoing);
+  a.stamp = p.queue;
+#endif
+  a.inc = static_cast<R*>(p.incoming);
+  a.threshold = (R)(p.threshold / p.rate_scale);
+  a.ctl = p.ctl;
+  a.timeout_ns = p.timeout_ns;
+  a.epoch = p.epoch;
+  a.epoch_base = p.epoch_base;
+  a.shape = stream_shape(p);
+  a.seg = p.lvl;
+  a.order = p.order;
+  a.cell_att = static_cast<const R*>(p.cell_att);
+  a.periodic = static_cast<const R*>(p.periodic);
+  a.Np = p.Np;
+  return a;
+}
+
+template <int W>
+cudaError_t launch_stream(const DevicePtrs& p, bool all, cudaStream_t s) {
+  const swk::StreamArgs<R> a = stream_args(p);
+  const size_t smem = swk::stream_smem_bytes<R>(a.shape);
+  auto fn = a.shape.far ? (all ? swk::k_sweep_stream<R, W, true, true> : swk::k_sweep_stream<R, W, true, false>)
+                        : (all ? swk::k_sweep_stream<R, W, false, true> : swk::k_sweep_stream<R, W, false, false>);
+  cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  fn<<<p.num_streams, 32 * W, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t sweep_stream(const DevicePtrs& p, int level, cudaStream_t s) {
+  if (p.sparse_sweep) {
+    cudaError_t e = compact_active(p, level, s);
+    if (e != cudaSuccess) return e;
+    swk::StreamArgs<R> a = stream_args(p);
+    a.act = p.act_lv[level];
+    a.act_range = p.act_range[level];
+    a.act_bits = p.act_bits_lv[level];
+    swk::k_sweep_stream_sparse<R><<<p.num_streams, swk::kStreamSparseThreads, 0, s>>>(a);
+    return cudaGetLastError();
+  }
+  swk::k_stream_gather<R><<<grid_for((int64_t)p.num_groups * 32, 256), 256, 0, s>>>(
+      static_cast<const swk::StreamGroup*>(p.stream_groups), p.num_groups, p.stream_data, p.order, p.Np,
+      static_cast<const R*>(p.cell_att), static_cast<const R*>(p.periodic));
+  const bool all = p.active_cells >= p.num_cells;
+  switch (p.stream_shape[3]) {
+    case 4: return launch_stream<4>(p, all, s);
+    case 8: return launch_stream<8>(p, all, s);
+    default: return launch_stream<16>(p, all, s);
+  }
 }
 
 cudaError_t occupancy(int* blocks_per_sm) {
@@ -111,6 +205,7 @@ cudaError_t sweep_levels(const DevicePtrs& p, int level, cudaStream_t s) {
   swk::SweepArgs<R> a = sweep_args(p, level);
   uint32_t total = (uint32_t)(p.num_cells * p.D);
 #if !SWK_PULL
+  if (p.stream_mode) return sweep_stream(p, level, s);
   if (p.push_rec) {
     const uint4* rec = static_cast<const uint4*>(p.push_rec);
     const uint32_t* tgt = p.push_tgt;
@@ -151,6 +246,47 @@ cudaError_t push_records(const DevicePtrs& p, int phase, unsigned long long* scr
 }
 #endif
 
+#if !SWK_PULL
+swk::FacePull face_pull(const DevicePtrs& p, const double* total) {
+  return {sweep_args(p, 0), p.order, p.pos_of_task, total};
+}
+
+// FP64 direction streams (the tasks' totals in `pending` until the pieces are written)
+cudaError_t stream_build64(const DevicePtrs& p, int phase, const StreamScratch& b, cudaStream_t s) {
+  const uint32_t total = (uint32_t)(p.num_cells * p.D);
+  double* totals = static_cast<double*>(p.pending);
+  const swk::FacePull f = face_pull(p, totals);
+  if (phase == 0) {
+    swk::k_invert_order<<<grid_for(total, 256), 256, 0, s>>>(p.order, total, p.pos_of_task);
+    swk::k_stream_group_segs<<<grid_for((int64_t)p.num_sched_levels * 32, 256), 256, 0, s>>>(
+        p.seg_group, p.num_sched_levels, b.gseg);
+    swk::k_task_totals<<<grid_for(total, 256), 256, 0, s>>>(f, totals);
+    return cudaGetLastError();
+  }
+  if (phase >= 3) {
+    if (p.n_periodic_cells > 0)
+      swk::k_fold_build64<<<grid_for((int64_t)p.n_periodic_cells * p.D, 256), 256, 0, s>>>(
+          f, p.periodic_cells, p.n_periodic_cells, p.fold_cnt, p.fold_off,
+          phase == 3 ? nullptr : static_cast<swk::FoldSlot64*>(p.fold_slots));
+    return cudaGetLastError();
+  }
+  const swk::StreamBuild sb{static_cast<swk::StreamGroup*>(p.stream_groups), p.num_groups, b.gseg, p.lvl, p.seg_group,
+                            b.sbase, b.sgroup, p.num_sched_levels, phase == 2 ? p.stream_data : nullptr, stream_shape(p)};
+  swk::k_stream_slots64<<<grid_for((int64_t)p.num_groups * 32, 256), 256, 0, s>>>(f, sb);
+  return cudaGetLastError();
+}
+
+// Incoming rates of every cell as after the last sweep, before they are exported: that sweep
+// left those of its inactive cells as they were.
+cudaError_t refresh(const DevicePtrs& p, cudaStream_t s) {
+  if (!p.stream_mode || p.active_cells >= p.num_cells) return cudaSuccess;
+  swk::k_stream_stale<<<grid_for(p.num_cells, 256), 256, 0, s>>>(sweep_args(p, 0), p.cell_sweep, p.stale);
+  const int y = std::max(1, (int)(8 * p.num_sms / std::max(1u, p.num_streams)));
+  swk::k_stream_refresh<<<dim3(p.num_streams, y), 256, 0, s>>>(stream_args(p), p.stale);
+  return cudaGetLastError();
+}
+#endif
+
 // Seed of the schedule: dependency counts with every cell active (the caller has set
 // all levels >= 0), tasks without dependencies appended to `order`.
 cudaError_t schedule_seed(const DevicePtrs& p, cudaStream_t s) {
@@ -175,6 +311,20 @@ cudaError_t kahn_round(const DevicePtrs& p, uint32_t begin, uint32_t end, uint16
 
 cudaError_t fold_periodic(const DevicePtrs& p, cudaStream_t s) {
   if (p.n_periodic_cells == 0) return cudaSuccess;
+#if !SWK_PULL
+  if (p.stream_mode) {
+    uint8_t* changed = nullptr;
+    if (p.active_cells < p.num_cells) {  // only entries next to an active cell
+      changed = p.fold_changed;
+      swk::k_fold_mark64<<<grid_for(p.n_periodic_cells, 256), 256, 0, s>>>(
+          sweep_args(p, 0), static_cast<const double*>(p.cell_att), p.periodic_cells, p.n_periodic_cells, changed);
+    }
+    swk::k_fold64<<<dim3((p.n_periodic_cells + 255) / 256, p.D), 256, 0, s>>>(
+        static_cast<const double*>(p.outgoing), static_cast<double*>(p.periodic), p.Np, p.periodic_cells,
+        p.n_periodic_cells, p.fold_off, static_cast<const swk::FoldSlot64*>(p.fold_slots), changed);
+    return cudaGetLastError();
+  }
+#endif
   swk::k_fold_periodic<R><<<grid_for((int64_t)p.n_periodic_cells * p.D, 256), 256, 0, s>>>(
       static_cast<R*>(p.periodic), static_cast<R*>(p.pending), p.periodic_cells, p.n_periodic_cells, p.D, p.Np);
   return cudaGetLastError();
@@ -428,110 +578,6 @@ cudaError_t sweep_pull_geo(const DevicePtrs& p, int level, cudaStream_t s) {
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(swk::kGeoThreads), args, 0, s);
 }
 
-// The compacted list of the level's active positions: mark the active cells' positions,
-// then compact the bitmap.
-cudaError_t compact_active(const DevicePtrs& p, int level, cudaStream_t s) {
-  uint32_t* act = p.act_lv[level];
-  uint32_t* cnt = p.act_counts + level;
-  if (!act) return cudaErrorInvalidValue;
-  if (!p.compact_now) return cudaSuccess;
-  const uint32_t words = (uint32_t)((p.num_cells * p.D + 31) / 32);
-  const uint32_t nb = (words + swk::kBitsThreads - 1) / swk::kBitsThreads;
-  uint32_t* bits = p.stream_mode ? p.act_bits_lv[level] : p.act_bits;
-  cudaError_t e = cudaMemsetAsync(bits, 0, (size_t)words * sizeof(uint32_t), s);
-  if (e != cudaSuccess) return e;
-  swk::k_mark_active<<<grid_for(p.num_cells, 256), 256, 0, s>>>(p.level, level, (uint32_t)p.num_cells, p.D, p.Np,
-                                                                  p.pos_of_task, bits);
-  swk::k_bits_count<<<nb, swk::kBitsThreads, 0, s>>>(bits, words, p.chunk);
-  swk::k_compact_scan<<<1, swk::kScanThreads, 0, s>>>(p.chunk, nb, cnt);
-  swk::k_bits_scatter<<<nb, swk::kBitsThreads, 0, s>>>(bits, words, p.chunk, act);
-  if (p.stream_mode)
-    swk::k_stream_act_range<<<grid_for((int64_t)p.num_streams * 64, 256), 256, 0, s>>>(
-        bits, p.chunk, static_cast<const swk::StreamDesc*>(p.streams), p.num_streams, (uint32_t)(p.num_cells * p.D),
-        cnt, p.act_range[level]);
-  return cudaGetLastError();
-}
-
-swk::StreamShape stream_shape(const DevicePtrs& p) {
-  return {p.stream_shape[0], p.stream_shape[1], p.stream_shape[2], p.stream_shape[3], p.stream_shape[4]};
-}
-
-swk::StreamArgs<R> stream_args(const DevicePtrs& p) {
-  swk::StreamArgs<R> a{};
-  a.streams = static_cast<const swk::StreamDesc*>(p.streams);
-  a.groups = static_cast<const swk::StreamGroup*>(p.stream_groups);
-  a.data = p.stream_data;
-  a.bytes = p.stream_bytes;
-  a.evict_first = p.stream_bytes > (64ull << 20);
-  a.seg_group = p.seg_group;
-  a.word = reinterpret_cast<swk::StreamArgs<R>::Word*>(p.qe);
-  a.inc = static_cast<R*>(p.incoming);
-  a.threshold = (R)(p.threshold / p.rate_scale);
-  a.ctl = p.ctl;
-  a.timeout_ns = p.timeout_ns;
-  a.epoch = p.epoch;
-  a.epoch_base = p.epoch_base;
-  a.shape = stream_shape(p);
-  return a;
-}
-
-template <int W>
-cudaError_t launch_stream(const DevicePtrs& p, bool all, cudaStream_t s) {
-  const swk::StreamArgs<R> a = stream_args(p);
-  const size_t smem = swk::stream_smem_bytes<R>(a.shape);
-  auto fn = a.shape.far ? (all ? swk::k_sweep_stream<R, W, true, true> : swk::k_sweep_stream<R, W, true, false>)
-                        : (all ? swk::k_sweep_stream<R, W, false, true> : swk::k_sweep_stream<R, W, false, false>);
-  cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  fn<<<p.num_streams, 32 * W, smem, s>>>(a);
-  return cudaGetLastError();
-}
-
-cudaError_t sweep_stream(const DevicePtrs& p, int level, cudaStream_t s) {
-  if (p.sparse_sweep) {
-    cudaError_t e = compact_active(p, level, s);
-    if (e != cudaSuccess) return e;
-    swk::StreamArgs<R> a = stream_args(p);
-    a.act = p.act_lv[level];
-    a.act_range = p.act_range[level];
-    a.act_bits = p.act_bits_lv[level];
-    a.seg = p.lvl;
-    a.order = p.order;
-    a.cell_att = static_cast<const R*>(p.cell_att);
-    a.periodic = static_cast<const R*>(p.periodic);
-    a.Np = p.Np;
-    swk::k_sweep_stream_sparse<R><<<p.num_streams, swk::kStreamSparseThreads, 0, s>>>(a);
-    return cudaGetLastError();
-  }
-  swk::k_stream_gather<R><<<grid_for((int64_t)p.num_groups * 32, 256), 256, 0, s>>>(
-      static_cast<const swk::StreamGroup*>(p.stream_groups), p.num_groups, p.stream_data, p.order, p.Np,
-      static_cast<const R*>(p.cell_att), static_cast<const R*>(p.periodic));
-  const bool all = p.active_cells >= p.num_cells;
-  switch (p.stream_shape[3]) {
-    case 4: return launch_stream<4>(p, all, s);
-    case 8: return launch_stream<8>(p, all, s);
-    default: return launch_stream<16>(p, all, s);
-  }
-}
-
-cudaError_t stream_build(const DevicePtrs& p, int phase, const StreamScratch& b, cudaStream_t s) {
-  const uint32_t total = (uint32_t)(p.num_cells * p.D);
-  swk::PullArgs a = pull_args(p, 0);
-  if (phase == 0) {
-    swk::k_invert_order<<<grid_for(total, 256), 256, 0, s>>>(p.order, total, p.pos_of_task);
-    swk::k_stream_group_segs<<<grid_for((int64_t)p.num_sched_levels * 32, 256), 256, 0, s>>>(
-        p.seg_group, p.num_sched_levels, b.gseg);
-    return cudaGetLastError();
-  }
-  const swk::StreamBuild sb{static_cast<swk::StreamGroup*>(p.stream_groups), p.num_groups, b.gseg, p.lvl, p.seg_group,
-                            b.sbase, b.sgroup, p.num_sched_levels, phase == 2 ? p.stream_data : nullptr, stream_shape(p)};
-  swk::k_stream_slots<<<grid_for((int64_t)p.num_groups * 32, 256), 256, 0, s>>>(a, sb);
-  if (phase == 2 && p.n_periodic_cells > 0)
-    swk::k_fold_build<<<grid_for((int64_t)p.n_periodic_cells * p.D, 256), 256, 0, s>>>(
-        a, p.periodic_cells, p.n_periodic_cells, p.fold_cnt, static_cast<uint2*>(p.fold_slots));
-  return cudaGetLastError();
-}
-
 cudaError_t sweep_pull(const DevicePtrs& p, int level, cudaStream_t s) {
   if (p.geo_mode) return sweep_pull_geo(p, level, s);
   if (p.stream_mode) return sweep_stream(p, level, s);
@@ -566,6 +612,24 @@ cudaError_t sweep_pull(const DevicePtrs& p, int level, cudaStream_t s) {
   cudaError_t e = coop_grid(p, fn, &grid);
   if (e != cudaSuccess) return e;
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(swk::kPullThreads), args, 0, s);
+}
+
+cudaError_t stream_build(const DevicePtrs& p, int phase, const StreamScratch& b, cudaStream_t s) {
+  const uint32_t total = (uint32_t)(p.num_cells * p.D);
+  swk::PullArgs a = pull_args(p, 0);
+  if (phase == 0) {
+    swk::k_invert_order<<<grid_for(total, 256), 256, 0, s>>>(p.order, total, p.pos_of_task);
+    swk::k_stream_group_segs<<<grid_for((int64_t)p.num_sched_levels * 32, 256), 256, 0, s>>>(
+        p.seg_group, p.num_sched_levels, b.gseg);
+    return cudaGetLastError();
+  }
+  const swk::StreamBuild sb{static_cast<swk::StreamGroup*>(p.stream_groups), p.num_groups, b.gseg, p.lvl, p.seg_group,
+                            b.sbase, b.sgroup, p.num_sched_levels, phase == 2 ? p.stream_data : nullptr, stream_shape(p)};
+  swk::k_stream_slots<<<grid_for((int64_t)p.num_groups * 32, 256), 256, 0, s>>>(a, sb);
+  if (phase == 2 && p.n_periodic_cells > 0)
+    swk::k_fold_build<<<grid_for((int64_t)p.n_periodic_cells * p.D, 256), 256, 0, s>>>(
+        a, p.periodic_cells, p.n_periodic_cells, p.fold_cnt, static_cast<uint2*>(p.fold_slots));
+  return cudaGetLastError();
 }
 
 cudaError_t fold_pull(const DevicePtrs& p, cudaStream_t s) {
@@ -614,23 +678,33 @@ cudaError_t export_rates(const DevicePtrs& p, int which, uint32_t last_epoch, do
   return cudaGetLastError();
 }
 #else
+// positions of the tasks' rates, or null where they lie by task
+const uint32_t* rate_pos(const DevicePtrs& p) { return p.stream_mode ? p.pos_of_task : nullptr; }
+
 cudaError_t photon_rate(const DevicePtrs& p, uint32_t, double* out, cudaStream_t s) {
+  const cudaError_t e = refresh(p, s);
+  if (e != cudaSuccess) return e;
   swk::k_photon_rate<R><<<grid_for(p.num_cells, 256), 256, 0, s>>>(
-      (uint32_t)p.num_cells, static_cast<const R*>(p.incoming), p.D, p.Np, p.rate_scale, out);
+      (uint32_t)p.num_cells, static_cast<const R*>(p.incoming), rate_pos(p), p.D, p.Np, p.rate_scale, out);
   return cudaGetLastError();
 }
 
 cudaError_t cell_rates(const DevicePtrs& p, uint32_t, double* out, cudaStream_t s) {
+  const cudaError_t e = refresh(p, s);
+  if (e != cudaSuccess) return e;
   swk::k_cell_rates<R><<<grid_for(p.num_cells, 256), 256, 0, s>>>(
-      (uint32_t)p.num_cells, static_cast<const R*>(p.incoming), static_cast<const R*>(p.periodic),
+      (uint32_t)p.num_cells, static_cast<const R*>(p.incoming), rate_pos(p), static_cast<const R*>(p.periodic),
       static_cast<const R*>(p.src_dir), p.D, p.Np, p.rate_scale, out);
   return cudaGetLastError();
 }
 
 cudaError_t export_rates(const DevicePtrs& p, int which, uint32_t, double* out, cudaStream_t s) {
+  const cudaError_t e = which == 0 ? refresh(p, s) : cudaSuccess;
+  if (e != cudaSuccess) return e;
   const void* src = which == 0 ? p.incoming : (which == 1 ? p.outgoing : p.periodic);
   swk::k_export_rates<R><<<grid_for(p.num_cells * p.D, 256), 256, 0, s>>>(
-      (uint32_t)p.num_cells, static_cast<const R*>(src), p.D, p.Np, p.rate_scale, out);
+      (uint32_t)p.num_cells, static_cast<const R*>(src), which == 2 ? nullptr : rate_pos(p), p.D, p.Np, p.rate_scale,
+      out);
   return cudaGetLastError();
 }
 #endif
@@ -642,14 +716,14 @@ extern const PrecisionOps SWK_OPS = {
     SWK_NAME,       (int)sizeof(R), true,       occupancy,     attenuation, init_counts, sweep,
     occupancy_pull, sweep_pull,     kahn_round, schedule_seed, fold_pull,   chemistry,   photon_rate,
     export_rates,   records,        cell_rates, SWK_CARRY != 0,
-    (int)(sizeof(kTuneVariants) / sizeof(int)), kTuneVariants, nullptr, stream_build,
+    (int)(sizeof(kTuneVariants) / sizeof(int)), kTuneVariants, nullptr, stream_build, nullptr,
 };
 #else
 extern const PrecisionOps SWK_OPS = {
     SWK_NAME,         (int)sizeof(R), false,      occupancy,     attenuation,   init_counts, sweep,
     occupancy_levels, sweep_levels,   kahn_round, schedule_seed, fold_periodic, chemistry,   photon_rate,
     export_rates,     nullptr,        cell_rates, SWK_CARRY != 0,
-    0, nullptr,       push_records, nullptr,
+    0, nullptr,       push_records, stream_build64, refresh,
 };
 #endif
 

@@ -36,9 +36,14 @@
 // tasks per ns).  A block barrier or an mbarrier per level instead of the counter: 64^3 1.2,
 // 24^3 0.20.
 //
-// The incoming rate is the sum of the pull kernels over the slots in face order: FP32
-// (mixed path) as eight partial sums combined pairwise, with the same roundings as the
-// lockstep kernels, so both give the same bits.
+// FP64 is bound by its unit instead: a warp's instruction takes 64 cycles of a quarter of the SM,
+// so a group of ~10 slots takes a warp 640 cycles for the products alone.  Its slots lie by upwind
+// position and all but those of the previous level are summed before that level is done: 64^3
+// 2.85 -> 2.0 ms per sweep, 24^3 0.40 -> 0.31 (push form with atomics 5.4 and 1.6).
+//
+// FP32 (mixed path): the incoming rate is the sum of the pull kernels over the slots in face
+// order, as eight partial sums combined pairwise, with the same roundings as the lockstep
+// kernels, so both give the same bits.  FP64: one sum of fused multiply-adds.
 #pragma once
 
 #include "sweep_device.cuh"
@@ -55,14 +60,28 @@ template <>
 struct StreamTraits<float> {
   using Word = unsigned long long;  // {q, sweep << 1}
 };
+template <>
+struct StreamTraits<double> {
+  using Word = double;  // the outgoing rate
+};
+
+// FP64: the slots of a task lie by upwind position, padding first, so that all but the last
+// `late` of them are words of levels before the previous one: they are summed while the previous
+// level is solved.
+struct alignas(16) StreamEarly {
+  uint32_t need;  // groups of the stream before the previous level
+  uint32_t skip;  // leading slots that are padding in every task
+  uint32_t late;  // trailing slots with words of the previous level in any task
+  uint32_t pad;
+};
 
 // A group's piece of data, 32 tasks (those past the group's read as padding): the group (16
-// bytes), attenuations [32], 1 / A_down [32] (FP32 rates only), weights [quad][32][4], 16-bit
-// slot indices [quad][32][4], periodic sources and cell sources / D [2][32] (kGroupExt),
+// bytes; FP64: and its StreamEarly), attenuations [32], 1 / A_down [32] (FP32 rates only), weights [quad][32][4]
+// (FP64: [pair][32][2]), 16-bit slot indices [quad][32][4], periodic sources and cell sources / D [2][32] (kGroupExt),
 // positions of the far words [far][32].  Slot k of task i is number 4 * (k / 4 * 32 + i) + k % 4.
 template <typename R>
 struct StreamPiece {
-  static constexpr uint32_t kAtt = sizeof(StreamGroup), kInv = kAtt + 32 * sizeof(R),
+  static constexpr uint32_t kAtt = sizeof(StreamGroup) + (sizeof(R) == 8 ? sizeof(StreamEarly) : 0u), kInv = kAtt + 32 * sizeof(R),
                             kW = kInv + (sizeof(R) == 4 ? 128u : 0u);
   const unsigned char* p;
   uint32_t quads, shape;
@@ -78,6 +97,9 @@ struct StreamPiece {
     return reinterpret_cast<const uint32_t*>(per() + ((shape & kGroupExt) ? 64 : 0));
   }
   __host__ __device__ static uint32_t slot(uint32_t k, uint32_t i) { return 4 * (k / 4 * 32 + i) + k % 4; }
+  // of its weight: in 16-byte loads
+  static constexpr uint32_t kVec = 16 / sizeof(R);
+  __host__ __device__ static uint32_t wslot(uint32_t k, uint32_t i) { return kVec * (k / kVec * 32 + i) + k % kVec; }
 };
 
 // The block's words: ring | zero word | far buffers of the warps [W][far][32].
@@ -120,6 +142,7 @@ struct StreamArgs {
   const uint32_t* order;
   const R *cell_att, *periodic;
   uint32_t Np;
+  uint32_t* stamp;  // FP64: per position, the last sparse sweep that solved it
 };
 
 __device__ __forceinline__ uint32_t st_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -152,7 +175,10 @@ __device__ __forceinline__ bool st_wait(Test test, SweepCtl* ctl, unsigned long 
 
 // whether an attenuation is one, not the mark of a cell that is not active in the sweep
 __device__ __forceinline__ bool st_live(float att) { return __float_as_uint(att) != 0xffffffffu; }
+__device__ __forceinline__ bool st_live(double att) { return __double_as_longlong(att) != -1ll; }
 // the q of a word in memory, the word of a q
+__device__ __forceinline__ double st_ldq(const double* w) { return __ldcg(w); }
+__device__ __forceinline__ double st_word(double q, uint32_t) { return q; }
 __device__ __forceinline__ float st_ldq(const unsigned long long* w) {
   return __uint_as_float(__ldcg(reinterpret_cast<const uint32_t*>(w)));
 }
@@ -178,11 +204,30 @@ struct StreamSum<float> {
   }
 };
 
+// FP64: one fused multiply-add per slot (the unit takes 64 cycles per warp and instruction,
+// whatever depends on what)
+template <>
+struct StreamSum<double> {
+  double sum;
+  __device__ __forceinline__ StreamSum() : sum(0.0) {}
+  __device__ __forceinline__ void add(int, double w, double q) { sum = fma(w, q, sum); }
+  __device__ __forceinline__ double total() const { return sum; }
+};
+
 // outgoing rate of the task (get_outgoing_rate of Site::get_rate), as the word's q
 __device__ __forceinline__ float st_solve(float in, float src, float per, float att, float threshold, float inv) {
   const float rt = (in + src) + per;                    // Site::get_rate, site.rs:53-56
   const float out = (rt < threshold) ? 0.f : rt * att;  // get_outgoing_rate
   return out * inv;
+}
+// FP64: the comparison on the bits, which order as the numbers do from the threshold up
+__device__ __forceinline__ double st_solve(double rt, double att, double threshold) {
+  const long long b = __double_as_longlong(rt), t = __double_as_longlong(threshold);
+  const bool below = t >= 0 ? b < t && (b & 0x7fffffffffffffffll) <= 0x7ff0000000000000ll : rt < threshold;
+  return below ? 0.0 : rt * att;
+}
+__device__ __forceinline__ double st_solve(double in, double src, double per, double att, double threshold, float) {
+  return st_solve((in + src) + per, att, threshold);
 }
 
 // Shared memory of a block: a barrier per warp, the count, the warps' buffers, the words.
@@ -210,13 +255,30 @@ constexpr uint32_t kStreamAhead = 98304;  // bytes between a group's piece and w
 
 // four weights and their slot indices
 template <typename R>
-struct StreamQuad;
+struct StreamWeights;
 template <>
-struct StreamQuad<float> {
-  float4 w;
-  uint2 x;
+struct StreamWeights<float> {
+  float4 v;
   __device__ __forceinline__ void load(const StreamPiece<float>& s, uint32_t k, uint32_t lane) {
-    w = reinterpret_cast<const float4*>(s.w())[k * 32 + lane];
+    v = reinterpret_cast<const float4*>(s.w())[k * 32 + lane];
+  }
+  __device__ __forceinline__ float get(int c) const { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
+};
+template <>
+struct StreamWeights<double> {
+  double2 a, b;
+  __device__ __forceinline__ void load(const StreamPiece<double>& s, uint32_t k, uint32_t lane) {
+    a = reinterpret_cast<const double2*>(s.w())[2 * k * 32 + lane];
+    b = reinterpret_cast<const double2*>(s.w())[(2 * k + 1) * 32 + lane];
+  }
+  __device__ __forceinline__ double get(int c) const { return c == 0 ? a.x : c == 1 ? a.y : c == 2 ? b.x : b.y; }
+};
+template <typename R>
+struct StreamQuad {
+  StreamWeights<R> w;
+  uint2 x;
+  __device__ __forceinline__ void load(const StreamPiece<R>& s, uint32_t k, uint32_t lane) {
+    w.load(s, k, lane);
     x = reinterpret_cast<const uint2*>(s.idx())[k * 32 + lane];
   }
 };
@@ -227,18 +289,35 @@ __device__ __forceinline__ void st_words(const StreamQuad<R>& t, const R* words,
   q[2] = words[t.x.y & 0xffffu];
   q[3] = words[t.x.y >> 16];
 }
-template <typename R, typename Sum>
-__device__ __forceinline__ void st_add(Sum& sum, bool odd, const StreamQuad<R>& t, const R (&q)[4]) {
+template <typename R>
+__device__ __forceinline__ void st_add(StreamSum<R>& sum, bool odd, const StreamWeights<R>& w, const R (&q)[4]) {
   if (odd) {
-    sum.add(4, t.w.x, q[0]);
-    sum.add(5, t.w.y, q[1]);
-    sum.add(6, t.w.z, q[2]);
-    sum.add(7, t.w.w, q[3]);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) sum.add(4 + c, w.get(c), q[c]);
   } else {
-    sum.add(0, t.w.x, q[0]);
-    sum.add(1, t.w.y, q[1]);
-    sum.add(2, t.w.z, q[2]);
-    sum.add(3, t.w.w, q[3]);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) sum.add(c, w.get(c), q[c]);
+  }
+}
+
+// FP64: adds the slots [lo, hi) of a group, in order
+__device__ __forceinline__ void st_sum(StreamSum<double>& sum, const StreamQuad<double> (&quad)[kStreamQuads],
+                                       const double* words, const StreamPiece<double>& s, uint32_t lane, uint32_t lo,
+                                       uint32_t hi) {
+  auto add = [&](const StreamQuad<double>& t, uint32_t k) {
+    double q[4];
+    st_words(t, words, q);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (k + c >= lo && k + c < hi) sum.add(0, t.w.get(c), q[c]);
+  };
+#pragma unroll
+  for (uint32_t c = 0; c < kStreamQuads; ++c)
+    if (4 * c + 4 > lo && 4 * c < hi) add(quad[c], 4 * c);
+  for (uint32_t c = max(kStreamQuads, lo / 4); 4 * c < hi; ++c) {
+    StreamQuad<double> t;
+    t.load(s, c, lane);
+    add(t, 4 * c);
   }
 }
 
@@ -308,6 +387,7 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
   uint32_t solved = 0, parity = 0, g = warp;
   // the group that the warp solves next, in registers
   StreamGroup gr{};
+  StreamEarly early{};
   StreamQuad<R> quad[kStreamQuads];
   R att = R(0), per = R(0), src = R(0), own = R(0);
   float inv = 0.f;
@@ -320,6 +400,7 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
     dead = !st_wait([&]() { return st_bar_test(bar, parity); }, a.ctl, a.timeout_ns) || dead;
     parity ^= 1;
     gr = *reinterpret_cast<const StreamGroup*>(buffer);
+    if constexpr (sizeof(R) == 8) early = *reinterpret_cast<const StreamEarly*>(buffer + sizeof(StreamGroup));
     const StreamPiece<R> s(buffer, gr);
     att = s.att()[lane];
     if (sizeof(R) == 4) inv = s.inv()[lane];
@@ -369,13 +450,22 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
   locate(warp + W);
   load();
   while (g < sd.groups) {
+    StreamSum<R> sum;
+    const uint32_t quads = group_slots(gr.shape) / 4;
+    uint32_t first = 0;  // slot that the sum goes on with
+    if constexpr (sizeof(R) == 8) {
+      const bool ahead = !kFar || !(gr.shape & (kGroupLate | kGroupSlow));
+      if (ahead && !dead) {
+        dead = !st_wait([&]() { return st_count(count) >= early.need; }, a.ctl, a.timeout_ns);
+        first = 4 * quads - early.late;
+        if (!dead) st_sum(sum, quad, words, StreamPiece<R>(buffer, gr), lane, early.skip, first);
+      }
+    }
     // the levels before this group's
     dead = dead || !st_wait([&]() { return st_count(count) >= gr.need; }, a.ctl, a.timeout_ns);
     const uint32_t n = group_tasks(gr.shape);
     rel = gr.pos - sd.base;
     if (!dead) {
-      StreamSum<R> sum;
-      const uint32_t quads = group_slots(gr.shape) / 4;
       if (kFar && (gr.shape & (kGroupLate | kGroupSlow))) {
         const StreamPiece<R> all(a.data + 16ull * gr.data, gr);
         const Word* base = a.word + sd.base;
@@ -390,7 +480,7 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
               const uint32_t x = all.idx()[StreamPiece<R>::slot(4 * j + c, lane)];
               q[c] = x >= far ? st_ldq(base + all.far()[(x - far) * 32 + lane]) : words[x];
             }
-            st_add(sum, j & 1u, t, q);
+            st_add(sum, j & 1u, t.w, q);
           }
         } else {
           for (uint32_t f = 0; f < group_far(gr.shape); ++f) {
@@ -400,24 +490,31 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
         }
       }
       if (!kFar || !(gr.shape & kGroupSlow)) {
-        R q[kStreamQuads][4];
-#pragma unroll
-        for (uint32_t c = 0; c < kStreamQuads; ++c)
-          if (c < quads) st_words(quad[c], words, q[c]);
-#pragma unroll
-        for (uint32_t c = 0; c < kStreamQuads; ++c)
-          if (c < quads) st_add(sum, c & 1u, quad[c], q[c]);
         const StreamPiece<R> s(buffer, gr);
-        for (uint32_t c = kStreamQuads; c < quads; ++c) {
-          StreamQuad<R> t;
-          t.load(s, c, lane);
-          R qc[4];
-          st_words(t, words, qc);
-          st_add(sum, c & 1u, t, qc);
+        if constexpr (sizeof(R) == 8) {
+          st_sum(sum, quad, words, s, lane, max(first, early.skip), 4 * quads);
+        } else {
+          R q[kStreamQuads][4];
+#pragma unroll
+          for (uint32_t c = 0; c < kStreamQuads; ++c)
+            if (c < quads) st_words(quad[c], words, q[c]);
+#pragma unroll
+          for (uint32_t c = 0; c < kStreamQuads; ++c)
+            if (c < quads) st_add(sum, c & 1u, quad[c].w, q[c]);
+          for (uint32_t c = kStreamQuads; c < quads; ++c) {
+            StreamQuad<R> t;
+            t.load(s, c, lane);
+            R qc[4];
+            st_words(t, words, qc);
+            st_add(sum, c & 1u, t.w, qc);
+          }
         }
       }
       in = sum.total();
-      out = st_solve(in, src, per, att, a.threshold, inv);
+      if constexpr (sizeof(R) == 8)
+        out = (gr.shape & kGroupExt) ? st_solve(in, src, per, att, a.threshold, inv) : st_solve(in, att, a.threshold);
+      else
+        out = st_solve(in, src, per, att, a.threshold, inv);
       mine = lane < n && (kAll || st_live(att));
       uint32_t slot = ring_slot(shape, rel) + lane;
       if (slot >= shape.ring) slot -= shape.ring;
@@ -474,6 +571,48 @@ __device__ __forceinline__ uint32_t stream_slot_position(const StreamShape& shap
 constexpr int kStreamSparseThreads = 512;
 constexpr uint32_t kSparseNone = 0x7fffffffu, kSparseActive = 0x80000000u;
 
+// The upwind words of four slots, and whether those that the sweep solves are there.  FP32: a
+// word carries the number of the sweep that wrote it; FP64: the stamp beside it, in the order of
+// the block (a stream is one block).
+__device__ __forceinline__ void st_try(const StreamArgs<float>&, const unsigned long long* word, uint32_t,
+                                       const uint32_t (&up)[4], uint32_t sweep, bool& ready, float (&q)[4]) {
+  unsigned long long v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] = up[k] != kSparseNone ? ld_relaxed64(word + (up[k] & kSparseNone)) : 0ull;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    ready = ready && (!(up[k] & kSparseActive) || (uint32_t)(v[k] >> 32) == sweep << 1);
+    q[k] = __uint_as_float((uint32_t)v[k]);
+  }
+}
+__device__ __forceinline__ void st_try(const StreamArgs<double>& a, const double* word, uint32_t base,
+                                       const uint32_t (&up)[4], uint32_t sweep, bool& ready, double (&q)[4]) {
+  uint32_t v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    v[k] = sweep;
+    if (up[k] & kSparseActive)
+      asm volatile("ld.acquire.cta.global.u32 %0, [%1];"
+                   : "=r"(v[k])
+                   : "l"(a.stamp + base + (up[k] & kSparseNone))
+                   : "memory");
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    ready = ready && v[k] == sweep;
+    q[k] = up[k] != kSparseNone ? st_ldq(word + (up[k] & kSparseNone)) : 0.0;
+  }
+}
+__device__ __forceinline__ void st_publish(const StreamArgs<float>&, unsigned long long* word, uint32_t, uint32_t rel,
+                                           float q, uint32_t sweep) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(word + rel), "l"(st_word(q, sweep)) : "memory");
+}
+__device__ __forceinline__ void st_publish(const StreamArgs<double>& a, double* word, uint32_t base, uint32_t rel,
+                                           double q, uint32_t sweep) {
+  word[rel] = q;
+  asm volatile("st.release.cta.global.u32 [%0], %1;" ::"l"(a.stamp + base + rel), "r"(sweep) : "memory");
+}
+
 template <typename R>
 __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(const __grid_constant__ StreamArgs<R> a) {
   using Word = typename StreamTraits<R>::Word;
@@ -491,9 +630,9 @@ __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(co
     uint32_t number = 0, i = 0, rel = 0, quads = 0;
     R att = R(0), per = R(0), src = R(0);
     float inv = 0.f;
-    float4 w[kStreamQuads];
+    StreamWeights<R> w[kStreamQuads];
     uint32_t up[kStreamQuads][4];  // positions of the upwind words, kSparseActive: solved in this sweep
-    auto quad = [&](const StreamPiece<R>& s, uint32_t c, float4& w4, uint32_t (&up4)[4]) {
+    auto quad = [&](const StreamPiece<R>& s, uint32_t c, StreamWeights<R>& w4, uint32_t (&up4)[4]) {
       StreamQuad<R> v;
       v.load(s, c, i);
       w4 = v.w;
@@ -538,20 +677,10 @@ __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(co
     auto attempt = [&]() {
       bool ready = true;
       StreamSum<R> sum;
-      auto add = [&](bool odd, const float4& w4, const uint32_t (&up4)[4]) {
+      auto add = [&](bool odd, const StreamWeights<R>& w4, const uint32_t (&up4)[4]) {
         R q[4];
-        Word v[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          v[k] = up4[k] != kSparseNone ? ld_relaxed_u64(word + (up4[k] & kSparseNone)) : 0ull;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          ready = ready && (!(up4[k] & kSparseActive) || (uint32_t)(v[k] >> 32) == sweep << 1);
-          q[k] = __uint_as_float((uint32_t)v[k]);
-        }
-        StreamQuad<R> t;
-        t.w = w4;
-        st_add(sum, odd, t, q);
+        st_try(a, word, sd.base, up4, sweep, ready, q);
+        st_add(sum, odd, w4, q);
       };
 #pragma unroll
       for (uint32_t c = 0; c < kStreamQuads; ++c)
@@ -559,7 +688,7 @@ __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(co
       if (quads > kStreamQuads) {
         const StreamPiece<R> s(a.data + 16ull * gr.data, gr);
         for (uint32_t c = kStreamQuads; c < quads; ++c) {
-          float4 w4;
+          StreamWeights<R> w4;
           uint32_t up4[4];
           quad(s, c, w4, up4);
           add(c & 1u, w4, up4);
@@ -567,7 +696,7 @@ __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(co
       }
       if (ready) {
         const R in = sum.total();
-        st_relaxed_u64(word + rel, st_word(st_solve(in, src, per, att, a.threshold, inv), sweep));
+        st_publish(a, word, sd.base, rel, st_solve(in, src, per, att, a.threshold, inv), sweep);
         inc[rel] = in;
         ++solved;
         todo = false;

@@ -1,0 +1,272 @@
+// Direction streams of the FP64 path: the pull form of Sweep::solve_task (src/sweep/mod.rs:423-485).
+//
+// The reference hands every downwind face the share (eff_f / total) of a task's outgoing rate,
+// with eff_f = area_f (n_f . d) and total the sum over the task's downwind faces in face order.
+// Here the receiving task sums the outgoing rates of its upwind tasks with the same fractions,
+// computed once per grid with the roundings of push_eff.  The share of face f of cell c comes
+// from the upwind cell's own face towards c (the reciprocal face, with the negated normal).
+//
+// The outgoing and incoming rates lie by schedule position.  Incoming rates of cells that were
+// not active lately are brought up to date when something asks for them (k_stream_refresh): a
+// sweep writes those of the active cells only.
+#pragma once
+
+#include "sweep_push_records.cuh"
+#include "sweep_stream.cuh"
+
+namespace swk {
+
+struct FacePull {
+  SweepArgs<double> a;
+  const uint32_t* order;
+  const uint32_t* pos_of_task;
+  const double* total;  // per task
+};
+
+__device__ __forceinline__ double task_total(const SweepArgs<double>& a, uint32_t c, uint32_t d) {
+  const double dx = a.dir64[3 * d], dy = a.dir64[3 * d + 1], dz = a.dir64[3 * d + 2];
+  const float fx = a.dir32[3 * d], fy = a.dir32[3 * d + 1], fz = a.dir32[3 * d + 2];
+  double tot = 0.0;  // face order, zeros for the other faces (solve_group)
+  for (uint32_t f = a.off[c]; f < a.off[c + 1]; ++f) tot += push_eff(a, f, dx, dy, dz, fx, fy, fz);
+  return tot;
+}
+
+static __global__ void k_task_totals(FacePull p, double* total) {
+  const size_t n = (size_t)p.a.N * p.a.D;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t d = (uint32_t)(i / p.a.N), c = (uint32_t)(i % p.a.N);
+    total[(size_t)d * p.a.Np + c] = task_total(p.a, c, d);
+  }
+}
+
+// Sign of face f against direction d (+1 downwind, -1 upwind).
+__device__ __forceinline__ int pull_sign(const SweepArgs<double>& a, uint32_t f, uint32_t d) {
+  const float4 g = a.geo32[f];
+  const float s = g.x * a.dir32[3 * d] + g.y * a.dir32[3 * d + 1] + g.z * a.dir32[3 * d + 2];
+  return face_sign(s, a.geo64 + f, a.dir64[3 * d], a.dir64[3 * d + 1], a.dir64[3 * d + 2], a.guard);
+}
+
+// The fraction that the cell across upwind face f of cell c hands to c in direction d: of its
+// face towards c with the negated normal (the k-th of equal ones, as f is the k-th of its equals).
+// Negative if there is none.
+__device__ __forceinline__ double pull_fraction(const FacePull& p, uint32_t c, uint32_t f, uint32_t d) {
+  const SweepArgs<double>& a = p.a;
+  const uint32_t nb = a.nbr[f], n = nb & kNbrMask, back = c | (nb & ~kNbrMask);
+  const Geo64 g = a.geo64[f];
+  int k = 0;
+  for (uint32_t e = a.off[c]; e < f; ++e)
+    if (a.nbr[e] == nb && a.geo64[e].x == g.x && a.geo64[e].y == g.y && a.geo64[e].z == g.z) ++k;
+  const double dx = a.dir64[3 * d], dy = a.dir64[3 * d + 1], dz = a.dir64[3 * d + 2];
+  const float fx = a.dir32[3 * d], fy = a.dir32[3 * d + 1], fz = a.dir32[3 * d + 2];
+  for (uint32_t q = a.off[n]; q < a.off[n + 1]; ++q) {
+    if (a.nbr[q] != back) continue;
+    if (a.geo64[q].x != -g.x || a.geo64[q].y != -g.y || a.geo64[q].z != -g.z || k-- > 0) continue;
+    const double eff = push_eff(a, q, dx, dy, dz, fx, fy, fz);
+    if (!(eff > 0.0)) return -1.0;
+    return eff / p.total[(size_t)d * a.Np + n];
+  }
+  return -1.0;
+}
+
+// Finds the flags and far words of every group (b.data null), or writes the groups' pieces, one
+// warp each (k_stream_slots of the mixed path).  The faces handed out and the faces found are
+// counted in ctl->head and ctl->tail: a grid where they differ keeps the push form.
+static __global__ void k_stream_slots64(FacePull p, StreamBuild b) {
+  const SweepArgs<double>& a = p.a;
+  const uint32_t lane = threadIdx.x & 31;
+  unsigned long long given = 0, found = 0;
+  for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / 32; g < b.num_groups; g += gridDim.x * blockDim.x / 32) {
+    const StreamGroup gr = b.groups[g];
+    const StreamPiece<double> piece(b.data + 16ull * gr.data, gr);
+    const uint32_t n = group_tasks(gr.shape), padded = group_slots(gr.shape);
+    StreamSlot s = stream_slots(b, g);
+    bool ext = false;
+    uint32_t* far = const_cast<uint32_t*>(piece.far()) + lane;
+    uint16_t* idx = const_cast<uint16_t*>(piece.idx());
+    double* w = const_cast<double*>(piece.w());
+    // upwind positions and faces, by position
+    uint32_t up[kMaxFaces];
+    uint8_t face[kMaxFaces];
+    uint32_t ups = 0, c = 0, d = 0;
+    double source = 0.0;
+    if (lane < n) {
+      const uint32_t t = p.order[gr.pos + lane];
+      d = t / a.Np;
+      c = t - d * a.Np;
+      source = a.src_dir[c];
+      ext = source != 0.0;
+      for (uint32_t f = a.off[c]; f < a.off[c + 1]; ++f) {
+        const uint32_t nb = a.nbr[f], kind = nb >> kKindShift;
+        if (kind == kKindBoundary) continue;
+        const int sign = pull_sign(a, f, d);
+        if (sign > 0) ++given;
+        if (sign >= 0) continue;
+        if (kind == kKindPeriodic) {
+          ext = true;
+          if (!b.data || pull_fraction(p, c, f, d) >= 0.0) ++found;
+          continue;
+        }
+        const uint32_t u = p.pos_of_task[d * a.Np + (nb & kNbrMask)] - s.base;
+        uint32_t i = ups++;
+        for (; i > 0 && up[i - 1] > u; --i) {
+          up[i] = up[i - 1];
+          face[i] = face[i - 1];
+        }
+        up[i] = u;
+        face[i] = (uint8_t)(f - a.off[c]);
+      }
+    }
+    if (ups > padded) {
+      atomicOr(&a.ctl->error, kErrRecords);
+      ups = padded;
+    }
+    const uint32_t k = b.gseg[g];
+    const uint32_t previous = s.number ? b.seg[k - (b.seg[k] > s.base ? 1 : 0)] - s.base : 0u;  // of the level before
+    uint32_t late = 0;
+    for (uint32_t i = 0; i < ups; ++i) {
+      const uint32_t f0 = s.far, x = stream_slot(b, s, gr.shape, lane, up[i]), j = padded - ups + i;
+      if (up[i] >= previous) ++late;
+      if (b.data) {
+        const double frac = pull_fraction(p, c, a.off[c] + face[i], d);
+        if (frac >= 0.0) ++found;
+        idx[piece.slot(j, lane)] = (uint16_t)x;
+        w[piece.wslot(j, lane)] = frac;
+        if (s.far > f0) far[f0 * 32] = up[i];
+      }
+    }
+    if (b.data) {
+      for (uint32_t j = 0; j < padded - ups; ++j) {
+        idx[piece.slot(j, lane)] = (uint16_t)b.shape.ring;  // the zero word
+        w[piece.wslot(j, lane)] = 0.0;
+      }
+      for (uint32_t f = s.far; f < group_far(gr.shape); ++f) far[f * 32] = 0xffffffffu;
+      const_cast<double*>(piece.att())[lane] = 0.0;
+      if (gr.shape & kGroupExt) {
+        const_cast<double*>(piece.per())[lane] = 0.0;
+        const_cast<double*>(piece.src())[lane] = source;
+      }
+      const uint32_t most = __reduce_max_sync(0xffffffffu, ups);
+      late = __reduce_max_sync(0xffffffffu, late);
+      if (lane == 0) {
+        unsigned char* at = b.data + 16ull * gr.data;
+        *reinterpret_cast<uint4*>(at) = reinterpret_cast<const uint4*>(b.groups)[g];
+        const uint32_t need = previous ? b.seg_group[k - 1] - b.sgroup[k] : 0u;
+        *reinterpret_cast<StreamEarly*>(at + sizeof(StreamGroup)) = {need, padded - most, late, 0u};
+      }
+    }
+    const uint32_t flags = stream_flags(ext, s, b.shape.far);
+    if (!b.data) {
+      if (lane == 0) atomicOr(&b.groups[g].shape, flags);
+    } else if (((gr.shape ^ flags) & ~(0xfffu | kGroupKeep)) != 0u) {
+      if (lane == 0) atomicOr(&a.ctl->error, kErrRecords);
+    }
+  }
+  if (!b.data) return;
+  for (int o = 16; o > 0; o >>= 1) {
+    given += __shfl_xor_sync(0xffffffffu, given, o);
+    found += __shfl_xor_sync(0xffffffffu, found, o);
+  }
+  if (lane == 0) {
+    atomicAdd(&a.ctl->head, given);
+    atomicAdd(&a.ctl->tail, found);
+  }
+}
+
+// Periodic sources after a sweep (snapshot semantics, k_fold_pull of the mixed path): entry
+// d * n_cells + (index of the cell in `cells`) has the slots [off[e], off[e + 1]), {upwind
+// position, fraction} in face order.  (Computing the fractions of wide entries here, a division
+// each, took 3.6 ms of a 64^3 sweep with 84 directions.)
+struct alignas(16) FoldSlot64 {
+  uint32_t pos, pad;
+  double frac;
+};
+
+// counts the entries' slots (slots null), or writes them
+static __global__ void k_fold_build64(FacePull p, const uint32_t* cells, uint32_t n_cells, uint8_t* cnt,
+                                      const uint32_t* off, FoldSlot64* slots) {
+  const SweepArgs<double>& a = p.a;
+  const size_t total = (size_t)n_cells * a.D;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t d = (uint32_t)(e / n_cells), c = cells[e % n_cells];
+    uint32_t n = 0;
+    for (uint32_t f = a.off[c]; f < a.off[c + 1]; ++f) {
+      const uint32_t nb = a.nbr[f];
+      if ((nb >> kKindShift) != kKindPeriodic || pull_sign(a, f, d) >= 0) continue;
+      if (slots)
+        slots[off[e] + n] = {p.pos_of_task[(size_t)d * a.Np + (nb & kNbrMask)], 0u, pull_fraction(p, c, f, d)};
+      ++n;
+    }
+    if (!slots) cnt[e] = (uint8_t)n;
+  }
+}
+
+// After a sweep that left cells inactive: the periodic cells with a periodic neighbour that was
+// active; the entries of the others stay as they are.
+static __global__ void k_fold_mark64(SweepArgs<double> a, const double* cell_att, const uint32_t* cells,
+                                     uint32_t n_cells, uint8_t* changed) {
+  for (uint32_t pc = blockIdx.x * blockDim.x + threadIdx.x; pc < n_cells; pc += gridDim.x * blockDim.x) {
+    const uint32_t c = cells[pc];
+    uint8_t ch = 0;
+    for (uint32_t f = a.off[c]; f < a.off[c + 1] && !ch; ++f) {
+      const uint32_t nb = a.nbr[f];
+      if ((nb >> kKindShift) == kKindPeriodic && st_live(cell_att[nb & kNbrMask])) ch = 1;
+    }
+    changed[pc] = ch;
+  }
+}
+
+// grid: (periodic cells / blockDim.x, D)
+static __global__ void k_fold64(const double* out, double* periodic, uint32_t Np, const uint32_t* cells,
+                                uint32_t n_cells, const uint32_t* off, const FoldSlot64* slots, const uint8_t* changed) {
+  const uint32_t d = blockIdx.y, pc = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pc >= n_cells || (changed && !changed[pc])) return;
+  const size_t e = (size_t)d * n_cells + pc;
+  double in = 0.0;
+  for (uint32_t k = off[e]; k < off[e + 1]; ++k) {
+    const FoldSlot64 s = slots[k];
+    in = fma(s.frac, out[s.pos], in);
+  }
+  periodic[(size_t)d * Np + cells[pc]] = in;
+}
+
+// Cells whose incoming rates are out of date: a LOCAL neighbour was solved in a later sweep.
+static __global__ void k_stream_stale(SweepArgs<double> a, const uint32_t* cell_sweep, uint8_t* stale) {
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < a.N; c += gridDim.x * blockDim.x) {
+    const uint32_t mine = cell_sweep[c];
+    uint8_t s = 0;
+    for (uint32_t f = a.off[c]; f < a.off[c + 1] && !s; ++f) {
+      const uint32_t nb = a.nbr[f];
+      if ((nb >> kKindShift) == kKindLocal && cell_sweep[nb & kNbrMask] > mine) s = 1;
+    }
+    stale[c] = s;
+  }
+}
+
+// Their incoming rates from the present words (the reference keeps adding corrections to
+// inactive cells), summed as the sweep does.  grid: (streams, any)
+static __global__ void k_stream_refresh(StreamArgs<double> a, const uint8_t* stale) {
+  const StreamDesc sd = a.streams[blockIdx.x];
+  const uint32_t lane = threadIdx.x & 31, warps = gridDim.y * (blockDim.x / 32);
+  const double* word = a.word + sd.base;
+  for (uint32_t number = blockIdx.y * (blockDim.x / 32) + threadIdx.x / 32; number < sd.groups; number += warps) {
+    const StreamGroup gr = a.groups[sd.group0 + number];
+    const bool mine = lane < group_tasks(gr.shape) && stale[a.order[gr.pos + lane] % a.Np] != 0;
+    if (!mine) continue;
+    const StreamPiece<double> s(a.data + 16ull * gr.data, gr);
+    const uint32_t rel = gr.pos - sd.base + lane;
+    StreamSum<double> sum;
+    for (uint32_t j = 0; j < s.quads; ++j) {
+      StreamQuad<double> t;
+      t.load(s, j, lane);
+      const uint32_t x[4] = {t.x.x & 0xffffu, t.x.x >> 16, t.x.y & 0xffffu, t.x.y >> 16};
+      double q[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        q[k] = x[k] == a.shape.ring ? 0.0 : st_ldq(word + stream_slot_position(a.shape, s, number, lane, rel, x[k]));
+      st_add(sum, j & 1u, t.w, q);
+    }
+    a.inc[sd.base + rel] = sum.total();
+  }
+}
+
+}  // namespace swk

@@ -1,7 +1,9 @@
-"""Direction streams against the levelled lockstep kernels, bit for bit (mixed path).
+"""Direction streams against the transports they replace.
 
-The two layouts solve the same tasks with the same roundings, so every field, rate, level
-and time series is compared exactly; checkpoints are written in one and read in the other.
+Mixed path: the levelled lockstep kernels solve the same tasks with the same roundings, so every
+field, rate, level and time series is compared exactly; checkpoints are written in one layout and
+read in the other.  FP64: the push form hands the same shares out, in an order of its own and as
+corrections, so the rates agree to rounding; the forms of the streams agree exactly.
 """
 import numpy as np
 import pytest
@@ -48,12 +50,12 @@ CASES = {
 }
 
 
-def make(w, monkeypatch, env):
+def make(w, monkeypatch, env, precision="mixed"):
     for k in ("SUBSWEEP_STREAMS", "SUBSWEEP_COMPACT", "SUBSWEEP_STREAM_WARPS", "SUBSWEEP_GRAPH"):
         monkeypatch.delenv(k, raising=False)
     for k, v in env.items():
         monkeypatch.setenv(k, v)
-    return Sweep(w.params, w.grid, w.density, w.ionized_hydrogen_fraction, w.temperature, w.source, precision="mixed",
+    return Sweep(w.params, w.grid, w.density, w.ionized_hydrogen_fraction, w.temperature, w.source, precision=precision,
                  autotune=False)
 
 
@@ -86,6 +88,52 @@ def test_streams_equal_lockstep(case, monkeypatch):
             same(expected, results(s))
             if "SUBSWEEP_COMPACT" not in env:
                 assert s.stats()["tasks"] == tasks
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_fp64_streams_equal_push(case, monkeypatch):
+    w = CASES[case]()
+    steps = 5
+    got = {}
+    forms = {"push": {"SUBSWEEP_STREAMS": "0"}, "streams": {"SUBSWEEP_STREAMS": "1"}}
+    forms.update({c: {"SUBSWEEP_STREAMS": "1", "SUBSWEEP_COMPACT": c} for c in ("never", "always")})
+    forms.update({"4": {"SUBSWEEP_STREAMS": "1", "SUBSWEEP_STREAM_WARPS": "4"},
+                  "graph": {"SUBSWEEP_STREAMS": "1", "SUBSWEEP_GRAPH": "1"}})
+    for name, env in forms.items():
+        with make(w, monkeypatch, env, "fp64") as s:
+            for _ in range(steps):
+                s.run_sweeps()
+            got[name] = results(s)
+            if name == "streams":
+                saved = s.save_state()
+    for name in forms:
+        if name not in ("push", "streams"):
+            same(got["streams"], got[name])
+    # A rate is a chain of at most a few hundred sums of fewer than 64 products: 300 * 70 * 2^-53 is
+    # 2e-12 of it, and the push form's corrections leave as much of the largest rate behind.
+    # (states that agree to 1e-10 leave the timestep, a state over its change in a step of at least
+    # max_timestep / 2^(levels - 1), its inverse to 1e-10 over that)
+    shortest = w.params.max_timestep / 2 ** (w.params.num_timestep_levels - 1)
+    for k, a in got["push"].items():
+        b = got["streams"][k]
+        if k == "level":
+            np.testing.assert_array_equal(a, b)
+            continue
+        finite = np.isfinite(a)
+        np.testing.assert_array_equal(finite, np.isfinite(b), err_msg=k)
+        a, b = a[finite], b[finite]
+        top = float(np.max(np.abs(a), initial=0.0))
+        if k == "timestep":
+            a, b, top = 1.0 / a, 1.0 / b, 100.0 / shortest
+        np.testing.assert_allclose(b, a, rtol=1e-10, atol=1e-12 * top, err_msg=k)
+    # a checkpoint of the streams goes on in both forms
+    for env in (forms["push"], forms["streams"]):
+        with make(w, monkeypatch, env, "fp64") as s:
+            s.load_state(saved)
+            after = results(s)
+            for k, a in got["streams"].items():
+                if k != "level":
+                    np.testing.assert_allclose(after[k], a, rtol=1e-13, err_msg=k)
 
 
 @pytest.mark.parametrize("case", ["lattice-20", "batch"])
