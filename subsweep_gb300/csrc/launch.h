@@ -107,7 +107,7 @@ struct DevicePtrs {
   void* cell_att;            // attenuation of every cell or the inactive mark (R)
   double* cell_rate;         // rate of every cell summed over the directions
   uint8_t* cell_periodic;    // whether the cell has a LOCAL_PERIODIC face
-  uint8_t* stale;            // FP64 streams: cells whose incoming rates are out of date (scratch)
+  uint8_t* stale;            // cells whose incoming rates are out of date (scratch)
   uint32_t stream_shape[5];  // StreamShape: ring, magic, far, warps, buffer
   // per level, lazily allocated: the active positions' bitmap, and their range in each stream
   uint32_t *act_bits_lv[32], *act_range[32];

@@ -656,12 +656,13 @@ __global__ void k_attenuation(uint32_t n, const uint8_t* level, int current_leve
 // Rate of cell c summed over the directions (Sweep::get_solver, src/sweep/mod.rs:613-631): FP64
 // in direction order; mixed path: a compensated FP32 sum of the scaled transported rates, the
 // source added in FP64.  `pos`: the incoming rates are indexed by position, else by task;
-// `has_periodic`: the cell has periodic faces (else its periodic sources are 0).  The rates are
-// loaded eight directions at a time.
-template <typename R>
+// `has_periodic`: the cell has periodic faces (else its periodic sources are 0).  The rates by
+// position are loaded kSumBatch directions at a time (latency: two loads per batch).
+constexpr int kRateBatch = 24;
+template <typename R, int kSumBatch>
 __device__ __forceinline__ double cell_sum(const R* incoming, const uint32_t* pos, const R* periodic, bool has_periodic,
                                            double source, int D, uint32_t Np, uint32_t c, double rate_scale) {
-  constexpr int kBatch = 8;
+  constexpr int kBatch = kSumBatch;
   const double src = source / (double)D;
   double rate = 0.0;
   float s = 0.f, comp = 0.f;
@@ -698,7 +699,7 @@ __global__ void __launch_bounds__(128) k_cell_sums(uint32_t n, const uint8_t* le
                                                    uint32_t Np, double rate_scale, double* out) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
     if (level[c] >= current_level)
-      out[c] = cell_sum(incoming, pos, periodic, cell_periodic[c] != 0, source[c], D, Np, c, rate_scale);
+      out[c] = cell_sum<R, kRateBatch>(incoming, pos, periodic, cell_periodic[c] != 0, source[c], D, Np, c, rate_scale);
 }
 
 template <typename R>
@@ -740,7 +741,7 @@ __global__ void k_chemistry(ChemArgs<R> a) {
     if (a.level[c] < a.current_level) continue;
     const double timestep = ldexp(a.max_timestep, -(int)a.level[c]);  // timestep_level.rs:42-48
     const double rate = a.cell_rate ? a.cell_rate[c]
-                                    : cell_sum(a.incoming, nullptr, a.periodic, true, a.source[c], a.D, a.Np, c,
+                                    : cell_sum<R, 8>(a.incoming, nullptr, a.periodic, true, a.source[c], a.D, a.Np, c,
                                                a.rate_scale);
     double relative_change;
     // chemistry/mod.rs:79-81.  The mixed path also treats a rate below the smallest
@@ -867,11 +868,19 @@ static __global__ void k_ionization_time(uint32_t n, const double* xhii, double*
 template <typename R>
 __global__ void k_photon_rate(uint32_t n, const R* incoming, const uint32_t* pos, int D, uint32_t Np, double rate_scale,
                               double* out) {
+  constexpr int kBatch = kRateBatch;
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
     double r = 0.0;
-    for (int d = 0; d < D; ++d) {
-      const size_t t = (size_t)d * Np + c;
-      r += (double)incoming[pos ? pos[t] : t];
+    for (int d0 = 0; d0 < D; d0 += kBatch) {
+      R in[kBatch];
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j) {
+        const size_t t = (size_t)min(d0 + j, D - 1) * Np + c;
+        in[j] = incoming[pos ? pos[t] : t];
+      }
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j)
+        if (d0 + j < D) r += (double)in[j];
     }
     out[c] = r * rate_scale;
   }

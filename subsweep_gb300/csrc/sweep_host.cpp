@@ -792,7 +792,7 @@ sw_status build_streams(sw_handle* h) {
   if (rb == 8) {  // what the push form does without
     uint32_t *pos = nullptr, *counts = nullptr, *cell_sweep = nullptr;
     if (!h->alloc(&pos, (size_t)h->Np * h->D) || !h->alloc(&counts, 32) || !h->alloc(&cell_sweep, h->Np) ||
-        !h->alloc(&p.stale, h->N) || !h->alloc(&p.fold_changed, p.n_periodic_cells) ||
+        !h->alloc(&p.fold_changed, p.n_periodic_cells) ||
         !h->alloc(&p.fold_off, (size_t)p.n_periodic_cells * h->D + 1)) {
       (void)cudaGetLastError();
       h->want_streams = false;
@@ -865,7 +865,8 @@ sw_status build_streams(sw_handle* h) {
   std::vector<uint8_t> has_periodic(h->N, 0);
   SW_CUDA(h, cudaMemcpy(pcells.data(), p.periodic_cells, pcells.size() * 4, cudaMemcpyDeviceToHost), "periodic cells");
   for (uint32_t c : pcells) has_periodic[c] = 1;
-  if (!h->alloc(&cell_att, (size_t)h->N * rb) || !h->alloc(&p.cell_rate, h->N) || !h->alloc(&p.cell_periodic, h->N))
+  if (!h->alloc(&cell_att, (size_t)h->N * rb) || !h->alloc(&p.cell_rate, h->N) || !h->alloc(&p.cell_periodic, h->N) ||
+      !h->alloc(&p.stale, h->N))
     return h->fail(SW_ERR_OOM, "device allocation of the streams failed");
   p.stream_bytes = at;
   p.cell_att = cell_att;
@@ -1542,9 +1543,9 @@ static bool pull_sparse(sw_handle* h, int level) {
   if (p.compact_mode == 2) return false;
   // Streams: a dense sweep takes the time of all tasks, 23 per ns, a sparse one ~5 per ns of
   // the active ones (128^3 x 84: 7.9 ms dense; sparse 14 ms with 39% of the cells active, the
-  // crossing near 20%; 64^3 x 84: 1.03 ms dense, 0.13 ms with 0.2% active).  FP64: a sparse sweep
-  // of all tasks takes twice a dense one's time (24^3 x 84, 32 sweeps: 19.8 and 9.8 ms).
-  if (p.stream_mode) return (int64_t)h->n_ge_host[level] * 5 < (h->ops->pull ? 1 : 2) * h->N;
+  // crossing near 20%; 64^3 x 84: 1.03 ms dense, 0.13 ms with 0.2% active).  FP64:
+  // 64^3 x 84 2.0 ms dense, 2.4 ms with a third of the cells active.
+  if (p.stream_mode) return (int64_t)h->n_ge_host[level] * 5 < h->N;
   return h->n_ge_host[level] * 2 < h->N;
 }
 
@@ -2307,6 +2308,7 @@ sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) {
     off += s.bytes;
   }
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "load state");
+  h->p.active_cells = 0;  // incoming rates of some cells may be out of date (mixed path)
   if (h->p.stream_mode && !h->ops->pull) {  // every incoming rate is current, no sweep is stamped
     h->p.active_cells = h->N;
     SW_CUDA(h, cudaMemset(h->p.cell_sweep, 0, (size_t)h->Np * 4), "load state");

@@ -155,6 +155,48 @@ cudaError_t sweep_stream(const DevicePtrs& p, int level, cudaStream_t s) {
   }
 }
 
+// Incoming rates of every cell as after the last sweep, before they are exported: that sweep
+// left those of its inactive cells as they were.
+cudaError_t refresh(const DevicePtrs& p, cudaStream_t s) {
+  if (!p.stream_mode || p.active_cells >= p.num_cells) return cudaSuccess;
+  swk::k_stream_stale<<<grid_for(p.num_cells, 256), 256, 0, s>>>((uint32_t)p.num_cells, p.off, p.nbr, p.cell_sweep,
+                                                                  p.stale);
+  const int y = std::max(8, (int)(8 * p.num_sms / std::max(1u, p.num_streams)));
+  swk::k_stream_refresh<R><<<dim3(p.num_streams, y), 256, 0, s>>>(stream_args(p), p.stale);
+  return cudaGetLastError();
+}
+
+// positions of the tasks' rates, or null where they lie by task
+const uint32_t* rate_pos(const DevicePtrs& p) { return p.stream_mode ? p.pos_of_task : nullptr; }
+
+// exports of the rates as they are stored (the push form's, and the streams' once brought up to date)
+cudaError_t photon_rate_stored(const DevicePtrs& p, double* out, cudaStream_t s) {
+  const cudaError_t e = refresh(p, s);
+  if (e != cudaSuccess) return e;
+  swk::k_photon_rate<R><<<grid_for(p.num_cells, 128), 128, 0, s>>>(
+      (uint32_t)p.num_cells, static_cast<const R*>(p.incoming), rate_pos(p), p.D, p.Np, p.rate_scale, out);
+  return cudaGetLastError();
+}
+
+cudaError_t cell_rates_stored(const DevicePtrs& p, double* out, cudaStream_t s) {
+  const cudaError_t e = refresh(p, s);
+  if (e != cudaSuccess) return e;
+  swk::k_cell_rates<R><<<grid_for(p.num_cells, 256), 256, 0, s>>>(
+      (uint32_t)p.num_cells, static_cast<const R*>(p.incoming), rate_pos(p), static_cast<const R*>(p.periodic),
+      static_cast<const R*>(p.src_dir), p.D, p.Np, p.rate_scale, out);
+  return cudaGetLastError();
+}
+
+cudaError_t export_rates_stored(const DevicePtrs& p, int which, double* out, cudaStream_t s) {
+  const cudaError_t e = which == 0 ? refresh(p, s) : cudaSuccess;
+  if (e != cudaSuccess) return e;
+  const void* src = which == 0 ? p.incoming : (which == 1 ? p.outgoing : p.periodic);
+  swk::k_export_rates<R><<<grid_for(p.num_cells * p.D, 256), 256, 0, s>>>(
+      (uint32_t)p.num_cells, static_cast<const R*>(src), which == 2 ? nullptr : rate_pos(p), p.D, p.Np, p.rate_scale,
+      out);
+  return cudaGetLastError();
+}
+
 cudaError_t occupancy(int* blocks_per_sm) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, swk::k_sweep<R>, swk::kSweepThreads, 0);
 }
@@ -276,15 +318,6 @@ cudaError_t stream_build64(const DevicePtrs& p, int phase, const StreamScratch& 
   return cudaGetLastError();
 }
 
-// Incoming rates of every cell as after the last sweep, before they are exported: that sweep
-// left those of its inactive cells as they were.
-cudaError_t refresh(const DevicePtrs& p, cudaStream_t s) {
-  if (!p.stream_mode || p.active_cells >= p.num_cells) return cudaSuccess;
-  swk::k_stream_stale<<<grid_for(p.num_cells, 256), 256, 0, s>>>(sweep_args(p, 0), p.cell_sweep, p.stale);
-  const int y = std::max(1, (int)(8 * p.num_sms / std::max(1u, p.num_streams)));
-  swk::k_stream_refresh<<<dim3(p.num_streams, y), 256, 0, s>>>(stream_args(p), p.stale);
-  return cudaGetLastError();
-}
 #endif
 
 // Seed of the schedule: dependency counts with every cell active (the caller has set
@@ -661,51 +694,30 @@ cudaError_t fold_pull(const DevicePtrs& p, cudaStream_t s) {
 }
 
 cudaError_t photon_rate(const DevicePtrs& p, uint32_t last_epoch, double* out, cudaStream_t s) {
+  if (p.stream_mode) return photon_rate_stored(p, out, s);
   swk::PullArgs a = pull_args(p, 0);
   swk::k_photon_rate_pull<<<grid_for(p.num_cells, 128), 128, 0, s>>>(a, last_epoch, p.rate_scale, out);
   return cudaGetLastError();
 }
 
 cudaError_t cell_rates(const DevicePtrs& p, uint32_t last_epoch, double* out, cudaStream_t s) {
+  if (p.stream_mode) return cell_rates_stored(p, out, s);
   swk::PullArgs a = pull_args(p, 0);
   swk::k_cell_rates_pull<<<grid_for(p.num_cells, 128), 128, 0, s>>>(a, last_epoch, p.rate_scale, out);
   return cudaGetLastError();
 }
 
 cudaError_t export_rates(const DevicePtrs& p, int which, uint32_t last_epoch, double* out, cudaStream_t s) {
+  if (p.stream_mode && which == 0) return export_rates_stored(p, which, out, s);
   swk::PullArgs a = pull_args(p, 0);
   swk::k_export_pull<<<grid_for(p.num_cells * p.D, 256), 256, 0, s>>>(a, last_epoch, which, p.rate_scale, out);
   return cudaGetLastError();
 }
 #else
-// positions of the tasks' rates, or null where they lie by task
-const uint32_t* rate_pos(const DevicePtrs& p) { return p.stream_mode ? p.pos_of_task : nullptr; }
-
-cudaError_t photon_rate(const DevicePtrs& p, uint32_t, double* out, cudaStream_t s) {
-  const cudaError_t e = refresh(p, s);
-  if (e != cudaSuccess) return e;
-  swk::k_photon_rate<R><<<grid_for(p.num_cells, 256), 256, 0, s>>>(
-      (uint32_t)p.num_cells, static_cast<const R*>(p.incoming), rate_pos(p), p.D, p.Np, p.rate_scale, out);
-  return cudaGetLastError();
-}
-
-cudaError_t cell_rates(const DevicePtrs& p, uint32_t, double* out, cudaStream_t s) {
-  const cudaError_t e = refresh(p, s);
-  if (e != cudaSuccess) return e;
-  swk::k_cell_rates<R><<<grid_for(p.num_cells, 256), 256, 0, s>>>(
-      (uint32_t)p.num_cells, static_cast<const R*>(p.incoming), rate_pos(p), static_cast<const R*>(p.periodic),
-      static_cast<const R*>(p.src_dir), p.D, p.Np, p.rate_scale, out);
-  return cudaGetLastError();
-}
-
+cudaError_t photon_rate(const DevicePtrs& p, uint32_t, double* out, cudaStream_t s) { return photon_rate_stored(p, out, s); }
+cudaError_t cell_rates(const DevicePtrs& p, uint32_t, double* out, cudaStream_t s) { return cell_rates_stored(p, out, s); }
 cudaError_t export_rates(const DevicePtrs& p, int which, uint32_t, double* out, cudaStream_t s) {
-  const cudaError_t e = which == 0 ? refresh(p, s) : cudaSuccess;
-  if (e != cudaSuccess) return e;
-  const void* src = which == 0 ? p.incoming : (which == 1 ? p.outgoing : p.periodic);
-  swk::k_export_rates<R><<<grid_for(p.num_cells * p.D, 256), 256, 0, s>>>(
-      (uint32_t)p.num_cells, static_cast<const R*>(src), which == 2 ? nullptr : rate_pos(p), p.D, p.Np, p.rate_scale,
-      out);
-  return cudaGetLastError();
+  return export_rates_stored(p, which, out, s);
 }
 #endif
 

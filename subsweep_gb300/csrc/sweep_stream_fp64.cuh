@@ -6,9 +6,7 @@
 // computed once per grid with the roundings of push_eff.  The share of face f of cell c comes
 // from the upwind cell's own face towards c (the reciprocal face, with the negated normal).
 //
-// The outgoing and incoming rates lie by schedule position.  Incoming rates of cells that were
-// not active lately are brought up to date when something asks for them (k_stream_refresh): a
-// sweep writes those of the active cells only.
+// The outgoing and incoming rates lie by schedule position.
 #pragma once
 
 #include "sweep_push_records.cuh"
@@ -227,46 +225,6 @@ static __global__ void k_fold64(const double* out, double* periodic, uint32_t Np
     in = fma(s.frac, out[s.pos], in);
   }
   periodic[(size_t)d * Np + cells[pc]] = in;
-}
-
-// Cells whose incoming rates are out of date: a LOCAL neighbour was solved in a later sweep.
-static __global__ void k_stream_stale(SweepArgs<double> a, const uint32_t* cell_sweep, uint8_t* stale) {
-  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < a.N; c += gridDim.x * blockDim.x) {
-    const uint32_t mine = cell_sweep[c];
-    uint8_t s = 0;
-    for (uint32_t f = a.off[c]; f < a.off[c + 1] && !s; ++f) {
-      const uint32_t nb = a.nbr[f];
-      if ((nb >> kKindShift) == kKindLocal && cell_sweep[nb & kNbrMask] > mine) s = 1;
-    }
-    stale[c] = s;
-  }
-}
-
-// Their incoming rates from the present words (the reference keeps adding corrections to
-// inactive cells), summed as the sweep does.  grid: (streams, any)
-static __global__ void k_stream_refresh(StreamArgs<double> a, const uint8_t* stale) {
-  const StreamDesc sd = a.streams[blockIdx.x];
-  const uint32_t lane = threadIdx.x & 31, warps = gridDim.y * (blockDim.x / 32);
-  const double* word = a.word + sd.base;
-  for (uint32_t number = blockIdx.y * (blockDim.x / 32) + threadIdx.x / 32; number < sd.groups; number += warps) {
-    const StreamGroup gr = a.groups[sd.group0 + number];
-    const bool mine = lane < group_tasks(gr.shape) && stale[a.order[gr.pos + lane] % a.Np] != 0;
-    if (!mine) continue;
-    const StreamPiece<double> s(a.data + 16ull * gr.data, gr);
-    const uint32_t rel = gr.pos - sd.base + lane;
-    StreamSum<double> sum;
-    for (uint32_t j = 0; j < s.quads; ++j) {
-      StreamQuad<double> t;
-      t.load(s, j, lane);
-      const uint32_t x[4] = {t.x.x & 0xffffu, t.x.x >> 16, t.x.y & 0xffffu, t.x.y >> 16};
-      double q[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        q[k] = x[k] == a.shape.ring ? 0.0 : st_ldq(word + stream_slot_position(a.shape, s, number, lane, rel, x[k]));
-      st_add(sum, j & 1u, t.w, q);
-    }
-    a.inc[sd.base + rel] = sum.total();
-  }
 }
 
 }  // namespace swk
