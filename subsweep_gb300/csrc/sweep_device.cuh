@@ -736,6 +736,7 @@ struct ChemArgs {
 // (hydrogen_only/mod.rs:90-119), one thread per cell (inactive cells skip).
 template <typename R, bool kCarryNeutral>
 __global__ void k_chemistry(ChemArgs<R> a) {
+  if (a.ctl->error & (kErrStall | kErrQueue)) return;  // a sweep of the step stalled
   uint32_t attempts = 0, failures = 0, cells = 0, invalid = 0;
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < a.n; c += gridDim.x * blockDim.x) {
     if (a.level[c] < a.current_level) continue;

@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstdarg>
@@ -100,6 +101,14 @@ struct sw_handle {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[8] = {};
+  // sweeps of a step in flight: their events (start, transport start and end, transport and
+  // fold end, chemistry end) and their error flags, read when the host waits for them
+  static constexpr int kMaxInFlight = 64;
+  std::vector<std::array<cudaEvent_t, 5>> sweep_ev;
+  struct Pinned {
+    swk::SweepCtl ctl;
+    uint32_t error[kMaxInFlight];
+  }* pinned = nullptr;
   swh::DevicePtrs p{};
   std::vector<void*> allocations;
   std::vector<uint32_t> n_ge_host;  // cells with level >= l at the start of the next step
@@ -149,6 +158,10 @@ struct sw_handle {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     for (cudaEvent_t e : graph_ev) cudaEventDestroy(e);
     if (graph_scalars) cudaFreeHost(graph_scalars);
+    for (auto& set : sweep_ev)
+      for (cudaEvent_t e : set)
+        if (e) cudaEventDestroy(e);
+    if (pinned) cudaFreeHost(pinned);
     for (void* a : allocations) cudaFree(a);
     for (cudaEvent_t e : ev)
       if (e) cudaEventDestroy(e);
@@ -293,9 +306,15 @@ bool check_acyclic(const sw_grid_csr* g, const std::vector<double>& dirs, int D,
 }
 
 sw_status sync_ctl(sw_handle* h) {
-  SW_CUDA(h, cudaMemcpyAsync(&h->ctl_host, h->p.ctl, sizeof(swk::SweepCtl), cudaMemcpyDeviceToHost, h->stream),
+  if (!h->pinned) {
+    void* ptr = nullptr;
+    SW_CUDA(h, cudaMallocHost(&ptr, sizeof(sw_handle::Pinned)), "pinned control block");
+    h->pinned = static_cast<sw_handle::Pinned*>(ptr);
+  }
+  SW_CUDA(h, cudaMemcpyAsync(&h->pinned->ctl, h->p.ctl, sizeof(swk::SweepCtl), cudaMemcpyDeviceToHost, h->stream),
           "read control block");
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "synchronize");
+  h->ctl_host = h->pinned->ctl;
   h->n_ge_host.assign(h->ctl_host.n_ge, h->ctl_host.n_ge + h->L);
   return SW_OK;
 }
@@ -1786,19 +1805,82 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
   float sweep_ms = 0.f, chem_ms = 0.f, level_ms = 0.f, kernel_ms = 0.f;
   int64_t launches = 0;
   SW_CUDA(h, cudaEventRecord(h->ev[5], h->stream), "event");
+  // The sweeps are launched one behind another and looked at when the host waits for them, at
+  // the step's end (or after kMaxInFlight, or one by one while variants are tried or traced).
+  // The error flag stays set across them: a stall ends the sweeps behind it at once, and they
+  // leave the cells alone.
+  SW_CUDA(h, cudaMemsetAsync(&h->p.ctl->error, 0, sizeof(uint32_t), h->stream), "reset error flag");
+  std::vector<int> in_flight;  // levels
+  bool trial = false;
+  auto look = [&]() -> sw_status {  // the stream has been synchronized
+    for (size_t k = 0; k < in_flight.size(); ++k) {
+      const auto& ev = h->sweep_ev[k];
+      const int level = in_flight[k];
+      float a = 0.f, b = 0.f, t = 0.f;
+      cudaEventElapsedTime(&a, ev[0], ev[3]);
+      cudaEventElapsedTime(&b, ev[3], ev[4]);
+      cudaEventElapsedTime(&t, ev[1], ev[2]);
+      (void)cudaGetLastError();  // timing queries are best effort
+      sweep_ms += a;
+      chem_ms += b;
+      kernel_ms += t;
+      if (trial && h->p.stream_mode) {  // the streams have one shape: nothing to choose
+        h->tuned = true;
+      } else if (trial) {  // one autotuning trial per sweep; the fastest variant per task is kept
+        h->tune_ns.push_back(1e6 * t / std::max(1.0, (double)h->n_ge_host[level] * h->D));
+        if (++h->tune_index == ops.num_tune_variants) {
+          int best = 0;
+          for (int i = 1; i < ops.num_tune_variants; ++i)
+            if (h->tune_ns[i] < h->tune_ns[best]) best = i;
+          h->p.pull_variant = ops.tune_variants[best];
+          h->tuned = true;
+        }
+      }
+      if (h->trace) {
+        swk::SweepCtl c{};
+        cudaMemcpy(&c, h->p.ctl, sizeof(c), cudaMemcpyDeviceToHost);
+        std::fprintf(stderr,
+                     "subsweep sweep level=%d active_tasks=%llu kernel_ms=%.3f transport_ms=%.3f chem_ms=%.3f "
+                     "attempts=%llu chem_cells=%llu chem_attempts=%llu\n",
+                     level, (unsigned long long)h->n_ge_host[level] * (unsigned long long)h->D, t, a, b,
+                     (unsigned long long)c.attempts, (unsigned long long)c.chem_cells,
+                     (unsigned long long)c.chem_attempts);
+      }
+      h->stats.level_sweeps += 1;
+      const uint32_t err = h->pinned->error[k];
+      if (err & (swk::kErrStall | swk::kErrQueue)) {
+        // leave the queue empty so the handle stays usable for inspection
+        if (h->p.queue) cudaMemsetAsync(h->p.queue, 0xff, (size_t)h->Np * h->D * sizeof(uint32_t), h->stream);
+        cudaStreamSynchronize(h->stream);
+        return h->fail(SW_ERR_STALLED,
+                       "level %d sweep stalled: tasks left unsolved after a %.1f s wait (dependency cycle; flags 0x%x)",
+                       level, h->p.timeout_ns * 1e-9, err);
+      }
+      if (err & swk::kErrClamp)
+        return h->fail(SW_ERR_INVALID_ARG, "x_HII floor above 1 - 1e-10 in the chemistry clamp (reference panics)");
+    }
+    in_flight.clear();
+    return SW_OK;
+  };
   for (int level : order) {
     // Sweep::run_sweeps skips levels without active cells (mod.rs:262)
     if (h->n_ge_host[level] == 0) continue;
     expected += (uint64_t)h->n_ge_host[level] * (uint64_t)h->D;
-    SW_CUDA(h, cudaMemsetAsync(h->p.ctl, 0, offsetof(swk::SweepCtl, tasks), h->stream), "reset queue");
-    SW_CUDA(h, cudaEventRecord(h->ev[0], h->stream), "event");
+    const size_t slot = in_flight.size();
+    if (slot == h->sweep_ev.size()) {
+      h->sweep_ev.push_back({});
+      for (cudaEvent_t& e : h->sweep_ev.back()) SW_CUDA(h, cudaEventCreate(&e), "event");
+    }
+    const std::array<cudaEvent_t, 5> ev = h->sweep_ev[slot];
+    SW_CUDA(h, cudaMemsetAsync(h->p.ctl, 0, offsetof(swk::SweepCtl, error), h->stream), "reset queue");
+    SW_CUDA(h, cudaEventRecord(ev[0], h->stream), "event");
     // Sweeps with at least 1/16 of the cells active walk the precomputed schedule;
     // sparser ones use the dependency-driven queue, which touches only active tasks.
     bool levelled = h->p.num_sched_levels > 0 && (uint64_t)h->n_ge_host[level] * 16 >= (uint64_t)h->N;
     if (h->force_path == 1) levelled = h->p.num_sched_levels > 0;
     if (h->force_path == 2) levelled = false;
     // autotuning trials on dense sweeps only: sparse ones always run the lockstep kernel
-    const bool trial = ops.pull && h->autotune && !h->tuned && !pull_sparse(h, level);
+    trial = ops.pull && h->autotune && !h->tuned && !pull_sparse(h, level);
     if (trial && !h->p.stream_mode) h->p.pull_variant = ops.tune_variants[h->tune_index];
     if (h->pulls()) {
       levelled = true;  // the pull path always walks the schedule (or the id order)
@@ -1823,80 +1905,48 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
       SW_CUDA(h, ops.init_counts(h->p, level, nullptr, !levelled, h->stream), "init_counts kernel");
       launches += 1;
     }
-    SW_CUDA(h, cudaEventRecord(h->ev[6], h->stream), "event");
+    SW_CUDA(h, cudaEventRecord(ev[1], h->stream), "event");
     if (levelled) {
       SW_CUDA(h, ops.sweep_levels(h->p, level, h->stream), "levelled sweep kernel");
       h->stats.levelled_sweeps += 1;
     } else {
       SW_CUDA(h, ops.sweep(h->p, level, h->stream), "sweep kernel");
     }
-    SW_CUDA(h, cudaEventRecord(h->ev[7], h->stream), "event");
+    SW_CUDA(h, cudaEventRecord(ev[2], h->stream), "event");
     SW_CUDA(h, ops.fold_periodic(h->p, h->stream), "periodic fold kernel");
     launches += 3 + (h->p.n_periodic_cells > 0 ? 1 : 0);
     if (h->p.stream_mode) launches += h->p.sparse_sweep ? 1 : 2;  // rates of the cells, gather of a dense sweep
     if (h->pulls() && h->p.n_periodic_cells > 0 && h->p.active_cells < h->N) launches += 1;  // fold marks
-    SW_CUDA(h, cudaEventRecord(h->ev[1], h->stream), "event");
+    SW_CUDA(h, cudaEventRecord(ev[3], h->stream), "event");
     SW_CUDA(h, ops.chemistry(h->p, level, h->stream), "chemistry kernel");
-    SW_CUDA(h, cudaEventRecord(h->ev[2], h->stream), "event");
-    SW_CUDA(h, cudaStreamSynchronize(h->stream), "level sweep");
-    float a = 0.f, b = 0.f, k = 0.f;
-    cudaEventElapsedTime(&a, h->ev[0], h->ev[1]);
-    cudaEventElapsedTime(&b, h->ev[1], h->ev[2]);
-    cudaEventElapsedTime(&k, h->ev[6], h->ev[7]);
-    (void)cudaGetLastError();  // timing queries are best effort
-    sweep_ms += a;
-    chem_ms += b;
-    kernel_ms += k;
-    if (trial && h->p.stream_mode) {  // the streams have one shape: nothing to choose
-      h->tuned = true;
-    } else if (trial) {  // one autotuning trial per sweep; the fastest variant per task is kept
-      h->tune_ns.push_back(1e6 * k / std::max(1.0, (double)h->n_ge_host[level] * h->D));
-      if (++h->tune_index == ops.num_tune_variants) {
-        int best = 0;
-        for (int i = 1; i < ops.num_tune_variants; ++i)
-          if (h->tune_ns[i] < h->tune_ns[best]) best = i;
-        h->p.pull_variant = ops.tune_variants[best];
-        h->tuned = true;
-      }
-    }
+    SW_CUDA(h, cudaEventRecord(ev[4], h->stream), "event");
+    SW_CUDA(h, cudaMemcpyAsync(&h->pinned->error[slot], &h->p.ctl->error, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                               h->stream), "read error flag");
+    in_flight.push_back(level);
     h->stats.transport_launches += 1;
-    if (h->trace) {
-      swk::SweepCtl c{};
-      cudaMemcpy(&c, h->p.ctl, sizeof(c), cudaMemcpyDeviceToHost);
-      std::fprintf(stderr,
-                   "subsweep sweep level=%d active_tasks=%llu kernel_ms=%.3f transport_ms=%.3f chem_ms=%.3f "
-                   "attempts=%llu chem_cells=%llu chem_attempts=%llu\n",
-                   level, (unsigned long long)h->n_ge_host[level] * (unsigned long long)h->D, k, a, b,
-                   (unsigned long long)c.attempts, (unsigned long long)c.chem_cells,
-                   (unsigned long long)c.chem_attempts);
+    if (trial || h->trace || (int)in_flight.size() == sw_handle::kMaxInFlight) {
+      SW_CUDA(h, cudaStreamSynchronize(h->stream), "level sweep");
+      const sw_status st = look();
+      if (st != SW_OK) return st;
     }
-    uint32_t err = 0;
-    SW_CUDA(h, cudaMemcpy(&err, &h->p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
-    h->stats.level_sweeps += 1;
-    if (err & (swk::kErrStall | swk::kErrQueue)) {
-      // leave the queue empty so the handle stays usable for inspection
-      if (h->p.queue) cudaMemsetAsync(h->p.queue, 0xff, (size_t)h->Np * h->D * sizeof(uint32_t), h->stream);
-      cudaStreamSynchronize(h->stream);
-      return h->fail(SW_ERR_STALLED,
-                     "level %d sweep stalled: tasks left unsolved after a %.1f s wait (dependency cycle; flags 0x%x)",
-                     level, h->p.timeout_ns * 1e-9, err);
-    }
-    if (err & swk::kErrClamp)
-      return h->fail(SW_ERR_INVALID_ARG, "x_HII floor above 1 - 1e-10 in the chemistry clamp (reference panics)");
   }
   // TimestepState bookkeeping and level reassignment (mod.rs:268-270)
   double elapsed = h->ts.current_max_timestep();
-  h->ts.advance();
+  TimestepState after = h->ts;
+  after.advance();
   SW_CUDA(h, cudaEventRecord(h->ev[3], h->stream), "event");
-  SW_CUDA(h, swh::launch_update_levels(h->p, h->ts.lowest, h->stream), "level kernels");
+  SW_CUDA(h, swh::launch_update_levels(h->p, after.lowest, h->stream), "level kernels");
   h->act_valid = 0;  // levels change: the compacted lists are rebuilt next step
   SW_CUDA(h, cudaEventRecord(h->ev[4], h->stream), "event");
-  h->sim_time += elapsed;
-  SW_CUDA(h, swh::launch_ionization_time(h->p, h->sim_time, h->stream), "ionization time kernel");
+  SW_CUDA(h, swh::launch_ionization_time(h->p, h->sim_time + elapsed, h->stream), "ionization time kernel");
   launches += 3;
   SW_CUDA(h, cudaEventRecord(h->ev[1], h->stream), "event");
   sw_status st = sync_ctl(h);
   if (st != SW_OK) return st;
+  st = look();
+  if (st != SW_OK) return st;
+  h->ts = after;
+  h->sim_time += elapsed;
   cudaEventElapsedTime(&level_ms, h->ev[3], h->ev[4]);
   float step_ms = 0.f;
   cudaEventElapsedTime(&step_ms, h->ev[5], h->ev[1]);
