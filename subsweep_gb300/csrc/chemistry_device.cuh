@@ -15,11 +15,18 @@
 // neutral density keeps full relative precision near complete ionisation; the
 // smaller of x and y is the accurate one and the other is re-derived from it.
 //
-// Work per try_timestep_update attempt: the FP64 path (the reference's expressions) 535
-// DFMA, 128 DADD and 169 DMUL thread instructions, 1367 FP64 flops (ncu, C2 64^3).  The
-// mixed path evaluates the rate fits in FP32 (Fits32), forms the per-cell factors once
-// per cell, and keeps the densities, the sums, the implicit updates and their accept /
-// reject tests in FP64: 55 DFMA, 41 DMUL and 9 DADD, 160 FP64 flops (ncu, C4 64^3).
+// What bounds it: the FP64 unit, 64 cycles for a warp's instruction in a quarter of an SM, and
+// in small runs the chain of the attempts of one cell (hundreds beside a source).  Hence
+//   what depends on the state alone is formed once per state (begin()) and not for every
+//   attempt from it: a rejected attempt is repeated with half the step for a few operations;
+//   the fits at the temperature that an attempt accepts are the next state's;
+//   a power is one logarithm and one exponential, the products of powers one exponential;
+//   the recommended steps are formed for the last accepted attempt only.
+// Whole first steps, where cells take up to hundreds of attempts: a column of 600 cells in FP64
+// 20.5 -> 11.8 ms, 64^3 lognormal 47 -> 34, a batch of 12 boxes 23-27 -> 18; 96^3 FP64 steps with
+// ~5 attempts a cell 113 -> 93 ms, 128^3 mixed 105 -> 100.
+// The mixed path evaluates the rate fits in FP32 (Fits32); the densities, the sums, the
+// implicit updates and their accept / reject tests are FP64 in both.
 #pragma once
 
 #include <cfloat>
@@ -114,8 +121,49 @@ __device__ __forceinline__ Fits32 fits32(float t) {
   return f;
 }
 
+// FP64: the fits' shared factors at one temperature.  The rate fits and their temperature
+// derivatives (hydrogen_only/mod.rs:161-302) are functions of these; each derivative is the
+// reference's formula with the common factors taken out.  s5 = sqrt(t / 1e5).
+struct Fits64 {
+  double t, inv_t, sq, inv_1s5;  // temperature, 1 / t, sqrt(t), 1 / (1 + s5)
+  double fit, fitd;              // collision_fit 161-166 and its derivative 167-173
+  double ln_lambda;              // lambda = 315614 / t
+  static constexpr double kS5 = 0.0031622776601683793;      // 1 / sqrt(1e5)
+  static constexpr double kInvS5 = 316.22776601683796;      // sqrt(1e5)
+};
+
+__device__ __forceinline__ Fits64 fits64(double t) {
+  Fits64 f;
+  f.t = t;
+  f.inv_t = 1.0 / t;
+  f.sq = sqrt(t);
+  const double s5 = f.sq * Fits64::kS5;
+  f.inv_1s5 = 1.0 / (1.0 + s5);
+  const double c1 = 1.0 / 1e5, c2 = 157809.1;
+  const double e = exp(-c2 / t);
+  f.fit = f.sq * f.inv_1s5 * e;
+  // 1 / (t^1.5 s5) = sqrt(1e5) / t^2
+  f.fitd = (e * (c1 * c2 * t + 0.5 * s5 * (2.0 * c2 + t))) *
+           ((Fits64::kInvS5 * (f.inv_t * f.inv_t)) * (f.inv_1s5 * f.inv_1s5));
+  f.ln_lambda = log(315614.0 / t);
+  return f;
+}
+
+__device__ __forceinline__ void set_fits(Fits64& f, double t) { f = fits64(t); }
+__device__ __forceinline__ void set_fits(Fits32& f, double t) { f = fits32((float)t); }
+
+template <bool kCarryNeutral>
+struct ChemFits {
+  using Type = Fits64;
+};
+template <>
+struct ChemFits<true> {
+  using Type = Fits32;
+};
+
 template <bool kCarryNeutral>
 struct ChemSolver {
+  using Fits = typename ChemFits<kCarryNeutral>::Type;
   double x;   // ionized hydrogen fraction
   double y;   // neutral fraction (only meaningful when kCarryNeutral)
   double temperature;
@@ -123,104 +171,82 @@ struct ChemSolver {
   bool has_floor;
   double floor_t, floor_x;
   bool clamp_invalid;
-  // Mixed path: the per-cell factors of the update, formed once per cell instead of once
-  // per attempt (prepare(); the FP64 path keeps the reference's expressions)
-  double nh_cell, k_cell, rate_per_volume, compton_cell, xx_cell;
+  // per-cell factors of the update (prepare())
+  double nh, k_cell, compton_cell, xx_cell;
+  double step_rate;  // photons of the whole timestep (FP64), rate per volume (mixed)
+  // factors of the state that every attempt from it shares (begin()), and the fits at its
+  // temperature
+  double m, photo, heat_step, cool_step;
+  Fits fits;
+  double fits_t;  // temperature of `fits`
+  // the last accepted attempt
+  double last_dt, rel_t, rel_x;
 
-  __device__ void prepare() {
-    if (!kCarryNeutral) return;
-    nh_cell = density / Units::kProtonMass;
+  __device__ void prepare(double timestep) {
+    nh = density / Units::kProtonMass;
     k_cell = (Units::kGamma - 1.0) * Units::kProtonMass / (density * Units::kBoltzmann);
-    rate_per_volume = rate / volume;
+    step_rate = kCarryNeutral ? rate / volume : timestep * rate;
     xx_cell = 2.727 / scale_factor;
     const double x2 = xx_cell * xx_cell;
     compton_cell = (1.017e-37 * (x2 * x2)) * Units::kErgsPerS;
+    fits_t = -1.0;  // of no cell
   }
 
   __device__ __forceinline__ double neutral() const { return kCarryNeutral ? y : (1.0 - x); }
-  __device__ __forceinline__ double nh() const {
-    return kCarryNeutral ? nh_cell : density / Units::kProtonMass;
-  }
-  __device__ __forceinline__ double n_ionized() const { return nh() * x; }
-  __device__ __forceinline__ double n_neutral() const { return nh() * neutral(); }
-  __device__ __forceinline__ double mu() const { return 1.0 / (x + 1.0); }
+  __device__ __forceinline__ double n_ionized() const { return nh * x; }
+  __device__ __forceinline__ double n_neutral() const { return nh * neutral(); }
 
-  // The rate fits and their temperature derivatives (161-302) share their powers and
-  // exponentials: each derivative below is the reference's formula with the common
-  // factor taken from the fit evaluated at the same temperature
-  // ((1 + p)^(-c - 1) = 1 / ((1 + p)^c (1 + p)), lambda^1.5 = lambda sqrt(lambda)).
-  // The values agree with separate evaluation to rounding.
-
-  // collision_fit 161-166 and collision_fit_derivative 167-173
-  __device__ static void collision_fits(double t, double sqrt_t, double s5, double& fit, double& fitd) {
-    const double c1 = 1.0 / 1e5, c2 = 157809.1;
-    const double e = exp(-c2 / t);
-    fit = sqrt_t / (1.0 + s5) * e;
-    fitd = (e * (c1 * c2 * t + 0.5 * s5 * (2.0 * c2 + t))) / ((t * sqrt_t) * s5 * ((s5 + 1.0) * (s5 + 1.0)));
-  }
-
-  // Mixed path: cooling_rate and its derivative from the FP32 fits; the densities, the
-  // sums and the unit factors in FP64.
-  __device__ void cooling32(double& lambda_c, double& dlambda_c) const {
-    const double t = temperature;
+  // cooling_rate 275-287 and cooling_rate_derivative 289-302 at the current state:
+  // collisional ionization / excitation cooling (237-253), case B recombination cooling
+  // (196-216), bremsstrahlung and Compton cooling (265-273).  Mixed path: from the FP32 fits;
+  // the densities, the sums and the unit factors in FP64.
+  __device__ void cooling(const Fits32& f, double& lambda_c, double& dlambda_c) const {
     const double ne = n_ionized();
     const double nhn = n_neutral();
-    const double nhi = n_ionized();
-    const Fits32 f = fits32((float)t);
     const double u = Units::kErgsCentimetersCubedPerS;
-    const double compton = compton_cell * (t - xx_cell);
-    const double dcompton = compton_cell;
+    const double compton = compton_cell * (temperature - xx_cell);
     const double coll = ((double)f.exc + 1.27e-21 * (double)f.fit) * u * ne * nhn;
     const double dcoll = ((double)f.dexc + 1.27e-21 * (double)f.fitd) * u * ne * nhn;
-    lambda_c = coll + ((double)f.recc + (double)f.brems) * u * ne * nhi + compton * ne;
-    dlambda_c = dcoll + ((double)f.drecc + (double)f.dbrems) * u * ne * nhi + dcompton * ne;
+    lambda_c = coll + ((double)f.recc + (double)f.brems) * u * ne * ne + compton * ne;
+    dlambda_c = dcoll + ((double)f.drecc + (double)f.dbrems) * u * ne * ne + compton_cell * ne;
   }
-
-  // cooling_rate 275-287 and cooling_rate_derivative 289-302 at the current temperature:
-  // collisional ionization / excitation cooling (237-253), case B recombination cooling
-  // (196-216), bremsstrahlung and Compton cooling (265-273).
-  __device__ void cooling(double& lambda_c, double& dlambda_c) const {
-    const double t = temperature;
+  __device__ void cooling(const Fits64& f, double& lambda_c, double& dlambda_c) const {
+    const double t = f.t;
     const double ne = n_ionized();
     const double nhn = n_neutral();
-    const double nhi = n_ionized();
-    const double sq = sqrt(t);
-    const double s5 = sqrt(t / 1e5);
-    double fit, fitd;
-    collision_fits(t, sq, s5, fit, fitd);
+    const double u = Units::kErgsCentimetersCubedPerS;
     // excitation cooling and its derivative
-    const double e_exc = exp(-118348.0 / t);
-    const double exc = (7.5e-19 / (1.0 + s5) * e_exc) * Units::kErgsCentimetersCubedPerS;
     const double c3 = 1.0 / 1e5, c2e = 118348.0;
-    const double dexc = ((7.5e-19 * e_exc * (c2e * c3 * t - 0.5 * c3 * (t * t) + c2e * s5)) /
-                         ((t * t) * s5 * ((1.0 + s5) * (1.0 + s5)))) *
-                        Units::kErgsCentimetersCubedPerS;
-    // case B recombination cooling and its derivative
-    const double lambda = 315614.0 / t;
-    // lambda^1.97 and (lambda / 2.25)^0.376 from one logarithm
-    const double ln_lambda = log(lambda);
-    const double l197 = exp(1.97 * ln_lambda);
-    const double q = exp(0.376 * (ln_lambda - 0.81093021621632877));  // ln 2.25
-    const double a = pow(1.0 + q, 3.72);
-    const double recomb_rate = (3.435e-30 * t * l197 / a) * Units::kErgsCentimetersCubedPerS;
+    const double e_exc = 7.5e-19 * exp(-c2e / t);
+    const double s5 = f.sq * Fits64::kS5;
+    const double exc = e_exc * f.inv_1s5;
+    // 1 / (t^2 s5) = sqrt(1e5) sqrt(t) / t^3
+    const double dexc = (e_exc * (c2e * c3 * t - 0.5 * c3 * (t * t) + c2e * s5)) *
+                        (((Fits64::kInvS5 * f.sq) * f.inv_t) * (f.inv_t * f.inv_t) * (f.inv_1s5 * f.inv_1s5));
+    // case B recombination cooling and its derivative, with lambda^1.97 / (1 + q)^3.72
     const double c2r = 1.97, c3r = 0.376, c4r = 3.72;
-    const double drecomb_rate = (3.435e-30 * ((1.0 / (a * (1.0 + q))) *
-                                             (1.0 - 1.0 * c2r + (1.0 - 1.0 * c2r + c3r * c4r) * q) * l197)) *
-                                Units::kErgsCentimetersCubedPerS;
-    // Compton
-    const double xx = 2.727 / scale_factor;
-    const double x2 = xx * xx;
-    const double compton = (1.017e-37 * (x2 * x2) * (t - xx)) * Units::kErgsPerS;
-    const double dcompton = (1.017e-37 * (x2 * x2)) * Units::kErgsPerS;
+    const double q = exp(c3r * (f.ln_lambda - 0.81093021621632877));  // ln 2.25
+    const double power = 3.435e-30 * exp(c2r * f.ln_lambda - c4r * log(1.0 + q));
+    const double recomb = power * t;
+    const double drecomb = power * ((1.0 - c2r + (1.0 - c2r + c3r * c4r) * q) / (1.0 + q));
+    const double brems = 1.42e-27 * f.sq;
+    const double dbrems = (0.5 * 1.42e-27) * (f.sq * f.inv_t);
+    const double compton = compton_cell * (temperature - xx_cell);
+    lambda_c = (exc + 1.27e-21 * f.fit) * u * ne * nhn + (recomb + brems) * u * ne * ne + compton * ne;
+    dlambda_c = (dexc + 1.27e-21 * f.fitd) * u * ne * nhn + (drecomb + dbrems) * u * ne * ne + compton_cell * ne;
+  }
 
-    const double coll = (exc + (1.27e-21 * fit) * Units::kErgsCentimetersCubedPerS) * ne * nhn;
-    const double recomb = recomb_rate * ne * nhi;
-    const double brems = ((1.42e-27 * sq) * Units::kErgsCentimetersCubedPerS) * ne * nhi;
-    lambda_c = coll + recomb + brems + compton * ne;
-    const double dcoll = (dexc + (1.27e-21 * fitd) * Units::kErgsCentimetersCubedPerS) * ne * nhn;
-    const double drecomb = drecomb_rate * ne * nhi;
-    const double dbrems = ((1.42e-27 / (2.0 * sq)) * Units::kErgsCentimetersCubedPerS) * ne * nhi;
-    dlambda_c = dcoll + drecomb + dbrems + dcompton * ne;
+  // case B recombination rate and its derivative, 175-194
+  __device__ static void recombination(const Fits32& f, double& alpha, double& dalpha) {
+    alpha = (double)f.alpha * Units::kCentimetersCubedPerS;
+    dalpha = (double)f.dalpha * Units::kCentimetersCubedPerS;
+  }
+  __device__ static void recombination(const Fits64& f, double& alpha, double& dalpha) {
+    const double c2a = 0.407, c3a = 2.242;
+    const double p = exp(c2a * (f.ln_lambda - 1.0079579203999789));  // ln 2.74
+    // lambda^1.5 / (1 + p)^2.242; the derivative by lambda times d lambda / dT = -lambda / T
+    alpha = (2.753e-14 * Units::kCentimetersCubedPerS) * exp(1.5 * f.ln_lambda - c3a * log(1.0 + p));
+    dalpha = (alpha * f.inv_t) * ((c2a * c3a * p - 1.5 * p - 1.5) / (p + 1.0));
   }
 
   // 312-319: photons absorbed per photon arriving, 1 - exp(-n_HI sigma size); both
@@ -231,62 +257,46 @@ struct ChemSolver {
     return 1.0 - exp(-n_neutral() * Units::kSigma * length);
   }
 
-  // 304-310 (+ photoheating_rate 321-325); m = mu() of the attempt
-  __device__ double temperature_change(double timestep, double absorbed, double m) const {
-    double k, heating, lc, dlc;
-    if (kCarryNeutral) {
-      k = k_cell;
-      heating = (rate_per_volume * absorbed) * (Units::kPhotonAverageEnergy - Units::kRydberg);
-      cooling32(lc, dlc);
-    } else {
-      k = (Units::kGamma - 1.0) * Units::kProtonMass / (density * Units::kBoltzmann);
-      heating = ((timestep * rate * absorbed) / volume) * (Units::kPhotonAverageEnergy - Units::kRydberg) / timestep;
-      cooling(lc, dlc);
+  // What the attempts from the current state share.  The reference forms the photon terms with
+  // the attempt's step and divides by it: a power of two times the whole timestep, so the whole
+  // one gives the same numbers.
+  __device__ void begin(double timestep) {
+    const double absorbed = absorbed_fraction();
+    m = 1.0 / (x + 1.0);  // mu
+    if (!(fits_t == temperature)) {
+      set_fits(fits, temperature);
+      fits_t = temperature;
     }
-    double lambda = heating - lc;
-    double dlambdadt = -dlc;
-    return k * m * lambda * timestep / (1.0 - k * m * dlambdadt * timestep);
+    double lc, dlc, heating;
+    cooling(fits, lc, dlc);
+    constexpr double kEnergy = Units::kPhotonAverageEnergy - Units::kRydberg;
+    if (kCarryNeutral) {  // photoheating_rate 321-325, photoionization_rate 327-332
+      heating = (step_rate * absorbed) * kEnergy;
+      photo = (step_rate * absorbed) / n_neutral();
+    } else {
+      heating = ((step_rate * absorbed) / volume) * kEnergy / timestep;
+      photo = ((step_rate * absorbed) / (n_neutral() * volume)) / timestep;
+    }
+    const double km = k_cell * m;
+    heat_step = km * (heating - lc);
+    cool_step = km * -dlc;
   }
-  // 334-354 (+ photoionization_rate 327-332), case B rate 175-194 at the current
-  // (already updated) temperature
-  __device__ double ionized_fraction_change(double timestep, double absorbed, double m) const {
-    const double t = temperature;
-    double n_h = nh();
-    double ne = n_ionized();
-    double alpha, dalpha, fit, fitd, photo;
-    const double c2a = 0.407, c3a = 2.242;
-    if (kCarryNeutral) {
-      const Fits32 f = fits32((float)t);
-      alpha = (double)f.alpha * Units::kCentimetersCubedPerS;
-      dalpha = (double)f.dalpha * Units::kCentimetersCubedPerS;
-      fit = (double)f.fit;
-      fitd = (double)f.fitd;
-      photo = (rate_per_volume * absorbed) / n_neutral();
-    } else {
-      const double lambda = 315614.0 / t;
-      const double dlambda_dt = -315614.0 / (t * t);
-      const double sl = sqrt(lambda);
-      const double p = pow(lambda / 2.74, 0.407);
-      const double b = pow(1.0 + p, 2.242);
-      alpha = (2.753e-14 * (lambda * sl) / b) * Units::kCentimetersCubedPerS;
-      const double da = -sl * (1.0 / (b * (p + 1.0))) * (c2a * c3a * p - 1.5 * p - 1.5);
-      dalpha = ((2.753e-14 * da) * Units::kCentimetersCubedPerS) * dlambda_dt;
-      const double sq = sqrt(t);
-      const double s5 = sqrt(t / 1e5);
-      collision_fits(t, sq, s5, fit, fitd);
-      photo = (((timestep * rate) * absorbed) / (n_neutral() * volume)) / timestep;
-    }
-    double beta = (5.85e-11 * fit) * Units::kCentimetersCubedPerS;
-    double dbeta = (5.85e-11 * fitd) * Units::kCentimetersCubedPerS;
-    double c = beta * ne + photo;
-    double d = alpha * ne;
-    double xhii = x;
-    double rhsc = ne * t * m * 1.0 * dbeta;
-    double dcdx = n_h * beta - rhsc;
-    double rhsd = ne * t * m * 1.0 * dalpha;
-    double dddx = n_h * alpha - rhsd;
-    double j = dcdx - (c + d) - xhii * (dcdx + dddx);
-    return timestep * (c - xhii * (c + d)) / (1.0 - j * timestep);
+
+  // 334-354, case B rate at the temperature t of `f` that the attempt has reached
+  __device__ double ionized_fraction_change(double timestep, const Fits& f, double t) const {
+    const double ne = n_ionized();
+    double alpha, dalpha;
+    recombination(f, alpha, dalpha);
+    const double beta = (5.85e-11 * (double)f.fit) * Units::kCentimetersCubedPerS;
+    const double dbeta = (5.85e-11 * (double)f.fitd) * Units::kCentimetersCubedPerS;
+    const double c = beta * ne + photo;
+    const double d = alpha * ne;
+    const double rhsc = ne * t * m * dbeta;
+    const double dcdx = nh * beta - rhsc;
+    const double rhsd = ne * t * m * dalpha;
+    const double dddx = nh * alpha - rhsd;
+    const double j = dcdx - (c + d) - x * (dcdx + dddx);
+    return timestep * (c - x * (c + d)) / (1.0 - j * timestep);
   }
 
   // 356-369 with Rust f64::clamp semantics (asserts min <= max: flagged here).
@@ -304,26 +314,26 @@ struct ChemSolver {
     if (has_floor && temperature < floor_t) temperature = floor_t;
   }
 
-  // update() 444-461
-  __device__ __forceinline__ static bool accept(double value, double change, double max_allowed,
-                                                double timestep, double& recommendation) {
-    double relative_change = fmin(fabs(change / value), 1.0 / DBL_EPSILON);
-    if (relative_change > max_allowed) return false;
-    recommendation = timestep * (max_allowed / relative_change);
-    return true;
+  // relative change of update() 444-461
+  __device__ __forceinline__ static double relative(double value, double change) {
+    return fmin(fabs(change / value), 1.0 / DBL_EPSILON);
   }
 
-  // try_timestep_update 371-392
-  __device__ bool try_update(double timestep, double safety, Timescale& out) {
-    const double absorbed = absorbed_fraction();
-    const double m = mu();  // both updates use the x of the attempt's start
-    double tc = temperature_change(timestep, absorbed, m);
-    double rec_t;
-    if (!accept(temperature, tc, safety, timestep, rec_t)) return false;
-    temperature += tc;
-    double xc = ionized_fraction_change(timestep, absorbed, m);
-    double rec_x;
-    if (!accept(x, xc, safety, timestep, rec_x)) return false;
+  // try_timestep_update 371-392; the state stays as it is unless both changes are accepted
+  // (temperature_change 304-310)
+  __device__ bool try_update(double timestep, double safety) {
+    const double tc = heat_step * timestep / (1.0 - cool_step * timestep);
+    const double change_t = relative(temperature, tc);
+    if (change_t > safety) return false;
+    const double t = temperature + tc;
+    Fits f;
+    set_fits(f, t);
+    const double xc = ionized_fraction_change(timestep, f, t);
+    const double change_x = relative(x, xc);
+    if (change_x > safety) return false;
+    temperature = t;
+    fits = f;
+    fits_t = t;
     x += xc;
     if (kCarryNeutral) {
       y -= xc;
@@ -331,7 +341,9 @@ struct ChemSolver {
       if (x < 0.5) y = 1.0 - x; else x = 1.0 - y;
     }
     clamp();
-    out = ts_min(Timescale{rec_t, kProcTemperature}, Timescale{rec_x, kProcIonization});
+    last_dt = timestep;
+    rel_t = change_t;
+    rel_x = change_x;
     return true;
   }
 
@@ -340,26 +352,21 @@ struct ChemSolver {
                                         uint32_t& attempts) {
     uint64_t pend_lo = 0, pend_hi = 0;  // pending second halves at depths 1..127
     int depth = 0;
-    Timescale last{0.0, kProcTemperature};
+    clamp();
+    begin(timestep);
     while (true) {
-      clamp();
-      double t0 = temperature, x0 = x, y0 = y;
       if (depth > kChemMaxDepth) {
         failed = true;
         return Timescale{timestep / 10.0, kProcTemperature};
       }
-      double sub = ldexp(timestep, -depth);  // == timestep / 2^depth, exact
+      // timestep / 2^depth, exact
+      const double sub = timestep * __longlong_as_double((long long)(1023 - depth) << 52);
       ++attempts;
-      Timescale r;
-      if (!try_update(sub, safety, r)) {
-        temperature = t0;
-        x = x0;
-        y = y0;
+      if (!try_update(sub, safety)) {
         ++depth;
         if (depth < 64) pend_lo |= (1ull << depth); else pend_hi |= (1ull << (depth - 64));
         continue;
       }
-      last = r;
       if (pend_hi) {
         depth = 127 - __clzll((long long)pend_hi);
         pend_hi &= ~(1ull << (depth - 64));
@@ -368,8 +375,10 @@ struct ChemSolver {
         pend_lo &= ~(1ull << depth);
       } else {
         failed = false;
-        return last;
+        return ts_min(Timescale{last_dt * (safety / rel_t), kProcTemperature},
+                      Timescale{last_dt * (safety / rel_x), kProcIonization});
       }
+      begin(timestep);
     }
   }
 };
