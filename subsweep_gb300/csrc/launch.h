@@ -108,7 +108,10 @@ struct DevicePtrs {
   double* cell_rate;         // rate of every cell summed over the directions
   uint8_t* cell_periodic;    // whether the cell has a LOCAL_PERIODIC face
   uint8_t* stale;            // cells whose incoming rates are out of date (scratch)
-  uint32_t stream_shape[5];  // StreamShape: ring, magic, far, warps, buffer
+  uint32_t stream_shape[6];  // StreamShape: ring, magic, far, warps, buffer, blocks
+  uint32_t num_pairs;        // pairs of blocks (stream_shape[5] == 2)
+  void* stream_parts;        // StreamPart of all pairs
+  uint32_t *stream_part0, *stream_flags;
   // per level, lazily allocated: the active positions' bitmap, and their range in each stream
   uint32_t *act_bits_lv[32], *act_range[32];
   int sparse_sweep;          // pull path: this launch runs over the compacted list of its level
@@ -172,6 +175,8 @@ struct PrecisionOps {
   // stream_data allocated, writes the groups' pieces; FP64: phase 3 counts the periodic fold's
   // slots, phase 4 writes them
   cudaError_t (*stream_build)(const DevicePtrs&, int phase, const StreamScratch&, cudaStream_t);
+  // direction streams: pairs of blocks that can be resident at once with the shape set
+  cudaError_t (*stream_pairs)(const DevicePtrs&, int* pairs);
   // FP64 streams: brings the incoming rates of inactive cells up to date; nullptr on the pull path
   cudaError_t (*refresh)(const DevicePtrs&, cudaStream_t);
 };

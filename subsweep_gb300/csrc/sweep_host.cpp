@@ -462,18 +462,22 @@ static void stream_order(const uint16_t* level, const uint8_t* up, uint32_t Np, 
 }
 
 // Whether direction streams are faster than the kernels over the levelled schedule: the longest
-// stream, at 3.6 ns a task of its block (FP64 7.7), against the time of a level, from word to word
+// stream, at 3.6 ns a task of its block (FP64 7.7, of a pair of blocks 5.9), against the time of a level, from word to word
 // 0.85 us (FP64 push form, from atomic to atomic: 4), times the levels, plus the tasks at 17 per
 // ns (12).  Measured on uniform boxes, ms per sweep, levelled and streams.  Mixed path: 84
 // directions 24^3 0.32 and 0.15, 48^3 0.89 and 0.52, 64^3 1.56 and 1.01, 128^3 10.3 and 7.6; 16
 // directions 64^3 0.95 and 0.87, but 101^3 1.87 and 2.98: sixteen blocks cannot keep up with the
 // whole device where levels are wide.  FP64: 84 directions 16^3 0.97 and 0.18, 24^3 1.61 and 0.31,
 // 32^3 2.10 and 0.46, 64^3 5.4 and 2.0, 96^3 13.8 and 7.9; 16 directions 64^3 4.8 and 1.8, 101^3
-// 7.8 and 7.5.
+// 7.8 and 6.0.
 static bool streams_pay(const std::vector<uint32_t>& parts, uint64_t tasks, size_t levels, bool mixed) {
   uint32_t longest = 0;
   for (size_t k = 1; k < parts.size(); ++k) longest = std::max(longest, parts[k] - parts[k - 1]);
-  if (!mixed) return 7.7 * longest < 4000.0 * (double)levels + (double)tasks / 12.0;
+  if (!mixed) {
+    double task = 7.7;
+    if (longest > 480.0 * (double)levels) task = 5.9 * std::max(1.0, (double)tasks / longest / 76.0);  // pairs
+    return task * longest < 4000.0 * (double)levels + (double)tasks / 12.0;
+  }
   return 3.6 * longest < 850.0 * (double)levels + (double)tasks / 17.0;
 }
 
@@ -711,6 +715,61 @@ static void plan_stream(const swk::StreamDesc& sd, const uint32_t* seg, const st
   }
 }
 
+// Whether pairs of blocks walk the streams faster than single blocks: cycles of a level with g
+// groups, times the levels of the longest stream, times the rounds (there are half as many
+// pairs).  Lines through the measured times of uniform boxes, ms per sweep of 84 directions with
+// single blocks and pairs: mixed path 96^3 (18 groups a level) 3.06 and 3.77, 128^3 (31) 7.68 and
+// 7.24; FP64 64^3 (8) 2.02 and 2.58, 96^3 7.90 and 6.72; 16 directions FP64 64^3 1.84 and 2.09,
+// 101^3 (19) 7.54 and 5.98.
+static bool pairs_pay(double levels, double groups, double total, int sms, bool mixed) {
+  const double g = groups / levels;
+  const double one = mixed ? 500.0 + 176.0 * g : std::max(670.0, 580.0 * g - 1300.0);
+  const double two = mixed ? 1850.0 + 103.0 * g : 1540.0 + 295.0 * g;
+  const auto rounds = [&](int blocks) { return std::max(1.0, total / (groups * blocks)); };
+  return two * rounds(sms / 2) < 0.95 * one * rounds(sms);
+}
+
+// The parts of `pairs` pairs of blocks: the streams' groups end to end, cut into equal shares at
+// the nearest level.  A stream that is cut has its beginning in front of the next pair's share and
+// the rest at the end of this one's, so the beginning is solved by the time the rest is due (no
+// stream is longer than a share).  Returns the number of cuts (flags).
+static uint32_t plan_parts(const std::vector<swk::StreamDesc>& streams, const std::vector<uint32_t>& seg_group,
+                           uint32_t pairs, std::vector<swk::StreamPart>& parts, std::vector<uint32_t>& part0) {
+  uint64_t total = 0, longest = 0;
+  for (const swk::StreamDesc& s : streams) {
+    total += s.groups;
+    longest = std::max<uint64_t>(longest, s.groups);
+  }
+  const uint64_t share = std::max(longest, (total + pairs - 1) / pairs);
+  uint32_t flags = 0;
+  uint64_t room = share;
+  parts.clear();
+  part0 = {0};
+  for (uint32_t i = 0; i < streams.size(); ++i) {
+    const swk::StreamDesc& s = streams[i];
+    uint32_t cut = 0;  // groups in front of the next pair's share
+    if (s.groups > room) {
+      const uint32_t want = (uint32_t)(s.groups - room), last = (uint32_t)(part0.size());
+      if (last < pairs) {
+        const uint32_t* lo = seg_group.data() + s.seg0;
+        const uint32_t* at = std::lower_bound(lo, lo + s.segs, s.group0 + want);
+        cut = (at == lo + s.segs ? s.group0 + s.groups : *at) - s.group0;
+      }
+    }
+    if (cut == 0) {
+      parts.push_back({i, 0, s.groups, 0, 0});
+      room -= std::min<uint64_t>(room, s.groups);
+      continue;
+    }
+    if (cut < s.groups) parts.push_back({i, cut, s.groups, flags + 1, 0});
+    part0.push_back((uint32_t)parts.size());
+    parts.push_back({i, 0, cut, 0, cut < s.groups ? ++flags : 0});
+    room = share - std::min<uint64_t>(share, cut);
+  }
+  part0.push_back((uint32_t)parts.size());
+  return flags;
+}
+
 // bytes of a group's piece (StreamPiece), rb bytes a rate
 static uint32_t piece_bytes(uint32_t shape, uint32_t rb) {
   const uint32_t slots = (shape >> 5) & 0x7fu, far = shape >> 17;
@@ -735,6 +794,19 @@ sw_status build_streams(sw_handle* h) {
     const int v = std::atoi(env);
     if (v == 4 || v == 8 || v == 16) warps = (uint32_t)v;
   }
+  bool pairs = false;
+  {
+    const double total = (double)h->N * h->D / swk::kStreamGroup;
+    double longest = 0, levels = 0;
+    for (const swk::StreamDesc& s : h->streams)
+      if (s.count > longest) {
+        longest = s.count;
+        levels = s.segs;
+      }
+    pairs = pairs_pay(levels, longest / swk::kStreamGroup, total, p.num_sms, rb == 4);
+    if (const char* env = std::getenv("SUBSWEEP_STREAM_PAIRS")) pairs = std::atoi(env) != 0;
+  }
+  if (pairs) warps = swk::kPairWarps;
   uint32_t slots = 0;  // per task of the largest group
   for (const auto& m : h->stream_gmax)
     for (uint8_t v : m) slots = std::max<uint32_t>(slots, (v + 3u) & ~3u);
@@ -763,7 +835,7 @@ sw_status build_streams(sw_handle* h) {
                              60000 - (int64_t)warps * far * 32);
   };
   size_t room = 0;
-  const int most = std::max(1, std::min(8, (int)(48 / warps)));  // blocks per SM that their registers allow
+  const int most = pairs ? 1 : std::max(1, std::min(8, (int)(48 / warps)));  // blocks per SM that their registers allow
   for (int k = std::max(1, std::min(most, (int)((h->streams.size() + p.num_sms - 1) / p.num_sms))); k >= 1; --k) {
     room = std::min((size_t)optin, (size_t)per_sm / k - 1024);
     if (words_for(room, swk::kStreamFar) >= (int64_t)std::min(longest, 8192u)) break;
@@ -835,6 +907,7 @@ sw_status build_streams(sw_handle* h) {
   SW_CUDA(h, h->ops->stream_build(p, 0, b, h->stream), "stream position kernels");
   uint32_t* shape = p.stream_shape;
   shape[3] = warps;
+  shape[5] = pairs ? 2u : 1u;
   bool far = false;
   int64_t late = 0, slow = 0;
   for (int pass = 0; pass < 2; ++pass) {
@@ -855,6 +928,28 @@ sw_status build_streams(sw_handle* h) {
       slow += (g.shape & swk::kGroupSlow) != 0;
     }
     if (!far) break;
+  }
+  if (pairs) {
+    int resident = 0;
+    SW_CUDA(h, h->ops->stream_pairs(p, &resident), "pairs of blocks");
+    if (const char* env = std::getenv("SUBSWEEP_STREAM_PAIRS"))
+      if (std::atoi(env) > 1) resident = std::min(resident, std::atoi(env));
+    if (resident < 1) {
+      shape[5] = 1u;
+    } else {
+      std::vector<swk::StreamPart> parts;
+      std::vector<uint32_t> part0;
+      plan_parts(h->streams, seg_group, (uint32_t)resident, parts, part0);
+      swk::StreamPart* d_parts = nullptr;
+      if (!h->alloc(&d_parts, parts.size()) || !h->alloc(&p.stream_part0, part0.size()) ||
+          !h->alloc(&p.stream_flags, part0.size()))
+        return h->fail(SW_ERR_OOM, "device allocation of the streams failed");
+      SW_CUDA(h, cudaMemcpy(d_parts, parts.data(), parts.size() * sizeof(parts[0]), cudaMemcpyHostToDevice), "streams");
+      SW_CUDA(h, cudaMemcpy(p.stream_part0, part0.data(), part0.size() * 4, cudaMemcpyHostToDevice), "streams");
+      SW_CUDA(h, cudaMemset(p.stream_flags, 0xff, part0.size() * 4), "streams");
+      p.stream_parts = d_parts;
+      p.num_pairs = (uint32_t)part0.size() - 1;
+    }
   }
   uint64_t at = 0;
   for (swk::StreamGroup& g : groups) {
@@ -933,8 +1028,8 @@ sw_status build_streams(sw_handle* h) {
   for (const swk::StreamGroup& g : groups) all_slots += (int64_t)((g.shape & 31u) + 1u) * ((g.shape >> 5) & 0x7fu);
   h->stats_upwind_slots = all_slots;
   if (h->trace)
-    std::fprintf(stderr, "subsweep streams: %u of %u warps, buffer %u, ring %u, far %u, %zu groups (%lld late, %lld slow), %llu bytes\n",
-                 p.num_streams, warps, shape[4], shape[0], shape[2], groups.size(), (long long)late, (long long)slow,
+    std::fprintf(stderr, "subsweep streams: %u (%u pairs) of %u warps, buffer %u, ring %u, far %u, %zu groups (%lld late, %lld slow), %llu bytes\n",
+                 p.num_streams, p.num_pairs, warps, shape[4], shape[0], shape[2], groups.size(), (long long)late, (long long)slow,
                  (unsigned long long)at);
   p.stream_mode = 1;
   return SW_OK;
@@ -2358,6 +2453,7 @@ sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) {
     off += s.bytes;
   }
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "load state");
+  if (h->p.num_pairs) SW_CUDA(h, cudaMemset(h->p.stream_flags, 0xff, (size_t)h->p.num_pairs * 4), "load state");
   h->p.active_cells = 0;  // incoming rates of some cells may be out of date (mixed path)
   if (h->p.stream_mode && !h->ops->pull) {  // every incoming rate is current, no sweep is stamped
     h->p.active_cells = h->N;

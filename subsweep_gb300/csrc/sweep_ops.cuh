@@ -89,7 +89,8 @@ cudaError_t compact_active(const DevicePtrs& p, int level, cudaStream_t s) {
 }
 
 swk::StreamShape stream_shape(const DevicePtrs& p) {
-  return {p.stream_shape[0], p.stream_shape[1], p.stream_shape[2], p.stream_shape[3], p.stream_shape[4]};
+  return {p.stream_shape[0], p.stream_shape[1], p.stream_shape[2],
+          p.stream_shape[3], p.stream_shape[4], p.stream_shape[5]};
 }
 
 swk::StreamArgs<R> stream_args(const DevicePtrs& p) {
@@ -118,6 +119,9 @@ swk::StreamArgs<R> stream_args(const DevicePtrs& p) {
   a.cell_att = static_cast<const R*>(p.cell_att);
   a.periodic = static_cast<const R*>(p.periodic);
   a.Np = p.Np;
+  a.parts = static_cast<const swk::StreamPart*>(p.stream_parts);
+  a.part0 = p.stream_part0;
+  a.flags = p.stream_flags;
   return a;
 }
 
@@ -131,6 +135,48 @@ cudaError_t launch_stream(const DevicePtrs& p, bool all, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   fn<<<p.num_streams, 32 * W, smem, s>>>(a);
   return cudaGetLastError();
+}
+
+// Pairs of blocks: clusters of two, all of them resident at once (a part may wait for another
+// pair's).
+using PairKernel = void (*)(const swk::StreamArgs<R>);
+PairKernel pair_kernel(bool far, bool all) {
+  constexpr int W = swk::kPairWarps;
+  return far ? (all ? swk::k_sweep_stream<R, W, true, true, true> : swk::k_sweep_stream<R, W, true, false, true>)
+             : (all ? swk::k_sweep_stream<R, W, false, true, true> : swk::k_sweep_stream<R, W, false, false, true>);
+}
+cudaError_t pair_config(const DevicePtrs& p, PairKernel fn, cudaLaunchConfig_t* c, cudaLaunchAttribute* at) {
+  const size_t smem = swk::stream_smem_bytes<R>(stream_shape(p));
+  c->blockDim = dim3(32 * (swk::kPairWarps + 1));
+  c->dynamicSmemBytes = smem;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim = {2, 1, 1};
+  at[1].id = cudaLaunchAttributeCooperative;
+  at[1].val.cooperative = 1;
+  c->attrs = at;
+  return cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+cudaError_t stream_pairs(const DevicePtrs& p, int* pairs) {
+  cudaLaunchConfig_t c{};
+  cudaLaunchAttribute at[2];
+  const PairKernel fn = pair_kernel(true, true);
+  cudaError_t e = pair_config(p, fn, &c, at);
+  if (e != cudaSuccess) return e;
+  c.gridDim = dim3(2);
+  c.numAttrs = 1;
+  return cudaOccupancyMaxActiveClusters(pairs, (const void*)fn, &c);
+}
+cudaError_t launch_pairs(const DevicePtrs& p, bool all, cudaStream_t s) {
+  cudaLaunchConfig_t c{};
+  cudaLaunchAttribute at[2];
+  const swk::StreamArgs<R> a = stream_args(p);
+  const PairKernel fn = pair_kernel(a.shape.far != 0, all);
+  cudaError_t e = pair_config(p, fn, &c, at);
+  if (e != cudaSuccess) return e;
+  c.gridDim = dim3(2 * p.num_pairs);
+  c.numAttrs = 2;
+  c.stream = s;
+  return cudaLaunchKernelEx(&c, fn, a);
 }
 
 cudaError_t sweep_stream(const DevicePtrs& p, int level, cudaStream_t s) {
@@ -148,6 +194,7 @@ cudaError_t sweep_stream(const DevicePtrs& p, int level, cudaStream_t s) {
       static_cast<const swk::StreamGroup*>(p.stream_groups), p.num_groups, p.stream_data, p.order, p.Np,
       static_cast<const R*>(p.cell_att), static_cast<const R*>(p.periodic));
   const bool all = p.active_cells >= p.num_cells;
+  if (p.stream_shape[5] == 2) return launch_pairs(p, all, s);
   switch (p.stream_shape[3]) {
     case 4: return launch_stream<4>(p, all, s);
     case 8: return launch_stream<8>(p, all, s);
@@ -728,14 +775,14 @@ extern const PrecisionOps SWK_OPS = {
     SWK_NAME,       (int)sizeof(R), true,       occupancy,     attenuation, init_counts, sweep,
     occupancy_pull, sweep_pull,     kahn_round, schedule_seed, fold_pull,   chemistry,   photon_rate,
     export_rates,   records,        cell_rates, SWK_CARRY != 0,
-    (int)(sizeof(kTuneVariants) / sizeof(int)), kTuneVariants, nullptr, stream_build, nullptr,
+    (int)(sizeof(kTuneVariants) / sizeof(int)), kTuneVariants, nullptr, stream_build, stream_pairs, nullptr,
 };
 #else
 extern const PrecisionOps SWK_OPS = {
     SWK_NAME,         (int)sizeof(R), false,      occupancy,     attenuation,   init_counts, sweep,
     occupancy_levels, sweep_levels,   kahn_round, schedule_seed, fold_periodic, chemistry,   photon_rate,
     export_rates,     nullptr,        cell_rates, SWK_CARRY != 0,
-    0, nullptr,       push_records, stream_build64, refresh,
+    0, nullptr,       push_records, stream_build64, stream_pairs, refresh,
 };
 #endif
 

@@ -109,6 +109,7 @@ struct StreamShape {
   uint32_t far;     // far words of a task in a warp's buffer
   uint32_t warps;   // solving warps
   uint32_t buffer;  // bytes of a warp's buffer: the largest piece without its far list
+  uint32_t blocks;  // blocks of a stream: 1, or the 2 of a cluster
 };
 constexpr uint32_t kStreamZero = 4;  // words between the ring and the far buffers: the zero word
 
@@ -143,6 +144,11 @@ struct StreamArgs {
   const R *cell_att, *periodic;
   uint32_t Np;
   uint32_t* stamp;  // FP64: per position, the last sparse sweep that solved it
+  // pairs of blocks: the parts of pair i are parts[part0[i]], ... up to part0[i + 1]; flags[i]: the
+  // last sweep in which the first part of a cut stream was solved
+  const StreamPart* parts;
+  const uint32_t* part0;
+  uint32_t* flags;
 };
 
 __device__ __forceinline__ uint32_t st_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -171,6 +177,37 @@ __device__ __forceinline__ bool st_wait(Test test, SweepCtl* ctl, unsigned long 
     if (!ok) atomicOr(&ctl->error, kErrStall);
   }
   return __all_sync(0xffffffffu, ok);
+}
+
+// Pairs of blocks (a cluster): the peer's words and count by their addresses in its shared memory.
+__device__ __forceinline__ uint32_t st_peer(uint32_t address, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(address), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_peer_word(uint32_t address, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(address), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_peer_word(uint32_t address, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(address), "d"(v) : "memory");
+}
+// A pair's counts: groups solved by this block, and by the other as far as it has told.  A group of
+// a level is solved only when all earlier levels are, so their sum reaches the groups before a
+// level exactly when those are solved.
+__device__ __forceinline__ uint32_t st_count_pair(const uint32_t* p) {
+  uint32_t own, other;
+  asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(own) : "r"(st_smem(p)) : "memory");
+  asm volatile("ld.acquire.cluster.shared::cta.u32 %0, [%1];" : "=r"(other) : "r"(st_smem(p + 1)) : "memory");
+  return own + other;
+}
+// the words counted so far are in the peer's ring: a fence for many groups, by a warp of its own
+__device__ __forceinline__ void st_tell_peer(uint32_t peer_other, uint32_t count) {
+  asm volatile("fence.acq_rel.cluster;" ::: "memory");
+  asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(peer_other), "r"(count) : "memory");
+}
+__device__ __forceinline__ void st_cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // whether an attenuation is one, not the mark of a cell that is not active in the sweep
@@ -325,8 +362,19 @@ __device__ __forceinline__ void st_sum(StreamSum<double>& sum, const StreamQuad<
 // groups w, w + W, ...; lanes past a group's tasks compute with padding.  kFar: some groups
 // have far words.  kAll: every cell is active; otherwise the tasks of inactive cells hand their
 // kept word on through the ring.
-template <typename R, int W, bool kFar, bool kAll>
-__global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__ StreamArgs<R> a) {
+//
+// kPair: a stream is walked by the two blocks of a cluster, with the warps of both taking its
+// groups in turn, where levels are wide (96^3 x 84 in FP64 7.9 -> 6.7 ms, 128^3 x 84 in the mixed
+// path 7.7 -> 7.2; at 64^3 slower).  Either block holds the whole ring and a word is stored into
+// both.  A warp of its own fences the words of all groups solved so far and tells the peer their
+// number: with a fence for every group 96^3 took 7.9 ms, since it waits for the stores of the SM.
+// There are fewer pairs of SMs than streams (76 for 84 directions), so the streams are laid end to
+// end and cut into equal shares: where a share ends inside a stream, the next pair starts with
+// that stream's beginning, and this one ends with the rest of it, once the beginning is solved
+// (flags), its ring filled from memory.
+template <typename R, int W, bool kFar, bool kAll, bool kPair = false>
+__global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const __grid_constant__ StreamArgs<R> a) {
+  constexpr uint32_t S = kPair ? 2 * W : W;  // warps that take the groups in turn
   using Word = typename StreamTraits<R>::Word;
   extern __shared__ __align__(16) unsigned char st_shared[];
   const StreamShape& shape = a.shape;
@@ -335,8 +383,18 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
   uint32_t* count = reinterpret_cast<uint32_t*>(st_shared + 8 * 32);  // solved groups of the stream
   unsigned char* buffer = st_shared + kStreamHead + warp * shape.buffer;
   R* words = reinterpret_cast<R*>(st_shared + kStreamHead + W * shape.buffer);
-  const StreamDesc sd = a.streams[blockIdx.x];
-  if (threadIdx.x == 0) *count = 0;
+  StreamDesc sd = a.streams[kPair ? 0 : blockIdx.x];
+  uint32_t me = warp, peer_words = 0, peer_count = 0, first_part = 0, parts = 1;
+  if constexpr (kPair) {
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    me = rank * W + warp;  // (the warp that tells the peer: (rank + 1) * W)
+    peer_words = st_peer(st_smem(words), rank ^ 1u);
+    peer_count = st_peer(st_smem(count + 1), rank ^ 1u);
+    first_part = a.part0[blockIdx.x / 2];
+    parts = a.part0[blockIdx.x / 2 + 1] - first_part;
+  }
+  if (threadIdx.x < 2) count[threadIdx.x] = 0;
   if (threadIdx.x < kStreamZero) words[shape.ring + threadIdx.x] = R(0);
   if (lane == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(st_smem(bar)) : "memory");
@@ -348,6 +406,8 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
   const StreamGroup* groups = a.groups + sd.group0;
   Word* word = a.word + sd.base + lane;
   R* inc = a.inc + sd.base + lane;
+  uint32_t begin = 0, stop = sd.groups;  // groups of the part
+  auto counted = [&](uint32_t need) { return (kPair ? st_count_pair(count) : st_count(count)) >= need; };
   R* far_words = words + shape.ring + kStreamZero + warp * shape.far * 32u + lane;
   uint64_t policy;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
@@ -355,7 +415,7 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
   StreamGroup next{};
   uint32_t end = 0;
   auto locate = [&](uint32_t g) {
-    if (g < sd.groups) {
+    if (g < stop) {
       next = groups[g];
       end = groups[g + 1].data;
     }
@@ -384,7 +444,7 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
     }
   };
   bool dead = false;
-  uint32_t solved = 0, parity = 0, g = warp;
+  uint32_t solved = 0, parity = 0, g = me;
   // the group that the warp solves next, in registers
   StreamGroup gr{};
   StreamEarly early{};
@@ -392,10 +452,14 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
   R att = R(0), per = R(0), src = R(0), own = R(0);
   float inv = 0.f;
   uint32_t up[kFar ? kStreamFar : 1], up_far = 0;
+  // kPair: the far words on their way (the other block wrote some of them, so they come from L2,
+  // not by the copies through L1)
+  R held[kFar && kPair ? kStreamFar : 1];
+  uint32_t held_far = 0;
   bool staged = false;  // its piece is still in the buffer: slots beyond the registers
   // loads group g and starts the copy of the one after it
   auto load = [&]() {
-    if (g >= sd.groups) return;
+    if (g >= stop) return;
     // (a dead block's copies still land before their buffer is used again or left)
     dead = !st_wait([&]() { return st_bar_test(bar, parity); }, a.ctl, a.timeout_ns) || dead;
     parity ^= 1;
@@ -414,7 +478,7 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
     }
     if (!kAll && lane < group_tasks(gr.shape)) own = st_ldq(word + (gr.pos - sd.base));
     staged = s.quads > kStreamQuads;
-    if (g + W < sd.groups) {
+    if (g + S < stop) {
       if (kFar) {  // the positions of the next group's far words
         up_far = (next.shape & (kGroupLate | kGroupSlow)) ? 0u : group_far(next.shape);
         if (up_far) {
@@ -426,12 +490,18 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
       }
       if (!staged) {
         copy();
-        locate(g + 2 * W);
+        locate(g + 2 * S);
       }
     } else {
       up_far = 0;
     }
-    if (kFar) asm volatile("cp.async.wait_all;" ::: "memory");  // this group's far words
+    if (kFar && !kPair) asm volatile("cp.async.wait_all;" ::: "memory");  // this group's far words
+    if (kFar && kPair) {
+#pragma unroll
+      for (int f = 0; f < (int)kStreamFar; ++f)
+        if ((uint32_t)f < held_far) far_words[f * 32] = held[f];
+      held_far = 0;
+    }
   };
   // what is left to store of the group solved: behind the count, off the levels' chain
   R in = R(0), out = R(0);
@@ -445,102 +515,168 @@ __global__ void __launch_bounds__(32 * W) k_sweep_stream(const __grid_constant__
     }
     mine = false;
   };
-  locate(warp);
-  if (warp < sd.groups) copy();
-  locate(warp + W);
-  load();
-  while (g < sd.groups) {
-    StreamSum<R> sum;
-    const uint32_t quads = group_slots(gr.shape) / 4;
-    uint32_t first = 0;  // slot that the sum goes on with
-    if constexpr (sizeof(R) == 8) {
-      const bool ahead = !kFar || !(gr.shape & (kGroupLate | kGroupSlow));
-      if (ahead && !dead) {
-        dead = !st_wait([&]() { return st_count(count) >= early.need; }, a.ctl, a.timeout_ns);
-        first = 4 * quads - early.late;
-        if (!dead) st_sum(sum, quad, words, StreamPiece<R>(buffer, gr), lane, early.skip, first);
+  for (uint32_t part = 0; part < parts; ++part) {
+    uint32_t post = 0;
+    bool fresh = false;  // the part's first groups: their far words have not been fetched ahead
+    if constexpr (kPair) {
+      const StreamPart pt = a.parts[first_part + part];
+      sd = a.streams[pt.stream];
+      groups = a.groups + sd.group0;
+      word = a.word + sd.base + lane;
+      inc = a.inc + sd.base + lane;
+      begin = pt.begin;
+      stop = pt.end;
+      post = pt.post;
+      if (pt.wait) {  // the pair that has the stream's beginning
+        const uint32_t* flag = a.flags + pt.wait - 1;
+        dead = !st_wait([&]() {
+          uint32_t v;
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+          return v == sweep;
+        }, a.ctl, a.timeout_ns) || dead;
       }
-    }
-    // the levels before this group's
-    dead = dead || !st_wait([&]() { return st_count(count) >= gr.need; }, a.ctl, a.timeout_ns);
-    const uint32_t n = group_tasks(gr.shape);
-    rel = gr.pos - sd.base;
-    if (!dead) {
-      if (kFar && (gr.shape & (kGroupLate | kGroupSlow))) {
-        const StreamPiece<R> all(a.data + 16ull * gr.data, gr);
-        const Word* base = a.word + sd.base;
-        if (gr.shape & kGroupSlow) {  // more far words than the buffer holds: index far + number
-          const uint32_t far = shape.ring + kStreamZero;
-          for (uint32_t j = 0; j < quads; ++j) {
-            R q[4];
-            StreamQuad<R> t;
-            t.load(all, j, lane);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const uint32_t x = all.idx()[StreamPiece<R>::slot(4 * j + c, lane)];
-              q[c] = x >= far ? st_ldq(base + all.far()[(x - far) * 32 + lane]) : words[x];
-            }
-            st_add(sum, j & 1u, t.w, q);
-          }
-        } else {
-          for (uint32_t f = 0; f < group_far(gr.shape); ++f) {
-            const uint32_t at = all.far()[f * 32 + lane];
-            far_words[f * 32u] = at != 0xffffffffu ? st_ldq(base + at) : R(0);
-          }
+      if (begin > 0) {
+        const uint32_t from = groups[begin].pos - sd.base;
+        for (uint32_t i = threadIdx.x; i < min(from, shape.ring); i += blockDim.x) {
+          const uint32_t at = from - 1 - i;
+          words[ring_slot(shape, at)] = st_ldq(a.word + sd.base + at);
         }
+        fresh = true;
       }
-      if (!kFar || !(gr.shape & kGroupSlow)) {
-        const StreamPiece<R> s(buffer, gr);
-        if constexpr (sizeof(R) == 8) {
-          st_sum(sum, quad, words, s, lane, max(first, early.skip), 4 * quads);
-        } else {
-          R q[kStreamQuads][4];
-#pragma unroll
-          for (uint32_t c = 0; c < kStreamQuads; ++c)
-            if (c < quads) st_words(quad[c], words, q[c]);
-#pragma unroll
-          for (uint32_t c = 0; c < kStreamQuads; ++c)
-            if (c < quads) st_add(sum, c & 1u, quad[c].w, q[c]);
-          for (uint32_t c = kStreamQuads; c < quads; ++c) {
-            StreamQuad<R> t;
-            t.load(s, c, lane);
-            R qc[4];
-            st_words(t, words, qc);
-            st_add(sum, c & 1u, t.w, qc);
-          }
+      // (the groups in front of the part count as this block's)
+      if (threadIdx.x < 2) count[threadIdx.x] = threadIdx.x == 0 ? begin : 0u;
+      st_cluster_sync();
+      g = begin - begin % S + me;
+      if (g < begin) g += S;
+      if (warp == W) {  // tells the peer of the groups that this block has solved, until all are
+        const uint32_t rank = me / W - 1;
+        uint32_t mine = 0;  // this block's groups of the part
+        for (uint32_t w = rank * W; w < (rank + 1) * W; ++w) {
+          const uint32_t f = begin - begin % S + w, from = f < begin ? f + S : f;
+          if (from < stop) mine += (stop - from + S - 1) / S;
         }
+        uint32_t told = 0, now = 0;
+        bool ok = true;
+        while (told < mine && ok) {
+          ok = st_wait([&]() { return (now = st_count(count) - begin) > told; }, a.ctl, a.timeout_ns);
+          now = __shfl_sync(0xffffffffu, now, 0);
+          if (lane == 0) st_tell_peer(peer_count, now);
+          told = now;
+        }
+        g = stop;
       }
-      in = sum.total();
-      if constexpr (sizeof(R) == 8)
-        out = (gr.shape & kGroupExt) ? st_solve(in, src, per, att, a.threshold, inv) : st_solve(in, att, a.threshold);
-      else
-        out = st_solve(in, src, per, att, a.threshold, inv);
-      mine = lane < n && (kAll || st_live(att));
-      uint32_t slot = ring_slot(shape, rel) + lane;
-      if (slot >= shape.ring) slot -= shape.ring;
-      if (lane < n) words[slot] = mine ? out : own;
-      // a word that another group reads from memory is there before the barrier
-      if (kFar && (gr.shape & kGroupKeep)) store();
     }
-    __syncwarp();
-    if (lane == 0) st_count_up(count);
-    if (kFar && up_far) {  // solved by now: their levels lie before this group's
-      const Word* base = a.word + sd.base;
-#pragma unroll
-      for (int f = 0; f < (int)kStreamFar; ++f)
-        if (up[f] != 0xffffffffu)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(st_smem(far_words + f * 32)),
-                       "l"(base + up[f]), "n"(sizeof(R))
-                       : "memory");  // the q leads a word
-      up_far = 0;
-    }
-    if (staged && g + W < sd.groups) {
-      copy();
-      locate(g + 2 * W);
-    }
-    store();
-    g += W;
+    locate(g);
+    if (g < stop) copy();
+    locate(g + S);
     load();
+    while (g < stop) {
+      StreamSum<R> sum;
+      const uint32_t quads = group_slots(gr.shape) / 4;
+      uint32_t first = 0;  // slot that the sum goes on with
+      if constexpr (sizeof(R) == 8) {
+        const bool ahead = !kFar || (!fresh && !(gr.shape & (kGroupLate | kGroupSlow)));
+        if (ahead && !dead) {
+          dead = !st_wait([&]() { return counted(early.need); }, a.ctl, a.timeout_ns);
+          first = 4 * quads - early.late;
+          if (!dead) st_sum(sum, quad, words, StreamPiece<R>(buffer, gr), lane, early.skip, first);
+        }
+      }
+      // the levels before this group's
+      dead = dead || !st_wait([&]() { return counted(gr.need); }, a.ctl, a.timeout_ns);
+      const uint32_t n = group_tasks(gr.shape);
+      rel = gr.pos - sd.base;
+      if (!dead) {
+        if (kFar && (fresh || (gr.shape & (kGroupLate | kGroupSlow)))) {
+          const StreamPiece<R> all(a.data + 16ull * gr.data, gr);
+          const Word* base = a.word + sd.base;
+          if (gr.shape & kGroupSlow) {  // more far words than the buffer holds: index far + number
+            const uint32_t far = shape.ring + kStreamZero;
+            for (uint32_t j = 0; j < quads; ++j) {
+              R q[4];
+              StreamQuad<R> t;
+              t.load(all, j, lane);
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                const uint32_t x = all.idx()[StreamPiece<R>::slot(4 * j + c, lane)];
+                q[c] = x >= far ? st_ldq(base + all.far()[(x - far) * 32 + lane]) : words[x];
+              }
+              st_add(sum, j & 1u, t.w, q);
+            }
+          } else {
+            for (uint32_t f = 0; f < group_far(gr.shape); ++f) {
+              const uint32_t at = all.far()[f * 32 + lane];
+              far_words[f * 32u] = at != 0xffffffffu ? st_ldq(base + at) : R(0);
+            }
+          }
+        }
+        if (!kFar || !(gr.shape & kGroupSlow)) {
+          const StreamPiece<R> s(buffer, gr);
+          if constexpr (sizeof(R) == 8) {
+            st_sum(sum, quad, words, s, lane, max(first, early.skip), 4 * quads);
+          } else {
+            R q[kStreamQuads][4];
+#pragma unroll
+            for (uint32_t c = 0; c < kStreamQuads; ++c)
+              if (c < quads) st_words(quad[c], words, q[c]);
+#pragma unroll
+            for (uint32_t c = 0; c < kStreamQuads; ++c)
+              if (c < quads) st_add(sum, c & 1u, quad[c].w, q[c]);
+            for (uint32_t c = kStreamQuads; c < quads; ++c) {
+              StreamQuad<R> t;
+              t.load(s, c, lane);
+              R qc[4];
+              st_words(t, words, qc);
+              st_add(sum, c & 1u, t.w, qc);
+            }
+          }
+        }
+        in = sum.total();
+        if constexpr (sizeof(R) == 8)
+          out = (gr.shape & kGroupExt) ? st_solve(in, src, per, att, a.threshold, inv) : st_solve(in, att, a.threshold);
+        else
+          out = st_solve(in, src, per, att, a.threshold, inv);
+        mine = lane < n && (kAll || st_live(att));
+        uint32_t slot = ring_slot(shape, rel) + lane;
+        if (slot >= shape.ring) slot -= shape.ring;
+        if (lane < n) {
+          const R q = mine ? out : own;
+          words[slot] = q;
+          if constexpr (kPair) st_peer_word(peer_words + slot * (uint32_t)sizeof(R), q);
+        }
+        // a word that another group reads from memory is there before the barrier
+        if (kFar && (gr.shape & kGroupKeep)) store();
+      }
+      __syncwarp();
+      if (lane == 0) st_count_up(count);
+      fresh = false;
+      if (kFar && up_far) {  // solved by now: their levels lie before this group's
+        const Word* base = a.word + sd.base;
+#pragma unroll
+        for (int f = 0; f < (int)kStreamFar; ++f)
+          if constexpr (kPair) {
+            held[f] = up[f] != 0xffffffffu ? st_ldq(base + up[f]) : R(0);
+          } else if (up[f] != 0xffffffffu)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(st_smem(far_words + f * 32)),
+                         "l"(base + up[f]), "n"(sizeof(R))
+                         : "memory");  // the q leads a word
+        if constexpr (kPair) held_far = up_far;
+        up_far = 0;
+      }
+      if (staged && g + S < stop) {
+        copy();
+        locate(g + 2 * S);
+      }
+      store();
+      g += S;
+      load();
+    }
+    if constexpr (kPair) {
+      st_cluster_sync();  // both blocks are done with the ring, and have stored all words
+      if (post && me == 0 && threadIdx.x == 0)
+        asm volatile("fence.acq_rel.gpu;\n\tst.relaxed.gpu.global.u32 [%0], %1;" ::"l"(a.flags + post - 1), "r"(sweep)
+                     : "memory");
+    }
   }
   for (int o = 16; o > 0; o >>= 1) solved += __shfl_xor_sync(0xffffffffu, solved, o);
   if (lane == 0 && solved) {
@@ -834,7 +970,8 @@ __device__ __forceinline__ StreamSlot stream_slots(const StreamBuild& b, uint32_
   s.number = g - b.sgroup[k];
   s.end = b.seg[k + 1] - s.base;
   // when a warp takes this group up it has waited for the levels before its previous group's
-  s.early = s.number >= b.shape.warps ? b.seg[b.gseg[g - b.shape.warps]] - s.base : 0u;
+  const uint32_t turn = b.shape.warps * b.shape.blocks;
+  s.early = s.number >= turn ? b.seg[b.gseg[g - turn]] - s.base : 0u;
   s.far = 0;
   s.late = false;
   return s;

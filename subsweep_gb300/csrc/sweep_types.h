@@ -38,7 +38,13 @@ struct alignas(16) StreamGroup {
   uint32_t pos;    // first position
   uint32_t shape;  // tasks - 1 | slots per task << 5 | kGroup* flags | far words per task << 17
 };
+// Groups [begin, end) of a stream, walked by a pair of blocks; wait, post: 1 + the flag to wait
+// for before them or to set after them, or 0.
+struct StreamPart {
+  uint32_t stream, begin, end, wait, post;
+};
 constexpr uint32_t kStreamGroup = 32;
+constexpr int kPairWarps = 15;             // of each block of a pair that solve, and one more
 constexpr uint32_t kGroupExt = 1u << 12;   // a task has a periodic source or a cell with a source
 constexpr uint32_t kGroupLate = 1u << 13;  // a far word may be solved after the warp's previous group
 constexpr uint32_t kGroupSlow = 1u << 14;  // more far words than the buffer holds

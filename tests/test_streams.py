@@ -51,7 +51,7 @@ CASES = {
 
 
 def make(w, monkeypatch, env, precision="mixed"):
-    for k in ("SUBSWEEP_STREAMS", "SUBSWEEP_COMPACT", "SUBSWEEP_STREAM_WARPS", "SUBSWEEP_GRAPH"):
+    for k in ("SUBSWEEP_STREAMS", "SUBSWEEP_COMPACT", "SUBSWEEP_STREAM_WARPS", "SUBSWEEP_STREAM_PAIRS", "SUBSWEEP_GRAPH"):
         monkeypatch.delenv(k, raising=False)
     for k, v in env.items():
         monkeypatch.setenv(k, v)
@@ -81,6 +81,9 @@ def test_streams_equal_lockstep(case, monkeypatch):
         expected, tasks = results(s), s.stats()["tasks"]
     forms = [{"SUBSWEEP_COMPACT": c} for c in ("never", "always")]
     forms += [{"SUBSWEEP_STREAM_WARPS": str(n)} for n in (4, 8, 16)] + [{"SUBSWEEP_GRAPH": "1"}]
+    # pairs of blocks: a stream each where there are enough, or 7 pairs with streams cut between them
+    forms += [{"SUBSWEEP_STREAM_PAIRS": n} for n in ("1", "7")]
+    forms += [{"SUBSWEEP_STREAM_PAIRS": "7", "SUBSWEEP_GRAPH": "1"}]
     for env in forms:
         with make(w, monkeypatch, {"SUBSWEEP_STREAMS": "1", **env}) as s:
             for _ in range(steps):
@@ -99,6 +102,7 @@ def test_fp64_streams_equal_push(case, monkeypatch):
     forms.update({c: {"SUBSWEEP_STREAMS": "1", "SUBSWEEP_COMPACT": c} for c in ("never", "always")})
     forms.update({"4": {"SUBSWEEP_STREAMS": "1", "SUBSWEEP_STREAM_WARPS": "4"},
                   "graph": {"SUBSWEEP_STREAMS": "1", "SUBSWEEP_GRAPH": "1"}})
+    forms.update({"pairs " + n: {"SUBSWEEP_STREAMS": "1", "SUBSWEEP_STREAM_PAIRS": n} for n in ("1", "7")})
     for name, env in forms.items():
         with make(w, monkeypatch, env, "fp64") as s:
             for _ in range(steps):
