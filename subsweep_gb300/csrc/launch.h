@@ -133,6 +133,7 @@ struct DevicePtrs {
 // device scratch of the streams' build (StreamBuild)
 struct StreamScratch {
   uint32_t *gseg, *sbase, *sgroup;
+  uint32_t* recip;  // FP64: per face, the face across it that leads back
 };
 
 struct PrecisionOps {
@@ -146,8 +147,9 @@ struct PrecisionOps {
   cudaError_t (*sweep)(const DevicePtrs&, int level, cudaStream_t);
   cudaError_t (*occupancy_levels)(int* blocks_per_sm);
   cudaError_t (*sweep_levels)(const DevicePtrs&, int level, cudaStream_t);
-  cudaError_t (*kahn_round)(const DevicePtrs&, uint32_t begin, uint32_t end, uint16_t* task_level, uint32_t round,
-                            cudaStream_t);
+  // Kahn rounds [round, round + rounds) of the schedule, over the bounds on the device
+  cudaError_t (*kahn_rounds)(const DevicePtrs&, uint32_t* bounds, uint32_t* done, uint16_t* task_level, uint32_t round,
+                             uint32_t rounds, cudaStream_t);
   cudaError_t (*schedule_seed)(const DevicePtrs&, cudaStream_t);
   cudaError_t (*fold_periodic)(const DevicePtrs&, cudaStream_t);
   cudaError_t (*chemistry)(const DevicePtrs&, int level, cudaStream_t);

@@ -370,10 +370,14 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep(SweepArgs<R> a) {
 
 // One Kahn round: release the downwind dependents of the tasks order[begin, end)
 // (all cells active), appending the tasks that become free at ctl->tail and recording
-// their level (round + 1) in task_level.
+// their level (round + 1) in task_level.  The rounds' bounds stay on the device, begin =
+// bounds[round] and end = bounds[round + 1]; the last block to finish writes the end of the
+// next one, so the host launches many rounds at once (with a wait for every round, 100 us,
+// the rounds took 0.21 s at 128^3 x 84; so 0.02 s).
 template <typename R>
-__global__ void k_kahn_round(SweepArgs<R> a, uint32_t* order, uint32_t begin, uint32_t end,
+__global__ void k_kahn_round(SweepArgs<R> a, uint32_t* order, uint32_t* bounds, uint32_t* done,
                              unsigned long long capacity, uint16_t* task_level, uint32_t round) {
+  const uint32_t begin = bounds[round], end = bounds[round + 1];
   const uint32_t nthreads = gridDim.x * blockDim.x;
   const uint32_t span = end - begin;
   const uint32_t iters = (span + nthreads - 1) / nthreads;
@@ -413,6 +417,14 @@ __global__ void k_kahn_round(SweepArgs<R> a, uint32_t* order, uint32_t begin, ui
         }
       }
       enqueue(ready, tn, a.ctl, order, capacity);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(done, 1u) == gridDim.x - 1) {
+      bounds[round + 2] = (uint32_t)ld_relaxed64(&a.ctl->tail);
+      *done = 0u;
     }
   }
 }

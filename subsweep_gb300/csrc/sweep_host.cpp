@@ -550,18 +550,33 @@ sw_status build_schedule(sw_handle* h) {
       up.resize((size_t)h->Np * q.D);
       SW_CUDA(h, cudaMemcpy(up.data(), p.counters, up.size(), cudaMemcpyDeviceToHost), "read upwind counts");
     }
-    uint32_t begin = 0;
-    uint32_t round = 0;
-    while (tail > begin) {
-      const uint32_t end = (uint32_t)tail;
-      lvl.push_back(end);
-      if (round + 1 >= 0xffffu) return h->fail(SW_ERR_UNSUPPORTED, "dependency graph deeper than 65534 levels");
-      SW_CUDA(h, h->ops->kahn_round(q, begin, end, task_level, round, h->stream), "schedule round kernel");
-      ++round;
-      SW_CUDA(h, cudaMemcpyAsync(&tail, &p.ctl->tail, sizeof(tail), cudaMemcpyDeviceToHost, h->stream), "read tail");
+    // the rounds, kRounds at a time (those after the last one find nothing to do)
+    constexpr uint32_t kRounds = 32, kMaxRounds = 0xffffu;
+    DeviceScratch bounds_scratch;
+    SW_CUDA(h, cudaMalloc(&bounds_scratch.ptr, (kMaxRounds + kRounds + 2) * sizeof(uint32_t)), "schedule scratch");
+    uint32_t* bounds = static_cast<uint32_t*>(bounds_scratch.ptr) + 1;  // behind the blocks' count
+    const uint32_t first[3] = {0u, 0u, (uint32_t)tail};
+    SW_CUDA(h, cudaMemcpy(bounds - 1, first, sizeof(first), cudaMemcpyHostToDevice), "schedule scratch");
+    uint32_t end = (uint32_t)tail;
+    if (end > 0) lvl.push_back(end);
+    for (uint32_t round = 0; end > 0;) {
+      uint32_t ends[kRounds];
+      SW_CUDA(h, h->ops->kahn_rounds(q, bounds, bounds - 1, task_level, round, kRounds, h->stream),
+              "schedule round kernel");
+      SW_CUDA(h, cudaMemcpyAsync(ends, bounds + round + 2, sizeof(ends), cudaMemcpyDeviceToHost, h->stream),
+              "read bounds");
       SW_CUDA(h, cudaStreamSynchronize(h->stream), "schedule round");
-      begin = end;
+      bool more = true;
+      for (uint32_t k = 0; k < kRounds && more; ++k) {
+        more = ends[k] > end;
+        if (more) lvl.push_back(end = ends[k]);
+      }
+      if (!more) break;
+      round += kRounds;
+      if (round >= kMaxRounds) return h->fail(SW_ERR_UNSUPPORTED, "dependency graph deeper than 65534 levels");
     }
+    tail = end;
+    if (lvl.size() - 1 >= kMaxRounds) return h->fail(SW_ERR_UNSUPPORTED, "dependency graph deeper than 65534 levels");
     uint32_t err = 0;
     SW_CUDA(h, cudaMemcpy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
     if (tail != total || err != 0) {
@@ -874,6 +889,7 @@ sw_status build_streams(sw_handle* h) {
   SW_CUDA(h, scratch.get((void**)&b.gseg, groups.size() * 4, nullptr), "stream scratch");
   SW_CUDA(h, scratch.get((void**)&b.sbase, sbase.size() * 4, sbase.data()), "stream scratch");
   SW_CUDA(h, scratch.get((void**)&b.sgroup, sgroup.size() * 4, sgroup.data()), "stream scratch");
+  if (rb == 8) SW_CUDA(h, scratch.get((void**)&b.recip, (size_t)h->E * 4, nullptr), "stream scratch");
   swk::StreamDesc* d_streams = nullptr;
   swk::StreamGroup* d_groups = nullptr;
   uint32_t* d_cell_sweep = nullptr;
@@ -910,8 +926,11 @@ sw_status build_streams(sw_handle* h) {
   shape[5] = pairs ? 2u : 1u;
   bool far = false;
   int64_t late = 0, slow = 0;
+  // room for far words is taken from the ring only if there are any: looked for with it where the
+  // ring is shorter than the longest stream, and without it again if there are none
+  const bool whole = words_for(room, 0) >= (int64_t)longest;
   for (int pass = 0; pass < 2; ++pass) {
-    shape[2] = pass == 0 ? 0u : swk::kStreamFar;
+    shape[2] = (pass == 0) == whole ? 0u : swk::kStreamFar;
     shape[4] = buffer;
     shape[0] = (uint32_t)std::min<int64_t>(words_for(room, shape[2]), longest);
     shape[1] = (uint32_t)((1ull << 32) / shape[0]) + 1u;
@@ -927,7 +946,7 @@ sw_status build_streams(sw_handle* h) {
       late += (g.shape & swk::kGroupLate) != 0;
       slow += (g.shape & swk::kGroupSlow) != 0;
     }
-    if (!far) break;
+    if (far == (shape[2] != 0u)) break;
   }
   if (pairs) {
     int resident = 0;

@@ -336,20 +336,21 @@ cudaError_t push_records(const DevicePtrs& p, int phase, unsigned long long* scr
 #endif
 
 #if !SWK_PULL
-swk::FacePull face_pull(const DevicePtrs& p, const double* total) {
-  return {sweep_args(p, 0), p.order, p.pos_of_task, total};
+swk::FacePull face_pull(const DevicePtrs& p, const double* total, uint32_t* recip) {
+  return {sweep_args(p, 0), p.order, p.pos_of_task, total, recip};
 }
 
 // FP64 direction streams (the tasks' totals in `pending` until the pieces are written)
 cudaError_t stream_build64(const DevicePtrs& p, int phase, const StreamScratch& b, cudaStream_t s) {
   const uint32_t total = (uint32_t)(p.num_cells * p.D);
   double* totals = static_cast<double*>(p.pending);
-  const swk::FacePull f = face_pull(p, totals);
+  const swk::FacePull f = face_pull(p, totals, b.recip);
   if (phase == 0) {
     swk::k_invert_order<<<grid_for(total, 256), 256, 0, s>>>(p.order, total, p.pos_of_task);
     swk::k_stream_group_segs<<<grid_for((int64_t)p.num_sched_levels * 32, 256), 256, 0, s>>>(
         p.seg_group, p.num_sched_levels, b.gseg);
     swk::k_task_totals<<<grid_for(total, 256), 256, 0, s>>>(f, totals);
+    swk::k_reciprocal_faces<<<grid_for(p.num_cells, 256), 256, 0, s>>>(f, b.recip);
     return cudaGetLastError();
   }
   if (phase >= 3) {
@@ -380,12 +381,13 @@ cudaError_t schedule_seed(const DevicePtrs& p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t kahn_round(const DevicePtrs& p, uint32_t begin, uint32_t end, uint16_t* task_level, uint32_t round,
-                       cudaStream_t s) {
+cudaError_t kahn_rounds(const DevicePtrs& p, uint32_t* bounds, uint32_t* done, uint16_t* task_level, uint32_t round,
+                        uint32_t rounds, cudaStream_t s) {
   swk::SweepArgs<R> a = sweep_args(p, 0);
   const unsigned long long capacity = (unsigned long long)p.D * p.Np;
-  swk::k_kahn_round<R><<<grid_for((int64_t)(end - begin), 256), 256, 0, s>>>(a, p.order, begin, end, capacity,
-                                                                              task_level, round);
+  const int grid = std::min(2 * p.num_sms, grid_for(p.num_cells * p.D / 16, 256));
+  for (uint32_t r = round; r < round + rounds; ++r)
+    swk::k_kahn_round<R><<<grid, 256, 0, s>>>(a, p.order, bounds, done, capacity, task_level, r);
   return cudaGetLastError();
 }
 
@@ -773,14 +775,14 @@ cudaError_t export_rates(const DevicePtrs& p, int which, uint32_t, double* out, 
 #if SWK_PULL
 extern const PrecisionOps SWK_OPS = {
     SWK_NAME,       (int)sizeof(R), true,       occupancy,     attenuation, init_counts, sweep,
-    occupancy_pull, sweep_pull,     kahn_round, schedule_seed, fold_pull,   chemistry,   photon_rate,
+    occupancy_pull, sweep_pull,     kahn_rounds, schedule_seed, fold_pull,   chemistry,   photon_rate,
     export_rates,   records,        cell_rates, SWK_CARRY != 0,
     (int)(sizeof(kTuneVariants) / sizeof(int)), kTuneVariants, nullptr, stream_build, stream_pairs, nullptr,
 };
 #else
 extern const PrecisionOps SWK_OPS = {
     SWK_NAME,         (int)sizeof(R), false,      occupancy,     attenuation,   init_counts, sweep,
-    occupancy_levels, sweep_levels,   kahn_round, schedule_seed, fold_periodic, chemistry,   photon_rate,
+    occupancy_levels, sweep_levels,   kahn_rounds, schedule_seed, fold_periodic, chemistry,   photon_rate,
     export_rates,     nullptr,        cell_rates, SWK_CARRY != 0,
     0, nullptr,       push_records, stream_build64, stream_pairs, refresh,
 };

@@ -18,7 +18,8 @@ struct FacePull {
   SweepArgs<double> a;
   const uint32_t* order;
   const uint32_t* pos_of_task;
-  const double* total;  // per task
+  const double* total;    // per task
+  const uint32_t* recip;  // per face (k_reciprocal_faces)
 };
 
 __device__ __forceinline__ double task_total(const SweepArgs<double>& a, uint32_t c, uint32_t d) {
@@ -44,26 +45,37 @@ __device__ __forceinline__ int pull_sign(const SweepArgs<double>& a, uint32_t f,
   return face_sign(s, a.geo64 + f, a.dir64[3 * d], a.dir64[3 * d + 1], a.dir64[3 * d + 2], a.guard);
 }
 
-// The fraction that the cell across upwind face f of cell c hands to c in direction d: of its
-// face towards c with the negated normal (the k-th of equal ones, as f is the k-th of its equals).
-// Negative if there is none.
-__device__ __forceinline__ double pull_fraction(const FacePull& p, uint32_t c, uint32_t f, uint32_t d) {
+// Of every face of a cell c towards a cell n: the face of n towards c of the same kind with the
+// negated normal (the k-th of equal ones, as the face is the k-th of its equals), or kNbrMask.
+static __global__ void k_reciprocal_faces(FacePull p, uint32_t* recip) {
   const SweepArgs<double>& a = p.a;
-  const uint32_t nb = a.nbr[f], n = nb & kNbrMask, back = c | (nb & ~kNbrMask);
-  const Geo64 g = a.geo64[f];
-  int k = 0;
-  for (uint32_t e = a.off[c]; e < f; ++e)
-    if (a.nbr[e] == nb && a.geo64[e].x == g.x && a.geo64[e].y == g.y && a.geo64[e].z == g.z) ++k;
-  const double dx = a.dir64[3 * d], dy = a.dir64[3 * d + 1], dz = a.dir64[3 * d + 2];
-  const float fx = a.dir32[3 * d], fy = a.dir32[3 * d + 1], fz = a.dir32[3 * d + 2];
-  for (uint32_t q = a.off[n]; q < a.off[n + 1]; ++q) {
-    if (a.nbr[q] != back) continue;
-    if (a.geo64[q].x != -g.x || a.geo64[q].y != -g.y || a.geo64[q].z != -g.z || k-- > 0) continue;
-    const double eff = push_eff(a, q, dx, dy, dz, fx, fy, fz);
-    if (!(eff > 0.0)) return -1.0;
-    return eff / p.total[(size_t)d * a.Np + n];
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < a.N; c += gridDim.x * blockDim.x) {
+    for (uint32_t f = a.off[c]; f < a.off[c + 1]; ++f) {
+      const uint32_t nb = a.nbr[f], n = nb & kNbrMask, back = c | (nb & ~kNbrMask);
+      uint32_t found = kNbrMask;
+      if ((nb >> kKindShift) != kKindBoundary) {
+        const Geo64 g = a.geo64[f];
+        int k = 0;
+        for (uint32_t e = a.off[c]; e < f; ++e)
+          if (a.nbr[e] == nb && a.geo64[e].x == g.x && a.geo64[e].y == g.y && a.geo64[e].z == g.z) ++k;
+        for (uint32_t q = a.off[n]; q < a.off[n + 1] && found == kNbrMask; ++q)
+          if (a.nbr[q] == back && a.geo64[q].x == -g.x && a.geo64[q].y == -g.y && a.geo64[q].z == -g.z && k-- == 0)
+            found = q;
+      }
+      recip[f] = found;
+    }
   }
-  return -1.0;
+}
+
+// The fraction that the cell across upwind face f hands on through it in direction d; negative if
+// its reciprocal face is not downwind or there is none.
+__device__ __forceinline__ double pull_fraction(const FacePull& p, uint32_t f, uint32_t d) {
+  const SweepArgs<double>& a = p.a;
+  const uint32_t q = p.recip[f];
+  if (q == kNbrMask) return -1.0;
+  const double eff = push_eff(a, q, a.dir64[3 * d], a.dir64[3 * d + 1], a.dir64[3 * d + 2], a.dir32[3 * d],
+                              a.dir32[3 * d + 1], a.dir32[3 * d + 2]);
+  return eff > 0.0 ? eff / p.total[(size_t)d * a.Np + (a.nbr[f] & kNbrMask)] : -1.0;
 }
 
 // Finds the flags and far words of every group (b.data null), or writes the groups' pieces, one
@@ -101,7 +113,7 @@ static __global__ void k_stream_slots64(FacePull p, StreamBuild b) {
         if (sign >= 0) continue;
         if (kind == kKindPeriodic) {
           ext = true;
-          if (!b.data || pull_fraction(p, c, f, d) >= 0.0) ++found;
+          if (!b.data || pull_fraction(p, f, d) >= 0.0) ++found;
           continue;
         }
         const uint32_t u = p.pos_of_task[d * a.Np + (nb & kNbrMask)] - s.base;
@@ -125,7 +137,7 @@ static __global__ void k_stream_slots64(FacePull p, StreamBuild b) {
       const uint32_t f0 = s.far, x = stream_slot(b, s, gr.shape, lane, up[i]), j = padded - ups + i;
       if (up[i] >= previous) ++late;
       if (b.data) {
-        const double frac = pull_fraction(p, c, a.off[c] + face[i], d);
+        const double frac = pull_fraction(p, a.off[c] + face[i], d);
         if (frac >= 0.0) ++found;
         idx[piece.slot(j, lane)] = (uint16_t)x;
         w[piece.wslot(j, lane)] = frac;
@@ -191,7 +203,7 @@ static __global__ void k_fold_build64(FacePull p, const uint32_t* cells, uint32_
       const uint32_t nb = a.nbr[f];
       if ((nb >> kKindShift) != kKindPeriodic || pull_sign(a, f, d) >= 0) continue;
       if (slots)
-        slots[off[e] + n] = {p.pos_of_task[(size_t)d * a.Np + (nb & kNbrMask)], 0u, pull_fraction(p, c, f, d)};
+        slots[off[e] + n] = {p.pos_of_task[(size_t)d * a.Np + (nb & kNbrMask)], 0u, pull_fraction(p, f, d)};
       ++n;
     }
     if (!slots) cnt[e] = (uint8_t)n;
