@@ -469,7 +469,9 @@ static void stream_order(const uint16_t* level, const uint8_t* up, uint32_t Np, 
 // directions 64^3 0.95 and 0.87, but 101^3 1.87 and 2.98: sixteen blocks cannot keep up with the
 // whole device where levels are wide.  FP64: 84 directions 16^3 0.97 and 0.18, 24^3 1.61 and 0.31,
 // 32^3 2.10 and 0.46, 64^3 5.4 and 2.0, 96^3 13.8 and 7.9; 16 directions 64^3 4.8 and 1.8, 101^3
-// 7.8 and 6.0.
+// 7.8 and 6.0; 84 directions 128^3 34 and 17, 160^3 66 and 34.  Where a level is wide, the ring
+// holds few levels and many words come from memory: mixed path 160^3 (1800 tasks a level) 20.2
+// and 15.8, 192^3 (2200) 35 and 34, 256^3 (3400) 83 and 114; hence the limit on the width.
 static bool streams_pay(const std::vector<uint32_t>& parts, uint64_t tasks, size_t levels, bool mixed) {
   uint32_t longest = 0;
   for (size_t k = 1; k < parts.size(); ++k) longest = std::max(longest, parts[k] - parts[k - 1]);
@@ -478,7 +480,7 @@ static bool streams_pay(const std::vector<uint32_t>& parts, uint64_t tasks, size
     if (longest > 480.0 * (double)levels) task = 5.9 * std::max(1.0, (double)tasks / longest / 76.0);  // pairs
     return task * longest < 4000.0 * (double)levels + (double)tasks / 12.0;
   }
-  return 3.6 * longest < 850.0 * (double)levels + (double)tasks / 17.0;
+  return longest < 2600.0 * (double)levels && 3.6 * longest < 850.0 * (double)levels + (double)tasks / 17.0;
 }
 
 // Compact state (mixed path): task spaces hold fewer than kSpaceTasks tasks each.  The
@@ -972,11 +974,11 @@ sw_status build_streams(sw_handle* h) {
   }
   uint64_t at = 0;
   for (swk::StreamGroup& g : groups) {
-    g.data = (uint32_t)(at / 16);
-    at += piece_bytes(g.shape, rb);
+    g.data = (uint32_t)(at / swk::kStreamUnit);
+    at += (piece_bytes(g.shape, rb) + swk::kStreamUnit - 1) / swk::kStreamUnit * swk::kStreamUnit;
   }
-  groups.push_back({0u, (uint32_t)(at / 16), 0u, 0u});  // where the last piece ends
-  if (at / 16 > 0xffffffffull) {  // past the pieces' 32-bit offsets: the levelled schedule
+  groups.push_back({0u, (uint32_t)(at / swk::kStreamUnit), 0u, 0u});  // where the last piece ends
+  if (at / swk::kStreamUnit > 0xffffffffull) {  // past the pieces' 32-bit offsets: the levelled schedule
     h->want_streams = false;
     return SW_OK;
   }

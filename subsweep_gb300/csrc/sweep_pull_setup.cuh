@@ -155,7 +155,7 @@ __global__ void k_stream_slots(PullArgs a, StreamBuild b) {
   const float inv_np = 1.0f / (float)a.Np;
   for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / 32; g < b.num_groups; g += gridDim.x * blockDim.x / 32) {
     const StreamGroup gr = b.groups[g];
-    const StreamPiece<float> piece(b.data + 16ull * gr.data, gr);
+    const StreamPiece<float> piece(b.data + kStreamUnit * gr.data, gr);
     const uint32_t n = group_tasks(gr.shape), padded = group_slots(gr.shape);
     StreamSlot s = stream_slots(b, g);
     bool ext = false;
@@ -210,7 +210,7 @@ __global__ void k_stream_slots(PullArgs a, StreamBuild b) {
         const_cast<float*>(piece.src())[lane] = source;
       }
     }
-    if (b.data && lane == 0) *reinterpret_cast<uint4*>(b.data + 16ull * gr.data) = reinterpret_cast<const uint4*>(b.groups)[g];
+    if (b.data && lane == 0) *reinterpret_cast<uint4*>(b.data + kStreamUnit * gr.data) = reinterpret_cast<const uint4*>(b.groups)[g];
     const uint32_t flags = stream_flags(ext, s, b.shape.far);
     if (!b.data) {
       if (lane == 0) atomicOr(&b.groups[g].shape, flags);

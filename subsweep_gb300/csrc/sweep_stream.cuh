@@ -425,8 +425,8 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
     __syncwarp();
     if (lane == 0) {
       // the far list, a piece's last part, need not fit
-      const uint32_t bytes = min((end - next.data) * 16u, shape.buffer);
-      const unsigned char* src = a.data + 16ull * next.data;
+      const uint32_t bytes = min((end - next.data) * (uint32_t)kStreamUnit, shape.buffer);
+      const unsigned char* src = a.data + kStreamUnit * next.data;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(st_smem(bar)), "r"(bytes) : "memory");
       if (a.evict_first)
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
                          st_smem(buffer)),
                      "l"(src), "r"(bytes), "r"(st_smem(bar))
                      : "memory");
-      if (16ull * end + kStreamAhead <= a.bytes)
+      if (kStreamUnit * end + kStreamAhead <= a.bytes)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + kStreamAhead), "r"(bytes) : "memory");
     }
   };
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
       if (kFar) {  // the positions of the next group's far words
         up_far = (next.shape & (kGroupLate | kGroupSlow)) ? 0u : group_far(next.shape);
         if (up_far) {
-          const StreamPiece<R> t(a.data + 16ull * next.data, next);
+          const StreamPiece<R> t(a.data + kStreamUnit * next.data, next);
 #pragma unroll
           for (int f = 0; f < (int)kStreamFar; ++f)
             up[f] = (uint32_t)f < up_far ? __ldcs(t.far() + f * 32 + lane) : 0xffffffffu;
@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
       rel = gr.pos - sd.base;
       if (!dead) {
         if (kFar && (fresh || (gr.shape & (kGroupLate | kGroupSlow)))) {
-          const StreamPiece<R> all(a.data + 16ull * gr.data, gr);
+          const StreamPiece<R> all(a.data + kStreamUnit * gr.data, gr);
           const Word* base = a.word + sd.base;
           if (gr.shape & kGroupSlow) {  // more far words than the buffer holds: index far + number
             const uint32_t far = shape.ring + kStreamZero;
@@ -799,7 +799,7 @@ __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(co
       gr = a.groups[g];
       const uint32_t id = a.order[p];
       att = a.cell_att[id % a.Np];
-      const StreamPiece<R> s(a.data + 16ull * gr.data, gr);
+      const StreamPiece<R> s(a.data + kStreamUnit * gr.data, gr);
       quads = s.quads;
       if (gr.shape & kGroupExt) {
         per = a.periodic[id];
@@ -822,7 +822,7 @@ __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(co
       for (uint32_t c = 0; c < kStreamQuads; ++c)
         if (c < quads) add(c & 1u, w[c], up[c]);
       if (quads > kStreamQuads) {
-        const StreamPiece<R> s(a.data + 16ull * gr.data, gr);
+        const StreamPiece<R> s(a.data + kStreamUnit * gr.data, gr);
         for (uint32_t c = kStreamQuads; c < quads; ++c) {
           StreamWeights<R> w4;
           uint32_t up4[4];
@@ -868,7 +868,7 @@ __global__ void k_stream_gather(const StreamGroup* groups, uint32_t ngroups, uns
   const float inv_np = 1.0f / (float)Np;
   for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / 32; g < ngroups; g += gridDim.x * blockDim.x / 32) {
     const StreamGroup gr = groups[g];
-    const StreamPiece<R> s(data + 16ull * gr.data, gr);
+    const StreamPiece<R> s(data + kStreamUnit * gr.data, gr);
     if (lane >= group_tasks(gr.shape)) continue;
     const uint32_t t = order[gr.pos + lane];
     // the cell: t modulo Np (the FP32 quotient is off by one at most)
@@ -907,7 +907,7 @@ __global__ void k_stream_refresh(StreamArgs<R> a, const uint8_t* stale) {
   for (uint32_t number = blockIdx.y * (blockDim.x / 32) + threadIdx.x / 32; number < sd.groups; number += warps) {
     const StreamGroup gr = a.groups[sd.group0 + number];
     if (lane >= group_tasks(gr.shape) || stale[a.order[gr.pos + lane] % a.Np] == 0) continue;
-    const StreamPiece<R> s(a.data + 16ull * gr.data, gr);
+    const StreamPiece<R> s(a.data + kStreamUnit * gr.data, gr);
     const uint32_t rel = gr.pos - sd.base + lane;
     R sum = R(0);
     for (uint32_t j = 0; j < s.quads; ++j) {

@@ -87,7 +87,7 @@ static __global__ void k_stream_slots64(FacePull p, StreamBuild b) {
   unsigned long long given = 0, found = 0;
   for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / 32; g < b.num_groups; g += gridDim.x * blockDim.x / 32) {
     const StreamGroup gr = b.groups[g];
-    const StreamPiece<double> piece(b.data + 16ull * gr.data, gr);
+    const StreamPiece<double> piece(b.data + kStreamUnit * gr.data, gr);
     const uint32_t n = group_tasks(gr.shape), padded = group_slots(gr.shape);
     StreamSlot s = stream_slots(b, g);
     bool ext = false;
@@ -158,7 +158,7 @@ static __global__ void k_stream_slots64(FacePull p, StreamBuild b) {
       const uint32_t most = __reduce_max_sync(0xffffffffu, ups);
       late = __reduce_max_sync(0xffffffffu, late);
       if (lane == 0) {
-        unsigned char* at = b.data + 16ull * gr.data;
+        unsigned char* at = b.data + kStreamUnit * gr.data;
         *reinterpret_cast<uint4*>(at) = reinterpret_cast<const uint4*>(b.groups)[g];
         const uint32_t need = previous ? b.seg_group[k - 1] - b.sgroup[k] : 0u;
         *reinterpret_cast<StreamEarly*>(at + sizeof(StreamGroup)) = {need, padded - most, late, 0u};

@@ -34,7 +34,7 @@ struct StreamDesc {
 };
 struct alignas(16) StreamGroup {
   uint32_t need;   // groups of the stream in earlier levels: solved before this one
-  uint32_t data;   // its piece of data, in units of 16 bytes
+  uint32_t data;   // its piece of data, in units of kStreamUnit bytes
   uint32_t pos;    // first position
   uint32_t shape;  // tasks - 1 | slots per task << 5 | kGroup* flags | far words per task << 17
 };
@@ -43,6 +43,7 @@ struct alignas(16) StreamGroup {
 struct StreamPart {
   uint32_t stream, begin, end, wait, post;
 };
+constexpr unsigned long long kStreamUnit = 64;  // pieces of up to 256 GB in 32 bits
 constexpr uint32_t kStreamGroup = 32;
 constexpr int kPairWarps = 15;             // of each block of a pair that solve, and one more
 constexpr uint32_t kGroupExt = 1u << 12;   // a task has a periodic source or a cell with a source
