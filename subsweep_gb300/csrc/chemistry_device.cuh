@@ -179,8 +179,6 @@ struct ChemSolver {
   double m, photo, heat_step, cool_step;
   Fits fits;
   double fits_t;  // temperature of `fits`
-  // the last accepted attempt
-  double last_dt, rel_t, rel_x;
 
   __device__ void prepare(double timestep) {
     nh = density / Units::kProtonMass;
@@ -196,6 +194,13 @@ struct ChemSolver {
   __device__ __forceinline__ double n_ionized() const { return nh * x; }
   __device__ __forceinline__ double n_neutral() const { return nh * neutral(); }
 
+  // collisional, recombination and free-free, and Compton cooling per volume
+  __device__ __forceinline__ void sum_cooling(double neutral_rate, double ion_rate, double ne, double nhn, double dt,
+                                              double& sum) const {
+    constexpr double u = Units::kErgsCentimetersCubedPerS;
+    sum = ne * ((neutral_rate * nhn + ion_rate * ne) * u + compton_cell * dt);
+  }
+
   // cooling_rate 275-287 and cooling_rate_derivative 289-302 at the current state:
   // collisional ionization / excitation cooling (237-253), case B recombination cooling
   // (196-216), bremsstrahlung and Compton cooling (265-273).  Mixed path: from the FP32 fits;
@@ -203,18 +208,14 @@ struct ChemSolver {
   __device__ void cooling(const Fits32& f, double& lambda_c, double& dlambda_c) const {
     const double ne = n_ionized();
     const double nhn = n_neutral();
-    const double u = Units::kErgsCentimetersCubedPerS;
-    const double compton = compton_cell * (temperature - xx_cell);
-    const double coll = ((double)f.exc + 1.27e-21 * (double)f.fit) * u * ne * nhn;
-    const double dcoll = ((double)f.dexc + 1.27e-21 * (double)f.fitd) * u * ne * nhn;
-    lambda_c = coll + ((double)f.recc + (double)f.brems) * u * ne * ne + compton * ne;
-    dlambda_c = dcoll + ((double)f.drecc + (double)f.dbrems) * u * ne * ne + compton_cell * ne;
+    sum_cooling((double)f.exc + 1.27e-21 * (double)f.fit, (double)f.recc + (double)f.brems, ne, nhn, temperature - xx_cell,
+                lambda_c);
+    sum_cooling((double)f.dexc + 1.27e-21 * (double)f.fitd, (double)f.drecc + (double)f.dbrems, ne, nhn, 1.0, dlambda_c);
   }
   __device__ void cooling(const Fits64& f, double& lambda_c, double& dlambda_c) const {
     const double t = f.t;
     const double ne = n_ionized();
     const double nhn = n_neutral();
-    const double u = Units::kErgsCentimetersCubedPerS;
     // excitation cooling and its derivative
     const double c3 = 1.0 / 1e5, c2e = 118348.0;
     const double e_exc = 7.5e-19 * exp(-c2e / t);
@@ -231,9 +232,8 @@ struct ChemSolver {
     const double drecomb = power * ((1.0 - c2r + (1.0 - c2r + c3r * c4r) * q) / (1.0 + q));
     const double brems = 1.42e-27 * f.sq;
     const double dbrems = (0.5 * 1.42e-27) * (f.sq * f.inv_t);
-    const double compton = compton_cell * (temperature - xx_cell);
-    lambda_c = (exc + 1.27e-21 * f.fit) * u * ne * nhn + (recomb + brems) * u * ne * ne + compton * ne;
-    dlambda_c = (dexc + 1.27e-21 * f.fitd) * u * ne * nhn + (drecomb + dbrems) * u * ne * ne + compton_cell * ne;
+    sum_cooling(exc + 1.27e-21 * f.fit, recomb + brems, ne, nhn, temperature - xx_cell, lambda_c);
+    sum_cooling(dexc + 1.27e-21 * f.fitd, drecomb + dbrems, ne, nhn, 1.0, dlambda_c);
   }
 
   // case B recombination rate and its derivative, 175-194
@@ -287,16 +287,16 @@ struct ChemSolver {
     const double ne = n_ionized();
     double alpha, dalpha;
     recombination(f, alpha, dalpha);
-    const double beta = (5.85e-11 * (double)f.fit) * Units::kCentimetersCubedPerS;
-    const double dbeta = (5.85e-11 * (double)f.fitd) * Units::kCentimetersCubedPerS;
+    constexpr double kBeta = 5.85e-11 * Units::kCentimetersCubedPerS;
+    const double beta = kBeta * (double)f.fit;
+    const double dbeta = kBeta * (double)f.fitd;
     const double c = beta * ne + photo;
-    const double d = alpha * ne;
-    const double rhsc = ne * t * m * dbeta;
-    const double dcdx = nh * beta - rhsc;
-    const double rhsd = ne * t * m * dalpha;
-    const double dddx = nh * alpha - rhsd;
-    const double j = dcdx - (c + d) - x * (dcdx + dddx);
-    return timestep * (c - x * (c + d)) / (1.0 - j * timestep);
+    const double cd = c + alpha * ne;
+    const double w = ne * t * m;
+    const double dcdx = nh * beta - w * dbeta;
+    const double both = nh * (beta + alpha) - w * (dbeta + dalpha);  // dcdx + dddx
+    const double j = (dcdx - cd) - x * both;
+    return timestep * (c - x * cd) / (1.0 - j * timestep);
   }
 
   // 356-369 with Rust f64::clamp semantics (asserts min <= max: flagged here).
@@ -314,40 +314,19 @@ struct ChemSolver {
     if (has_floor && temperature < floor_t) temperature = floor_t;
   }
 
-  // relative change of update() 444-461
+  // relative change of update() 444-461, and whether it is small enough (a change that is no
+  // number, or of a value of 0, is not)
   __device__ __forceinline__ static double relative(double value, double change) {
     return fmin(fabs(change / value), 1.0 / DBL_EPSILON);
   }
-
-  // try_timestep_update 371-392; the state stays as it is unless both changes are accepted
-  // (temperature_change 304-310)
-  __device__ bool try_update(double timestep, double safety) {
-    const double tc = heat_step * timestep / (1.0 - cool_step * timestep);
-    const double change_t = relative(temperature, tc);
-    if (change_t > safety) return false;
-    const double t = temperature + tc;
-    Fits f;
-    set_fits(f, t);
-    const double xc = ionized_fraction_change(timestep, f, t);
-    const double change_x = relative(x, xc);
-    if (change_x > safety) return false;
-    temperature = t;
-    fits = f;
-    fits_t = t;
-    x += xc;
-    if (kCarryNeutral) {
-      y -= xc;
-      // keep the smaller fraction exact and derive the other from it
-      if (x < 0.5) y = 1.0 - x; else x = 1.0 - y;
-    }
-    clamp();
-    last_dt = timestep;
-    rel_t = change_t;
-    rel_x = change_x;
-    return true;
+  __device__ __forceinline__ static bool small(double value, double change, double safety) {
+    return fabs(change) < safety * fabs(value);
   }
 
-  // perform_timestep 426-441 with perform_timestep_internal 394-424 unrolled.
+  // perform_timestep 426-441 with perform_timestep_internal 394-424 unrolled, and the attempts
+  // (try_timestep_update 371-392, temperature_change 304-310): the state changes when both changes
+  // of an attempt are small enough.  The temperature's test takes a few operations, so a lane
+  // repeats it until it holds before the warp goes on to the fits at the new temperature.
   __device__ Timescale perform_timestep(double timestep, double safety, bool& failed,
                                         uint32_t& attempts) {
     uint64_t pend_lo = 0, pend_hi = 0;  // pending second halves at depths 1..127
@@ -355,18 +334,38 @@ struct ChemSolver {
     clamp();
     begin(timestep);
     while (true) {
-      if (depth > kChemMaxDepth) {
-        failed = true;
-        return Timescale{timestep / 10.0, kProcTemperature};
+      double sub, tc;
+      while (true) {
+        if (depth > kChemMaxDepth) {
+          failed = true;
+          return Timescale{timestep / 10.0, kProcTemperature};
+        }
+        // timestep / 2^depth, exact
+        sub = timestep * __longlong_as_double((long long)(1023 - depth) << 52);
+        ++attempts;
+        tc = heat_step * sub / (1.0 - cool_step * sub);
+        if (small(temperature, tc, safety)) break;
+        reject(depth, pend_lo, pend_hi);
       }
-      // timestep / 2^depth, exact
-      const double sub = timestep * __longlong_as_double((long long)(1023 - depth) << 52);
-      ++attempts;
-      if (!try_update(sub, safety)) {
-        ++depth;
-        if (depth < 64) pend_lo |= (1ull << depth); else pend_hi |= (1ull << (depth - 64));
+      const double t = temperature + tc;
+      Fits f;
+      set_fits(f, t);
+      const double xc = ionized_fraction_change(sub, f, t);
+      if (!small(x, xc, safety)) {
+        reject(depth, pend_lo, pend_hi);
         continue;
       }
+      const double t0 = temperature, x0 = x;
+      temperature = t;
+      fits = f;
+      fits_t = t;
+      x += xc;
+      if (kCarryNeutral) {
+        y -= xc;
+        // keep the smaller fraction exact and derive the other from it
+        if (x < 0.5) y = 1.0 - x; else x = 1.0 - y;
+      }
+      clamp();
       if (pend_hi) {
         depth = 127 - __clzll((long long)pend_hi);
         pend_hi &= ~(1ull << (depth - 64));
@@ -375,11 +374,17 @@ struct ChemSolver {
         pend_lo &= ~(1ull << depth);
       } else {
         failed = false;
-        return ts_min(Timescale{last_dt * (safety / rel_t), kProcTemperature},
-                      Timescale{last_dt * (safety / rel_x), kProcIonization});
+        return ts_min(Timescale{sub * (safety / relative(t0, tc)), kProcTemperature},
+                      Timescale{sub * (safety / relative(x0, xc)), kProcIonization});
       }
       begin(timestep);
     }
+  }
+
+  // halves the step: its second half is pending
+  __device__ __forceinline__ static void reject(int& depth, uint64_t& pend_lo, uint64_t& pend_hi) {
+    ++depth;
+    if (depth < 64) pend_lo |= (1ull << depth); else pend_hi |= (1ull << (depth - 64));
   }
 };
 
