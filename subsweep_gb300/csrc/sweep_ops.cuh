@@ -137,8 +137,7 @@ cudaError_t launch_stream(const DevicePtrs& p, bool all, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// Pairs of blocks: clusters of two, all of them resident at once (a part may wait for another
-// pair's).
+// Pairs of blocks: clusters of two, no more than can be resident at once.
 using PairKernel = void (*)(const swk::StreamArgs<R>);
 PairKernel pair_kernel(bool far, bool all) {
   constexpr int W = swk::kPairWarps;
@@ -151,30 +150,27 @@ cudaError_t pair_config(const DevicePtrs& p, PairKernel fn, cudaLaunchConfig_t* 
   c->dynamicSmemBytes = smem;
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim = {2, 1, 1};
-  at[1].id = cudaLaunchAttributeCooperative;
-  at[1].val.cooperative = 1;
   c->attrs = at;
+  c->numAttrs = 1;
   return cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 cudaError_t stream_pairs(const DevicePtrs& p, int* pairs) {
   cudaLaunchConfig_t c{};
-  cudaLaunchAttribute at[2];
+  cudaLaunchAttribute at[1];
   const PairKernel fn = pair_kernel(true, true);
   cudaError_t e = pair_config(p, fn, &c, at);
   if (e != cudaSuccess) return e;
   c.gridDim = dim3(2);
-  c.numAttrs = 1;
   return cudaOccupancyMaxActiveClusters(pairs, (const void*)fn, &c);
 }
 cudaError_t launch_pairs(const DevicePtrs& p, bool all, cudaStream_t s) {
   cudaLaunchConfig_t c{};
-  cudaLaunchAttribute at[2];
+  cudaLaunchAttribute at[1];
   const swk::StreamArgs<R> a = stream_args(p);
   const PairKernel fn = pair_kernel(a.shape.far != 0, all);
   cudaError_t e = pair_config(p, fn, &c, at);
   if (e != cudaSuccess) return e;
   c.gridDim = dim3(2 * p.num_pairs);
-  c.numAttrs = 2;
   c.stream = s;
   return cudaLaunchKernelEx(&c, fn, a);
 }

@@ -371,7 +371,8 @@ __device__ __forceinline__ void st_sum(StreamSum<double>& sum, const StreamQuad<
 // There are fewer pairs of SMs than streams (76 for 84 directions), so the streams are laid end to
 // end and cut into equal shares: where a share ends inside a stream, the next pair starts with
 // that stream's beginning, and this one ends with the rest of it, once the beginning is solved
-// (flags), its ring filled from memory.
+// (flags), its ring filled from memory.  The last pair is launched first, so a cluster waits only
+// for one launched before it and not for all to be resident.
 template <typename R, int W, bool kFar, bool kAll, bool kPair = false>
 __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const __grid_constant__ StreamArgs<R> a) {
   constexpr uint32_t S = kPair ? 2 * W : W;  // warps that take the groups in turn
@@ -386,13 +387,19 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
   StreamDesc sd = a.streams[kPair ? 0 : blockIdx.x];
   uint32_t me = warp, peer_words = 0, peer_count = 0, first_part = 0, parts = 1;
   if constexpr (kPair) {
-    uint32_t rank;
+    uint32_t rank, size;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+    if (size != 2) {  // launched without its peer
+      if (threadIdx.x == 0) atomicOr(&a.ctl->error, kErrStall);
+      return;
+    }
+    const uint32_t pair = (gridDim.x - 1 - blockIdx.x) / 2;  // the last pair first
     me = rank * W + warp;  // (the warp that tells the peer: (rank + 1) * W)
     peer_words = st_peer(st_smem(words), rank ^ 1u);
     peer_count = st_peer(st_smem(count + 1), rank ^ 1u);
-    first_part = a.part0[blockIdx.x / 2];
-    parts = a.part0[blockIdx.x / 2 + 1] - first_part;
+    first_part = a.part0[pair];
+    parts = a.part0[pair + 1] - first_part;
   }
   if (threadIdx.x < 2) count[threadIdx.x] = 0;
   if (threadIdx.x < kStreamZero) words[shape.ring + threadIdx.x] = R(0);
