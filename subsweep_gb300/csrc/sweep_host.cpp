@@ -875,6 +875,17 @@ sw_status build_streams(sw_handle* h) {
     for (auto& x : th) x.join();
   }
   h->stream_gmax.clear();
+  // No room: the levelled schedule.  FP64: as for the push form's records, room is what leaves a
+  // reserve of 1/16 of the device (at least 4 GiB) for later allocations.
+  size_t free_b = 0, total_b = 0;
+  SW_CUDA(h, cudaMemGetInfo(&free_b, &total_b), "memory info");
+  const size_t reserve = rb == 8 ? std::max(total_b / 16, (size_t)4 << 30) : 0;
+  uint64_t least = 0;
+  for (const swk::StreamGroup& g : groups) least += piece_bytes(g.shape, rb);
+  if (least + reserve > free_b) {
+    h->want_streams = false;
+    return SW_OK;
+  }
   struct Scratch {
     std::vector<void*> mem;
     ~Scratch() {
@@ -984,11 +995,7 @@ sw_status build_streams(sw_handle* h) {
   }
   SW_CUDA(h, cudaMemcpy(d_groups, groups.data(), groups.size() * sizeof(groups[0]), cudaMemcpyHostToDevice), "groups");
   groups.pop_back();
-  // no room: the levelled schedule.  FP64: as for the push form's records, room is what leaves a
-  // reserve of 1/16 of the device (at least 4 GiB) for later allocations.
-  size_t free_b = 0, total_b = 0;
   SW_CUDA(h, cudaMemGetInfo(&free_b, &total_b), "memory info");
-  const size_t reserve = rb == 8 ? std::max(total_b / 16, (size_t)4 << 30) : 0;
   if (at + reserve > free_b || !h->alloc(&p.stream_data, at)) {
     (void)cudaGetLastError();
     p.stream_data = nullptr;
@@ -1037,7 +1044,6 @@ sw_status build_streams(sw_handle* h) {
     SW_CUDA(h, cudaMemset(p.ctl, 0, offsetof(swk::SweepCtl, error)), "reset control");
     if (faces[0] != faces[1]) {  // faces without a partner of their own: only the push form tells them apart
       h->want_streams = false;
-      p.cell_att = nullptr;
       return SW_OK;
     }
     p.cell_sweep = d_cell_sweep;
@@ -1060,9 +1066,20 @@ sw_status build_streams(sw_handle* h) {
 // schedule, or the id order of a cyclic grid, is in place).
 sw_status build_records(sw_handle* h) {
   if (h->want_streams) {
+    const swh::DevicePtrs before = h->p;
+    const size_t allocations = h->allocations.size();
+    const int64_t device_bytes = h->device_bytes;
     sw_status st = build_streams(h);
     if (st != SW_OK || h->want_streams) return st;
-    st = build_schedule(h);  // a level too wide for a ring: the levelled schedule
+    // a level too wide for a ring, or no room: the levelled schedule
+    for (size_t k = allocations; k < h->allocations.size(); ++k) cudaFree(h->allocations[k]);
+    h->allocations.resize(allocations);
+    h->device_bytes = device_bytes;
+    h->p = before;
+    h->streams.clear();
+    h->stream_seg.clear();
+    h->stream_gmax.clear();
+    st = build_schedule(h);
     if (st != SW_OK) return st;
   }
   if (!h->ops->records) return SW_OK;
