@@ -1680,7 +1680,7 @@ sw_status sw_create(const sw_params* params, const sw_grid_csr* grid, const sw_c
 // reset, attenuation, dependency counts on the push path, transport, periodic fold,
 // chemistry; then the level update and the ionization times), captured once per step
 // shape (lowest allowed level before and after, and each sweep's level and kernel
-// choice).  The sweep
+// choice, and with streams whether it takes every cell).  The sweep
 // numbers and the end time live in the control block, copied from pinned host memory by
 // the graph's first node; the error flag stays set across the step's sweeps, so a stall
 // ends the remaining sweeps at once, and is read when the step has finished.  Event
@@ -1744,7 +1744,9 @@ static sw_status step_graph(sw_handle* h, double* time_elapsed_out) {
       if (h->force_path == 2) variant = false;
     }
     variants.push_back(variant);
-    key.push_back(level * 2 + (variant ? 1 : 0));
+    // (a sweep of every cell runs another kernel of the streams than one that leaves some out)
+    const bool all = (int64_t)h->n_ge_host[level] >= h->N;
+    key.push_back(level * 4 + (variant ? 2 : 0) + (p.stream_mode && all ? 1 : 0));
   }
   if (!h->graph_scalars) {
     void* ptr = nullptr;

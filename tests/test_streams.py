@@ -140,6 +140,32 @@ def test_fp64_streams_equal_push(case, monkeypatch):
                     np.testing.assert_allclose(after[k], a, rtol=1e-13, err_msg=k)
 
 
+def everywhere_a_source(seed=1, n=400, levels=3):
+    # all cells stay at the deepest level for some steps, then leave it one by one
+    rng = np.random.default_rng(seed)
+    box = 30 * 3.0857e16 * n ** (1 / 3)
+    g = gridmod.voronoi(gridmod.poisson_points(n, box, seed), box, periodic=False, nthreads=8)
+    source = 1e46 * np.exp(0.5 * rng.standard_normal(g.num_cells))
+    params = SweepParameters(directions=21, num_timestep_levels=levels, periodic=False, max_timestep=0.01 * MEGAYEAR,
+                             significant_rate_threshold=1e-5)
+    return workloads.Workload("sources", params, g, np.full(g.num_cells, float(mass_density_from_number_density(1e-2))),
+                              np.full(g.num_cells, 1e-10), np.full(g.num_cells, 1e4), source, steps=8)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_captured_steps_follow_the_cells_that_leave_a_level(precision, monkeypatch):
+    w = everywhere_a_source()
+    seen = set()
+    with make(w, monkeypatch, {"SUBSWEEP_STREAMS": "1"}, precision) as direct, \
+            make(w, monkeypatch, {"SUBSWEEP_STREAMS": "1", "SUBSWEEP_GRAPH": "1"}, precision) as captured:
+        for _ in range(8):
+            direct.run_sweeps()
+            captured.run_sweeps()
+            same(results(direct), results(captured))
+            seen.add(int(direct.level_counts()[-1]) == w.grid.num_cells)
+    assert seen == {True, False}
+
+
 @pytest.mark.parametrize("case", ["lattice-20", "batch"])
 def test_checkpoints_move_between_layouts(case, monkeypatch):
     w = CASES[case]()
