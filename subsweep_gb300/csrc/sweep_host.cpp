@@ -388,11 +388,25 @@ static uint64_t grouped_level_order(const uint16_t* level, uint32_t Np, uint32_t
 // Closed parts of a grid: contiguous cell ranges that no LOCAL face leaves (the boxes of
 // a batch; the whole grid otherwise), at least `min_cells` each.  Returns their offsets.
 static std::vector<uint32_t> closed_parts(const sw_grid_csr* g, int64_t min_cells) {
+  std::vector<int32_t> farthest(g->num_cells);  // LOCAL neighbour of every cell
+  {
+    const int nt = (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    std::vector<std::thread> th;
+    for (int t = 0; t < nt; ++t)
+      th.emplace_back([&, t]() {
+        for (int64_t c = g->num_cells * t / nt; c < g->num_cells * (t + 1) / nt; ++c) {
+          int32_t n = 0;
+          for (int64_t f = g->row_ptr[c]; f < g->row_ptr[c + 1]; ++f)
+            if (g->kind[f] == SW_FACE_LOCAL) n = std::max(n, (int32_t)g->nbr[f]);
+          farthest[c] = n;
+        }
+      });
+    for (auto& x : th) x.join();
+  }
   std::vector<uint32_t> parts = {0};
   int64_t reach = 0;
   for (int64_t c = 0; c < g->num_cells; ++c) {
-    for (int64_t f = g->row_ptr[c]; f < g->row_ptr[c + 1]; ++f)
-      if (g->kind[f] == SW_FACE_LOCAL) reach = std::max<int64_t>(reach, g->nbr[f]);
+    reach = std::max<int64_t>(reach, farthest[c]);
     if (reach <= c && c + 1 - parts.back() >= min_cells && g->num_cells - (c + 1) >= min_cells)
       parts.push_back((uint32_t)(c + 1));
   }
