@@ -26,8 +26,8 @@
 // What bounds it: the SM's load/store pipe and the warps' instructions.  A group of 32 tasks
 // with 12 slots takes ~90 cycles of the pipe (12 gathers from shared memory at ~3.5 bank
 // conflicts each, 20 to fill the buffer and 18 to read the slots, the rest small), 84 SMs for
-// 84 directions; hence the slots in quads of 16-byte loads at fixed strides.  Hence everything that would touch a memory line
-// per task is done elsewhere: the attenuations are gathered into the groups' pieces before the
+// 84 directions; hence the slots in quads of 16-byte loads at fixed strides, and everything that
+// would touch a memory line per task is done elsewhere: the attenuations are gathered into the groups' pieces before the
 // sweep (k_stream_gather, the whole device), the incoming rates are stored by position and
 // gathered by the sums over directions (k_cell_sums).
 //
@@ -376,6 +376,7 @@ __device__ __forceinline__ void st_sum(StreamSum<double>& sum, const StreamQuad<
 template <typename R, int W, bool kFar, bool kAll, bool kPair = false>
 __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const __grid_constant__ StreamArgs<R> a) {
   constexpr uint32_t S = kPair ? 2 * W : W;  // warps that take the groups in turn
+  constexpr bool kAddress = sizeof(R) == 4 && !kFar && !kPair;  // slots' addresses ahead of the wait
   using Word = typename StreamTraits<R>::Word;
   extern __shared__ __align__(16) unsigned char st_shared[];
   const StreamShape& shape = a.shape;
@@ -589,10 +590,23 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
           if (!dead) st_sum(sum, quad, words, StreamPiece<R>(buffer, gr), lane, early.skip, first);
         }
       }
-      // the levels before this group's
-      dead = dead || !st_wait([&]() { return counted(gr.need); }, a.ctl, a.timeout_ns);
+      // (all that needs no word of this level, ahead of the wait)
       const uint32_t n = group_tasks(gr.shape);
       rel = gr.pos - sd.base;
+      uint32_t slot = ring_slot(shape, rel) + lane;
+      if (slot >= shape.ring) slot -= shape.ring;
+      uint32_t at[kAddress ? kStreamQuads : 1][4];
+      if constexpr (kAddress) {
+#pragma unroll
+        for (uint32_t c = 0; c < kStreamQuads; ++c) {
+          at[c][0] = st_smem(words) + (quad[c].x.x & 0xffffu) * (uint32_t)sizeof(R);
+          at[c][1] = st_smem(words) + (quad[c].x.x >> 16) * (uint32_t)sizeof(R);
+          at[c][2] = st_smem(words) + (quad[c].x.y & 0xffffu) * (uint32_t)sizeof(R);
+          at[c][3] = st_smem(words) + (quad[c].x.y >> 16) * (uint32_t)sizeof(R);
+        }
+      }
+      // the levels before this group's
+      dead = dead || !st_wait([&]() { return counted(gr.need); }, a.ctl, a.timeout_ns);
       if (!dead) {
         if (kFar && (fresh || (gr.shape & (kGroupLate | kGroupSlow)))) {
           const StreamPiece<R> all(a.data + kStreamUnit * gr.data, gr);
@@ -625,7 +639,15 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
             R q[kStreamQuads][4];
 #pragma unroll
             for (uint32_t c = 0; c < kStreamQuads; ++c)
-              if (c < quads) st_words(quad[c], words, q[c]);
+              if (c < quads) {
+                if constexpr (kAddress) {
+#pragma unroll
+                  for (int k = 0; k < 4; ++k)
+                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(q[c][k]) : "r"(at[c][k]) : "memory");
+                } else {
+                  st_words(quad[c], words, q[c]);
+                }
+              }
 #pragma unroll
             for (uint32_t c = 0; c < kStreamQuads; ++c)
               if (c < quads) st_add(sum, c & 1u, quad[c].w, q[c]);
@@ -644,8 +666,6 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
         else
           out = st_solve(in, src, per, att, a.threshold, inv);
         mine = lane < n && (kAll || st_live(att));
-        uint32_t slot = ring_slot(shape, rel) + lane;
-        if (slot >= shape.ring) slot -= shape.ring;
         if (lane < n) {
           const R q = mine ? out : own;
           words[slot] = q;
