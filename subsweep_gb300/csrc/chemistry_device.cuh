@@ -19,7 +19,7 @@
 // in small runs the chain of the attempts of one cell (hundreds beside a source).  Hence
 //   what depends on the state alone is formed once per state (begin()) and not for every
 //   attempt from it: a rejected attempt is repeated with half the step for a few operations;
-//   the fits at the temperature that an attempt accepts are the next state's;
+//   FP64: the fits at the temperature that an attempt accepts are the next state's;
 //   a power is one logarithm and one exponential, the products of powers one exponential;
 //   the recommended steps are formed for the last accepted attempt only.
 // Whole first steps, where cells take up to hundreds of attempts: a column of 600 cells in FP64
@@ -205,12 +205,19 @@ struct ChemSolver {
   // collisional ionization / excitation cooling (237-253), case B recombination cooling
   // (196-216), bremsstrahlung and Compton cooling (265-273).  Mixed path: from the FP32 fits;
   // the densities, the sums and the unit factors in FP64.
+  // (every term in the order in which it has always been rounded)
   __device__ void cooling(const Fits32& f, double& lambda_c, double& dlambda_c) const {
+    const double t = temperature;
     const double ne = n_ionized();
     const double nhn = n_neutral();
-    sum_cooling((double)f.exc + 1.27e-21 * (double)f.fit, (double)f.recc + (double)f.brems, ne, nhn, temperature - xx_cell,
-                lambda_c);
-    sum_cooling((double)f.dexc + 1.27e-21 * (double)f.fitd, (double)f.drecc + (double)f.dbrems, ne, nhn, 1.0, dlambda_c);
+    const double nhi = n_ionized();
+    const double u = Units::kErgsCentimetersCubedPerS;
+    const double compton = compton_cell * (t - xx_cell);
+    const double dcompton = compton_cell;
+    const double coll = ((double)f.exc + 1.27e-21 * (double)f.fit) * u * ne * nhn;
+    const double dcoll = ((double)f.dexc + 1.27e-21 * (double)f.fitd) * u * ne * nhn;
+    lambda_c = coll + ((double)f.recc + (double)f.brems) * u * ne * nhi + compton * ne;
+    dlambda_c = dcoll + ((double)f.drecc + (double)f.dbrems) * u * ne * nhi + dcompton * ne;
   }
   __device__ void cooling(const Fits64& f, double& lambda_c, double& dlambda_c) const {
     const double t = f.t;
@@ -263,12 +270,18 @@ struct ChemSolver {
   __device__ void begin(double timestep) {
     const double absorbed = absorbed_fraction();
     m = 1.0 / (x + 1.0);  // mu
-    if (!(fits_t == temperature)) {
-      set_fits(fits, temperature);
-      fits_t = temperature;
-    }
     double lc, dlc, heating;
-    cooling(fits, lc, dlc);
+    if (kCarryNeutral) {  // (FP32: evaluated apart for either use, so that both keep their roundings)
+      Fits f;
+      set_fits(f, temperature);
+      cooling(f, lc, dlc);
+    } else {
+      if (!(fits_t == temperature)) {
+        set_fits(fits, temperature);
+        fits_t = temperature;
+      }
+      cooling(fits, lc, dlc);
+    }
     constexpr double kEnergy = Units::kPhotonAverageEnergy - Units::kRydberg;
     if (kCarryNeutral) {  // photoheating_rate 321-325, photoionization_rate 327-332
       heating = (step_rate * absorbed) * kEnergy;
@@ -277,9 +290,10 @@ struct ChemSolver {
       heating = ((step_rate * absorbed) / volume) * kEnergy / timestep;
       photo = ((step_rate * absorbed) / (n_neutral() * volume)) / timestep;
     }
-    const double km = k_cell * m;
-    heat_step = km * (heating - lc);
-    cool_step = km * -dlc;
+    const double lambda = heating - lc;
+    const double dlambdadt = -dlc;
+    heat_step = k_cell * m * lambda;
+    cool_step = k_cell * m * dlambdadt;
   }
 
   // 334-354, case B rate at the temperature t of `f` that the attempt has reached
@@ -287,6 +301,20 @@ struct ChemSolver {
     const double ne = n_ionized();
     double alpha, dalpha;
     recombination(f, alpha, dalpha);
+    if (kCarryNeutral) {
+      const double n_h = nh;
+      double beta = (5.85e-11 * (double)f.fit) * Units::kCentimetersCubedPerS;
+      double dbeta = (5.85e-11 * (double)f.fitd) * Units::kCentimetersCubedPerS;
+      double c = beta * ne + photo;
+      double d = alpha * ne;
+      double xhii = x;
+      double rhsc = ne * t * m * 1.0 * dbeta;
+      double dcdx = n_h * beta - rhsc;
+      double rhsd = ne * t * m * 1.0 * dalpha;
+      double dddx = n_h * alpha - rhsd;
+      double j = dcdx - (c + d) - xhii * (dcdx + dddx);
+      return timestep * (c - xhii * (c + d)) / (1.0 - j * timestep);
+    }
     constexpr double kBeta = 5.85e-11 * Units::kCentimetersCubedPerS;
     const double beta = kBeta * (double)f.fit;
     const double dbeta = kBeta * (double)f.fitd;
@@ -332,8 +360,10 @@ struct ChemSolver {
     uint64_t pend_lo = 0, pend_hi = 0;  // pending second halves at depths 1..127
     int depth = 0;
     clamp();
-    begin(timestep);
+    bool moved = true;  // (one place for begin(): the same roundings for every state)
     while (true) {
+      if (moved) begin(timestep);
+      moved = false;
       double sub, tc;
       while (true) {
         if (depth > kChemMaxDepth) {
@@ -357,8 +387,10 @@ struct ChemSolver {
       }
       const double t0 = temperature, x0 = x;
       temperature = t;
-      fits = f;
-      fits_t = t;
+      if (!kCarryNeutral) {
+        fits = f;
+        fits_t = t;
+      }
       x += xc;
       if (kCarryNeutral) {
         y -= xc;
@@ -377,7 +409,7 @@ struct ChemSolver {
         return ts_min(Timescale{sub * (safety / relative(t0, tc)), kProcTemperature},
                       Timescale{sub * (safety / relative(x0, xc)), kProcIonization});
       }
-      begin(timestep);
+      moved = true;
     }
   }
 
