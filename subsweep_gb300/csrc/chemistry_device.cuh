@@ -20,11 +20,9 @@
 //   what depends on the state alone is formed once per state (begin()) and not for every
 //   attempt from it: a rejected attempt is repeated with half the step for a few operations;
 //   FP64: the fits at the temperature that an attempt accepts are the next state's;
-//   a power is one logarithm and one exponential, the products of powers one exponential;
 //   the recommended steps are formed for the last accepted attempt only.
-// Whole first steps, where cells take up to hundreds of attempts: a column of 600 cells in FP64
-// 20.5 -> 11.8 ms, 64^3 lognormal 47 -> 34, a batch of 12 boxes 23-27 -> 18; 96^3 FP64 steps with
-// ~5 attempts a cell 113 -> 93 ms, 128^3 mixed 105 -> 100.
+// None of it changes a rounding: near equilibrium a state's timescale is its value over a small
+// difference of large terms, which shows the last bits of every one of them.
 // The mixed path evaluates the rate fits in FP32 (Fits32); the densities, the sums, the
 // implicit updates and their accept / reject tests are FP64 in both.
 #pragma once
@@ -121,31 +119,23 @@ __device__ __forceinline__ Fits32 fits32(float t) {
   return f;
 }
 
-// FP64: the fits' shared factors at one temperature.  The rate fits and their temperature
-// derivatives (hydrogen_only/mod.rs:161-302) are functions of these; each derivative is the
-// reference's formula with the common factors taken out.  s5 = sqrt(t / 1e5).
+// FP64: what the rate fits and their temperature derivatives (hydrogen_only/mod.rs:161-302) share
+// at one temperature.
 struct Fits64 {
-  double t, inv_t, sq, inv_1s5;  // temperature, 1 / t, sqrt(t), 1 / (1 + s5)
-  double fit, fitd;              // collision_fit 161-166 and its derivative 167-173
-  double ln_lambda;              // lambda = 315614 / t
-  static constexpr double kS5 = 0.0031622776601683793;      // 1 / sqrt(1e5)
-  static constexpr double kInvS5 = 316.22776601683796;      // sqrt(1e5)
+  double t, sq, s5, lambda;  // temperature, sqrt(t), sqrt(t / 1e5), 315614 / t
+  double fit, fitd;          // collision_fit 161-166 and its derivative 167-173
 };
 
 __device__ __forceinline__ Fits64 fits64(double t) {
   Fits64 f;
   f.t = t;
-  f.inv_t = 1.0 / t;
   f.sq = sqrt(t);
-  const double s5 = f.sq * Fits64::kS5;
-  f.inv_1s5 = 1.0 / (1.0 + s5);
+  f.s5 = sqrt(t / 1e5);
+  f.lambda = 315614.0 / t;
   const double c1 = 1.0 / 1e5, c2 = 157809.1;
   const double e = exp(-c2 / t);
-  f.fit = f.sq * f.inv_1s5 * e;
-  // 1 / (t^1.5 s5) = sqrt(1e5) / t^2
-  f.fitd = (e * (c1 * c2 * t + 0.5 * s5 * (2.0 * c2 + t))) *
-           ((Fits64::kInvS5 * (f.inv_t * f.inv_t)) * (f.inv_1s5 * f.inv_1s5));
-  f.ln_lambda = log(315614.0 / t);
+  f.fit = f.sq / (1.0 + f.s5) * e;
+  f.fitd = (e * (c1 * c2 * t + 0.5 * f.s5 * (2.0 * c2 + t))) / ((t * f.sq) * f.s5 * ((f.s5 + 1.0) * (f.s5 + 1.0)));
   return f;
 }
 
@@ -186,20 +176,14 @@ struct ChemSolver {
     step_rate = kCarryNeutral ? rate / volume : timestep * rate;
     xx_cell = 2.727 / scale_factor;
     const double x2 = xx_cell * xx_cell;
-    compton_cell = (1.017e-37 * (x2 * x2)) * Units::kErgsPerS;
+    compton_cell = 1.017e-37 * (x2 * x2);
+    if (kCarryNeutral) compton_cell *= Units::kErgsPerS;
     fits_t = -1.0;  // of no cell
   }
 
   __device__ __forceinline__ double neutral() const { return kCarryNeutral ? y : (1.0 - x); }
   __device__ __forceinline__ double n_ionized() const { return nh * x; }
   __device__ __forceinline__ double n_neutral() const { return nh * neutral(); }
-
-  // collisional, recombination and free-free, and Compton cooling per volume
-  __device__ __forceinline__ void sum_cooling(double neutral_rate, double ion_rate, double ne, double nhn, double dt,
-                                              double& sum) const {
-    constexpr double u = Units::kErgsCentimetersCubedPerS;
-    sum = ne * ((neutral_rate * nhn + ion_rate * ne) * u + compton_cell * dt);
-  }
 
   // cooling_rate 275-287 and cooling_rate_derivative 289-302 at the current state:
   // collisional ionization / excitation cooling (237-253), case B recombination cooling
@@ -219,28 +203,40 @@ struct ChemSolver {
     lambda_c = coll + ((double)f.recc + (double)f.brems) * u * ne * nhi + compton * ne;
     dlambda_c = dcoll + ((double)f.drecc + (double)f.dbrems) * u * ne * nhi + dcompton * ne;
   }
+  // FP64: each derivative is the reference's formula with the powers taken from the fit; the
+  // values agree with separate evaluation to rounding.
   __device__ void cooling(const Fits64& f, double& lambda_c, double& dlambda_c) const {
     const double t = f.t;
     const double ne = n_ionized();
     const double nhn = n_neutral();
+    const double nhi = n_ionized();
+    constexpr double u = Units::kErgsCentimetersCubedPerS;
     // excitation cooling and its derivative
     const double c3 = 1.0 / 1e5, c2e = 118348.0;
-    const double e_exc = 7.5e-19 * exp(-c2e / t);
-    const double s5 = f.sq * Fits64::kS5;
-    const double exc = e_exc * f.inv_1s5;
-    // 1 / (t^2 s5) = sqrt(1e5) sqrt(t) / t^3
-    const double dexc = (e_exc * (c2e * c3 * t - 0.5 * c3 * (t * t) + c2e * s5)) *
-                        (((Fits64::kInvS5 * f.sq) * f.inv_t) * (f.inv_t * f.inv_t) * (f.inv_1s5 * f.inv_1s5));
-    // case B recombination cooling and its derivative, with lambda^1.97 / (1 + q)^3.72
+    const double e_exc = exp(-c2e / t);
+    const double exc = (7.5e-19 / (1.0 + f.s5) * e_exc) * u;
+    const double dexc = ((7.5e-19 * e_exc * (c2e * c3 * t - 0.5 * c3 * (t * t) + c2e * f.s5)) /
+                         ((t * t) * f.s5 * ((1.0 + f.s5) * (1.0 + f.s5)))) * u;
+    // case B recombination cooling and its derivative: lambda^1.97 and (lambda / 2.25)^0.376 from
+    // one logarithm
     const double c2r = 1.97, c3r = 0.376, c4r = 3.72;
-    const double q = exp(c3r * (f.ln_lambda - 0.81093021621632877));  // ln 2.25
-    const double power = 3.435e-30 * exp(c2r * f.ln_lambda - c4r * log(1.0 + q));
-    const double recomb = power * t;
-    const double drecomb = power * ((1.0 - c2r + (1.0 - c2r + c3r * c4r) * q) / (1.0 + q));
-    const double brems = 1.42e-27 * f.sq;
-    const double dbrems = (0.5 * 1.42e-27) * (f.sq * f.inv_t);
-    sum_cooling(exc + 1.27e-21 * f.fit, recomb + brems, ne, nhn, temperature - xx_cell, lambda_c);
-    sum_cooling(dexc + 1.27e-21 * f.fitd, drecomb + dbrems, ne, nhn, 1.0, dlambda_c);
+    const double ln_lambda = log(f.lambda);
+    const double l197 = exp(c2r * ln_lambda);
+    const double q = exp(c3r * (ln_lambda - 0.81093021621632877));  // ln 2.25
+    const double a = pow(1.0 + q, c4r);
+    const double recomb_rate = (3.435e-30 * t * l197 / a) * u;
+    const double drecomb_rate =
+        (3.435e-30 * ((1.0 / (a * (1.0 + q))) * (1.0 - c2r + (1.0 - c2r + c3r * c4r) * q) * l197)) * u;
+    const double compton = (compton_cell * (temperature - xx_cell)) * Units::kErgsPerS;
+    const double dcompton = compton_cell * Units::kErgsPerS;
+    const double coll = (exc + (1.27e-21 * f.fit) * u) * ne * nhn;
+    const double recomb = recomb_rate * ne * nhi;
+    const double brems = ((1.42e-27 * f.sq) * u) * ne * nhi;
+    lambda_c = coll + recomb + brems + compton * ne;
+    const double dcoll = (dexc + (1.27e-21 * f.fitd) * u) * ne * nhn;
+    const double drecomb = drecomb_rate * ne * nhi;
+    const double dbrems = ((1.42e-27 / (2.0 * f.sq)) * u) * ne * nhi;
+    dlambda_c = dcoll + drecomb + dbrems + dcompton * ne;
   }
 
   // case B recombination rate and its derivative, 175-194
@@ -250,10 +246,13 @@ struct ChemSolver {
   }
   __device__ static void recombination(const Fits64& f, double& alpha, double& dalpha) {
     const double c2a = 0.407, c3a = 2.242;
-    const double p = exp(c2a * (f.ln_lambda - 1.0079579203999789));  // ln 2.74
-    // lambda^1.5 / (1 + p)^2.242; the derivative by lambda times d lambda / dT = -lambda / T
-    alpha = (2.753e-14 * Units::kCentimetersCubedPerS) * exp(1.5 * f.ln_lambda - c3a * log(1.0 + p));
-    dalpha = (alpha * f.inv_t) * ((c2a * c3a * p - 1.5 * p - 1.5) / (p + 1.0));
+    const double dlambda_dt = -315614.0 / (f.t * f.t);
+    const double sl = sqrt(f.lambda);
+    const double p = pow(f.lambda / 2.74, c2a);
+    const double b = pow(1.0 + p, c3a);
+    alpha = (2.753e-14 * (f.lambda * sl) / b) * Units::kCentimetersCubedPerS;
+    const double da = -sl * (1.0 / (b * (p + 1.0))) * (c2a * c3a * p - 1.5 * p - 1.5);
+    dalpha = ((2.753e-14 * da) * Units::kCentimetersCubedPerS) * dlambda_dt;
   }
 
   // 312-319: photons absorbed per photon arriving, 1 - exp(-n_HI sigma size); both
@@ -301,30 +300,18 @@ struct ChemSolver {
     const double ne = n_ionized();
     double alpha, dalpha;
     recombination(f, alpha, dalpha);
-    if (kCarryNeutral) {
-      const double n_h = nh;
-      double beta = (5.85e-11 * (double)f.fit) * Units::kCentimetersCubedPerS;
-      double dbeta = (5.85e-11 * (double)f.fitd) * Units::kCentimetersCubedPerS;
-      double c = beta * ne + photo;
-      double d = alpha * ne;
-      double xhii = x;
-      double rhsc = ne * t * m * 1.0 * dbeta;
-      double dcdx = n_h * beta - rhsc;
-      double rhsd = ne * t * m * 1.0 * dalpha;
-      double dddx = n_h * alpha - rhsd;
-      double j = dcdx - (c + d) - xhii * (dcdx + dddx);
-      return timestep * (c - xhii * (c + d)) / (1.0 - j * timestep);
-    }
-    constexpr double kBeta = 5.85e-11 * Units::kCentimetersCubedPerS;
-    const double beta = kBeta * (double)f.fit;
-    const double dbeta = kBeta * (double)f.fitd;
-    const double c = beta * ne + photo;
-    const double cd = c + alpha * ne;
-    const double w = ne * t * m;
-    const double dcdx = nh * beta - w * dbeta;
-    const double both = nh * (beta + alpha) - w * (dbeta + dalpha);  // dcdx + dddx
-    const double j = (dcdx - cd) - x * both;
-    return timestep * (c - x * cd) / (1.0 - j * timestep);
+    const double n_h = nh;
+    double beta = (5.85e-11 * (double)f.fit) * Units::kCentimetersCubedPerS;
+    double dbeta = (5.85e-11 * (double)f.fitd) * Units::kCentimetersCubedPerS;
+    double c = beta * ne + photo;
+    double d = alpha * ne;
+    double xhii = x;
+    double rhsc = ne * t * m * 1.0 * dbeta;
+    double dcdx = n_h * beta - rhsc;
+    double rhsd = ne * t * m * 1.0 * dalpha;
+    double dddx = n_h * alpha - rhsd;
+    double j = dcdx - (c + d) - xhii * (dcdx + dddx);
+    return timestep * (c - xhii * (c + d)) / (1.0 - j * timestep);
   }
 
   // 356-369 with Rust f64::clamp semantics (asserts min <= max: flagged here).
@@ -342,13 +329,21 @@ struct ChemSolver {
     if (has_floor && temperature < floor_t) temperature = floor_t;
   }
 
-  // relative change of update() 444-461, and whether it is small enough (a change that is no
-  // number, or of a value of 0, is not)
+  // relative change of update() 444-461, and whether it is small enough.  Away from equality the
+  // product decides as the quotient does (2^-50 covers the roundings of both); at it, and where
+  // the product leaves the normal range or the cap of the relative change plays a part, the
+  // quotient itself.
   __device__ __forceinline__ static double relative(double value, double change) {
     return fmin(fabs(change / value), 1.0 / DBL_EPSILON);
   }
   __device__ __forceinline__ static bool small(double value, double change, double safety) {
-    return fabs(change) < safety * fabs(value);
+    constexpr double kNear = 8.8817841970012523e-16;  // 2^-50
+    const double c = fabs(change), most = safety * fabs(value);
+    if (most > 1e-290 && safety < 1.0 / DBL_EPSILON) {
+      if (c < most * (1.0 - kNear)) return true;
+      if (c > most * (1.0 + kNear)) return false;
+    }
+    return !(relative(value, change) > safety);
   }
 
   // perform_timestep 426-441 with perform_timestep_internal 394-424 unrolled, and the attempts
