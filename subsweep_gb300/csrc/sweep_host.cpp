@@ -120,6 +120,7 @@ struct sw_handle {
   // direction streams: whether the schedule is to be laid out in streams, the closed cell
   // ranges of the grid ([parts] offsets), and the layout until the records are built
   bool want_streams = false, force_streams = false;
+  uint64_t stream_limit = ~0ull;  // bytes that their pieces may take (SUBSWEEP_STREAM_BYTES)
   // whether sweeps pull (and are numbered): the mixed path and the FP64 streams
   bool pulls() const { return ops->pull || p.stream_mode; }
   std::vector<uint32_t> parts;
@@ -896,7 +897,7 @@ sw_status build_streams(sw_handle* h) {
   const size_t reserve = rb == 8 ? std::max(total_b / 16, (size_t)4 << 30) : 0;
   uint64_t least = 0;
   for (const swk::StreamGroup& g : groups) least += piece_bytes(g.shape, rb);
-  if (least + reserve > free_b) {
+  if (least + reserve > free_b || least > h->stream_limit) {
     h->want_streams = false;
     return SW_OK;
   }
@@ -1010,7 +1011,7 @@ sw_status build_streams(sw_handle* h) {
   SW_CUDA(h, cudaMemcpy(d_groups, groups.data(), groups.size() * sizeof(groups[0]), cudaMemcpyHostToDevice), "groups");
   groups.pop_back();
   SW_CUDA(h, cudaMemGetInfo(&free_b, &total_b), "memory info");
-  if (at + reserve > free_b || !h->alloc(&p.stream_data, at)) {
+  if (at + reserve > free_b || at > h->stream_limit || !h->alloc(&p.stream_data, at)) {
     (void)cudaGetLastError();
     p.stream_data = nullptr;
     h->want_streams = false;
@@ -1090,6 +1091,12 @@ sw_status build_records(sw_handle* h) {
     h->allocations.resize(allocations);
     h->device_bytes = device_bytes;
     h->p = before;
+    // (the push form adds what `pending` holds to the periodic sources: the tasks' totals were there)
+    if (h->p.pending)
+      SW_CUDA(h, cudaMemsetAsync(h->p.pending, 0, (size_t)h->Np * h->D * (size_t)h->ops->rate_bytes, h->stream),
+              "pending rates");
+    SW_CUDA(h, cudaMemsetAsync(h->p.ctl, 0, offsetof(swk::SweepCtl, tasks), h->stream), "reset control");
+    SW_CUDA(h, cudaStreamSynchronize(h->stream), "levelled schedule");
     h->streams.clear();
     h->stream_seg.clear();
     h->stream_gmax.clear();
@@ -1603,6 +1610,7 @@ sw_status sw_create(const sw_params* params, const sw_grid_csr* grid, const sw_c
       h->want_streams = h->want_streams && std::atoi(env) != 0;
       h->force_streams = h->want_streams;
     }
+    if (const char* env = std::getenv("SUBSWEEP_STREAM_BYTES")) h->stream_limit = std::strtoull(env, nullptr, 10);
     if (h->want_streams) h->parts = closed_parts(grid, 256);
   }
   {
