@@ -121,6 +121,7 @@ struct sw_handle {
   // ranges of the grid ([parts] offsets), and the layout until the records are built
   bool want_streams = false, force_streams = false;
   uint64_t stream_limit = ~0ull;  // bytes that their pieces may take (SUBSWEEP_STREAM_BYTES)
+  int64_t stream_allocs_left = INT64_MAX;  // of their arrays (SUBSWEEP_STREAM_ARRAYS)
   // whether sweeps pull (and are numbered): the mixed path and the FP64 streams
   bool pulls() const { return ops->pull || p.stream_mode; }
   std::vector<uint32_t> parts;
@@ -176,6 +177,12 @@ struct sw_handle {
     allocations.push_back((void*)*ptr);
     device_bytes += (int64_t)(count * sizeof(T));
     return true;
+  }
+
+  // one of the streams' arrays: counted, so that a test can let any of them find no memory
+  template <typename T>
+  bool stream_alloc(T** ptr, size_t count) {
+    return stream_allocs_left-- > 0 && alloc(ptr, count);
   }
 
   sw_status fail(sw_status st, const char* fmt, ...) {
@@ -816,6 +823,18 @@ sw_status build_streams(sw_handle* h) {
   const std::vector<uint32_t>& seg = h->stream_seg;
   const uint32_t segs = (uint32_t)seg.size() - 1;
   const uint32_t rb = (uint32_t)h->ops->rate_bytes;
+  // no room, at any point: the levelled schedule (build_records frees what was allocated)
+  const auto give_up = [h]() {
+    (void)cudaGetLastError();
+    h->want_streams = false;
+    return SW_OK;
+  };
+#define SW_ROOM(h, call, where)                                  \
+  do {                                                           \
+    const cudaError_t _r = (call);                               \
+    if (_r == cudaErrorMemoryAllocation) return give_up();       \
+    if (_r != cudaSuccess) return (h)->cuda_fail(_r, where);     \
+  } while (0)
   const double width = (double)h->N * h->D / segs;  // of a level, on average
   // warps of a block: as many as find a group of a level to work on.  Mixed path, 84 directions,
   // ms per sweep with 4, 8 and 16: 24^3 (35 tasks a level) 0.159, 0.152, 0.185; 32^3 (62) 0.289,
@@ -874,8 +893,7 @@ sw_status build_streams(sw_handle* h) {
   }
   // a ring must not wrap inside a level: with a wider one the grid keeps the levelled schedule
   if (words_for(room, swk::kStreamFar) < (int64_t)std::min(longest, widest)) {
-    h->want_streams = false;
-    return SW_OK;
+    return give_up();
   }
   std::vector<swk::StreamGroup> groups(seg_group[segs]);
   {
@@ -898,8 +916,7 @@ sw_status build_streams(sw_handle* h) {
   uint64_t least = 0;
   for (const swk::StreamGroup& g : groups) least += piece_bytes(g.shape, rb);
   if (least + reserve > free_b || least > h->stream_limit) {
-    h->want_streams = false;
-    return SW_OK;
+    return give_up();
   }
   struct Scratch {
     std::vector<void*> mem;
@@ -914,25 +931,22 @@ sw_status build_streams(sw_handle* h) {
     }
   } scratch;
   swh::StreamScratch b{};
-  SW_CUDA(h, scratch.get((void**)&b.gseg, groups.size() * 4, nullptr), "stream scratch");
-  SW_CUDA(h, scratch.get((void**)&b.sbase, sbase.size() * 4, sbase.data()), "stream scratch");
-  SW_CUDA(h, scratch.get((void**)&b.sgroup, sgroup.size() * 4, sgroup.data()), "stream scratch");
-  if (rb == 8) SW_CUDA(h, scratch.get((void**)&b.recip, (size_t)h->E * 4, nullptr), "stream scratch");
+  SW_ROOM(h, scratch.get((void**)&b.gseg, groups.size() * 4, nullptr), "stream scratch");
+  SW_ROOM(h, scratch.get((void**)&b.sbase, sbase.size() * 4, sbase.data()), "stream scratch");
+  SW_ROOM(h, scratch.get((void**)&b.sgroup, sgroup.size() * 4, sgroup.data()), "stream scratch");
+  if (rb == 8) SW_ROOM(h, scratch.get((void**)&b.recip, (size_t)h->E * 4, nullptr), "stream scratch");
   swk::StreamDesc* d_streams = nullptr;
   swk::StreamGroup* d_groups = nullptr;
   uint32_t* d_cell_sweep = nullptr;
-  if (!h->alloc(&d_streams, h->streams.size()) || !h->alloc(&d_groups, groups.size() + 1) ||
-      !h->alloc(&p.seg_group, seg_group.size()))
-    return h->fail(SW_ERR_OOM, "device allocation of the streams failed");
+  if (!h->stream_alloc(&d_streams, h->streams.size()) || !h->stream_alloc(&d_groups, groups.size() + 1) ||
+      !h->stream_alloc(&p.seg_group, seg_group.size()))
+    return give_up();
   if (rb == 8) {  // what the push form does without
     uint32_t *pos = nullptr, *counts = nullptr, *cell_sweep = nullptr;
-    if (!h->alloc(&pos, (size_t)h->Np * h->D) || !h->alloc(&counts, 32) || !h->alloc(&cell_sweep, h->Np) ||
-        !h->alloc(&p.fold_changed, p.n_periodic_cells) ||
-        !h->alloc(&p.fold_off, (size_t)p.n_periodic_cells * h->D + 1)) {
-      (void)cudaGetLastError();
-      h->want_streams = false;
-      return SW_OK;
-    }
+    if (!h->stream_alloc(&pos, (size_t)h->Np * h->D) || !h->stream_alloc(&counts, 32) ||
+        !h->stream_alloc(&cell_sweep, h->Np) || !h->stream_alloc(&p.fold_changed, p.n_periodic_cells) ||
+        !h->stream_alloc(&p.fold_off, (size_t)p.n_periodic_cells * h->D + 1))
+      return give_up();
     SW_CUDA(h, cudaMemset(cell_sweep, 0, h->Np * sizeof(uint32_t)), "streams");
     p.pos_of_task = pos;
     p.act_counts = counts;
@@ -988,9 +1002,9 @@ sw_status build_streams(sw_handle* h) {
       std::vector<uint32_t> part0;
       plan_parts(h->streams, seg_group, (uint32_t)resident, parts, part0);
       swk::StreamPart* d_parts = nullptr;
-      if (!h->alloc(&d_parts, parts.size()) || !h->alloc(&p.stream_part0, part0.size()) ||
-          !h->alloc(&p.stream_flags, part0.size()))
-        return h->fail(SW_ERR_OOM, "device allocation of the streams failed");
+      if (!h->stream_alloc(&d_parts, parts.size()) || !h->stream_alloc(&p.stream_part0, part0.size()) ||
+          !h->stream_alloc(&p.stream_flags, part0.size()))
+        return give_up();
       SW_CUDA(h, cudaMemcpy(d_parts, parts.data(), parts.size() * sizeof(parts[0]), cudaMemcpyHostToDevice), "streams");
       SW_CUDA(h, cudaMemcpy(p.stream_part0, part0.data(), part0.size() * 4, cudaMemcpyHostToDevice), "streams");
       SW_CUDA(h, cudaMemset(p.stream_flags, 0xff, part0.size() * 4), "streams");
@@ -1005,26 +1019,20 @@ sw_status build_streams(sw_handle* h) {
   }
   groups.push_back({0u, (uint32_t)(at / swk::kStreamUnit), 0u, 0u});  // where the last piece ends
   if (at / swk::kStreamUnit > 0xffffffffull) {  // past the pieces' 32-bit offsets: the levelled schedule
-    h->want_streams = false;
-    return SW_OK;
+    return give_up();
   }
   SW_CUDA(h, cudaMemcpy(d_groups, groups.data(), groups.size() * sizeof(groups[0]), cudaMemcpyHostToDevice), "groups");
   groups.pop_back();
   SW_CUDA(h, cudaMemGetInfo(&free_b, &total_b), "memory info");
-  if (at + reserve > free_b || at > h->stream_limit || !h->alloc(&p.stream_data, at)) {
-    (void)cudaGetLastError();
-    p.stream_data = nullptr;
-    h->want_streams = false;
-    return SW_OK;
-  }
+  if (at + reserve > free_b || at > h->stream_limit || !h->stream_alloc(&p.stream_data, at)) return give_up();
   char* cell_att = nullptr;
   std::vector<uint32_t> pcells(p.n_periodic_cells);
   std::vector<uint8_t> has_periodic(h->N, 0);
   SW_CUDA(h, cudaMemcpy(pcells.data(), p.periodic_cells, pcells.size() * 4, cudaMemcpyDeviceToHost), "periodic cells");
   for (uint32_t c : pcells) has_periodic[c] = 1;
-  if (!h->alloc(&cell_att, (size_t)h->N * rb) || !h->alloc(&p.cell_rate, h->N) || !h->alloc(&p.cell_periodic, h->N) ||
-      !h->alloc(&p.stale, h->N))
-    return h->fail(SW_ERR_OOM, "device allocation of the streams failed");
+  if (!h->stream_alloc(&cell_att, (size_t)h->N * rb) || !h->stream_alloc(&p.cell_rate, h->N) ||
+      !h->stream_alloc(&p.cell_periodic, h->N) || !h->stream_alloc(&p.stale, h->N))
+    return give_up();
   p.stream_bytes = at;
   p.cell_att = cell_att;
   SW_CUDA(h, cudaMemcpy(p.cell_periodic, has_periodic.data(), h->N, cudaMemcpyHostToDevice), "periodic cells");
@@ -1034,7 +1042,7 @@ sw_status build_streams(sw_handle* h) {
   if (rb == 8 && p.n_periodic_cells > 0) {  // the periodic fold's slots
     const size_t entries = (size_t)p.n_periodic_cells * h->D;
     void* cnt = nullptr;
-    SW_CUDA(h, scratch.get(&cnt, entries, nullptr), "fold scratch");
+    SW_ROOM(h, scratch.get(&cnt, entries, nullptr), "fold scratch");
     p.fold_cnt = static_cast<uint8_t*>(cnt);
     SW_CUDA(h, h->ops->stream_build(p, 3, b, h->stream), "periodic fold entries");
     SW_CUDA(h, cudaStreamSynchronize(h->stream), "periodic fold entries");
@@ -1045,7 +1053,7 @@ sw_status build_streams(sw_handle* h) {
     for (size_t e = 0; e < entries; ++e) off[e + 1] = off[e] + n[e];
     SW_CUDA(h, cudaMemcpy(p.fold_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice), "periodic fold entries");
     uint4* fslots = nullptr;
-    if (!h->alloc(&fslots, off[entries])) return h->fail(SW_ERR_OOM, "device allocation of the periodic fold slots failed");
+    if (!h->stream_alloc(&fslots, off[entries])) return give_up();
     p.fold_slots = fslots;
     SW_CUDA(h, h->ops->stream_build(p, 4, b, h->stream), "periodic fold entries");
     SW_CUDA(h, cudaStreamSynchronize(h->stream), "periodic fold entries");
@@ -1057,10 +1065,8 @@ sw_status build_streams(sw_handle* h) {
     const size_t nd = (size_t)h->Np * h->D;
     SW_CUDA(h, cudaMemset(p.pending, 0, nd * 8), "pending rates");
     SW_CUDA(h, cudaMemset(p.ctl, 0, offsetof(swk::SweepCtl, error)), "reset control");
-    if (faces[0] != faces[1]) {  // faces without a partner of their own: only the push form tells them apart
-      h->want_streams = false;
-      return SW_OK;
-    }
+    // faces without a partner of their own: only the push form tells them apart
+    if (faces[0] != faces[1]) return give_up();
     p.cell_sweep = d_cell_sweep;
   }
   uint32_t err = 0;
@@ -1076,6 +1082,7 @@ sw_status build_streams(sw_handle* h) {
   p.stream_mode = 1;
   return SW_OK;
 }
+#undef SW_ROOM
 
 // Pull path: task records and upwind slots of every schedule position (after the
 // schedule, or the id order of a cyclic grid, is in place).
@@ -1611,6 +1618,7 @@ sw_status sw_create(const sw_params* params, const sw_grid_csr* grid, const sw_c
       h->force_streams = h->want_streams;
     }
     if (const char* env = std::getenv("SUBSWEEP_STREAM_BYTES")) h->stream_limit = std::strtoull(env, nullptr, 10);
+    if (const char* env = std::getenv("SUBSWEEP_STREAM_ARRAYS")) h->stream_allocs_left = std::strtoll(env, nullptr, 10);
     if (h->want_streams) h->parts = closed_parts(grid, 256);
   }
   {

@@ -12,7 +12,8 @@ STEPS = 5
 
 
 def make(w, monkeypatch, env, precision):
-    for k in ("SUBSWEEP_STREAMS", "SUBSWEEP_STREAM_BYTES", "SUBSWEEP_STREAM_PAIRS", "SUBSWEEP_STREAM_WARPS"):
+    for k in ("SUBSWEEP_STREAMS", "SUBSWEEP_STREAM_BYTES", "SUBSWEEP_STREAM_PAIRS", "SUBSWEEP_STREAM_WARPS",
+              "SUBSWEEP_STREAM_ARRAYS"):
         monkeypatch.delenv(k, raising=False)
     for k, v in env.items():
         monkeypatch.setenv(k, v)
@@ -75,3 +76,19 @@ def test_grids_whose_pieces_do_not_fit(precision, monkeypatch, capfd):
         with make(w, monkeypatch, env, precision) as s:
             same(w, precision, expected, results(s))
     assert streams_bytes(w, monkeypatch, capfd, precision, {**on, "SUBSWEEP_STREAM_BYTES": str(size)}) == size
+
+
+@pytest.mark.parametrize("pairs", ["0", "1"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_grids_whose_streams_run_out_of_memory(precision, pairs, monkeypatch, capfd):
+    w = periodic()
+    with make(w, monkeypatch, {"SUBSWEEP_STREAMS": "0"}, precision) as s:
+        expected = results(s)
+    env = {"SUBSWEEP_STREAMS": "1", "SUBSWEEP_STREAM_PAIRS": pairs}
+    for arrays in range(64):  # the first so many arrays are found room for
+        env["SUBSWEEP_STREAM_ARRAYS"] = str(arrays)
+        if streams_bytes(w, monkeypatch, capfd, precision, env) is not None:
+            break
+        with make(w, monkeypatch, env, precision) as s:
+            same(w, precision, expected, results(s))
+    assert 8 <= arrays < 63
