@@ -96,7 +96,7 @@ struct DevicePtrs {
   uint32_t space_lvl_words[kMaxSpaces];
   // direction streams (sweep_stream.cuh): stream_mode != 0 when the handle's schedule is
   // laid out in streams.  The FP64 path then keeps incoming and outgoing by schedule position,
-  // the sparse sweeps' stamps in queue, and no pending rates
+  // the changes of the outgoing rates in a sweep in pending and the sparse sweeps' stamps in queue
   int stream_mode;
   void* streams;             // StreamDesc per stream, in launch order (longest first)
   void* stream_groups;       // StreamGroup per group
@@ -107,13 +107,15 @@ struct DevicePtrs {
   void* cell_att;            // attenuation of every cell or the inactive mark (R)
   double* cell_rate;         // rate of every cell summed over the directions
   uint8_t* cell_periodic;    // whether the cell has a LOCAL_PERIODIC face
-  uint8_t* stale;            // cells whose incoming rates are out of date (scratch)
+  uint8_t* stale;            // cells whose incoming rates are out of date (scratch; FP64: after a sparse
+                             // sweep, inactive cells beside an active one)
   uint32_t stream_shape[6];  // StreamShape: ring, magic, far, warps, buffer, blocks
   uint32_t num_pairs;        // pairs of blocks (stream_shape[5] == 2)
   void* stream_parts;        // StreamPart of all pairs
   uint32_t *stream_part0, *stream_flags;
   // per level, lazily allocated: the active positions' bitmap, and their range in each stream
   uint32_t *act_bits_lv[32], *act_range[32];
+  int sweep_level;           // pull path: level of this launch
   int sparse_sweep;          // pull path: this launch runs over the compacted list of its level
   int compact_now;           // pull path: ... and builds that list first
   uint32_t* chunk;           // pull path: compaction chunk offsets, count at [num_chunks]
@@ -179,8 +181,6 @@ struct PrecisionOps {
   cudaError_t (*stream_build)(const DevicePtrs&, int phase, const StreamScratch&, cudaStream_t);
   // direction streams: pairs of blocks that can be resident at once with the shape set
   cudaError_t (*stream_pairs)(const DevicePtrs&, int* pairs);
-  // FP64 streams: brings the incoming rates of inactive cells up to date; nullptr on the pull path
-  cudaError_t (*refresh)(const DevicePtrs&, cudaStream_t);
 };
 
 // pull path: transport kernel variant used without autotuning (the lockstep kernel with

@@ -937,20 +937,17 @@ sw_status build_streams(sw_handle* h) {
   if (rb == 8) SW_ROOM(h, scratch.get((void**)&b.recip, (size_t)h->E * 4, nullptr), "stream scratch");
   swk::StreamDesc* d_streams = nullptr;
   swk::StreamGroup* d_groups = nullptr;
-  uint32_t* d_cell_sweep = nullptr;
   if (!h->stream_alloc(&d_streams, h->streams.size()) || !h->stream_alloc(&d_groups, groups.size() + 1) ||
       !h->stream_alloc(&p.seg_group, seg_group.size()))
     return give_up();
   if (rb == 8) {  // what the push form does without
-    uint32_t *pos = nullptr, *counts = nullptr, *cell_sweep = nullptr;
+    uint32_t *pos = nullptr, *counts = nullptr;
     if (!h->stream_alloc(&pos, (size_t)h->Np * h->D) || !h->stream_alloc(&counts, 32) ||
-        !h->stream_alloc(&cell_sweep, h->Np) || !h->stream_alloc(&p.fold_changed, p.n_periodic_cells) ||
+        !h->stream_alloc(&p.fold_changed, p.n_periodic_cells) ||
         !h->stream_alloc(&p.fold_off, (size_t)p.n_periodic_cells * h->D + 1))
       return give_up();
-    SW_CUDA(h, cudaMemset(cell_sweep, 0, h->Np * sizeof(uint32_t)), "streams");
     p.pos_of_task = pos;
     p.act_counts = counts;
-    d_cell_sweep = cell_sweep;
   }
   p.streams = d_streams;
   p.stream_groups = d_groups;
@@ -1067,7 +1064,6 @@ sw_status build_streams(sw_handle* h) {
     SW_CUDA(h, cudaMemset(p.ctl, 0, offsetof(swk::SweepCtl, error)), "reset control");
     // faces without a partner of their own: only the push form tells them apart
     if (faces[0] != faces[1]) return give_up();
-    p.cell_sweep = d_cell_sweep;
   }
   uint32_t err = 0;
   SW_CUDA(h, cudaMemcpy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
@@ -1806,7 +1802,8 @@ static sw_status step_graph(sw_handle* h, double* time_elapsed_out) {
       // attenuation, transport, chemistry, the periodic fold, and the counts (push) or
       // the compaction at a sparse level's first sweep (pull)
       kernels += 3 + (p.n_periodic_cells > 0 ? 1 : 0);
-      if (p.stream_mode) kernels += variants[k] ? 1 : 2;  // rates of the cells, gather of a dense sweep
+      // rates of the cells, gather of a dense sweep, the changes beside a sparse one (FP64)
+      if (p.stream_mode) kernels += variants[k] ? (ops.pull ? 1 : 3) : 2;
       // the fold's mark pass after a sweep that leaves cells inactive (pull path)
       if (h->pulls() && p.n_periodic_cells > 0 && h->n_ge_host[levels[k]] < h->N) kernels += 1;
       if (!h->pulls()) {
@@ -1821,6 +1818,7 @@ static sw_status step_graph(sw_handle* h, double* time_elapsed_out) {
       const int level = levels[k];
       q.epoch = (uint32_t)(k + 1);
       q.active_cells = h->n_ge_host[level];
+      q.sweep_level = level;
       q.sparse_sweep = (h->pulls() && variants[k]) ? 1 : 0;
       q.compact_now = compact_now[k];
       ce = cudaMemsetAsync(p.ctl, 0, offsetof(swk::SweepCtl, error), h->stream);
@@ -2052,6 +2050,7 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
       h->p.epoch += 1;
       h->last_epoch = h->p.epoch;
       h->p.active_cells = h->n_ge_host[level];
+      h->p.sweep_level = level;
       h->p.sparse_sweep = pull_sparse(h, level) ? 1 : 0;
       h->p.compact_now = 0;
       if (h->p.sparse_sweep) {
@@ -2080,7 +2079,8 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
     SW_CUDA(h, cudaEventRecord(ev[2], h->stream), "event");
     SW_CUDA(h, ops.fold_periodic(h->p, h->stream), "periodic fold kernel");
     launches += 3 + (h->p.n_periodic_cells > 0 ? 1 : 0);
-    if (h->p.stream_mode) launches += h->p.sparse_sweep ? 1 : 2;  // rates of the cells, gather of a dense sweep
+    // rates of the cells, gather of a dense sweep, the changes beside a sparse one (FP64)
+    if (h->p.stream_mode) launches += h->p.sparse_sweep ? (ops.pull ? 1 : 3) : 2;
     if (h->pulls() && h->p.n_periodic_cells > 0 && h->p.active_cells < h->N) launches += 1;  // fold marks
     SW_CUDA(h, cudaEventRecord(ev[3], h->stream), "event");
     SW_CUDA(h, ops.chemistry(h->p, level, h->stream), "chemistry kernel");
@@ -2339,6 +2339,7 @@ static void reorder_rates(sw_handle* h, char* end, const std::vector<uint32_t>& 
   } else {
     reorder(end - 3 * nd * 8, nd, 8, own, nullptr, save);
     reorder(end - 2 * nd * 8, nd, 8, own, nullptr, save);
+    std::memset(end - nd * 8, 0, nd * 8);  // no pending rates: the last sweep's changes are there
   }
 }
 
@@ -2469,7 +2470,6 @@ sw_status sw_save_state(sw_handle* h, void* buffer, size_t bytes) {
     const sw_status st = levelled_schedule(h, own, order, schedule);
     if (st != SW_OK) return st;
     if (h->ops->pull) hd.schedule_hash = schedule;
-    if (h->ops->refresh) SW_CUDA(h, h->ops->refresh(h->p, h->stream), "incoming rates");
   }
   char* out = static_cast<char*>(buffer);
   std::memcpy(out, &hd, sizeof(hd));
@@ -2525,11 +2525,8 @@ sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) {
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "load state");
   if (h->p.num_pairs) SW_CUDA(h, cudaMemset(h->p.stream_flags, 0xff, (size_t)h->p.num_pairs * 4), "load state");
   h->p.active_cells = 0;  // incoming rates of some cells may be out of date (mixed path)
-  if (h->p.stream_mode && !h->ops->pull) {  // every incoming rate is current, no sweep is stamped
-    h->p.active_cells = h->N;
-    SW_CUDA(h, cudaMemset(h->p.cell_sweep, 0, (size_t)h->Np * 4), "load state");
+  if (h->p.stream_mode && !h->ops->pull)  // no sweep is stamped
     SW_CUDA(h, cudaMemset(h->p.queue, 0xff, (size_t)h->Np * h->D * 4), "load state");
-  }
   h->sim_time = hd.sim_time;
   h->ts.lowest = hd.ts_lowest;
   h->ts.first_done = hd.ts_first_done != 0;

@@ -104,7 +104,8 @@ swk::StreamArgs<R> stream_args(const DevicePtrs& p) {
 #if SWK_PULL
   a.word = p.qe;
 #else
-  a.word = static_cast<double*>(p.outgoing);
+  a.word = static_cast<double*>(p.pending);
+  a.out = static_cast<double*>(p.outgoing);
   a.stamp = p.queue;
 #endif
   a.inc = static_cast<R*>(p.incoming);
@@ -184,6 +185,12 @@ cudaError_t sweep_stream(const DevicePtrs& p, int level, cudaStream_t s) {
     a.act_range = p.act_range[level];
     a.act_bits = p.act_bits_lv[level];
     swk::k_sweep_stream_sparse<R><<<p.num_streams, swk::kStreamSparseThreads, 0, s>>>(a);
+#if !SWK_PULL
+    swk::k_cells_near64<<<grid_for(p.num_cells, 256), 256, 0, s>>>((uint32_t)p.num_cells, p.level, level, p.off, p.nbr,
+                                                                    p.stale);
+    const int y = std::max(8, (int)(16 * p.num_sms / std::max(1u, p.num_streams)));
+    swk::k_stream_take64<<<dim3(p.num_streams, y), 256, 0, s>>>(a, p.stale);
+#endif
     return cudaGetLastError();
   }
   swk::k_stream_gather<R><<<grid_for((int64_t)p.num_groups * 32, 256), 256, 0, s>>>(
@@ -198,14 +205,16 @@ cudaError_t sweep_stream(const DevicePtrs& p, int level, cudaStream_t s) {
   }
 }
 
-// Incoming rates of every cell as after the last sweep, before they are exported: that sweep
-// left those of its inactive cells as they were.
+// Incoming rates of every cell as after the last sweep, before they are exported: a sweep of the
+// mixed path leaves those of its inactive cells as they were.
 cudaError_t refresh(const DevicePtrs& p, cudaStream_t s) {
+#if SWK_PULL
   if (!p.stream_mode || p.active_cells >= p.num_cells) return cudaSuccess;
   swk::k_stream_stale<<<grid_for(p.num_cells, 256), 256, 0, s>>>((uint32_t)p.num_cells, p.off, p.nbr, p.cell_sweep,
                                                                   p.stale);
   const int y = std::max(8, (int)(8 * p.num_sms / std::max(1u, p.num_streams)));
-  swk::k_stream_refresh<R><<<dim3(p.num_streams, y), 256, 0, s>>>(stream_args(p), p.stale);
+  swk::k_stream_refresh<<<dim3(p.num_streams, y), 256, 0, s>>>(stream_args(p), p.stale);
+#endif
   return cudaGetLastError();
 }
 
@@ -398,8 +407,9 @@ cudaError_t fold_periodic(const DevicePtrs& p, cudaStream_t s) {
           sweep_args(p, 0), static_cast<const double*>(p.cell_att), p.periodic_cells, p.n_periodic_cells, changed);
     }
     swk::k_fold64<<<dim3((p.n_periodic_cells + 255) / 256, p.D), 256, 0, s>>>(
-        static_cast<const double*>(p.outgoing), static_cast<double*>(p.periodic), p.Np, p.periodic_cells,
-        p.n_periodic_cells, p.fold_off, static_cast<const swk::FoldSlot64*>(p.fold_slots), changed);
+        static_cast<const double*>(p.pending), static_cast<double*>(p.periodic), p.Np, p.periodic_cells,
+        p.n_periodic_cells, p.fold_off, static_cast<const swk::FoldSlot64*>(p.fold_slots), changed,
+        p.sparse_sweep ? p.act_bits_lv[p.sweep_level] : nullptr);
     return cudaGetLastError();
   }
 #endif
@@ -773,14 +783,14 @@ extern const PrecisionOps SWK_OPS = {
     SWK_NAME,       (int)sizeof(R), true,       occupancy,     attenuation, init_counts, sweep,
     occupancy_pull, sweep_pull,     kahn_rounds, schedule_seed, fold_pull,   chemistry,   photon_rate,
     export_rates,   records,        cell_rates, SWK_CARRY != 0,
-    (int)(sizeof(kTuneVariants) / sizeof(int)), kTuneVariants, nullptr, stream_build, stream_pairs, nullptr,
+    (int)(sizeof(kTuneVariants) / sizeof(int)), kTuneVariants, nullptr, stream_build, stream_pairs,
 };
 #else
 extern const PrecisionOps SWK_OPS = {
     SWK_NAME,         (int)sizeof(R), false,      occupancy,     attenuation,   init_counts, sweep,
     occupancy_levels, sweep_levels,   kahn_rounds, schedule_seed, fold_periodic, chemistry,   photon_rate,
     export_rates,     nullptr,        cell_rates, SWK_CARRY != 0,
-    0, nullptr,       push_records, stream_build64, stream_pairs, refresh,
+    0, nullptr,       push_records, stream_build64, stream_pairs,
 };
 #endif
 

@@ -39,11 +39,14 @@
 // FP64 is bound by its unit instead: a warp's instruction takes 64 cycles of a quarter of the SM,
 // so a group of ~10 slots takes a warp 640 cycles for the products alone.  Its slots lie by upwind
 // position and all but those of the previous level are summed before that level is done: 64^3
-// 2.85 -> 2.0 ms per sweep, 24^3 0.40 -> 0.31 (push form with atomics 5.4 and 1.6).
+// 2.85 -> 2.0 ms per sweep, 24^3 0.40 -> 0.31 (push form with atomics 5.4 and 1.6).  Its words are
+// the changes of the outgoing rates, added to the incoming rates of before, as the push form adds
+// them: with gather and fold 2.24 ms, where sums of the outgoing rates themselves took 2.12, but
+// left other last bits in the rates; with the products rounded as well 30% more.
 //
 // FP32 (mixed path): the incoming rate is the sum of the pull kernels over the slots in face
 // order, as eight partial sums combined pairwise, with the same roundings as the lockstep
-// kernels, so both give the same bits.  FP64: one sum of fused multiply-adds.
+// kernels, so both give the same bits.  FP64: fused multiply-adds one by one.
 #pragma once
 
 #include "sweep_device.cuh"
@@ -62,7 +65,7 @@ struct StreamTraits<float> {
 };
 template <>
 struct StreamTraits<double> {
-  using Word = double;  // the outgoing rate
+  using Word = double;  // what the sweep changes the outgoing rate by (0: the cell is not active)
 };
 
 // FP64: the slots of a task lie by upwind position, padding first, so that all but the last
@@ -127,6 +130,7 @@ struct StreamArgs {
   unsigned long long bytes;    // of them
   Word* word;                  // per position
   R* inc;                      // per position: the incoming rate
+  R* out;                      // FP64, per position: the outgoing rate
   R threshold;
   SweepCtl* ctl;
   unsigned long long timeout_ns;
@@ -231,7 +235,7 @@ struct StreamSum;
 template <>
 struct StreamSum<float> {
   float part[8];
-  __device__ __forceinline__ StreamSum() {
+  __device__ __forceinline__ explicit StreamSum(float) {
 #pragma unroll
     for (int k = 0; k < 8; ++k) part[k] = 0.f;
   }
@@ -241,12 +245,12 @@ struct StreamSum<float> {
   }
 };
 
-// FP64: one fused multiply-add per slot (the unit takes 64 cycles per warp and instruction,
-// whatever depends on what)
+// FP64: the incoming rate of before and, one by one, the shares of the upwind tasks' changes, which
+// the push form adds in any order (the product is not rounded: half the instructions).
 template <>
 struct StreamSum<double> {
   double sum;
-  __device__ __forceinline__ StreamSum() : sum(0.0) {}
+  __device__ __forceinline__ explicit StreamSum(double before) : sum(before) {}
   __device__ __forceinline__ void add(int, double w, double q) { sum = fma(w, q, sum); }
   __device__ __forceinline__ double total() const { return sum; }
 };
@@ -256,6 +260,11 @@ __device__ __forceinline__ float st_solve(float in, float src, float per, float 
   const float rt = (in + src) + per;                    // Site::get_rate, site.rs:53-56
   const float out = (rt < threshold) ? 0.f : rt * att;  // get_outgoing_rate
   return out * inv;
+}
+// Photons::make_positive (chemistry/mod.rs:61-65), on the bits: a number below 0 becomes 0
+__device__ __forceinline__ double st_positive(double in) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(in);
+  return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull ? 0.0 : in;
 }
 // FP64: the comparison on the bits, which order as the numbers do from the threshold up
 __device__ __forceinline__ double st_solve(double rt, double att, double threshold) {
@@ -377,6 +386,7 @@ template <typename R, int W, bool kFar, bool kAll, bool kPair = false>
 __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const __grid_constant__ StreamArgs<R> a) {
   constexpr uint32_t S = kPair ? 2 * W : W;  // warps that take the groups in turn
   constexpr bool kAddress = sizeof(R) == 4 && !kFar && !kPair;  // slots' addresses ahead of the wait
+  constexpr bool kChange = sizeof(R) == 8;  // words are changes, added to the incoming rate of before
   using Word = typename StreamTraits<R>::Word;
   extern __shared__ __align__(16) unsigned char st_shared[];
   const StreamShape& shape = a.shape;
@@ -414,6 +424,7 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
   const StreamGroup* groups = a.groups + sd.group0;
   Word* word = a.word + sd.base + lane;
   R* inc = a.inc + sd.base + lane;
+  R* outgoing = a.out + sd.base + lane;
   uint32_t begin = 0, stop = sd.groups;  // groups of the part
   auto counted = [&](uint32_t need) { return (kPair ? st_count_pair(count) : st_count(count)) >= need; };
   R* far_words = words + shape.ring + kStreamZero + warp * shape.far * 32u + lane;
@@ -457,7 +468,12 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
   StreamGroup gr{};
   StreamEarly early{};
   StreamQuad<R> quad[kStreamQuads];
-  R att = R(0), per = R(0), src = R(0), own = R(0);
+  R att = R(0), per = R(0), src = R(0);
+  R own = R(0);  // the word kept by an inactive task; FP64: the outgoing rate of before
+  R before = R(0), before_next = R(0);  // FP64: the incoming rate of before, and that of the group `next`
+  auto ask = [&]() {
+    if constexpr (kChange) before_next = lane < group_tasks(next.shape) ? __ldcg(inc + (next.pos - sd.base)) : R(0);
+  };
   float inv = 0.f;
   uint32_t up[kFar ? kStreamFar : 1], up_far = 0;
   // kPair: the far words on their way (the other block wrote some of them, so they come from L2,
@@ -484,9 +500,15 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
       per = s.per()[lane];
       src = s.src()[lane];
     }
-    if (!kAll && lane < group_tasks(gr.shape)) own = st_ldq(word + (gr.pos - sd.base));
+    if constexpr (kChange) {
+      before = before_next;
+      if (lane < group_tasks(gr.shape)) own = __ldcg(outgoing + (gr.pos - sd.base));
+    } else if (!kAll && lane < group_tasks(gr.shape)) {
+      own = st_ldq(word + (gr.pos - sd.base));
+    }
     staged = s.quads > kStreamQuads;
     if (g + S < stop) {
+      ask();
       if (kFar) {  // the positions of the next group's far words
         up_far = (next.shape & (kGroupLate | kGroupSlow)) ? 0u : group_far(next.shape);
         if (up_far) {
@@ -512,16 +534,19 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
     }
   };
   // what is left to store of the group solved: behind the count, off the levels' chain
-  R in = R(0), out = R(0);
+  R in = R(0), out = R(0), q = R(0);
   uint32_t rel = 0;
-  bool mine = false;
+  bool mine = false, other = false;  // other: FP64, of an inactive cell, which takes the changes upwind
   auto store = [&]() {
-    if (mine) {
-      word[rel] = st_word(out, sweep);
+    if (mine || other) {
+      word[rel] = st_word(q, sweep);
       inc[rel] = in;
+    }
+    if (mine) {
+      if constexpr (kChange) outgoing[rel] = out;
       ++solved;
     }
-    mine = false;
+    mine = other = false;
   };
   for (uint32_t part = 0; part < parts; ++part) {
     uint32_t post = 0;
@@ -532,6 +557,7 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
       groups = a.groups + sd.group0;
       word = a.word + sd.base + lane;
       inc = a.inc + sd.base + lane;
+      outgoing = a.out + sd.base + lane;
       begin = pt.begin;
       stop = pt.end;
       post = pt.post;
@@ -575,11 +601,14 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
       }
     }
     locate(g);
-    if (g < stop) copy();
+    if (g < stop) {
+      ask();
+      copy();
+    }
     locate(g + S);
     load();
     while (g < stop) {
-      StreamSum<R> sum;
+      StreamSum<R> sum(before);
       const uint32_t quads = group_slots(gr.shape) / 4;
       uint32_t first = 0;  // slot that the sum goes on with
       if constexpr (sizeof(R) == 8) {
@@ -661,13 +690,17 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
           }
         }
         in = sum.total();
-        if constexpr (sizeof(R) == 8)
-          out = (gr.shape & kGroupExt) ? st_solve(in, src, per, att, a.threshold, inv) : st_solve(in, att, a.threshold);
-        else
-          out = st_solve(in, src, per, att, a.threshold, inv);
         mine = lane < n && (kAll || st_live(att));
+        if constexpr (kChange) {
+          if (mine) in = st_positive(in);
+          out = (gr.shape & kGroupExt) ? st_solve(in, src, per, att, a.threshold, inv) : st_solve(in, att, a.threshold);
+          other = lane < n && !mine;
+          q = mine ? out - own : R(0);
+        } else {
+          out = st_solve(in, src, per, att, a.threshold, inv);
+          q = mine ? out : own;
+        }
         if (lane < n) {
-          const R q = mine ? out : own;
           words[slot] = q;
           if constexpr (kPair) st_peer_word(peer_words + slot * (uint32_t)sizeof(R), q);
         }
@@ -748,6 +781,7 @@ __device__ __forceinline__ void st_try(const StreamArgs<float>&, const unsigned 
     q[k] = __uint_as_float((uint32_t)v[k]);
   }
 }
+// (FP64: the word of a cell that is not active is 0)
 __device__ __forceinline__ void st_try(const StreamArgs<double>& a, const double* word, uint32_t base,
                                        const uint32_t (&up)[4], uint32_t sweep, bool& ready, double (&q)[4]) {
   uint32_t v[4];
@@ -763,7 +797,7 @@ __device__ __forceinline__ void st_try(const StreamArgs<double>& a, const double
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     ready = ready && v[k] == sweep;
-    q[k] = up[k] != kSparseNone ? st_ldq(word + (up[k] & kSparseNone)) : 0.0;
+    q[k] = (up[k] & kSparseActive) ? st_ldq(word + (up[k] & kSparseNone)) : 0.0;
   }
 }
 __device__ __forceinline__ void st_publish(const StreamArgs<float>&, unsigned long long* word, uint32_t, uint32_t rel,
@@ -780,6 +814,7 @@ template <typename R>
 __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(const __grid_constant__ StreamArgs<R> a) {
   using Word = typename StreamTraits<R>::Word;
   constexpr uint32_t T = kStreamSparseThreads;
+  constexpr bool kChange = sizeof(R) == 8;
   const StreamDesc sd = a.streams[blockIdx.x];
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t sweep = a.epoch_base ? *a.epoch_base + a.epoch : a.epoch;
@@ -789,6 +824,7 @@ __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(co
   uint32_t solved = 0;
   for (uint32_t j0 = a.act_range[2 * blockIdx.x] + (threadIdx.x & ~31u); j0 < end; j0 += T) {
     bool todo = j0 + lane < end;
+    R before = R(0), own = R(0);
     StreamGroup gr{};
     uint32_t number = 0, i = 0, rel = 0, quads = 0;
     R att = R(0), per = R(0), src = R(0);
@@ -826,6 +862,10 @@ __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(co
       gr = a.groups[g];
       const uint32_t id = a.order[p];
       att = a.cell_att[id % a.Np];
+      if constexpr (kChange) {
+        before = __ldcg(inc + rel);
+        own = __ldcg(a.out + p);
+      }
       const StreamPiece<R> s(a.data + kStreamUnit * gr.data, gr);
       quads = s.quads;
       if (gr.shape & kGroupExt) {
@@ -839,7 +879,7 @@ __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(co
     }
     auto attempt = [&]() {
       bool ready = true;
-      StreamSum<R> sum;
+      StreamSum<R> sum(before);
       auto add = [&](bool odd, const StreamWeights<R>& w4, const uint32_t (&up4)[4]) {
         R q[4];
         st_try(a, word, sd.base, up4, sweep, ready, q);
@@ -858,8 +898,15 @@ __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(co
         }
       }
       if (ready) {
-        const R in = sum.total();
-        st_publish(a, word, sd.base, rel, st_solve(in, src, per, att, a.threshold, inv), sweep);
+        R in = sum.total();
+        if constexpr (kChange) {
+          in = st_positive(in);
+          const R out = st_solve(in, src, per, att, a.threshold, inv);
+          st_publish(a, word, sd.base, rel, out - own, sweep);
+          a.out[sd.base + rel] = out;
+        } else {
+          st_publish(a, word, sd.base, rel, st_solve(in, src, per, att, a.threshold, inv), sweep);
+        }
         inc[rel] = in;
         ++solved;
         todo = false;
@@ -907,7 +954,7 @@ __global__ void k_stream_gather(const StreamGroup* groups, uint32_t ngroups, uns
   }
 }
 
-// A sweep writes the incoming rates of the active cells only; those of the others are brought up
+// Mixed path: a sweep writes the incoming rates of the active cells only; those of the others are brought up
 // to date when something asks for them, as the reference keeps adding corrections to inactive
 // cells.  Out of date: a LOCAL neighbour was solved in a later sweep.
 static __global__ void k_stream_stale(uint32_t n, const uint32_t* off, const uint32_t* nbr, const uint32_t* cell_sweep,
@@ -923,28 +970,27 @@ static __global__ void k_stream_stale(uint32_t n, const uint32_t* off, const uin
   }
 }
 
-// From the words in memory, one fused multiply-add per slot in order (FP32: in face order, as
-// gather_in sums them).  grid: (streams, any).  Bound by the pieces' bytes: 64^3 x 84 in the mixed
+// From the words in memory, one fused multiply-add per slot in order (in face order, as gather_in
+// sums them).  grid: (streams, any).  Bound by the pieces' bytes: 64^3 x 84 in the mixed
 // path 1.5 ms per export from the geometry, 0.4 ms so.
-template <typename R>
-__global__ void k_stream_refresh(StreamArgs<R> a, const uint8_t* stale) {
+static __global__ void k_stream_refresh(StreamArgs<float> a, const uint8_t* stale) {
   const StreamDesc sd = a.streams[blockIdx.x];
   const uint32_t lane = threadIdx.x & 31, warps = gridDim.y * (blockDim.x / 32);
   const auto* word = a.word + sd.base;
   for (uint32_t number = blockIdx.y * (blockDim.x / 32) + threadIdx.x / 32; number < sd.groups; number += warps) {
     const StreamGroup gr = a.groups[sd.group0 + number];
     if (lane >= group_tasks(gr.shape) || stale[a.order[gr.pos + lane] % a.Np] == 0) continue;
-    const StreamPiece<R> s(a.data + kStreamUnit * gr.data, gr);
+    const StreamPiece<float> s(a.data + kStreamUnit * gr.data, gr);
     const uint32_t rel = gr.pos - sd.base + lane;
-    R sum = R(0);
+    float sum = 0.f;
     for (uint32_t j = 0; j < s.quads; ++j) {
-      StreamQuad<R> t;
+      StreamQuad<float> t;
       t.load(s, j, lane);
       const uint32_t x[4] = {t.x.x & 0xffffu, t.x.x >> 16, t.x.y & 0xffffu, t.x.y >> 16};
-      R q[4];
+      float q[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        q[k] = x[k] == a.shape.ring ? R(0) : st_ldq(word + stream_slot_position(a.shape, s, number, lane, rel, x[k]));
+        q[k] = x[k] == a.shape.ring ? 0.f : st_ldq(word + stream_slot_position(a.shape, s, number, lane, rel, x[k]));
 #pragma unroll
       for (int k = 0; k < 4; ++k) sum = fma(t.w.get(k), q[k], sum);
     }

@@ -1,12 +1,15 @@
 // Direction streams of the FP64 path: the pull form of Sweep::solve_task (src/sweep/mod.rs:423-485).
 //
-// The reference hands every downwind face the share (eff_f / total) of a task's outgoing rate,
-// with eff_f = area_f (n_f . d) and total the sum over the task's downwind faces in face order.
-// Here the receiving task sums the outgoing rates of its upwind tasks with the same fractions,
-// computed once per grid with the roundings of push_eff.  The share of face f of cell c comes
-// from the upwind cell's own face towards c (the reciprocal face, with the negated normal).
+// The reference hands every downwind face the share (eff_f / total) of the change of a task's
+// outgoing rate, with eff_f = area_f (n_f . d) and total the sum over the task's downwind faces in
+// face order, and the receiving task adds it to its incoming rate.  Here the receiving task adds
+// the shares of its upwind tasks' changes itself, with the same fractions, computed once per grid
+// with the roundings of push_eff.  The share of face f of cell c comes from the upwind cell's own
+// face towards c (the reciprocal face, with the negated normal).  The changes are summed, and not
+// the outgoing rates anew: near equilibrium the timescale of a cell shows the last bits of its rate,
+// those that a history of changes left in it among them.
 //
-// The outgoing and incoming rates lie by schedule position.
+// The outgoing and incoming rates and the changes lie by schedule position.
 #pragma once
 
 #include "sweep_push_records.cuh"
@@ -225,18 +228,65 @@ static __global__ void k_fold_mark64(SweepArgs<double> a, const double* cell_att
   }
 }
 
-// grid: (periodic cells / blockDim.x, D)
-static __global__ void k_fold64(const double* out, double* periodic, uint32_t Np, const uint32_t* cells,
-                                uint32_t n_cells, const uint32_t* off, const FoldSlot64* slots, const uint8_t* changed) {
+// grid: (periodic cells / blockDim.x, D).  active: bitmap of the positions that a sparse sweep has
+// solved (the changes of the others are of an earlier sweep), or null
+static __global__ void k_fold64(const double* change, double* periodic, uint32_t Np, const uint32_t* cells,
+                                uint32_t n_cells, const uint32_t* off, const FoldSlot64* slots, const uint8_t* changed,
+                                const uint32_t* active) {
   const uint32_t d = blockIdx.y, pc = blockIdx.x * blockDim.x + threadIdx.x;
   if (pc >= n_cells || (changed && !changed[pc])) return;
   const size_t e = (size_t)d * n_cells + pc;
   double in = 0.0;
   for (uint32_t k = off[e]; k < off[e + 1]; ++k) {
     const FoldSlot64 s = slots[k];
-    in = fma(s.frac, out[s.pos], in);
+    if (active && !(active[s.pos >> 5] >> (s.pos & 31u) & 1u)) continue;
+    in = fma(s.frac, change[s.pos], in);
   }
-  periodic[(size_t)d * Np + cells[pc]] = in;
+  if (in != 0.0) periodic[(size_t)d * Np + cells[pc]] += in;
+}
+
+// After a sparse sweep: its changes reach the tasks of inactive cells as well.
+// The inactive cells beside an active one.
+static __global__ void k_cells_near64(uint32_t n, const uint8_t* level, int cur, const uint32_t* off,
+                                      const uint32_t* nbr, uint8_t* near) {
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+    uint8_t s = 0;
+    if (level[c] < cur)
+      for (uint32_t f = off[c]; f < off[c + 1] && !s; ++f)
+        s = (nbr[f] >> kKindShift) == kKindLocal && level[nbr[f] & kNbrMask] >= cur;
+    near[c] = s;
+  }
+}
+
+// Adds the changes upwind to their incoming rates, in the order of the dense sweep.  grid: (streams,
+// any).  A pass over the whole device and not part of the streams' walk, where such tasks would
+// be waited for like those that others depend on.
+static __global__ void k_stream_take64(StreamArgs<double> a, const uint8_t* near) {
+  const StreamDesc sd = a.streams[blockIdx.x];
+  const uint32_t lane = threadIdx.x & 31, warps = gridDim.y * (blockDim.x / 32);
+  const double* word = a.word + sd.base;
+  for (uint32_t number = blockIdx.y * (blockDim.x / 32) + threadIdx.x / 32; number < sd.groups; number += warps) {
+    const StreamGroup gr = a.groups[sd.group0 + number];
+    if (lane >= group_tasks(gr.shape) || near[a.order[gr.pos + lane] % a.Np] == 0) continue;
+    const StreamPiece<double> s(a.data + kStreamUnit * gr.data, gr);
+    const uint32_t rel = gr.pos - sd.base + lane;
+    double sum = 0.0;
+    bool any = false;
+    for (uint32_t j = 0; j < s.quads; ++j) {
+      const uint2 v = reinterpret_cast<const uint2*>(s.idx())[j * 32 + lane];
+      const uint32_t x[4] = {v.x & 0xffffu, v.x >> 16, v.y & 0xffffu, v.y >> 16};
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) {
+        if (x[k] == a.shape.ring) continue;
+        const uint32_t u = stream_slot_position(a.shape, s, number, lane, rel, x[k]), q = sd.base + u;
+        if (!(a.act_bits[q >> 5] >> (q & 31u) & 1u)) continue;
+        if (!any) sum = a.inc[sd.base + rel];
+        any = true;
+        sum = fma(s.w()[StreamPiece<double>::wslot(4 * j + k, lane)], st_ldq(word + u), sum);
+      }
+    }
+    if (any) a.inc[sd.base + rel] = sum;
+  }
 }
 
 }  // namespace swk
