@@ -857,7 +857,6 @@ sw_status build_streams(sw_handle* h) {
     pairs = pairs_pay(levels, longest / swk::kStreamGroup, total, p.num_sms, rb == 4);
     if (const char* env = std::getenv("SUBSWEEP_STREAM_PAIRS")) pairs = std::atoi(env) != 0;
   }
-  if (pairs) warps = swk::kPairWarps;
   uint32_t slots = 0;  // per task of the largest group
   for (const auto& m : h->stream_gmax)
     for (uint8_t v : m) slots = std::max<uint32_t>(slots, (v + 3u) & ~3u);
@@ -886,14 +885,35 @@ sw_status build_streams(sw_handle* h) {
                              60000 - (int64_t)warps * far * 32);
   };
   size_t room = 0;
-  const int most = pairs ? 1 : std::max(1, std::min(8, (int)(48 / warps)));  // blocks per SM that their registers allow
-  for (int k = std::max(1, std::min(most, (int)((h->streams.size() + p.num_sms - 1) / p.num_sms))); k >= 1; --k) {
-    room = std::min((size_t)optin, (size_t)per_sm / k - 1024);
-    if (words_for(room, swk::kStreamFar) >= (int64_t)std::min(longest, 8192u)) break;
-  }
-  // a ring must not wrap inside a level: with a wider one the grid keeps the levelled schedule
-  if (words_for(room, swk::kStreamFar) < (int64_t)std::min(longest, widest)) {
-    return give_up();
+  uint32_t* shape = p.stream_shape;
+  int resident = 0;  // pairs at once
+  const uint32_t single = warps;
+  for (;; pairs = false) {
+    warps = pairs ? swk::kPairWarps : single;
+    const int most = pairs ? 1 : std::max(1, std::min(8, (int)(48 / warps)));  // blocks per SM that registers allow
+    for (int k = std::max(1, std::min(most, (int)((h->streams.size() + p.num_sms - 1) / p.num_sms))); k >= 1; --k) {
+      room = std::min((size_t)optin, (size_t)per_sm / k - 1024);
+      if (words_for(room, swk::kStreamFar) >= (int64_t)std::min(longest, 8192u)) break;
+    }
+    const int64_t ring = words_for(room, swk::kStreamFar);
+    // a ring must not wrap inside a level: with a wider one the grid keeps the levelled schedule
+    if (ring < (int64_t)std::min(longest, widest)) {
+      if (pairs) continue;
+      return give_up();
+    }
+    if (!pairs) break;
+    // with the most shared memory that the layout may ask for; none: single blocks
+    const uint32_t largest[6] = {(uint32_t)ring, 0u, swk::kStreamFar, warps, buffer, 2u};
+    std::copy(largest, largest + 6, shape);
+    if (h->ops->stream_pairs(p, &resident) != cudaSuccess) {
+      (void)cudaGetLastError();
+      resident = 0;
+    }
+    if (const char* env = std::getenv("SUBSWEEP_STREAM_PAIRS")) {  // at most so many, or (-1) none
+      const int v = std::atoi(env);
+      if (v > 1 || v < 0) resident = std::min(resident, std::max(v, 0));
+    }
+    if (resident >= 1) break;
   }
   std::vector<swk::StreamGroup> groups(seg_group[segs]);
   {
@@ -960,7 +980,6 @@ sw_status build_streams(sw_handle* h) {
           "streams");
   SW_CUDA(h, cudaMemcpy(p.seg_group, seg_group.data(), seg_group.size() * 4, cudaMemcpyHostToDevice), "streams");
   SW_CUDA(h, h->ops->stream_build(p, 0, b, h->stream), "stream position kernels");
-  uint32_t* shape = p.stream_shape;
   shape[3] = warps;
   shape[5] = pairs ? 2u : 1u;
   bool far = false;
@@ -988,26 +1007,18 @@ sw_status build_streams(sw_handle* h) {
     if (far == (shape[2] != 0u)) break;
   }
   if (pairs) {
-    int resident = 0;
-    SW_CUDA(h, h->ops->stream_pairs(p, &resident), "pairs of blocks");
-    if (const char* env = std::getenv("SUBSWEEP_STREAM_PAIRS"))
-      if (std::atoi(env) > 1) resident = std::min(resident, std::atoi(env));
-    if (resident < 1) {
-      shape[5] = 1u;
-    } else {
-      std::vector<swk::StreamPart> parts;
-      std::vector<uint32_t> part0;
-      plan_parts(h->streams, seg_group, (uint32_t)resident, parts, part0);
-      swk::StreamPart* d_parts = nullptr;
-      if (!h->stream_alloc(&d_parts, parts.size()) || !h->stream_alloc(&p.stream_part0, part0.size()) ||
-          !h->stream_alloc(&p.stream_flags, part0.size()))
-        return give_up();
-      SW_CUDA(h, cudaMemcpy(d_parts, parts.data(), parts.size() * sizeof(parts[0]), cudaMemcpyHostToDevice), "streams");
-      SW_CUDA(h, cudaMemcpy(p.stream_part0, part0.data(), part0.size() * 4, cudaMemcpyHostToDevice), "streams");
-      SW_CUDA(h, cudaMemset(p.stream_flags, 0xff, part0.size() * 4), "streams");
-      p.stream_parts = d_parts;
-      p.num_pairs = (uint32_t)part0.size() - 1;
-    }
+    std::vector<swk::StreamPart> parts;
+    std::vector<uint32_t> part0;
+    plan_parts(h->streams, seg_group, (uint32_t)resident, parts, part0);
+    swk::StreamPart* d_parts = nullptr;
+    if (!h->stream_alloc(&d_parts, parts.size()) || !h->stream_alloc(&p.stream_part0, part0.size()) ||
+        !h->stream_alloc(&p.stream_flags, part0.size()))
+      return give_up();
+    SW_CUDA(h, cudaMemcpy(d_parts, parts.data(), parts.size() * sizeof(parts[0]), cudaMemcpyHostToDevice), "streams");
+    SW_CUDA(h, cudaMemcpy(p.stream_part0, part0.data(), part0.size() * 4, cudaMemcpyHostToDevice), "streams");
+    SW_CUDA(h, cudaMemset(p.stream_flags, 0xff, part0.size() * 4), "streams");
+    p.stream_parts = d_parts;
+    p.num_pairs = (uint32_t)part0.size() - 1;
   }
   uint64_t at = 0;
   for (swk::StreamGroup& g : groups) {

@@ -201,7 +201,8 @@ cudaError_t sweep_stream(const DevicePtrs& p, int level, cudaStream_t s) {
   switch (p.stream_shape[3]) {
     case 4: return launch_stream<4>(p, all, s);
     case 8: return launch_stream<8>(p, all, s);
-    default: return launch_stream<16>(p, all, s);
+    case 16: return launch_stream<16>(p, all, s);
+    default: return cudaErrorInvalidValue;  // (the layout goes by the number of warps)
   }
 }
 

@@ -92,3 +92,17 @@ def test_grids_whose_streams_run_out_of_memory(precision, pairs, monkeypatch, ca
         with make(w, monkeypatch, env, precision) as s:
             same(w, precision, expected, results(s))
     assert 8 <= arrays < 63
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_pairs_that_cannot_be_resident_are_single_blocks(precision, monkeypatch, capfd):
+    # (40^3: far words, whose slots go by the warps of a block)
+    w = workloads.c4_grf(n_per_side=40, num_sources=3, num_directions=16, nthreads=8, grid_device="gpu")
+    got = {}
+    for pairs in ("0", "-1"):
+        env = {"SUBSWEEP_STREAMS": "1", "SUBSWEEP_STREAM_PAIRS": pairs}
+        assert streams_bytes(w, monkeypatch, capfd, precision, env)
+        with make(w, monkeypatch, env, precision) as s:
+            got[pairs] = results(s)
+    for k, a in got["0"].items():
+        np.testing.assert_array_equal(a, got["-1"][k], err_msg=k)
