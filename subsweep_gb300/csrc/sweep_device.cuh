@@ -834,6 +834,7 @@ __device__ __forceinline__ int desired_level(double max_timestep, double desired
 // level histogram.
 static __global__ void k_update_levels(uint32_t n, const double* change_timescale, uint8_t* level, double safety,
                                        double max_timestep, int num_levels, int lowest, SweepCtl* ctl) {
+  if (ctl->error & kErrFailed) return;  // a failed step leaves the levels alone
   __shared__ uint32_t hist[32];
   if (threadIdx.x < 32) hist[threadIdx.x] = 0;
   __syncthreads();
@@ -859,6 +860,7 @@ static __global__ void k_level_hist(uint32_t n, const uint8_t* level, int num_le
 
 // n_ge[l] = #cells with level >= l, from the histogram (which is then cleared).
 static __global__ void k_level_counts(SweepCtl* ctl, int num_levels) {
+  if (ctl->error & kErrFailed) return;
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     uint32_t acc = 0;
     for (int l = num_levels - 1; l >= 0; --l) {
@@ -871,7 +873,8 @@ static __global__ void k_level_counts(SweepCtl* ctl, int num_levels) {
 
 // IonizationTime write-back of run_sweep_system (src/sweep/mod.rs:731-738).
 static __global__ void k_ionization_time(uint32_t n, const double* xhii, double* ionization_time, double time,
-                                         const double* time_dev) {
+                                         const double* time_dev, const SweepCtl* ctl) {
+  if (ctl->error & kErrFailed) return;
   if (time_dev) time = *time_dev;
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
     if (xhii[c] > 0.5 && isinf(ionization_time[c])) ionization_time[c] = time;

@@ -154,6 +154,12 @@ struct sw_handle {
   int tune_index = 0;
   std::vector<double> tune_ns;  // ns per task of each candidate
   std::vector<cudaEvent_t> graph_ev;  // start / end of each sweep's transport inside the graph
+  // whether a cell's x_HII may lie above what the chemistry's clamp takes for a floor
+  bool floor_unsafe = false;
+  void look_at_floors(const double* x) {
+    floor_unsafe = !(params.chemistry_timestep_safety_factor < 1.0);  // (a change of any size may pass)
+    for (int64_t c = 0; c < N && !floor_unsafe; ++c) floor_unsafe = !(x[c] <= 1.0 - 1e-10);
+  }
   uint32_t last_epoch = 0;  // pull path: sweep number of the last sweep of the last step
 
   ~sw_handle() {
@@ -1311,6 +1317,7 @@ sw_status sw_create(const sw_params* params, const sw_grid_csr* grid, const sw_c
   h->N = N;
   h->E = E;
   h->ts.init(P.max_timestep, P.num_timestep_levels);
+  h->look_at_floors(init->ionized_hydrogen_fraction);
 
   auto bail = [&](sw_status st) {
     g_create_error = h->last_error;
@@ -1981,8 +1988,11 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
   SW_CUDA(h, cudaEventRecord(h->ev[5], h->stream), "event");
   // The sweeps are launched one behind another and looked at when the host waits for them, at
   // the step's end (or after kMaxInFlight, or one by one while variants are tried or traced).
-  // The error flag stays set across them: a stall ends the sweeps behind it at once, and they
-  // leave the cells alone.
+  // A failure that can be foreseen is looked for sweep by sweep, and the first one ends the step:
+  // the stall of a grid without a schedule, and a floor that the chemistry refuses.  Otherwise the
+  // error flag stays set across the sweeps: after a stall no stream waits any longer, and no kernel
+  // changes a cell, its level or its ionization time.
+  const bool may_fail = h->p.num_sched_levels == 0 || (h->params.prevent_cooling && h->floor_unsafe);
   SW_CUDA(h, cudaMemsetAsync(&h->p.ctl->error, 0, sizeof(uint32_t), h->stream), "reset error flag");
   std::vector<int> in_flight;  // levels
   bool trial = false;
@@ -2100,7 +2110,7 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
                                h->stream), "read error flag");
     in_flight.push_back(level);
     h->stats.transport_launches += 1;
-    if (trial || h->trace || (int)in_flight.size() == sw_handle::kMaxInFlight) {
+    if (trial || h->trace || may_fail || (int)in_flight.size() == sw_handle::kMaxInFlight) {
       SW_CUDA(h, cudaStreamSynchronize(h->stream), "level sweep");
       const sw_status st = look();
       if (st != SW_OK) return st;
@@ -2186,6 +2196,7 @@ sw_status sw_set_fields(sw_handle* h, const double* x, const double* T) {
   if (x) {
     std::vector<double> y(h->N);
     for (int64_t c = 0; c < h->N; ++c) y[c] = 1.0 - x[c];
+    h->look_at_floors(x);
     SW_CUDA(h, cudaMemcpy(h->p.xhii, x, nb, cudaMemcpyHostToDevice), "copy x");
     SW_CUDA(h, cudaMemcpy(h->p.yneu, y.data(), nb, cudaMemcpyHostToDevice), "copy y");
   }
@@ -2530,6 +2541,11 @@ sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) {
   }
   size_t off = sizeof(hd);
   for (const CheckpointSection& s : checkpoint_sections(h)) {
+    if (s.dev == h->p.xhii) {
+      std::vector<double> x(h->N);
+      std::memcpy(x.data(), in + off, s.bytes);
+      h->look_at_floors(x.data());
+    }
     SW_CUDA(h, cudaMemcpyAsync(s.dev, in + off, s.bytes, cudaMemcpyHostToDevice, h->stream), "load state");
     off += s.bytes;
   }
@@ -2551,8 +2567,9 @@ sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) {
     q.active_cells = h->N;  // every entry
     SW_CUDA(h, h->ops->fold_periodic(q, h->stream), "periodic fold kernel");
   }
-  // cells per level for the next step
+  // cells per level for the next step (an earlier step's failure is over)
   h->act_valid = 0;
+  SW_CUDA(h, cudaMemsetAsync(&h->p.ctl->error, 0, sizeof(uint32_t), h->stream), "reset error flag");
   SW_CUDA(h, swh::launch_level_hist(h->p, h->stream), "level histogram");
   return sync_ctl(h);
 }

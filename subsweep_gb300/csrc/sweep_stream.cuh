@@ -164,6 +164,12 @@ __device__ __forceinline__ uint32_t st_count(const uint32_t* p) {
 __device__ __forceinline__ void st_count_up(uint32_t* p) {
   asm volatile("red.release.cta.shared::cta.add.u32 [%0], 1;" ::"r"(st_smem(p)) : "memory");
 }
+// whether a sweep of the step has stalled
+__device__ __forceinline__ bool st_stalled(const SweepCtl* ctl) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&ctl->error) : "memory");
+  return (v & kErrStall) != 0;
+}
 // bounded wait of a warp; on a timeout sets kErrStall and returns false, and the caller goes
 // on without waiting or solving (it still counts its groups, so no other warp waits for them)
 template <typename Test>
@@ -175,7 +181,7 @@ __device__ __forceinline__ bool st_wait(Test test, SweepCtl* ctl, unsigned long 
       if ((k & 255u) == 0) {
         const unsigned long long now = globaltimer_ns();
         if (w0 == 0) w0 = now;
-        if (now - w0 > limit) break;
+        if (now - w0 > limit || st_stalled(ctl)) break;
       }
     }
     if (!ok) atomicOr(&ctl->error, kErrStall);
@@ -918,7 +924,7 @@ __global__ void __launch_bounds__(kStreamSparseThreads) k_sweep_stream_sparse(co
       if ((k & 255u) == 0) {
         const unsigned long long now = __shfl_sync(0xffffffffu, globaltimer_ns(), 0);
         if (w0 == 0) w0 = now;
-        if (now - w0 > a.timeout_ns) break;
+        if (now - w0 > a.timeout_ns || __any_sync(0xffffffffu, st_stalled(a.ctl))) break;
       }
     }
     if (__any_sync(0xffffffffu, todo)) {  // stalled: those that wait for this warp's tasks run out as well

@@ -53,6 +53,7 @@ constexpr uint32_t kGroupKeep = 1u << 15;  // a word of it is a far word of anot
 constexpr uint32_t kStreamFar = 8;         // far words of a task in the buffer at most
 
 enum : uint32_t { kErrStall = 1u, kErrQueue = 2u, kErrClamp = 8u, kErrRecords = 16u };
+constexpr uint32_t kErrFailed = kErrStall | kErrQueue | kErrClamp;  // of a step
 
 // Control block of one handle (device memory).
 struct SweepCtl {
