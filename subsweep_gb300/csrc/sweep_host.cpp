@@ -1994,12 +1994,16 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
   // changes a cell, its level or its ionization time.
   const bool may_fail = h->p.num_sched_levels == 0 || (h->params.prevent_cooling && h->floor_unsafe);
   SW_CUDA(h, cudaMemsetAsync(&h->p.ctl->error, 0, sizeof(uint32_t), h->stream), "reset error flag");
-  std::vector<int> in_flight;  // levels
-  bool trial = false;
+  struct InFlight {
+    int level;
+    bool trial;  // of a transport variant
+  };
+  std::vector<InFlight> in_flight;
   auto look = [&]() -> sw_status {  // the stream has been synchronized
     for (size_t k = 0; k < in_flight.size(); ++k) {
       const auto& ev = h->sweep_ev[k];
-      const int level = in_flight[k];
+      const int level = in_flight[k].level;
+      const bool trial = in_flight[k].trial;
       float a = 0.f, b = 0.f, t = 0.f;
       cudaEventElapsedTime(&a, ev[0], ev[3]);
       cudaEventElapsedTime(&b, ev[3], ev[4]);
@@ -2064,7 +2068,7 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
     if (h->force_path == 1) levelled = h->p.num_sched_levels > 0;
     if (h->force_path == 2) levelled = false;
     // autotuning trials on dense sweeps only: sparse ones always run the lockstep kernel
-    trial = ops.pull && h->autotune && !h->tuned && !pull_sparse(h, level);
+    const bool trial = ops.pull && h->autotune && !h->tuned && !pull_sparse(h, level);
     if (trial && !h->p.stream_mode) h->p.pull_variant = ops.tune_variants[h->tune_index];
     if (h->pulls()) {
       levelled = true;  // the pull path always walks the schedule (or the id order)
@@ -2108,7 +2112,7 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
     SW_CUDA(h, cudaEventRecord(ev[4], h->stream), "event");
     SW_CUDA(h, cudaMemcpyAsync(&h->pinned->error[slot], &h->p.ctl->error, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                h->stream), "read error flag");
-    in_flight.push_back(level);
+    in_flight.push_back({level, trial});
     h->stats.transport_launches += 1;
     if (trial || h->trace || may_fail || (int)in_flight.size() == sw_handle::kMaxInFlight) {
       SW_CUDA(h, cudaStreamSynchronize(h->stream), "level sweep");
