@@ -185,6 +185,13 @@ struct sw_handle {
     return true;
   }
 
+  // The stream does not wait for the default stream, nor that for it: copies and sets of the arrays
+  // that kernels use go by the stream.  Returns when the host's side of the copy is free.
+  cudaError_t copy(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
+  }
+
   // one of the streams' arrays: counted, so that a test can let any of them find no memory
   template <typename T>
   bool stream_alloc(T** ptr, size_t count) {
@@ -578,7 +585,7 @@ sw_status build_schedule(sw_handle* h) {
     std::vector<uint8_t> up;  // upwind LOCAL faces of every task (the rounds count them down)
     if (h->want_streams) {
       up.resize((size_t)h->Np * q.D);
-      SW_CUDA(h, cudaMemcpy(up.data(), p.counters, up.size(), cudaMemcpyDeviceToHost), "read upwind counts");
+      SW_CUDA(h, h->copy(up.data(), p.counters, up.size(), cudaMemcpyDeviceToHost), "read upwind counts");
     }
     // the rounds, kRounds at a time (those after the last one find nothing to do)
     constexpr uint32_t kRounds = 32, kMaxRounds = 0xffffu;
@@ -586,7 +593,7 @@ sw_status build_schedule(sw_handle* h) {
     SW_CUDA(h, cudaMalloc(&bounds_scratch.ptr, (kMaxRounds + kRounds + 2) * sizeof(uint32_t)), "schedule scratch");
     uint32_t* bounds = static_cast<uint32_t*>(bounds_scratch.ptr) + 1;  // behind the blocks' count
     const uint32_t first[3] = {0u, 0u, (uint32_t)tail};
-    SW_CUDA(h, cudaMemcpy(bounds - 1, first, sizeof(first), cudaMemcpyHostToDevice), "schedule scratch");
+    SW_CUDA(h, h->copy(bounds - 1, first, sizeof(first), cudaMemcpyHostToDevice), "schedule scratch");
     uint32_t end = (uint32_t)tail;
     if (end > 0) lvl.push_back(end);
     for (uint32_t round = 0; end > 0;) {
@@ -608,7 +615,7 @@ sw_status build_schedule(sw_handle* h) {
     tail = end;
     if (lvl.size() - 1 >= kMaxRounds) return h->fail(SW_ERR_UNSUPPORTED, "dependency graph deeper than 65534 levels");
     uint32_t err = 0;
-    SW_CUDA(h, cudaMemcpy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
+    SW_CUDA(h, h->copy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
     if (tail != total || err != 0) {
       if (p.geo_mode) return h->fail(SW_ERR_STALLED, "the dependency graph has a cycle (compact state)");
       // cyclic dependency graph: no schedule.  The push path falls back to the
@@ -621,7 +628,7 @@ sw_status build_schedule(sw_handle* h) {
         ids.reserve(total);
         for (uint32_t d = 0; d < (uint32_t)h->D; ++d)
           for (uint32_t c = 0; c < (uint32_t)h->N; ++c) ids.push_back(d * h->Np + c);
-        SW_CUDA(h, cudaMemcpy(p.order, ids.data(), ids.size() * sizeof(uint32_t), cudaMemcpyHostToDevice), "order");
+        SW_CUDA(h, h->copy(p.order, ids.data(), ids.size() * sizeof(uint32_t), cudaMemcpyHostToDevice), "order");
       }
       SW_CUDA(h, cudaMemsetAsync(p.ctl, 0, offsetof(swk::SweepCtl, tasks), h->stream), "reset control");
       return SW_OK;
@@ -644,7 +651,7 @@ sw_status build_schedule(sw_handle* h) {
     std::vector<uint32_t> seg = {0};
     {
       std::vector<uint16_t> tl((size_t)h->Np * q.D);
-      SW_CUDA(h, cudaMemcpy(tl.data(), task_level, tl.size() * sizeof(uint16_t), cudaMemcpyDeviceToHost),
+      SW_CUDA(h, h->copy(tl.data(), task_level, tl.size() * sizeof(uint16_t), cudaMemcpyDeviceToHost),
               "read task levels");
       std::vector<uint32_t> order(total);
       if (h->want_streams) {
@@ -655,15 +662,15 @@ sw_status build_schedule(sw_handle* h) {
                  total) {
         return h->fail(SW_ERR_CUDA, "schedule order incomplete");
       }
-      SW_CUDA(h, cudaMemcpy(q.order, order.data(), order.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
+      SW_CUDA(h, h->copy(q.order, order.data(), order.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
               "upload order");
     }
     uint32_t* d_lvl;
     // padded to a multiple of four entries: the staged wavefront kernel copies them whole
     const size_t lvl_words = (seg.size() + 3) & ~(size_t)3;
     if (!h->alloc(&d_lvl, lvl_words)) return h->fail(SW_ERR_OOM, "device allocation of the schedule failed");
-    SW_CUDA(h, cudaMemset(d_lvl, 0, lvl_words * sizeof(uint32_t)), "schedule");
-    SW_CUDA(h, cudaMemcpy(d_lvl, seg.data(), seg.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
+    SW_CUDA(h, cudaMemsetAsync(d_lvl, 0, lvl_words * sizeof(uint32_t), h->stream), "schedule");
+    SW_CUDA(h, h->copy(d_lvl, seg.data(), seg.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
             "upload schedule");
     p.space_lvl[sp] = d_lvl;
     p.space_segments[sp] = (uint32_t)(seg.size() - 1);
@@ -732,7 +739,7 @@ sw_status build_push_records(sw_handle* h) {
   ce = h->ops->push_records(p, 1, chunk_off, h->stream);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);
   uint32_t err = 0;
-  if (ce == cudaSuccess) ce = cudaMemcpy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost);
+  if (ce == cudaSuccess) ce = h->copy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost);
   if (ce != cudaSuccess) {
     p.push_rec = nullptr;
     return h->cuda_fail(ce, "downwind fraction kernel");
@@ -945,6 +952,7 @@ sw_status build_streams(sw_handle* h) {
     return give_up();
   }
   struct Scratch {
+    sw_handle* h;
     std::vector<void*> mem;
     ~Scratch() {
       for (void* m : mem) cudaFree(m);
@@ -953,9 +961,9 @@ sw_status build_streams(sw_handle* h) {
       cudaError_t e = cudaMalloc(out, std::max<size_t>(bytes, 4));
       if (e != cudaSuccess) return e;
       mem.push_back(*out);
-      return src ? cudaMemcpy(*out, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
+      return src ? h->copy(*out, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
     }
-  } scratch;
+  } scratch{h, {}};
   swh::StreamScratch b{};
   SW_ROOM(h, scratch.get((void**)&b.gseg, groups.size() * 4, nullptr), "stream scratch");
   SW_ROOM(h, scratch.get((void**)&b.sbase, sbase.size() * 4, sbase.data()), "stream scratch");
@@ -982,9 +990,9 @@ sw_status build_streams(sw_handle* h) {
   const size_t group_bytes = groups.size() * sizeof(groups[0]);
   std::stable_sort(h->streams.begin(), h->streams.end(),  // launch order: the longest first
                    [](const swk::StreamDesc& x, const swk::StreamDesc& y) { return x.count > y.count; });
-  SW_CUDA(h, cudaMemcpy(d_streams, h->streams.data(), h->streams.size() * sizeof(h->streams[0]), cudaMemcpyHostToDevice),
+  SW_CUDA(h, h->copy(d_streams, h->streams.data(), h->streams.size() * sizeof(h->streams[0]), cudaMemcpyHostToDevice),
           "streams");
-  SW_CUDA(h, cudaMemcpy(p.seg_group, seg_group.data(), seg_group.size() * 4, cudaMemcpyHostToDevice), "streams");
+  SW_CUDA(h, h->copy(p.seg_group, seg_group.data(), seg_group.size() * 4, cudaMemcpyHostToDevice), "streams");
   SW_CUDA(h, h->ops->stream_build(p, 0, b, h->stream), "stream position kernels");
   shape[3] = warps;
   shape[5] = pairs ? 2u : 1u;
@@ -999,10 +1007,10 @@ sw_status build_streams(sw_handle* h) {
     shape[0] = (uint32_t)std::min<int64_t>(words_for(room, shape[2]), longest);
     shape[1] = (uint32_t)((1ull << 32) / shape[0]) + 1u;
     for (swk::StreamGroup& g : groups) g.shape &= 0xfffu;
-    SW_CUDA(h, cudaMemcpy(d_groups, groups.data(), group_bytes, cudaMemcpyHostToDevice), "groups");
+    SW_CUDA(h, h->copy(d_groups, groups.data(), group_bytes, cudaMemcpyHostToDevice), "groups");
     SW_CUDA(h, h->ops->stream_build(p, 1, b, h->stream), "stream flag kernel");
     SW_CUDA(h, cudaStreamSynchronize(h->stream), "stream flags");
-    SW_CUDA(h, cudaMemcpy(groups.data(), d_groups, group_bytes, cudaMemcpyDeviceToHost), "groups");
+    SW_CUDA(h, h->copy(groups.data(), d_groups, group_bytes, cudaMemcpyDeviceToHost), "groups");
     far = false;
     late = slow = 0;
     for (const swk::StreamGroup& g : groups) {
@@ -1020,9 +1028,9 @@ sw_status build_streams(sw_handle* h) {
     if (!h->stream_alloc(&d_parts, parts.size()) || !h->stream_alloc(&p.stream_part0, part0.size()) ||
         !h->stream_alloc(&p.stream_flags, part0.size()))
       return give_up();
-    SW_CUDA(h, cudaMemcpy(d_parts, parts.data(), parts.size() * sizeof(parts[0]), cudaMemcpyHostToDevice), "streams");
-    SW_CUDA(h, cudaMemcpy(p.stream_part0, part0.data(), part0.size() * 4, cudaMemcpyHostToDevice), "streams");
-    SW_CUDA(h, cudaMemset(p.stream_flags, 0xff, part0.size() * 4), "streams");
+    SW_CUDA(h, h->copy(d_parts, parts.data(), parts.size() * sizeof(parts[0]), cudaMemcpyHostToDevice), "streams");
+    SW_CUDA(h, h->copy(p.stream_part0, part0.data(), part0.size() * 4, cudaMemcpyHostToDevice), "streams");
+    SW_CUDA(h, cudaMemsetAsync(p.stream_flags, 0xff, part0.size() * 4, h->stream), "streams");
     p.stream_parts = d_parts;
     p.num_pairs = (uint32_t)part0.size() - 1;
   }
@@ -1035,21 +1043,21 @@ sw_status build_streams(sw_handle* h) {
   if (at / swk::kStreamUnit > 0xffffffffull) {  // past the pieces' 32-bit offsets: the levelled schedule
     return give_up();
   }
-  SW_CUDA(h, cudaMemcpy(d_groups, groups.data(), groups.size() * sizeof(groups[0]), cudaMemcpyHostToDevice), "groups");
+  SW_CUDA(h, h->copy(d_groups, groups.data(), groups.size() * sizeof(groups[0]), cudaMemcpyHostToDevice), "groups");
   groups.pop_back();
   SW_CUDA(h, cudaMemGetInfo(&free_b, &total_b), "memory info");
   if (at + reserve > free_b || at > h->stream_limit || !h->stream_alloc(&p.stream_data, at)) return give_up();
   char* cell_att = nullptr;
   std::vector<uint32_t> pcells(p.n_periodic_cells);
   std::vector<uint8_t> has_periodic(h->N, 0);
-  SW_CUDA(h, cudaMemcpy(pcells.data(), p.periodic_cells, pcells.size() * 4, cudaMemcpyDeviceToHost), "periodic cells");
+  SW_CUDA(h, h->copy(pcells.data(), p.periodic_cells, pcells.size() * 4, cudaMemcpyDeviceToHost), "periodic cells");
   for (uint32_t c : pcells) has_periodic[c] = 1;
   if (!h->stream_alloc(&cell_att, (size_t)h->N * rb) || !h->stream_alloc(&p.cell_rate, h->N) ||
       !h->stream_alloc(&p.cell_periodic, h->N) || !h->stream_alloc(&p.stale, h->N))
     return give_up();
   p.stream_bytes = at;
   p.cell_att = cell_att;
-  SW_CUDA(h, cudaMemcpy(p.cell_periodic, has_periodic.data(), h->N, cudaMemcpyHostToDevice), "periodic cells");
+  SW_CUDA(h, h->copy(p.cell_periodic, has_periodic.data(), h->N, cudaMemcpyHostToDevice), "periodic cells");
   SW_CUDA(h, cudaMemsetAsync(p.ctl, 0, offsetof(swk::SweepCtl, tasks), h->stream), "reset control");
   SW_CUDA(h, h->ops->stream_build(p, 2, b, h->stream), "upwind slot kernel");
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "upwind slots");
@@ -1062,10 +1070,10 @@ sw_status build_streams(sw_handle* h) {
     SW_CUDA(h, cudaStreamSynchronize(h->stream), "periodic fold entries");
     p.fold_cnt = nullptr;
     std::vector<uint8_t> n(entries);
-    SW_CUDA(h, cudaMemcpy(n.data(), cnt, entries, cudaMemcpyDeviceToHost), "periodic fold entries");
+    SW_CUDA(h, h->copy(n.data(), cnt, entries, cudaMemcpyDeviceToHost), "periodic fold entries");
     std::vector<uint32_t> off(entries + 1, 0u);
     for (size_t e = 0; e < entries; ++e) off[e + 1] = off[e] + n[e];
-    SW_CUDA(h, cudaMemcpy(p.fold_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice), "periodic fold entries");
+    SW_CUDA(h, h->copy(p.fold_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice), "periodic fold entries");
     uint4* fslots = nullptr;
     if (!h->stream_alloc(&fslots, off[entries])) return give_up();
     p.fold_slots = fslots;
@@ -1074,16 +1082,16 @@ sw_status build_streams(sw_handle* h) {
   }
   if (rb == 8) {
     unsigned long long faces[2] = {0, 0};  // handed out, found
-    SW_CUDA(h, cudaMemcpy(&faces[0], &p.ctl->head, 8, cudaMemcpyDeviceToHost), "upwind slots");
-    SW_CUDA(h, cudaMemcpy(&faces[1], &p.ctl->tail, 8, cudaMemcpyDeviceToHost), "upwind slots");
+    SW_CUDA(h, h->copy(&faces[0], &p.ctl->head, 8, cudaMemcpyDeviceToHost), "upwind slots");
+    SW_CUDA(h, h->copy(&faces[1], &p.ctl->tail, 8, cudaMemcpyDeviceToHost), "upwind slots");
     const size_t nd = (size_t)h->Np * h->D;
-    SW_CUDA(h, cudaMemset(p.pending, 0, nd * 8), "pending rates");
-    SW_CUDA(h, cudaMemset(p.ctl, 0, offsetof(swk::SweepCtl, error)), "reset control");
+    SW_CUDA(h, cudaMemsetAsync(p.pending, 0, nd * 8, h->stream), "pending rates");
+    SW_CUDA(h, cudaMemsetAsync(p.ctl, 0, offsetof(swk::SweepCtl, error), h->stream), "reset control");
     // faces without a partner of their own: only the push form tells them apart
     if (faces[0] != faces[1]) return give_up();
   }
   uint32_t err = 0;
-  SW_CUDA(h, cudaMemcpy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
+  SW_CUDA(h, h->copy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
   if (err & swk::kErrRecords) return h->fail(SW_ERR_CUDA, "upwind slot classification disagrees with its count");
   int64_t all_slots = 0;
   for (const swk::StreamGroup& g : groups) all_slots += (int64_t)((g.shape & 31u) + 1u) * ((g.shape >> 5) & 0x7fu);
@@ -1157,7 +1165,7 @@ sw_status build_records(sw_handle* h) {
   SW_CUDA(h, h->ops->records(p, 1, chunk_off, h->stream), "upwind slot kernel");
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "upwind slots");
   uint32_t err = 0;
-  SW_CUDA(h, cudaMemcpy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
+  SW_CUDA(h, h->copy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
   if (err & swk::kErrRecords) return h->fail(SW_ERR_CUDA, "upwind slot classification disagrees with its count");
   h->stats_upwind_slots = (int64_t)total;
   return SW_OK;
@@ -2026,7 +2034,7 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
       }
       if (h->trace) {
         swk::SweepCtl c{};
-        cudaMemcpy(&c, h->p.ctl, sizeof(c), cudaMemcpyDeviceToHost);
+        h->copy(&c, h->p.ctl, sizeof(c), cudaMemcpyDeviceToHost);
         std::fprintf(stderr,
                      "subsweep sweep level=%d active_tasks=%llu kernel_ms=%.3f transport_ms=%.3f chem_ms=%.3f "
                      "attempts=%llu chem_cells=%llu chem_attempts=%llu\n",
@@ -2201,10 +2209,10 @@ sw_status sw_set_fields(sw_handle* h, const double* x, const double* T) {
     std::vector<double> y(h->N);
     for (int64_t c = 0; c < h->N; ++c) y[c] = 1.0 - x[c];
     h->look_at_floors(x);
-    SW_CUDA(h, cudaMemcpy(h->p.xhii, x, nb, cudaMemcpyHostToDevice), "copy x");
-    SW_CUDA(h, cudaMemcpy(h->p.yneu, y.data(), nb, cudaMemcpyHostToDevice), "copy y");
+    SW_CUDA(h, h->copy(h->p.xhii, x, nb, cudaMemcpyHostToDevice), "copy x");
+    SW_CUDA(h, h->copy(h->p.yneu, y.data(), nb, cudaMemcpyHostToDevice), "copy y");
   }
-  if (T) SW_CUDA(h, cudaMemcpy(h->p.temperature, T, nb, cudaMemcpyHostToDevice), "copy T");
+  if (T) SW_CUDA(h, h->copy(h->p.temperature, T, nb, cudaMemcpyHostToDevice), "copy T");
   return SW_OK;
 }
 
@@ -2318,7 +2326,7 @@ static sw_status levelled_schedule(sw_handle* h, std::vector<uint32_t>& own, std
   const swh::DevicePtrs& p = h->p;
   const uint32_t total = (uint32_t)(h->N * (int64_t)h->D);
   own.resize(total);
-  SW_CUDA(h, cudaMemcpy(own.data(), p.order, (size_t)total * 4, cudaMemcpyDeviceToHost), "read order");
+  SW_CUDA(h, h->copy(own.data(), p.order, (size_t)total * 4, cudaMemcpyDeviceToHost), "read order");
   std::vector<uint16_t> level((size_t)h->Np * h->D, 0);
   uint32_t depth = 0;
   for (const swk::StreamDesc& s : h->streams) {
@@ -2554,10 +2562,10 @@ sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) {
     off += s.bytes;
   }
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "load state");
-  if (h->p.num_pairs) SW_CUDA(h, cudaMemset(h->p.stream_flags, 0xff, (size_t)h->p.num_pairs * 4), "load state");
+  if (h->p.num_pairs) SW_CUDA(h, cudaMemsetAsync(h->p.stream_flags, 0xff, (size_t)h->p.num_pairs * 4, h->stream), "load state");
   h->p.active_cells = 0;  // incoming rates of some cells may be out of date (mixed path)
   if (h->p.stream_mode && !h->ops->pull)  // no sweep is stamped
-    SW_CUDA(h, cudaMemset(h->p.queue, 0xff, (size_t)h->Np * h->D * 4), "load state");
+    SW_CUDA(h, cudaMemsetAsync(h->p.queue, 0xff, (size_t)h->Np * h->D * 4, h->stream), "load state");
   h->sim_time = hd.sim_time;
   h->ts.lowest = hd.ts_lowest;
   h->ts.first_done = hd.ts_first_done != 0;
