@@ -83,7 +83,8 @@ __device__ __forceinline__ double pull_fraction(const FacePull& p, uint32_t f, u
 
 // Finds the flags and far words of every group (b.data null), or writes the groups' pieces, one
 // warp each (k_stream_slots of the mixed path).  The faces handed out and the faces found are
-// counted in ctl->head and ctl->tail: a grid where they differ keeps the push form.
+// counted in ctl->head and ctl->tail: a grid where they differ keeps the push form.  An upwind face
+// without a partner counts as handed out and not found.
 static __global__ void k_stream_slots64(FacePull p, StreamBuild b) {
   const SweepArgs<double>& a = p.a;
   const uint32_t lane = threadIdx.x & 31;
@@ -117,6 +118,7 @@ static __global__ void k_stream_slots64(FacePull p, StreamBuild b) {
         if (kind == kKindPeriodic) {
           ext = true;
           if (!b.data || pull_fraction(p, f, d) >= 0.0) ++found;
+          else ++given;  // nothing is handed out through it: no face may be taken for its partner
           continue;
         }
         const uint32_t u = p.pos_of_task[d * a.Np + (nb & kNbrMask)] - s.base;
@@ -142,6 +144,7 @@ static __global__ void k_stream_slots64(FacePull p, StreamBuild b) {
       if (b.data) {
         const double frac = pull_fraction(p, a.off[c] + face[i], d);
         if (frac >= 0.0) ++found;
+        else ++given;
         idx[piece.slot(j, lane)] = (uint16_t)x;
         w[piece.wslot(j, lane)] = frac;
         if (s.far > f0) far[f0 * 32] = up[i];

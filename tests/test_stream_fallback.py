@@ -106,3 +106,36 @@ def test_pairs_that_cannot_be_resident_are_single_blocks(precision, monkeypatch,
             got[pairs] = results(s)
     for k, a in got["0"].items():
         np.testing.assert_array_equal(a, got["-1"][k], err_msg=k)
+
+
+def test_upwind_faces_without_a_partner_keep_the_push_form(monkeypatch, capfd):
+    # A column along z, closed on itself, whose first cell has its periodic face to the last one
+    # twice: the last cell hands its rate out once, so the second face stands without a partner.
+    # (Against the direction both would hand out; along it only the receiving side counts them.)
+    from subsweep_gb300 import grid as gridmod
+    from subsweep_gb300.sweep import SweepParameters
+    n = 40
+    up, down = np.array([0.0, 0.0, 1.0]), np.array([0.0, 0.0, -1.0])
+    row, nbr, kind, normal = [0], [], [], []
+    for c in range(n):
+        faces = [((c + 1) % n, 1 if c == n - 1 else 0, up)]
+        faces += [((c - 1) % n, 1 if c == 0 else 0, down)] * (2 if c == 0 else 1)
+        for a, k, v in faces:
+            nbr.append(a)
+            kind.append(k)
+            normal.append(v)
+        row.append(len(nbr))
+    e = len(nbr)
+    length = 3e17
+    g = gridmod.Grid(row_ptr=np.array(row, np.int64), nbr=np.array(nbr, np.int32), kind=np.array(kind, np.uint8),
+                     area=np.full(e, length ** 2), normal=np.array(normal), volume=np.full(n, length ** 3),
+                     size=np.full(n, length), position=np.zeros((n, 3)), box_size=np.ones(3), periodic=True)
+    params = SweepParameters(directions=[[0.0, 0.0, 1.0]], num_timestep_levels=2, periodic=True, max_timestep=1e12)
+    w = workloads.Workload("ring", params, g, np.full(n, 1.67e-24), np.full(n, 0.9), np.full(n, 1e4),
+                           np.full(n, 1e45), steps=4)
+    got = {}
+    for streams in ("0", "1"):
+        with make(w, monkeypatch, {"SUBSWEEP_STREAMS": streams}, "fp64") as s:
+            got[streams] = results(s)
+    same(w, "fp64", got["0"], got["1"])
+    assert streams_bytes(w, monkeypatch, capfd, "fp64", {"SUBSWEEP_STREAMS": "1"}) is None
