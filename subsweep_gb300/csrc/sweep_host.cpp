@@ -894,7 +894,7 @@ sw_status build_streams(sw_handle* h) {
   SW_CUDA(h, cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device), "attribute");
   const uint32_t buffer = piece_bytes(31u | (slots << 5) | swk::kGroupExt, rb);
   auto words_for = [&](size_t room, uint32_t far) -> int64_t {
-    return std::min<int64_t>(((int64_t)room - 272 - 4 * rb - (int64_t)warps * buffer) / rb - (int64_t)warps * far * 32,
+    return std::min<int64_t>(((int64_t)room - 288 - 4 * rb - (int64_t)warps * buffer) / rb - (int64_t)warps * far * 32,
                              60000 - (int64_t)warps * far * 32);
   };
   size_t room = 0;

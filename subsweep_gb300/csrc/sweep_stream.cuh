@@ -282,8 +282,8 @@ __device__ __forceinline__ double st_solve(double in, double src, double per, do
   return st_solve((in + src) + per, att, threshold);
 }
 
-// Shared memory of a block: a barrier per warp, the count, the warps' buffers, the words.
-constexpr uint32_t kStreamHead = 8 * 34;
+// Shared memory of a block: a barrier per warp, the counts and parts, the warps' buffers, the words.
+constexpr uint32_t kStreamHead = 8 * 36;
 template <typename R>
 constexpr size_t stream_smem_bytes(const StreamShape& s) {
   return kStreamHead + (size_t)s.warps * s.buffer +
@@ -386,8 +386,9 @@ __device__ __forceinline__ void st_sum(StreamSum<double>& sum, const StreamQuad<
 // There are fewer pairs of SMs than streams (76 for 84 directions), so the streams are laid end to
 // end and cut into equal shares: where a share ends inside a stream, the next pair starts with
 // that stream's beginning, and this one ends with the rest of it, once the beginning is solved
-// (flags), its ring filled from memory.  The last pair is launched first, so a cluster waits only
-// for one launched before it and not for all to be resident.
+// (flags), its ring filled from memory.  The clusters take the pairs in the order in which they
+// start, the last pair first, so one waits only for another that runs already, in whatever order
+// and however many at a time the device starts them.
 template <typename R, int W, bool kFar, bool kAll, bool kPair = false>
 __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const __grid_constant__ StreamArgs<R> a) {
   constexpr uint32_t S = kPair ? 2 * W : W;  // warps that take the groups in turn
@@ -399,10 +400,12 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
   const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x & 31;
   uint64_t* bar = reinterpret_cast<uint64_t*>(st_shared) + warp;
   uint32_t* count = reinterpret_cast<uint32_t*>(st_shared + 8 * 32);  // solved groups of the stream
+  // kPair: the parts of the pair [first, end) (read where they are needed: registers)
+  volatile uint32_t* parts_of = count + 4;
   unsigned char* buffer = st_shared + kStreamHead + warp * shape.buffer;
   R* words = reinterpret_cast<R*>(st_shared + kStreamHead + W * shape.buffer);
   StreamDesc sd = a.streams[kPair ? 0 : blockIdx.x];
-  uint32_t me = warp, peer_words = 0, peer_count = 0, first_part = 0, parts = 1;
+  uint32_t me = warp, peer_words = 0, peer_count = 0;
   if constexpr (kPair) {
     uint32_t rank, size;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -411,12 +414,22 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
       if (threadIdx.x == 0) atomicOr(&a.ctl->error, kErrStall);
       return;
     }
-    const uint32_t pair = (gridDim.x - 1 - blockIdx.x) / 2;  // the last pair first
+    // the last pair goes to the cluster that starts first (ctl->head is 0 before every sweep)
+    if (rank == 0 && threadIdx.x == 0) count[2] = (uint32_t)atomicAdd(&a.ctl->head, 1ull);
+    st_cluster_sync();
+    if (threadIdx.x == 0) {
+      uint32_t started;
+      asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(started) : "r"(st_peer(st_smem(count + 2), 0u)) : "memory");
+      const bool spare = started >= gridDim.x / 2;  // more clusters than pairs: none
+      if (spare) atomicOr(&a.ctl->error, kErrStall);
+      const uint32_t* at = a.part0 + (gridDim.x / 2 - 1 - started);
+      parts_of[0] = spare ? 0u : at[0];
+      parts_of[1] = spare ? 0u : at[1];
+    }
+    st_cluster_sync();
     me = rank * W + warp;  // (the warp that tells the peer: (rank + 1) * W)
     peer_words = st_peer(st_smem(words), rank ^ 1u);
     peer_count = st_peer(st_smem(count + 1), rank ^ 1u);
-    first_part = a.part0[pair];
-    parts = a.part0[pair + 1] - first_part;
   }
   if (threadIdx.x < 2) count[threadIdx.x] = 0;
   if (threadIdx.x < kStreamZero) words[shape.ring + threadIdx.x] = R(0);
@@ -554,11 +567,11 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
     }
     mine = other = false;
   };
-  for (uint32_t part = 0; part < parts; ++part) {
+  for (uint32_t part = kPair ? parts_of[0] : 0u; part < (kPair ? parts_of[1] : 1u); ++part) {
     uint32_t post = 0;
     bool fresh = false;  // the part's first groups: their far words have not been fetched ahead
     if constexpr (kPair) {
-      const StreamPart pt = a.parts[first_part + part];
+      const StreamPart pt = a.parts[part];
       sd = a.streams[pt.stream];
       groups = a.groups + sd.group0;
       word = a.word + sd.base + lane;

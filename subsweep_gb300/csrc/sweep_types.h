@@ -57,7 +57,8 @@ constexpr uint32_t kErrFailed = kErrStall | kErrQueue | kErrClamp;  // of a step
 
 // Control block of one handle (device memory).
 struct SweepCtl {
-  unsigned long long head;  // next ready-queue slot to claim (consumers); pull wavefront: barrier arrivals
+  unsigned long long head;  // next ready-queue slot to claim (consumers); pull wavefront: barrier arrivals;
+                            // pairs of blocks: clusters that have started
   unsigned long long tail;  // next ready-queue slot to fill (producers)
   uint32_t error;           // kErr* bits
   uint32_t pad;
