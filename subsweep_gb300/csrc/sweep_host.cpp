@@ -135,6 +135,7 @@ struct sw_handle {
   int64_t stats_upwind_slots = 0;
   int force_path = 0;  // 0 automatic, 1 always levelled, 2 always dependency-driven
   bool trace = false;  // SUBSWEEP_TRACE: one stderr line per level sweep
+  uint32_t no_act_list = 0;  // streams: levels whose compacted list found no room
   uint32_t act_valid = 0;  // pull path: levels whose compacted list is current this step
   double* series_dev = nullptr;  // time-series partial sums and result (allocated on first use)
   // graph replay of a step (pull path): the instantiated graph, the step shape it was
@@ -1742,7 +1743,7 @@ sw_status sw_create(const sw_params* params, const sw_grid_csr* grid, const sw_c
 // overrides), and that list's buffer, allocated on first use.
 static bool pull_sparse(sw_handle* h, int level) {
   const swh::DevicePtrs& p = h->p;
-  if (level <= 0) return false;
+  if (level <= 0 || ((h->no_act_list >> level) & 1u)) return false;
   if (p.compact_mode == 1) return true;
   if (p.compact_mode == 2) return false;
   // Streams: a dense sweep takes the time of all tasks, 23 per ns, a sparse one ~5 per ns of
@@ -1753,19 +1754,35 @@ static bool pull_sparse(sw_handle* h, int level) {
   return h->n_ge_host[level] * 2 < h->N;
 }
 
-static sw_status ensure_act_list(sw_handle* h, int level) {
+// The buffer of the list, allocated on first use (outside of a capture).  Streams: without room for
+// it `sparse` becomes false, and the level's sweeps visit every position, now and later; the
+// lockstep kernels have no such form.
+static sw_status ensure_act_list(sw_handle* h, int level, bool& sparse) {
   if (h->p.act_lv[level]) return SW_OK;
+  const size_t tasks = (size_t)h->Np * h->D;
+  uint32_t* list = nullptr;
   if (h->p.stream_mode) {
+    const size_t allocations = h->allocations.size();
+    const int64_t device_bytes = h->device_bytes;
     uint32_t *bits = nullptr, *range = nullptr;
-    if (!h->alloc(&bits, ((size_t)h->Np * h->D + 31) / 32) || !h->alloc(&range, 2 * (size_t)h->p.num_streams))
-      return h->fail(SW_ERR_OOM, "device allocation of the active positions of level %d failed", level);
-    h->p.act_bits_lv[level] = bits;
-    h->p.act_range[level] = range;
+    if (h->stream_alloc(&bits, (tasks + 31) / 32) &&
+        h->stream_alloc(&range, 2 * (size_t)h->p.num_streams) && h->stream_alloc(&list, tasks)) {
+      h->p.act_bits_lv[level] = bits;
+      h->p.act_range[level] = range;
+      h->p.act_lv[level] = list;
+      return SW_OK;
+    }
+    (void)cudaGetLastError();
+    for (size_t k = allocations; k < h->allocations.size(); ++k) cudaFree(h->allocations[k]);
+    h->allocations.resize(allocations);
+    h->device_bytes = device_bytes;
+    h->no_act_list |= 1u << level;
+    sparse = false;
+    return SW_OK;
   }
-  uint32_t* buf = nullptr;
-  if (!h->alloc(&buf, (size_t)h->Np * h->D))
+  if (!h->alloc(&list, tasks))
     return h->fail(SW_ERR_OOM, "device allocation of the active positions of level %d failed", level);
-  h->p.act_lv[level] = buf;
+  h->p.act_lv[level] = list;
   return SW_OK;
 }
 
@@ -1787,7 +1804,7 @@ static sw_status step_graph(sw_handle* h, double* time_elapsed_out) {
     if (h->pulls()) {
       variant = pull_sparse(h, level);
       if (variant) {
-        sw_status st = ensure_act_list(h, level);  // allocations stay outside the capture
+        sw_status st = ensure_act_list(h, level, variant);  // allocations stay outside the capture
         if (st != SW_OK) return st;
       }
     } else {
@@ -2084,11 +2101,14 @@ sw_status sw_step(sw_handle* h, double* time_elapsed_out) {
       h->last_epoch = h->p.epoch;
       h->p.active_cells = h->n_ge_host[level];
       h->p.sweep_level = level;
-      h->p.sparse_sweep = pull_sparse(h, level) ? 1 : 0;
-      h->p.compact_now = 0;
-      if (h->p.sparse_sweep) {
-        sw_status st = ensure_act_list(h, level);
+      bool sparse = pull_sparse(h, level);
+      if (sparse) {
+        sw_status st = ensure_act_list(h, level, sparse);
         if (st != SW_OK) return st;
+      }
+      h->p.sparse_sweep = sparse ? 1 : 0;
+      h->p.compact_now = 0;
+      if (sparse) {
         if (!((h->act_valid >> level) & 1u)) {  // first sweep of this level in the step
           h->p.compact_now = 1;
           h->act_valid |= 1u << level;

@@ -139,3 +139,23 @@ def test_upwind_faces_without_a_partner_keep_the_push_form(monkeypatch, capfd):
             got[streams] = results(s)
     same(w, "fp64", got["0"], got["1"])
     assert streams_bytes(w, monkeypatch, capfd, "fp64", {"SUBSWEEP_STREAMS": "1"}) is None
+
+
+@pytest.mark.parametrize("graph", ["0", "1"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_sparse_sweeps_without_room_for_their_lists(precision, graph, monkeypatch, capfd):
+    w = periodic()
+    env = {"SUBSWEEP_STREAMS": "1", "SUBSWEEP_GRAPH": graph, "SUBSWEEP_COMPACT": "always"}
+    monkeypatch.setenv("SUBSWEEP_COMPACT", "always")
+    with make(w, monkeypatch, env, precision) as s:
+        expected = results(s)
+    for arrays in range(64):  # the first with which a handle has streams leaves none for a list
+        env["SUBSWEEP_STREAM_ARRAYS"] = str(arrays)
+        if streams_bytes(w, monkeypatch, capfd, precision, env) is not None:
+            break
+    for more in (0, 1, 2, 3, 4):  # a list takes three: the second level's finds no room, or less
+        env["SUBSWEEP_STREAM_ARRAYS"] = str(arrays + more)
+        with make(w, monkeypatch, env, precision) as s:
+            got = results(s)
+        for k, a in expected.items():
+            np.testing.assert_array_equal(a, got[k], err_msg=k)
