@@ -497,10 +497,24 @@ static void stream_order(const uint16_t* level, const uint8_t* up, uint32_t Np, 
   }
 }
 
+// Whether pairs of blocks walk the streams faster than single blocks: cycles of a level with g
+// groups, times the levels of the longest stream, times the rounds (there are half as many
+// pairs).  Lines through the measured times of uniform boxes, ms per sweep of 84 directions with
+// single blocks and pairs: mixed path 96^3 (18 groups a level) 3.06 and 3.77, 128^3 (31) 7.68 and
+// 7.24; FP64 64^3 (8) 2.02 and 2.58, 96^3 7.90 and 6.72; 16 directions FP64 64^3 1.84 and 2.09,
+// 101^3 (19) 7.54 and 5.98.
+static bool pairs_pay(double levels, double groups, double total, int sms, bool mixed) {
+  const double g = groups / levels;
+  const double one = mixed ? 500.0 + 176.0 * g : std::max(670.0, 580.0 * g - 1300.0);
+  const double two = mixed ? 1850.0 + 103.0 * g : 1540.0 + 295.0 * g;
+  const auto rounds = [&](int blocks) { return std::max(1.0, total / (groups * blocks)); };
+  return two * rounds(sms / 2) < 0.95 * one * rounds(sms);
+}
+
 // Whether direction streams are faster than the kernels over the levelled schedule: the longest
-// stream, at 3.6 ns a task of its block (FP64 7.7, of a pair of blocks 5.9), against the time of a level, from word to word
-// 0.85 us (FP64 push form, from atomic to atomic: 4), times the levels, plus the tasks at 17 per
-// ns (12).  Measured on uniform boxes, ms per sweep, levelled and streams.  Mixed path: 84
+// stream, at 3.6 ns a task of its block (FP64 7.7, of a pair of blocks 5.9 where pairs_pay takes them,
+// times the streams that a pair has), against the time of a level, from word to word 0.85 us (FP64
+// push form, from atomic to atomic: 4), times the levels, plus the tasks at 17 per ns (12).  Measured on uniform boxes, ms per sweep, levelled and streams.  Mixed path: 84
 // directions 24^3 0.32 and 0.15, 48^3 0.89 and 0.52, 64^3 1.56 and 1.01, 128^3 10.3 and 7.6; 16
 // directions 64^3 0.95 and 0.87, but 101^3 1.87 and 2.98: sixteen blocks cannot keep up with the
 // whole device where levels are wide.  FP64: 84 directions 16^3 0.97 and 0.18, 24^3 1.61 and 0.31,
@@ -508,12 +522,13 @@ static void stream_order(const uint16_t* level, const uint8_t* up, uint32_t Np, 
 // 7.8 and 6.0; 84 directions 128^3 34 and 17, 160^3 66 and 34.  Where a level is wide, the ring
 // holds few levels and many words come from memory: mixed path 160^3 (1800 tasks a level) 20.2
 // and 15.8, 192^3 (2200) 35 and 34, 256^3 (3400) 83 and 114; hence the limit on the width.
-static bool streams_pay(const std::vector<uint32_t>& parts, uint64_t tasks, size_t levels, bool mixed) {
+static bool streams_pay(const std::vector<uint32_t>& parts, uint64_t tasks, size_t levels, int sms, bool mixed) {
   uint32_t longest = 0;
   for (size_t k = 1; k < parts.size(); ++k) longest = std::max(longest, parts[k] - parts[k - 1]);
   if (!mixed) {
     double task = 7.7;
-    if (longest > 480.0 * (double)levels) task = 5.9 * std::max(1.0, (double)tasks / longest / 76.0);  // pairs
+    if (pairs_pay((double)levels, longest / (double)swk::kStreamGroup, (double)tasks / swk::kStreamGroup, sms, false))
+      task = 5.9 * std::max(1.0, 2.0 * (double)tasks / ((double)longest * sms));
     return task * longest < 4000.0 * (double)levels + (double)tasks / 12.0;
   }
   return longest < 2600.0 * (double)levels && 3.6 * longest < 850.0 * (double)levels + (double)tasks / 17.0;
@@ -646,7 +661,7 @@ sw_status build_schedule(sw_handle* h) {
     // and checkpoints hold them in that order.
     const size_t L = lvl.size() - 1;
     depth = std::max(depth, (uint32_t)L);
-    if (h->want_streams) h->want_streams = h->force_streams || streams_pay(h->parts, total, L, h->ops->pull);
+    if (h->want_streams) h->want_streams = h->force_streams || streams_pay(h->parts, total, L, p.num_sms, h->ops->pull);
     int groups = schedule_dir_groups(q.D, total, L);
     if (p.geo_mode && !std::getenv("SUBSWEEP_DIR_GROUPS")) groups = 1;
     std::vector<uint32_t> seg = {0};
@@ -766,20 +781,6 @@ static void plan_stream(const swk::StreamDesc& sd, const uint32_t* seg, const st
       out[g] = {need, 0u, p, (n - 1) | (slots << 5)};
     }
   }
-}
-
-// Whether pairs of blocks walk the streams faster than single blocks: cycles of a level with g
-// groups, times the levels of the longest stream, times the rounds (there are half as many
-// pairs).  Lines through the measured times of uniform boxes, ms per sweep of 84 directions with
-// single blocks and pairs: mixed path 96^3 (18 groups a level) 3.06 and 3.77, 128^3 (31) 7.68 and
-// 7.24; FP64 64^3 (8) 2.02 and 2.58, 96^3 7.90 and 6.72; 16 directions FP64 64^3 1.84 and 2.09,
-// 101^3 (19) 7.54 and 5.98.
-static bool pairs_pay(double levels, double groups, double total, int sms, bool mixed) {
-  const double g = groups / levels;
-  const double one = mixed ? 500.0 + 176.0 * g : std::max(670.0, 580.0 * g - 1300.0);
-  const double two = mixed ? 1850.0 + 103.0 * g : 1540.0 + 295.0 * g;
-  const auto rounds = [&](int blocks) { return std::max(1.0, total / (groups * blocks)); };
-  return two * rounds(sms / 2) < 0.95 * one * rounds(sms);
 }
 
 // The parts of `pairs` pairs of blocks: the streams' groups end to end, cut into equal shares at
