@@ -667,36 +667,37 @@ __global__ void k_attenuation(uint32_t n, const uint8_t* level, int current_leve
 
 // Rate of cell c summed over the directions (Sweep::get_solver, src/sweep/mod.rs:613-631): FP64
 // in direction order; mixed path: a compensated FP32 sum of the scaled transported rates, the
-// source added in FP64.  `pos`: the incoming rates are indexed by position, else by task;
-// `has_periodic`: the cell has periodic faces (else its periodic sources are 0).  The rates by
-// position are loaded kSumBatch directions at a time (latency: two loads per batch).
+// source added in FP64.
+__device__ __forceinline__ void add_compensated(float& s, float& comp, float v) {
+  const float yv = v - comp;
+  const float tt = s + yv;
+  comp = (tt - s) - yv;
+  s = tt;
+}
+
+// Rates by position, kRateBatch directions at a time (latency: two loads per batch).  has_periodic:
+// the cell has periodic faces (else its periodic sources are 0).
 constexpr int kRateBatch = 24;
-template <typename R, int kSumBatch>
-__device__ __forceinline__ double cell_sum(const R* incoming, const uint32_t* pos, const R* periodic, bool has_periodic,
-                                           double source, int D, uint32_t Np, uint32_t c, double rate_scale) {
-  constexpr int kBatch = kSumBatch;
+template <typename R>
+__device__ __forceinline__ double cell_sum_gathered(const R* incoming, const uint32_t* pos, const R* periodic,
+                                                    bool has_periodic, double source, int D, uint32_t Np, uint32_t c,
+                                                    double rate_scale) {
   const double src = source / (double)D;
   double rate = 0.0;
   float s = 0.f, comp = 0.f;
-  for (int d0 = 0; d0 < D; d0 += kBatch) {
-    R in[kBatch], per[kBatch];
+  for (int d0 = 0; d0 < D; d0 += kRateBatch) {
+    R in[kRateBatch], per[kRateBatch];
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
+    for (int j = 0; j < kRateBatch; ++j) {
       const size_t t = (size_t)min(d0 + j, D - 1) * Np + c;
-      in[j] = incoming[pos ? pos[t] : t];
+      in[j] = incoming[pos[t]];
       per[j] = has_periodic ? periodic[t] : R(0);
     }
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
+    for (int j = 0; j < kRateBatch; ++j) {
       if (d0 + j >= D) break;
-      if (sizeof(R) == 8) {
-        rate += ((double)in[j] + src) + (double)per[j];  // Site::get_rate
-      } else {
-        const float yv = ((float)in[j] + (float)per[j]) - comp;
-        const float tt = s + yv;
-        comp = (tt - s) - yv;
-        s = tt;
-      }
+      if (sizeof(R) == 8) rate += ((double)in[j] + src) + (double)per[j];  // Site::get_rate
+      else add_compensated(s, comp, (float)in[j] + (float)per[j]);
     }
   }
   return sizeof(R) == 8 ? rate : (double)s * rate_scale + source;
@@ -711,7 +712,7 @@ __global__ void __launch_bounds__(128) k_cell_sums(uint32_t n, const uint8_t* le
                                                    uint32_t Np, double rate_scale, double* out) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
     if (level[c] >= current_level)
-      out[c] = cell_sum<R, kRateBatch>(incoming, pos, periodic, cell_periodic[c] != 0, source[c], D, Np, c, rate_scale);
+      out[c] = cell_sum_gathered<R>(incoming, pos, periodic, cell_periodic[c] != 0, source[c], D, Np, c, rate_scale);
 }
 
 template <typename R>
@@ -744,6 +745,39 @@ struct ChemArgs {
   int prevent_cooling;
 };
 
+// The rate of a cell from the rates by task, inside the chemistry: eight directions' loads at a time,
+// the two rates of a direction added as they come (128^3 x 84, mixed path, one attempt a cell: 0.91
+// ms of chemistry a sweep; with 16 rates held until all have come 1.29).  Its operands come from the
+// kernel's arguments: handed on one by one they took the chemistry from 80 registers to 117.
+template <typename R>
+__device__ __forceinline__ double cell_sum(const ChemArgs<R>& a, uint32_t c) {
+  if (sizeof(R) == 8) {
+    const double src = a.source[c] / (double)a.D;
+    double rate = 0.0;
+    for (int d = 0; d < a.D; ++d) {
+      const size_t t = (size_t)d * a.Np + c;
+      rate += ((double)a.incoming[t] + src) + (double)a.periodic[t];  // Site::get_rate
+    }
+    return rate;
+  }
+  constexpr int kBatch = 8;
+  float s = 0.f, comp = 0.f;
+  for (int d0 = 0; d0 < a.D; d0 += kBatch) {
+    float v[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const size_t t = (size_t)(d0 + j) * a.Np + c;
+      v[j] = d0 + j < a.D ? (float)a.incoming[t] + (float)a.periodic[t] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      if (d0 + j >= a.D) break;
+      add_compensated(s, comp, v[j]);
+    }
+  }
+  return (double)s * a.rate_scale + a.source[c];
+}
+
 // Sweep::update_chemistry (src/sweep/mod.rs:549-574) + HydrogenOnly::update_abundances
 // (hydrogen_only/mod.rs:90-119), one thread per cell (inactive cells skip).
 template <typename R, bool kCarryNeutral>
@@ -753,9 +787,7 @@ __global__ void k_chemistry(ChemArgs<R> a) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < a.n; c += gridDim.x * blockDim.x) {
     if (a.level[c] < a.current_level) continue;
     const double timestep = ldexp(a.max_timestep, -(int)a.level[c]);  // timestep_level.rs:42-48
-    const double rate = a.cell_rate ? a.cell_rate[c]
-                                    : cell_sum<R, 8>(a.incoming, nullptr, a.periodic, true, a.source[c], a.D, a.Np, c,
-                                               a.rate_scale);
+    const double rate = a.cell_rate ? a.cell_rate[c] : cell_sum(a, c);
     double relative_change;
     // chemistry/mod.rs:79-81.  The mixed path also treats a rate below the smallest
     // value its FP32 transport carries at full precision as insignificant: there the
@@ -887,6 +919,7 @@ __global__ void k_photon_rate(uint32_t n, const R* incoming, const uint32_t* pos
   constexpr int kBatch = kRateBatch;
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
     double r = 0.0;
+#pragma unroll 1
     for (int d0 = 0; d0 < D; d0 += kBatch) {
       R in[kBatch];
 #pragma unroll
