@@ -1749,9 +1749,10 @@ static bool pull_sparse(sw_handle* h, int level) {
   if (p.compact_mode == 2) return false;
   // Streams: a dense sweep takes the time of all tasks, 23 per ns, a sparse one ~5 per ns of
   // the active ones (128^3 x 84: 7.9 ms dense; sparse 14 ms with 39% of the cells active, the
-  // crossing near 20%; 64^3 x 84: 1.03 ms dense, 0.13 ms with 0.2% active).  FP64:
-  // 64^3 x 84 2.0 ms dense, 2.4 ms with a third of the cells active.
-  if (p.stream_mode) return (int64_t)h->n_ge_host[level] * 5 < h->N;
+  // crossing near 20%; 64^3 x 84: 1.03 ms dense, 0.13 ms with 0.2% active).  FP64, whose
+  // sparse sweeps pass their changes on to the cells beside: six boxes x 84 0.54 ms dense, 0.45 with
+  // 6% active, 0.56 with 9%, 0.88 with 24%; 64^3 x 84 2.2 dense, 3.0 with a third.
+  if (p.stream_mode) return (int64_t)h->n_ge_host[level] * (h->ops->pull ? 5 : 10) < h->N;
   return h->n_ge_host[level] * 2 < h->N;
 }
 
