@@ -49,7 +49,6 @@ def test_a_refused_floor_ends_the_step_at_its_sweep(streams, precision, monkeypa
                 s.run_sweeps()
             x = s.fields()["ionized_hydrogen_fraction"]
             at = np.argmax(x)
-            assert x[at] > 0.9
             x[at] = 1.0
             s.set_fields(ionized_hydrogen_fraction=x)
             before, sweeps = state(s), s.stats()["level_sweeps"]
