@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -2499,7 +2500,7 @@ sw_status sw_checkpoint_size(sw_handle* h, size_t* bytes) {
   return SW_OK;
 }
 
-sw_status sw_save_state(sw_handle* h, void* buffer, size_t bytes) {
+sw_status sw_save_state(sw_handle* h, void* buffer, size_t bytes) try {
   if (!h || !buffer) return SW_ERR_INVALID_ARG;
   h->last_error.clear();
   if (bytes < checkpoint_bytes(h)) return h->fail(SW_ERR_INVALID_ARG, "checkpoint buffer too small");
@@ -2537,9 +2538,11 @@ sw_status sw_save_state(sw_handle* h, void* buffer, size_t bytes) {
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "save state");
   if (h->p.stream_mode) reorder_rates(h, out + off, own, order, true);
   return SW_OK;
+} catch (const std::bad_alloc&) {  // the streams' rates are reordered on the host
+  return h->fail(SW_ERR_OOM, "no host memory to reorder the checkpoint's rates");
 }
 
-sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) {
+sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) try {
   if (!h || !buffer) return SW_ERR_INVALID_ARG;
   h->last_error.clear();
   CheckpointHeader hd{};
@@ -2606,6 +2609,8 @@ sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) {
   SW_CUDA(h, cudaMemsetAsync(&h->p.ctl->error, 0, sizeof(uint32_t), h->stream), "reset error flag");
   SW_CUDA(h, swh::launch_level_hist(h->p, h->stream), "level histogram");
   return sync_ctl(h);
+} catch (const std::bad_alloc&) {  // the streams' rates are reordered on the host
+  return h->fail(SW_ERR_OOM, "no host memory to reorder the checkpoint's rates");
 }
 
 sw_status sw_get_time_series(sw_handle* h, sw_time_series* out) {
