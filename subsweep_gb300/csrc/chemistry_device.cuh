@@ -22,7 +22,9 @@
 //   FP64: the fits at the temperature that an attempt accepts are the next state's;
 //   the recommended steps are formed for the last accepted attempt only.
 // None of it changes a rounding: near equilibrium a state's timescale is its value over a small
-// difference of large terms, which shows the last bits of every one of them.
+// difference of large terms, which shows the last bits of every one of them.  Against factors formed
+// per attempt, ms a sweep: 128^3 mixed, 14 attempts a cell 10.9 -> 9.4, one 0.97 -> 0.91; 64^3 FP64,
+// 27 attempts 15.9 -> 14.0, 1.6 attempts 0.88 -> 0.74, one 0.33 -> 0.32; 256^3 FP64 219 -> 181.
 // The mixed path evaluates the rate fits in FP32 (Fits32); the densities, the sums, the
 // implicit updates and their accept / reject tests are FP64 in both.
 #pragma once
