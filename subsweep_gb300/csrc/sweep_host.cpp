@@ -127,6 +127,7 @@ struct sw_handle {
   bool pulls() const { return ops->pull || p.stream_mode; }
   std::vector<uint32_t> parts;
   std::vector<uint32_t> stream_seg;
+  std::vector<uint16_t> kept_levels;  // of every task, until the streams are laid out or given up
   std::vector<std::vector<uint8_t>> stream_gmax;  // per stream: the largest count of every group
   std::vector<swk::StreamDesc> streams;
   // fingerprint of the levelled schedule (direction groups and segment offsets): the pull
@@ -567,6 +568,68 @@ struct ScheduleHash {
   }
 };
 
+// The Kahn levels of a space's tasks (all cells active), on the host: levels[t], their number, and
+// for streams the upwind LOCAL faces of every task.  cyclic: some task has no level.
+static sw_status kahn_levels(sw_handle* h, const swh::DevicePtrs& q, std::vector<uint16_t>& levels, size_t& depth,
+                             std::vector<uint8_t>& up, bool& cyclic) {
+  const swh::DevicePtrs& p = h->p;
+  const uint64_t total = (uint64_t)h->N * (uint64_t)q.D;
+  struct DeviceScratch {
+    void* ptr = nullptr;
+    ~DeviceScratch() {
+      if (ptr) cudaFree(ptr);
+    }
+  } level_scratch, bounds_scratch;
+  SW_CUDA(h, cudaMalloc(&level_scratch.ptr, (size_t)h->Np * q.D * sizeof(uint16_t)), "schedule scratch");
+  uint16_t* task_level = static_cast<uint16_t*>(level_scratch.ptr);
+  SW_CUDA(h, cudaMemsetAsync(p.ctl, 0, offsetof(swk::SweepCtl, tasks), h->stream), "reset control");
+  SW_CUDA(h, cudaMemsetAsync(task_level, 0, (size_t)h->Np * q.D * sizeof(uint16_t), h->stream), "schedule scratch");
+  SW_CUDA(h, h->ops->schedule_seed(q, h->stream), "schedule seed kernel");
+  std::vector<uint32_t> lvl = {0};
+  unsigned long long tail = 0;
+  SW_CUDA(h, cudaMemcpyAsync(&tail, &p.ctl->tail, sizeof(tail), cudaMemcpyDeviceToHost, h->stream), "read tail");
+  SW_CUDA(h, cudaStreamSynchronize(h->stream), "schedule seed");
+  if (h->want_streams) {  // (the rounds count them down)
+    up.resize((size_t)h->Np * q.D);
+    SW_CUDA(h, h->copy(up.data(), p.counters, up.size(), cudaMemcpyDeviceToHost), "read upwind counts");
+  }
+  // the rounds, kRounds at a time (those after the last one find nothing to do)
+  constexpr uint32_t kRounds = 32, kMaxRounds = 0xffffu;
+  SW_CUDA(h, cudaMalloc(&bounds_scratch.ptr, (kMaxRounds + kRounds + 2) * sizeof(uint32_t)), "schedule scratch");
+  uint32_t* bounds = static_cast<uint32_t*>(bounds_scratch.ptr) + 1;  // behind the blocks' count
+  const uint32_t first[3] = {0u, 0u, (uint32_t)tail};
+  SW_CUDA(h, h->copy(bounds - 1, first, sizeof(first), cudaMemcpyHostToDevice), "schedule scratch");
+  uint32_t end = (uint32_t)tail;
+  if (end > 0) lvl.push_back(end);
+  for (uint32_t round = 0; end > 0;) {
+    uint32_t ends[kRounds];
+    SW_CUDA(h, h->ops->kahn_rounds(q, bounds, bounds - 1, task_level, round, kRounds, h->stream),
+            "schedule round kernel");
+    SW_CUDA(h, cudaMemcpyAsync(ends, bounds + round + 2, sizeof(ends), cudaMemcpyDeviceToHost, h->stream),
+            "read bounds");
+    SW_CUDA(h, cudaStreamSynchronize(h->stream), "schedule round");
+    bool more = true;
+    for (uint32_t k = 0; k < kRounds && more; ++k) {
+      more = ends[k] > end;
+      if (more) lvl.push_back(end = ends[k]);
+    }
+    if (!more) break;
+    round += kRounds;
+    if (round >= kMaxRounds) return h->fail(SW_ERR_UNSUPPORTED, "dependency graph deeper than 65534 levels");
+  }
+  tail = end;
+  if (lvl.size() - 1 >= kMaxRounds) return h->fail(SW_ERR_UNSUPPORTED, "dependency graph deeper than 65534 levels");
+  uint32_t err = 0;
+  SW_CUDA(h, h->copy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
+  cyclic = tail != total || err != 0;
+  if (cyclic) return SW_OK;
+  depth = lvl.size() - 1;
+  levels.resize((size_t)h->Np * q.D);
+  SW_CUDA(h, h->copy(levels.data(), task_level, levels.size() * sizeof(uint16_t), cudaMemcpyDeviceToHost),
+          "read task levels");
+  return SW_OK;
+}
+
 // Levelled schedule (Kahn levels of all N*D tasks with every cell active), built once
 // per grid on the device, per task space (one space unless the compact state splits the
 // directions; task ids and positions are local to a space).  A dependency cycle leaves
@@ -575,16 +638,6 @@ struct ScheduleHash {
 // such path, refuses the grid).
 sw_status build_schedule(sw_handle* h) {
   swh::DevicePtrs& p = h->p;
-  struct DeviceScratch {
-    void* ptr = nullptr;
-    ~DeviceScratch() {
-      if (ptr) cudaFree(ptr);
-    }
-  } level_scratch;
-  int max_ds = 0;
-  for (int sp = 0; sp < p.num_spaces; ++sp) max_ds = std::max(max_ds, p.space_d0[sp + 1] - p.space_d0[sp]);
-  SW_CUDA(h, cudaMalloc(&level_scratch.ptr, (size_t)h->Np * max_ds * sizeof(uint16_t)), "schedule scratch");
-  uint16_t* task_level = static_cast<uint16_t*>(level_scratch.ptr);
   ScheduleHash hash;
   hash.mix((uint32_t)p.geo_mode);
   hash.mix((uint32_t)p.num_spaces);
@@ -592,48 +645,16 @@ sw_status build_schedule(sw_handle* h) {
   for (int sp = 0; sp < p.num_spaces; ++sp) {
     const swh::DevicePtrs q = swh::space_view(p, sp);
     const uint64_t total = (uint64_t)h->N * (uint64_t)q.D;
-    SW_CUDA(h, cudaMemsetAsync(p.ctl, 0, offsetof(swk::SweepCtl, tasks), h->stream), "reset control");
-    SW_CUDA(h, cudaMemsetAsync(task_level, 0, (size_t)h->Np * q.D * sizeof(uint16_t), h->stream), "schedule scratch");
-    SW_CUDA(h, h->ops->schedule_seed(q, h->stream), "schedule seed kernel");
-    std::vector<uint32_t> lvl = {0};
-    unsigned long long tail = 0;
-    SW_CUDA(h, cudaMemcpyAsync(&tail, &p.ctl->tail, sizeof(tail), cudaMemcpyDeviceToHost, h->stream), "read tail");
-    SW_CUDA(h, cudaStreamSynchronize(h->stream), "schedule seed");
-    std::vector<uint8_t> up;  // upwind LOCAL faces of every task (the rounds count them down)
-    if (h->want_streams) {
-      up.resize((size_t)h->Np * q.D);
-      SW_CUDA(h, h->copy(up.data(), p.counters, up.size(), cudaMemcpyDeviceToHost), "read upwind counts");
+    // (of a grid whose streams were given up, the levels are known)
+    std::vector<uint16_t> tl = std::move(h->kept_levels);
+    size_t L = h->stats_schedule_levels;
+    std::vector<uint8_t> up;
+    bool cyclic = false;
+    if (tl.empty()) {
+      const sw_status st = kahn_levels(h, q, tl, L, up, cyclic);
+      if (st != SW_OK) return st;
     }
-    // the rounds, kRounds at a time (those after the last one find nothing to do)
-    constexpr uint32_t kRounds = 32, kMaxRounds = 0xffffu;
-    DeviceScratch bounds_scratch;
-    SW_CUDA(h, cudaMalloc(&bounds_scratch.ptr, (kMaxRounds + kRounds + 2) * sizeof(uint32_t)), "schedule scratch");
-    uint32_t* bounds = static_cast<uint32_t*>(bounds_scratch.ptr) + 1;  // behind the blocks' count
-    const uint32_t first[3] = {0u, 0u, (uint32_t)tail};
-    SW_CUDA(h, h->copy(bounds - 1, first, sizeof(first), cudaMemcpyHostToDevice), "schedule scratch");
-    uint32_t end = (uint32_t)tail;
-    if (end > 0) lvl.push_back(end);
-    for (uint32_t round = 0; end > 0;) {
-      uint32_t ends[kRounds];
-      SW_CUDA(h, h->ops->kahn_rounds(q, bounds, bounds - 1, task_level, round, kRounds, h->stream),
-              "schedule round kernel");
-      SW_CUDA(h, cudaMemcpyAsync(ends, bounds + round + 2, sizeof(ends), cudaMemcpyDeviceToHost, h->stream),
-              "read bounds");
-      SW_CUDA(h, cudaStreamSynchronize(h->stream), "schedule round");
-      bool more = true;
-      for (uint32_t k = 0; k < kRounds && more; ++k) {
-        more = ends[k] > end;
-        if (more) lvl.push_back(end = ends[k]);
-      }
-      if (!more) break;
-      round += kRounds;
-      if (round >= kMaxRounds) return h->fail(SW_ERR_UNSUPPORTED, "dependency graph deeper than 65534 levels");
-    }
-    tail = end;
-    if (lvl.size() - 1 >= kMaxRounds) return h->fail(SW_ERR_UNSUPPORTED, "dependency graph deeper than 65534 levels");
-    uint32_t err = 0;
-    SW_CUDA(h, h->copy(&err, &p.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error flag");
-    if (tail != total || err != 0) {
+    if (cyclic) {
       if (p.geo_mode) return h->fail(SW_ERR_STALLED, "the dependency graph has a cycle (compact state)");
       // cyclic dependency graph: no schedule.  The push path falls back to the
       // dependency-driven queue; the pull path visits tasks in id order and its waits run
@@ -660,21 +681,18 @@ sw_status build_schedule(sw_handle* h) {
     // order is a stable counting sort on the host, so every handle on the same grid
     // gets the same schedule: the pull path's words are indexed by schedule position,
     // and checkpoints hold them in that order.
-    const size_t L = lvl.size() - 1;
     depth = std::max(depth, (uint32_t)L);
     if (h->want_streams) h->want_streams = h->force_streams || streams_pay(h->parts, total, L, p.num_sms, h->ops->pull);
     int groups = schedule_dir_groups(q.D, total, L);
     if (p.geo_mode && !std::getenv("SUBSWEEP_DIR_GROUPS")) groups = 1;
     std::vector<uint32_t> seg = {0};
     {
-      std::vector<uint16_t> tl((size_t)h->Np * q.D);
-      SW_CUDA(h, h->copy(tl.data(), task_level, tl.size() * sizeof(uint16_t), cudaMemcpyDeviceToHost),
-              "read task levels");
       std::vector<uint32_t> order(total);
       if (h->want_streams) {
         stream_order(tl.data(), up.data(), h->Np, (uint32_t)h->N, (uint32_t)q.D, h->parts, order.data(), seg,
                      h->streams, h->stream_gmax);
         h->stream_seg = seg;
+        h->kept_levels = std::move(tl);
       } else if (grouped_level_order(tl.data(), h->Np, (uint32_t)h->N, (uint32_t)q.D, L, groups, order.data(), seg) !=
                  total) {
         return h->fail(SW_ERR_CUDA, "schedule order incomplete");
@@ -1116,7 +1134,10 @@ sw_status build_records(sw_handle* h) {
     const size_t allocations = h->allocations.size();
     const int64_t device_bytes = h->device_bytes;
     sw_status st = build_streams(h);
-    if (st != SW_OK || h->want_streams) return st;
+    if (st != SW_OK || h->want_streams) {
+      h->kept_levels = {};
+      return st;
+    }
     // a level too wide for a ring, or no room: the levelled schedule
     for (size_t k = allocations; k < h->allocations.size(); ++k) cudaFree(h->allocations[k]);
     h->allocations.resize(allocations);
