@@ -503,8 +503,8 @@ static void stream_order(const uint16_t* level, const uint8_t* up, uint32_t Np, 
 // groups, times the levels of the longest stream, times the rounds (there are half as many
 // pairs).  Lines through the measured times of uniform boxes, ms per sweep of 84 directions with
 // single blocks and pairs: mixed path 96^3 (18 groups a level) 3.06 and 3.77, 128^3 (31) 7.68 and
-// 7.24; FP64 64^3 (8) 2.02 and 2.58, 96^3 7.90 and 6.72; 16 directions FP64 64^3 1.84 and 2.09,
-// 101^3 (19) 7.54 and 5.98.
+// 7.24; FP64 64^3 (8) 2.14 and 2.68, 72^3 3.12 and 3.35, 80^3 4.51 and 4.14, 96^3 8.48 and 7.42; 16
+// directions FP64 64^3 1.94 and 2.19, 80^3 3.98 and 3.24, 101^3 (19) 8.02 and 6.56.
 static bool pairs_pay(double levels, double groups, double total, int sms, bool mixed) {
   const double g = groups / levels;
   const double one = mixed ? 500.0 + 176.0 * g : std::max(670.0, 580.0 * g - 1300.0);
@@ -514,23 +514,24 @@ static bool pairs_pay(double levels, double groups, double total, int sms, bool 
 }
 
 // Whether direction streams are faster than the kernels over the levelled schedule: the longest
-// stream, at 3.6 ns a task of its block (FP64 7.7, of a pair of blocks 5.9 where pairs_pay takes them,
+// stream, at 3.6 ns a task of its block (FP64 8.1, of a pair of blocks 6.4 where pairs_pay takes them,
 // times the streams that a pair has), against the time of a level, from word to word 0.85 us (FP64
-// push form, from atomic to atomic: 4), times the levels, plus the tasks at 17 per ns (12).  Measured on uniform boxes, ms per sweep, levelled and streams.  Mixed path: 84
-// directions 24^3 0.32 and 0.15, 48^3 0.89 and 0.52, 64^3 1.56 and 1.01, 128^3 10.3 and 7.6; 16
-// directions 64^3 0.95 and 0.87, but 101^3 1.87 and 2.98: sixteen blocks cannot keep up with the
-// whole device where levels are wide.  FP64: 84 directions 16^3 0.97 and 0.18, 24^3 1.61 and 0.31,
-// 32^3 2.10 and 0.46, 64^3 5.4 and 2.0, 96^3 13.8 and 7.9; 16 directions 64^3 4.8 and 1.8, 101^3
-// 7.8 and 6.0; 84 directions 128^3 34 and 17, 160^3 66 and 34.  Where a level is wide, the ring
-// holds few levels and many words come from memory: mixed path 160^3 (1800 tasks a level) 20.2
-// and 15.8, 192^3 (2200) 35 and 34, 256^3 (3400) 83 and 114; hence the limit on the width.
+// push form, from atomic to atomic: 4), times the levels, plus the tasks at 17 per ns (12).
+// Measured on uniform boxes, ms per sweep, levelled and streams.  Mixed path: 84 directions 24^3 0.32
+// and 0.15, 48^3 0.97 and 0.50, 64^3 1.67 and 1.04, 128^3 10.6 and 7.3; 16 directions 64^3 0.99 and
+// 0.87, but 101^3 2.0 and 3.0: sixteen blocks cannot keep up with the whole device where levels are
+// wide.  FP64: 84 directions 16^3 0.95 and 0.18, 24^3 1.60 and 0.32, 32^3 2.08 and 0.47, 64^3 5.4 and
+// 2.1, 96^3 13.8 and 7.4, 128^3 34 and 19.5, 160^3 66 and 38; 16 directions 64^3 4.8 and 1.9, 101^3
+// 7.8 and 6.6.  Where a level is wide, the ring holds few levels and many words come from memory:
+// mixed path 160^3 (1800 tasks a level) 20.8 and 16.1, 192^3 (2200) 35 and 34, 256^3 (3400) 83 and
+// 114; hence the limit on the width.
 static bool streams_pay(const std::vector<uint32_t>& parts, uint64_t tasks, size_t levels, int sms, bool mixed) {
   uint32_t longest = 0;
   for (size_t k = 1; k < parts.size(); ++k) longest = std::max(longest, parts[k] - parts[k - 1]);
   if (!mixed) {
-    double task = 7.7;
+    double task = 8.1;
     if (pairs_pay((double)levels, longest / (double)swk::kStreamGroup, (double)tasks / swk::kStreamGroup, sms, false))
-      task = 5.9 * std::max(1.0, 2.0 * (double)tasks / ((double)longest * sms));
+      task = 6.4 * std::max(1.0, 2.0 * (double)tasks / ((double)longest * sms));
     return task * longest < 4000.0 * (double)levels + (double)tasks / 12.0;
   }
   return longest < 2600.0 * (double)levels && 3.6 * longest < 850.0 * (double)levels + (double)tasks / 17.0;
@@ -873,7 +874,8 @@ sw_status build_streams(sw_handle* h) {
   // warps of a block: as many as find a group of a level to work on.  Mixed path, 84 directions,
   // ms per sweep with 4, 8 and 16: 24^3 (35 tasks a level) 0.159, 0.152, 0.185; 32^3 (62) 0.289,
   // 0.235, 0.274; 48^3 (138) 0.80, 0.57, 0.52; 64^3 (250) 2.5, 1.55, 1.01.  FP64, whose warps also
-  // sum ahead: 24^3 0.36, 0.31, 0.31; 32^3 0.69, 0.48, 0.46; 48^3 2.2, 1.38, 1.02.
+  // sum ahead: 24^3 0.36, 0.31, 0.31; 32^3 0.69, 0.48, 0.46; 48^3 2.2, 1.38, 1.02 (sums made anew; of
+  // changes with 16 warps 0.32, 0.47, 1.07).
   uint32_t warps = width <= 32 ? 4 : (width <= (rb == 4 ? 96 : 48) ? 8 : 16);
   if (const char* env = std::getenv("SUBSWEEP_STREAM_WARPS")) {
     const int v = std::atoi(env);
@@ -2608,7 +2610,8 @@ sw_status sw_load_state(sw_handle* h, const void* buffer, size_t bytes) try {
     off += s.bytes;
   }
   SW_CUDA(h, cudaStreamSynchronize(h->stream), "load state");
-  if (h->p.num_pairs) SW_CUDA(h, cudaMemsetAsync(h->p.stream_flags, 0xff, (size_t)h->p.num_pairs * 4, h->stream), "load state");
+  if (h->p.num_pairs)
+    SW_CUDA(h, cudaMemsetAsync(h->p.stream_flags, 0xff, (size_t)h->p.num_pairs * 4, h->stream), "load state");
   h->p.active_cells = 0;  // incoming rates of some cells may be out of date (mixed path)
   if (h->p.stream_mode && !h->ops->pull)  // no sweep is stamped
     SW_CUDA(h, cudaMemsetAsync(h->p.queue, 0xff, (size_t)h->Np * h->D * 4, h->stream), "load state");

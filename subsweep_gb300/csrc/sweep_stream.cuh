@@ -379,8 +379,8 @@ __device__ __forceinline__ void st_sum(StreamSum<double>& sum, const StreamQuad<
 // kept word on through the ring.
 //
 // kPair: a stream is walked by the two blocks of a cluster, with the warps of both taking its
-// groups in turn, where levels are wide (96^3 x 84 in FP64 7.9 -> 6.7 ms, 128^3 x 84 in the mixed
-// path 7.7 -> 7.2; at 64^3 slower).  Either block holds the whole ring and a word is stored into
+// groups in turn, where levels are wide (96^3 x 84 in FP64 8.5 -> 7.4 ms, 128^3 x 84 in the mixed
+// path 7.8 -> 7.3; at 64^3 slower).  Either block holds the whole ring and a word is stored into
 // both.  A warp of its own fences the words of all groups solved so far and tells the peer their
 // number: with a fence for every group 96^3 took 7.9 ms, since it waits for the stores of the SM.
 // There are fewer pairs of SMs than streams (76 for 84 directions), so the streams are laid end to
@@ -419,7 +419,10 @@ __global__ void __launch_bounds__(32 * (kPair ? W + 1 : W)) k_sweep_stream(const
     st_cluster_sync();
     if (threadIdx.x == 0) {
       uint32_t started;
-      asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(started) : "r"(st_peer(st_smem(count + 2), 0u)) : "memory");
+      asm volatile("ld.shared::cluster.u32 %0, [%1];"
+                   : "=r"(started)
+                   : "r"(st_peer(st_smem(count + 2), 0u))
+                   : "memory");
       const bool spare = started >= gridDim.x / 2;  // more clusters than pairs: none
       if (spare) atomicOr(&a.ctl->error, kErrStall);
       const uint32_t* at = a.part0 + (gridDim.x / 2 - 1 - started);

@@ -43,8 +43,8 @@ def test_fits_are_exact_to_a_few_roundings(host):
             a = mp.mpf(2.753e-14) * lam ** mp.mpf(1.5) / (1 + p) ** mp.mpf(2.242) * cm3
             c, d = mp.mpf(0.407), mp.mpf(2.242)
             # d alpha / d lambda (175-194) times d lambda / d t
-            slope = (mp.mpf(2.753e-14) * -mp.sqrt(lam) / (1 + p) ** (d + 1) * (c * d * p - mp.mpf(1.5) * p - mp.mpf(1.5))
-                     * cm3 * (-315614 / v ** 2))
+            poly = c * d * p - mp.mpf(1.5) * p - mp.mpf(1.5)
+            slope = mp.mpf(2.753e-14) * -mp.sqrt(lam) / (1 + p) ** (d + 1) * poly * cm3 * (-315614 / v ** 2)
             q = (lam / mp.mpf(2.25)) ** mp.mpf(0.376)
             r = (mp.mpf(3.435e-30) * v * lam ** mp.mpf(1.97) / (1 + q) ** mp.mpf(3.72) + mp.mpf(1.42e-27) * mp.sqrt(v))
             err[:, i] = off(alpha[i], a), off(dalpha[i], slope), off(cooling[i], r * erg_cm3)
